@@ -270,11 +270,47 @@ cudaError_t for_item_classes(const lcp_orbs* o, int* launches, F launch) {
   return cudaSuccess;
 }
 
+// Whether an FP64 contraction takes the tensor-core kernels, with their brick
+// lists and workspaces made if need be.  Always, except for cells beyond the
+// kernels' limits and inside a caller's stream capture before anything was
+// made (allocating and synchronising there would break the capture): those
+// take the pair kernels (64-atom 96^3 cell: 36.8 ms for density and matrix
+// elements, against 3.3 ms; 2-atom 24^3 cell: 0.62 ms against 0.15).
+static lcp_status f64_ready(lcp_ctx* ctx, const lcp_orbs* orbs, bool* tc) {
+  *tc = false;
+  if (ctx->precision != LCP_PREC_FP64) return LCP_OK;
+  lcp_orbs* o = const_cast<lcp_orbs*>(orbs);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  API_CUDA(cudaStreamIsCapturing(ctx->stream, &cap), "capture status");
+  if (cap != cudaStreamCaptureStatusNone) {
+    if (o->f64_state == 1) return ensure_f64_workspace(ctx, o, tc);
+    return LCP_OK;
+  }
+  lcp_status s = ensure_f64(ctx, o);
+  if (s || o->f64_state != 1) return s;
+  if ((s = ensure_f64_workspace(ctx, o))) return s;
+  *tc = true;
+  return LCP_OK;
+}
+
 lcp_status density_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nspin, const double* const* dm, double* const* rho,
                           int64_t nn) {
   int prec = ctx->precision;
   if (prec == LCP_PREC_BF16X3) return density_tc_device(ctx, orbs, nspin, dm, rho);
   if (orbs->phi_released) return fail(LCP_ESTATE, "the FP64 orbital tables were released (split-BF16 only)");
+  bool tc = false;
+  lcp_status fs = f64_ready(ctx, orbs, &tc);
+  if (fs) return fs;
+  if (tc) {
+    const lcp::F64DensWork w{ctx->w_f64d.as<double>() + orbs->ucell->u.total_hsize, ctx->w_f64d.as<uint64_t>(),
+                             ctx->w_f64c.as<uint32_t>(), ctx->w_f64e.as<int32_t>()};
+    for (int c = 0; c < nspin; ++c)
+      API_CUDA(lcp::launch_f64_density(orbs->f64_density.g, orbs->f64_pairs, dm[c], w, rho[c], ctx->w_status.as<int>(),
+                                       ctx->stream),
+               "density kernel");
+    ctx->launches += 4 * nspin;
+    return LCP_OK;
+  }
   for (int s = 0; s < nspin; ++s) API_CUDA(cudaMemsetAsync(rho[s], 0, nn * sizeof(double), ctx->stream), "memset");
   if (prec == LCP_PREC_FP32) {
     lcp_status s = ensure_phi32(ctx, const_cast<lcp_orbs*>(orbs));
@@ -336,6 +372,19 @@ lcp_status hamiltonian_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nch, const
   int prec = ctx->precision;
   if (prec == LCP_PREC_BF16X3) return hamiltonian_tc_device(ctx, orbs, nch, vpot, hks);
   if (orbs->phi_released) return fail(LCP_ESTATE, "the FP64 orbital tables were released (split-BF16 only)");
+  bool tc = false;
+  lcp_status fs = f64_ready(ctx, orbs, &tc);
+  if (fs) return fs;
+  if (tc) {
+    const lcp::F64HamWork w{ctx->w_f64v.as<int64_t>(), ctx->w_f64e.as<int32_t>(),
+                            ctx->w_f64d.as<double>()};
+    for (int c = 0; c < nch; ++c)
+      API_CUDA(lcp::launch_f64_hamiltonian(orbs->f64_elements.g, orbs->pairs, orbs->geom.numorbs, vpot[c], w,
+                                           orbs->ucell->u.gridvol, hks[c], hsize, ctx->w_status.as<int>(), ctx->stream),
+               "hamiltonian kernel");
+    ctx->launches += 3 * nch;
+    return LCP_OK;
+  }
   for (int c = 0; c < nch; ++c) API_CUDA(cudaMemsetAsync(hks[c], 0, hsize * sizeof(double), ctx->stream), "memset");
   if (prec == LCP_PREC_FP32) {
     lcp_status s = ensure_phi32(ctx, const_cast<lcp_orbs*>(orbs));
@@ -1772,6 +1821,9 @@ lcp_status lcp_job_footprint(const lcp_job* job, int64_t* bytes) {
                         &o->b_redslot, &o->b_subpair, &o->b_subchunks, &o->b_sbfold, &o->b_sbchunks, &o->o_atom,
                         &o->o_jatom, &o->o_boff, &o->o_partner, &o->b_scale, &o->b_tmp})
     add(*d);
+  for (const F64Set* f : {&o->f64_density, &o->f64_elements})
+    for (const DBuf* d : {&f->bricks, &f->rows, &f->table, &f->ptexp, &f->tab}) add(*d);
+  for (const DBuf& d : o->f64_pair_buf) add(d);
   *bytes = b;
   return LCP_OK;
 }
@@ -1780,7 +1832,7 @@ lcp_status lcp_job_footprint(const lcp_job* job, int64_t* bytes) {
 
 // Device bytes the job will hold once its tables for `precision` exist: its
 // footprint now plus, when not built yet, the split-BF16 brick tables (from
-// the host brick geometry) or the FP32 orbital copy.
+// the host brick geometry), the FP32 orbital copy or the FP64 kernels' tables.
 int64_t job_footprint_estimate(lcp_job* job, int32_t precision) {
   int64_t fp = 0;
   if (lcp_job_footprint(job, &fp) != LCP_OK) return -1;
@@ -1794,6 +1846,8 @@ int64_t job_footprint_estimate(lcp_job* job, int32_t precision) {
                     b.sb_chunks.size()) * 4;
   } else if (precision == LCP_PREC_FP32 && !o->phi32.p) {
     fp += o->table_elems * 4;
+  } else if (precision == LCP_PREC_FP64 && o->f64_state == 0 && !o->phi_released) {
+    fp += f64_footprint_estimate(o);
   }
   return fp;
 }
@@ -1806,6 +1860,10 @@ lcp_status lcp_job_prepare(lcp_ctx* ctx, lcp_job* job) {
   if (!job) return fail(LCP_EINVAL, "NULL job");
   lcp_orbs* o = const_cast<lcp_orbs*>(job->orbs);
   if (ctx->precision == LCP_PREC_BF16X3) return ensure_bricks(ctx, o);
+  if (ctx->precision == LCP_PREC_FP64 && !o->phi_released) {
+    bool tc = false;
+    if ((s = f64_ready(ctx, o, &tc))) return s;
+  }
   if (ctx->precision == LCP_PREC_FP32) {
     if ((s = ensure_phi32(ctx, o))) return s;
     API_CUDA(cudaStreamSynchronize(ctx->stream), "prepare");

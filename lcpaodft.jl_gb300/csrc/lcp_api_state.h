@@ -7,6 +7,7 @@
 
 #include <atomic>
 #include <map>
+#include <mutex>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -110,6 +111,7 @@ struct lcp_ctx {
   // workspaces of the host-buffer entry points
   DBuf w_in[4], w_out[4], w_aux[4], w_real, w_spec, w_part, w_scal, w_a, w_b;
   DBuf w_dsym, w_status, w_hscratch, w_dscale, w_dtmp, w_vw, w_vscale, w_pfac;
+  DBuf w_f64d, w_f64c, w_f64v, w_f64e;  // FP64 contractions (ensure_f64_workspace)
   // second stream of the step: the xc pass runs there beside the FFT Poisson solve
   cudaStream_t aux = nullptr;
   // device address of the no-allocation density's fixed scratch array, looked
@@ -131,6 +133,16 @@ struct lcp_ctx {
     if (ev_join) cudaEventDestroy(ev_join);
     if (aux) cudaStreamDestroy(aux);
     if (own) cudaStreamDestroy(own);
+  }
+};
+
+// One brick tiling of the FP64 tensor-core contractions (lcp_f64bricks.cu).
+struct F64Set {
+  lcp::F64Bricks g{};
+  DBuf bricks, rows, table, ptexp, tab;
+  void release() {
+    for (DBuf* d : {&bricks, &rows, &table, &ptexp, &tab}) d->release();
+    g = lcp::F64Bricks{};
   }
 };
 
@@ -163,6 +175,12 @@ struct lcp_orbs {
   DBuf o_atom, o_jatom, o_boff, o_partner;  // ordered pair list
   DBuf b_scale, b_tmp;                       // fixed-point scale of the tables: [S_phi, 1/S_phi]
   double phi_scale = 1.0;
+  // brick tilings of the FP64 contractions (ensure_f64: 0 not built, 1 built, -1 beyond the kernels' limits)
+  std::mutex f64_mutex;
+  int f64_state = 0;
+  F64Set f64_density, f64_elements;
+  lcp::F64Pairs f64_pairs{};
+  DBuf f64_pair_buf[8];
   // device times of the last tabulation and split-table build (ms)
   float tab_ms = 0.f, split_ms = 0.f;
 };
@@ -209,6 +227,9 @@ lcp_status check_ctx(lcp_ctx* ctx);
 lcp_status check_pair(const lcp_ucell* ucell, const lcp_orbs* orbs);
 lcp_status ensure_bricks(lcp_ctx* ctx, lcp_orbs* o);
 lcp_status device_status(lcp_ctx* ctx);
+lcp_status ensure_f64(lcp_ctx* ctx, lcp_orbs* o);
+int64_t f64_footprint_estimate(const lcp_orbs* o);
+lcp_status ensure_f64_workspace(lcp_ctx* ctx, const lcp_orbs* o, bool* ready = nullptr);
 lcp_status density_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nspin, const double* const* dm, double* const* rho,
                           int64_t nn);
 lcp_status hamiltonian_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nch, const double* const* vpot,

@@ -349,4 +349,89 @@ cudaError_t launch_h_reduce(int64_t nsb, const int64_t* red_off, const int64_t* 
                             const int32_t* sb_chunks, const float* scratch, const DevPairs& pr,
                             const int32_t* numorbs, double dv, double* H, cudaStream_t st);
 
+// ---------------------------------------------------------------- FP64 contractions on the tensor cores
+// Brick lists and tables of the FP64 tensor-core kernels (device pointers).
+// The home cell is tiled by bricks of at most P points (slot (l0*bdim1 +
+// l1)*bdim2 + l2); a brick lists the atom images whose spheres hold one of its
+// points, sorted by (atom, unrolled brick), and packs their orbitals densely as
+// rows, in chunks of 32 (the last one padded with zeros).  The table holds
+// every row's phi at every slot as a 56-bit fixed-point integer t + kF64Bias
+// (phi = t 2^-55 2^(E - 1023)), scaled per point (density, P = 128) or per row
+// (matrix elements, P = 64); chunk layout [P/8 groups][4 pairs][32 rows][2 points].
+struct F64Row {
+  uint32_t info;     // orbitals of the atom | matrix elements: E of the row, density: atom * 32 + orbital, << 6
+  uint32_t img_orb;  // image within the brick << 8 | orbital
+};
+struct alignas(16) F64Brick {
+  uint32_t row, chunk, tab;  // its first row, table chunk and pair table entry
+  uint32_t size;             // rows | images << 16
+};
+constexpr uint64_t kF64Bias = 0x0080808080808080ull;  // 128 in each of the seven bytes
+struct F64Bricks {
+  int32_t P, npts;             // point slots per brick (64 or 128) and points of a whole brick
+  int32_t bdim[3], nb[3], ngrid[3];
+  int32_t max_rows;            // of a brick
+  int64_t nbricks, nimg, nrows, nchunks;
+  const F64Brick* bricks;      // [nbricks]
+  const F64Row* rows;          // [nrows]
+  const uint64_t* table;       // [nchunks * 32 * P]
+  const int32_t* ptexp;        // density: [nbricks * P] E of a point
+  const int32_t* tab;          // m x m per brick: offset of the block of the ordered pair (s, t) (density) or of
+                               // its partner (t, s), where the matrix elements are accumulated; -1: no pair
+};
+constexpr int kF64MaxRows = 1000;  // packed rows of a brick the kernels take
+// Ordered pair list of the cell (device pointers) for the brick pair tables and the symmetrised D.
+struct F64Pairs {
+  int32_t natom, ncell, cpy;
+  int64_t npairs;
+  const int32_t* atom;         // [npairs] 0-based, ascending
+  const int32_t* jatom;
+  const int32_t* cell;
+  const int32_t* partner;
+  const int64_t* boff;
+  const int64_t* first;        // [natom+1] first pair of each atom (its self pair)
+  const int32_t* ijk;          // [ncell * 3]
+  const int32_t* ratv;         // [(2 cpy + 1)^3]
+  const int32_t* numorbs;      // [natom]
+};
+// rho (one channel) from D.  Workspace: dsym (hsize doubles) and dfix (hsize
+// words: D symmetrised per ordered pair, as FP64 and on the grids of its
+// columns' scales), cmax (natom * 32 words: the columns' largest magnitudes)
+// and btop (nbricks ints: the bricks' largest column scales).
+struct F64DensWork {
+  double* dsym;
+  uint64_t* dfix;
+  uint32_t* cmax;
+  int32_t* btop;
+};
+cudaError_t launch_f64_density(const F64Bricks& b, const F64Pairs& pr, const double* dm, const F64DensWork& w,
+                               double* rho, int* status, cudaStream_t st);
+// H (one channel) from V, in both orientations, times gridvol.  Workspace: vb
+// (nbricks * 64 words: V by brick), vexp (nbricks ints: its scales) and acc
+// (kF64Copies * hsize doubles: the sums).
+constexpr int kF64Copies = 8;
+struct F64HamWork {
+  int64_t* vb;
+  int32_t* vexp;
+  double* acc;
+};
+cudaError_t launch_f64_hamiltonian(const F64Bricks& b, const DevPairs& folded, const int32_t* numorbs,
+                                   const double* vpot, const F64HamWork& w, double gridvol, double* hks, int64_t hsize,
+                                   int* status, cudaStream_t st);
+// The rows, scales and table of a tiling from the FP64 orbital tables.
+struct F64Build {
+  const double* phi;
+  const int64_t* phi_off;
+  const int32_t* numorbs;
+  const int64_t* img_off;   // [nbricks+1]
+  const int32_t* img_atom;  // [nimg]
+  const int32_t* img_row0;  // [nimg] first row of an image within its brick
+  const int32_t* slot;      // [nimg * P] sphere point of the image's atom at each slot (-1: outside)
+};
+cudaError_t launch_f64_table(const F64Bricks& b, const F64Build& f, F64Row* rows, int32_t* ptexp, uint64_t* table,
+                             cudaStream_t st);
+// Exclusive scan of n int32 into n + 1 int64 (totals: scan_blocks(n) + 1 int64 of scratch).
+int64_t scan_blocks(int64_t n);
+cudaError_t exclusive_scan_i32(const int32_t* in, int64_t n, int64_t* out, int64_t* totals, cudaStream_t st);
+
 }  // namespace lcp

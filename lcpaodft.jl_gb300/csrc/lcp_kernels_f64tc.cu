@@ -1,0 +1,1206 @@
+// FP64 density assembly and grid matrix elements on the tensor cores.
+//
+// GB300 issues 2 FP64 FMAs per clock and SM, and the pair kernels of
+// lcp_kernels_pair.cu keep that pipe 95 % busy: 16.9 ms (density) and 19.9 ms
+// (matrix elements) on the 64-atom 96^3 cell, where the kernels below take 1.75
+// and 1.5 ms.  The tensor cores do 4,096 FP16 multiply-adds per clock and SM
+// with FP32 accumulation, which is exact for integers below 2^24.  So each FP64
+// operand is put on a fixed-point grid of 56 bits,
+//
+//   x = t 2^-55 2^E,  |x| < 2^E,  t = sum_i d_i 256^(7-i),  |d_i| <= 128,
+//
+// whose seven base-256 digits are exact FP16 values, and a contraction of two
+// operands is the 28 digit products d_i d_j' with i + j <= 8, each group of
+// equal weight (i + j = d + 1) in its own FP32 accumulator a_d.  Over 64 terms
+// |a_d| <= d 2^20 < 2^24, so every sum is exact in the matrix elements; in the
+// density (up to R packed rows) the first R d <= 1024 groups are exact for any
+// values.  The dropped groups are below 2^-62 of the scales' product.  What is
+// rounded: each operand once to 2^-56 of its row's (column's, point's) largest
+// value, the assembled sum once to 2^-55 of the scales' product, and the FP64
+// additions that follow.  An FP64 FMA chain rounds every partial sum to 2^-53
+// of itself.  Against 113-bit sums over the same tables, on cells of 2 to 6
+// atoms and 4 to 18 orbitals, the errors over the result's norm are 1.3e-16 to
+// 2.1e-16 in H (pair kernels 2.0e-16 to 3.7e-16) and 1.3e-16 to 1.5e-16 in rho
+// (1.4e-16 to 2.8e-16).  Elements of H far below the largest, where two
+// orbitals' tails meet, carry fewer digits of their own than the pair
+// kernels' (99th percentile of the elements' relative errors 3e-14 to 2e-13,
+// against 1e-14).
+//
+// The split is integer work: the mantissa shifted to the scale's grid, rounded,
+// biased by 128 in every byte, and each byte turned into FP16 by placing it
+// under the exponent of 1024 and subtracting 1152 (two digits per instruction).
+// FP16 rather than BF16 because a byte fits FP16's eleven-bit integers without
+// a sign trick; the tensor rate is the same.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include "lcp_bounds.cuh"
+#include "lcp_device.h"
+#include "lcp_tc.cuh"
+
+namespace lcp {
+
+namespace {
+
+constexpr int kDig = 7;       // digits per operand
+constexpr int kWin = 32;      // columns of a window (7 * 32 TMEM columns per buffer)
+constexpr int kBadExp = 4095; // scale of a column or brick that holds Inf or NaN
+constexpr uint32_t kBufCols = 256;
+
+// |x| as a 53-bit integer m and a biased exponent e: |x| = m 2^(e - 1075) (subnormals too).
+__device__ __forceinline__ uint64_t mantissa(double x, int& e) {
+  const uint32_t hi = (uint32_t)__double2hiint(x);
+  const int f = (int)((hi >> 20) & 0x7ffu);
+  e = max(f, 1);
+  return ((uint64_t)((hi & 0xfffffu) | (f > 0 ? 0x100000u : 0u)) << 32) | (uint32_t)__double2loint(x);
+}
+
+// t + sum_k 128 * 256^k of x on the grid of exponent E (biased; |x| < 2^(E - 1023)):
+// rounded to nearest, ties away from zero.
+__device__ __forceinline__ uint64_t fx_biased(double x, int E) {
+  int e;
+  const uint64_t m = mantissa(x, e) << 4;
+  const uint64_t t = ((m >> min((uint32_t)(E - e), 63u)) + 1) >> 1;
+  const uint64_t s = (uint64_t)(int64_t)(__double2hiint(x) >> 31);
+  return (t ^ s) - s + kF64Bias;
+}
+
+// FP16 pairs of the seven digits of two values (d[0]: the leading digits).
+__device__ __forceinline__ uint32_t half_digits(uint32_t biased) {  // 0x64bb64bb: 1024 + byte
+  const uint32_t k = 0x64806480u;                                   // 1152
+  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&biased), *reinterpret_cast<const __half2*>(&k));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ void digit_pairs(uint64_t x, uint64_t y, uint32_t* d) {
+  const uint32_t xl = (uint32_t)x, xh = (uint32_t)(x >> 32), yl = (uint32_t)y, yh = (uint32_t)(y >> 32);
+  const uint32_t k = 0x64646464u;
+  const uint32_t z0 = __byte_perm(xl, yl, 0x5140);  // bytes 0 and 1 of x and y interleaved
+  const uint32_t z1 = __byte_perm(xl, yl, 0x7362);  // 2 and 3
+  const uint32_t z2 = __byte_perm(xh, yh, 0x5140);  // 4 and 5
+  // the leading digit keeps the carry byte: 128 + 128 = 256 is possible
+  d[0] = half_digits(__byte_perm(xh, yh, 0x7632) | 0x64006400u);
+  d[1] = half_digits(__byte_perm(z2, k, 0x4342));
+  d[2] = half_digits(__byte_perm(z2, k, 0x4140));
+  d[3] = half_digits(__byte_perm(z1, k, 0x4342));
+  d[4] = half_digits(__byte_perm(z1, k, 0x4140));
+  d[5] = half_digits(__byte_perm(z0, k, 0x4342));
+  d[6] = half_digits(__byte_perm(z0, k, 0x4140));
+}
+
+// The digits of eight values into seven 16-byte pieces, `step` bytes apart.
+__device__ __forceinline__ void store_digits(uint8_t* dst, uint32_t step, const uint64_t* t) {
+  uint32_t d[4][kDig];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) digit_pairs(t[2 * q], t[2 * q + 1], d[q]);
+#pragma unroll
+  for (int i = 0; i < kDig; ++i)
+    *reinterpret_cast<uint4*>(dst + i * step) = make_uint4(d[0][i], d[1][i], d[2][i], d[3][i]);
+}
+
+// Biased exponent bound of the magnitude whose high word is h: |x| < 2^(E - 1023).
+__device__ __forceinline__ int exp_bound(uint32_t h) {
+  const int e = (int)(h >> 20);
+  return e == 0x7ff ? kBadExp : e + 1;
+}
+
+constexpr uint32_t idesc_f16_f32(int M, int N, int a_mn, int b_mn) {  // FP16 operands, FP32 accumulator
+  return (1u << 4) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) | ((uint32_t)(N >> 3) << 17) |
+         ((uint32_t)(M >> 4) << 24);
+}
+
+// The seven accumulators of four columns from `col` on, lanes of `quarter`.
+__device__ __forceinline__ void tmem_ld4_nowait(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void load_acc(uint32_t tmem, uint32_t quarter, uint32_t col, uint32_t (&y)[kDig][4]) {
+#pragma unroll
+  for (int i = 0; i < kDig; ++i) tmem_ld4_nowait(tc::tmem_addr(tmem, quarter * 32, col + i * kWin), y[i]);
+  tc::tmem_wait_ld();
+#pragma unroll
+  for (int i = 0; i < kDig; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) asm volatile("" : "+r"(y[i][j]));  // no use before the wait
+}
+
+// Eight consecutive slots of row `row` of a 32-row table chunk staged in
+// shared memory; piece: the 2 KB of that slot group ([4 pairs][32 rows][2]).
+__device__ __forceinline__ void read_piece(const uint8_t* piece, int row, uint64_t* t) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(piece + i * 512 + row * 16);
+    t[2 * i] = w.x;
+    t[2 * i + 1] = w.y;
+  }
+}
+
+// Table pieces of kRawBytes on their way into a ring of shared-memory slots
+// (bulk copies).  The issuing warp keeps the ring full; a slot is refilled
+// once every reading warp has arrived on its empty barrier.
+constexpr uint32_t kRawBytes = 16384;
+template <int SLOTS>
+struct RawRing {
+  uint8_t* buf;
+  uint64_t *full, *empty;
+  uint32_t slot = 0, par = 1, issued = 0;  // par: parity of the slot's last release
+  __device__ __forceinline__ bool issue(const uint8_t* src, const volatile int* abort_flag) {  // the whole warp
+    if (issued >= SLOTS && !tc::mbar_wait_warp(&empty[slot], par, abort_flag)) return false;
+    if (tc::elect_one()) {
+      tc::mbar_arrive_expect_tx(&full[slot], kRawBytes);
+      tc::bulk_g2s(buf + slot * kRawBytes, src, kRawBytes, &full[slot]);
+    }
+    __syncwarp();
+    ++issued;
+    if (++slot == SLOTS) {
+      slot = 0;
+      par ^= 1;
+    }
+    return true;
+  }
+  // the last copies have landed (before the shared memory goes away)
+  __device__ __forceinline__ void drain() {
+    for (uint32_t i = 0; i < SLOTS && i < issued; ++i) {
+      const uint32_t n = issued - 1 - i;
+      tc::mbar_wait(&full[n % SLOTS], (n / SLOTS) & 1, 1u << 22);
+    }
+  }
+};
+
+__device__ __forceinline__ F64Row load_meta(const F64Row* p) {
+  const uint2 w = __ldg(reinterpret_cast<const uint2*>(p));
+  return F64Row{w.x, w.y};
+}
+__device__ __forceinline__ int row_no(uint32_t info) { return (int)(info & 63u); }
+__device__ __forceinline__ int row_exp(uint32_t info) { return (int)(info >> 6); }  // matrix elements
+__device__ __forceinline__ int row_col(uint32_t info) { return (int)(info >> 6); }  // density: column of D
+
+__device__ __forceinline__ F64Brick load_brick(const F64Brick* p) {
+  const uint4 w = __ldg(reinterpret_cast<const uint4*>(p));
+  return F64Brick{w.x, w.y, w.z, w.w};
+}
+
+// A CTA's bricks with rows, in order; AHEAD: each one is loaded a brick ahead
+// (four registers).
+template <bool AHEAD>
+struct BrickIterT {
+  int k, nb;
+  F64Brick b, n;
+  __device__ __forceinline__ int R() const { return (int)(b.size & 0xffffu); }
+  __device__ __forceinline__ int m() const { return (int)(b.size >> 16); }
+  __device__ __forceinline__ bool valid() const { return k < nb; }
+  __device__ __forceinline__ void settle(const F64Bricks& B) {
+    for (; k < nb; k += gridDim.x) {
+      b = AHEAD ? n : load_brick(B.bricks + k);
+      if (AHEAD && k + (int)gridDim.x < nb) n = load_brick(B.bricks + k + gridDim.x);
+      if (R() > 0) return;
+    }
+  }
+  __device__ __forceinline__ void start(const F64Bricks& B) {
+    k = blockIdx.x;
+    nb = (int)B.nbricks;
+    if (AHEAD && k < nb) n = load_brick(B.bricks + k);
+    settle(B);
+  }
+  __device__ __forceinline__ void next(const F64Bricks& B) {
+    k += gridDim.x;
+    settle(B);
+  }
+};
+using BrickIter = BrickIterT<true>;
+
+int device_sms() {
+  int dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+}  // namespace
+
+// ==========================================================================
+// Scales and tables of a tiling.
+// ==========================================================================
+namespace {
+
+// Rows and scales, one warp per image (lane = orbital): each row's exponent
+// bound over the brick's points, or each point's over all rows.
+__global__ void __launch_bounds__(256) f64_scales_kernel(F64Bricks b, F64Build f, F64Row* __restrict__ rows,
+                                                         int32_t* __restrict__ ptexp) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int64_t hb = blockIdx.x; hb < b.nbricks; hb += gridDim.x) {
+    const int64_t i0 = f.img_off[hb];
+    const int m = (int)(f.img_off[hb + 1] - i0);
+    for (int i = warp; i < m; i += nw) {
+      const int a = f.img_atom[i0 + i], no = f.numorbs[a];
+      const double* src = f.phi + f.phi_off[a] + lane;
+      const int32_t* sl = f.slot + (i0 + i) * b.P;
+      uint32_t mx = 0;
+#pragma unroll 8
+      for (int p = 0; p < b.P; ++p) {
+        const int k = sl[p];
+        const uint32_t h = (k >= 0 && lane < no) ? (uint32_t)__double2hiint(__ldg(src + (int64_t)k * no)) & 0x7fffffffu : 0u;
+        mx = max(mx, h);
+        if (k >= 0 && ptexp) {
+          const uint32_t pm = __reduce_max_sync(0xffffffffu, h);
+          if (lane == 0) atomicMax(ptexp + hb * b.P + p, exp_bound(pm));
+        }
+      }
+      if (lane < no)
+        rows[(int64_t)b.bricks[hb].row + f.img_row0[i0 + i] + lane] =
+            F64Row{(uint32_t)no | ((ptexp ? (uint32_t)(a * 32 + lane) : (uint32_t)exp_bound(mx)) << 6),
+                   ((uint32_t)i << 8) | (uint32_t)lane};
+    }
+  }
+}
+
+// phi of every row at every slot on its scale's grid: lane = row of a chunk,
+// two slots per store (the phi rows of a point are contiguous over its lanes).
+__global__ void __launch_bounds__(256) f64_table_kernel(F64Bricks b, F64Build f, uint64_t* __restrict__ table) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int64_t hb = blockIdx.x; hb < b.nbricks; hb += gridDim.x) {
+    const F64Brick br = load_brick(b.bricks + hb);
+    const int R = (int)(br.size & 0xffffu);
+    const int64_t i0 = f.img_off[hb];
+    for (int c = 0; c * 32 < R; ++c) {
+      const int r = c * 32 + lane;
+      F64Row m{};
+      const double* src = f.phi;
+      const int32_t* sl = f.slot;
+      if (r < R) {
+        m = load_meta(b.rows + br.row + r);
+        const int64_t im = i0 + (m.img_orb >> 8);
+        src = f.phi + f.phi_off[f.img_atom[im]] + (m.img_orb & 255u);
+        sl = f.slot + im * b.P;
+      }
+      const int no = row_no(m.info), e = row_exp(m.info);
+      for (int w = warp; w < b.P / 2; w += nw) {
+        const int p = 2 * w;
+        uint64_t t[2] = {kF64Bias, kF64Bias};
+        if (r < R) {
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int k = __ldg(sl + p + q);
+            if (k >= 0) t[q] = fx_biased(__ldg(src + (int64_t)k * no), b.P == 128 ? __ldg(b.ptexp + hb * b.P + p + q) : e);
+          }
+        }
+        reinterpret_cast<ulonglong2*>(table + (int64_t)(br.chunk + c) * 32 * b.P)[w * 32 + lane] = make_ulonglong2(t[0], t[1]);
+      }
+    }
+  }
+}
+
+}  // namespace
+
+// ==========================================================================
+// Matrix elements.  Per brick of 64 points, over its R packed rows,
+//
+//   G[r][c] = sum_p phi_r(p) V(p) phi_c(p),   r <= c  (G is symmetric),
+//
+// as tiles of 128 rows x windows of 32 columns: A holds the V-weighted rows
+// (split once per tile), B a window's plain columns, both K-major.  64 points
+// because the seven digit planes of A take 112 KB of shared memory at that K;
+// packed rows because 13 orbitals in 16-row blocks would waste a third of the
+// products, and 4- and 18-orbital atoms more.
+//
+// A pair's bricks (over a thousand for a self pair) are summed by FP64 atomic
+// adds into one of eight copies of H, the brick's number mod 8, which
+// f64_finish_kernel adds up: with one copy the matrix was 2.5 to 4 times
+// further from the exact one than the pair kernels' (8e-16 against 3e-16 of
+// its norm, one rounding per brick instead of one per 512 points).  Exact sums
+// in two 64-bit integers (5e-17) cost a second atomic per element, 14 clocks
+// per warp and SM each, and the adds are what the epilogue waits for most.
+//
+// A step is one window.  Since only r <= c counts, window w of a tile needs
+// the tile's row blocks up to its own: the first four steps split their chunk
+// twice, as the window's B and, V-weighted, as row block w of A, and no step
+// waits for a whole A tile.  (Rows of A left from an earlier tile only feed
+// results with r > c, which nobody reads.)
+//
+// Roles (640 threads, one CTA per SM, persistent over bricks; warp w runs on
+// scheduler w % 4, and the epilogue warps of one quarter of the TMEM lanes
+// have to sit on one scheduler.  The first quarter holds the lowest rows,
+// which count in every window, the last one the fewest, so the schedulers get
+// 4, 3, 2 and 2 epilogue warps and the split warps fill the others):
+//   epilogue: a warp takes its share of a window's eight column groups: the
+//             seven accumulators as integers, assembled in 64 bits, one FP64
+//             atomic add into the pair's accumulated block (lanes are
+//             consecutive orbitals of one image: consecutive addresses);
+//   MMA:      4 K steps x 7 MMAs, digit i of A against digits 1 .. 8-i of B
+//             stacked along N (N = 32 (8 - i)), so that every product lands
+//             in the accumulator of its weight;
+//   split:    8 warps, one k group (8 points) each, lane = row of the chunk.
+// Every wait is bounded; a timeout sets *status and stops all roles.
+// ==========================================================================
+namespace {
+
+constexpr int kHP = 64;
+constexpr int kHEpi = 11, kHConv = 8;
+constexpr int kHThreads = 32 * (kHEpi + 1 + kHConv);
+constexpr uint32_t kHADigit = 128 * kHP * 2;           // 16 KB: [k group][128 rows][16 B]
+constexpr uint32_t kHBLbo = kDig * kWin * 16;          // 3,584 B per k group: [digit][32 columns][16 B]
+constexpr uint32_t kHBStage = (kHP / 8) * kHBLbo;      // 28 KB
+constexpr int kHRaw = 3;                               // table chunks in shared memory
+constexpr size_t kHSmemBytes = kDig * (size_t)kHADigit + 2 * (size_t)kHBStage + kHRaw * (size_t)kRawBytes;  // 216 KB
+static_assert(kRawBytes == 32 * kHP * 8, "a raw slot is a chunk");
+
+// sum a_d 256^(7-d) / 256 for |a_d| <= d 2^20 (64 products of each kind, |digit| <= 128), rounded;
+// below 2^61.  a_1 .. a_4 lie within 2^22, where adding 1.5 2^23 leaves the
+// integer in the low bits; a_7 only counts in units of 256.  Conversions run
+// at a quarter of the rate of these additions.
+__device__ __forceinline__ int64_t assemble_bounded(uint32_t u1, uint32_t u2, uint32_t u3, uint32_t u4, uint32_t u5,
+                                                    uint32_t u6, uint32_t u7) {
+  constexpr float M = 12582912.0f;
+  constexpr int K = 0x4B400000;  // bits of M
+  const int b1 = __float_as_int(__fadd_rn(__uint_as_float(u1), M)), b2 = __float_as_int(__fadd_rn(__uint_as_float(u2), M)),
+            b3 = __float_as_int(__fadd_rn(__uint_as_float(u3), M)), b4 = __float_as_int(__fadd_rn(__uint_as_float(u4), M));
+  const float f7 = __fadd_rn(__fmaf_rn(__uint_as_float(u7), 0.00390625f, M), -M);
+  const int i6 = __float2int_rn(__fadd_rn(__uint_as_float(u6), f7)), i5 = __float2int_rn(__uint_as_float(u5));
+  const int p23 = (int)((uint32_t)b2 * 256u + (uint32_t)b3 - (uint32_t)K * 257u);
+  const int p45 = (int)((uint32_t)b4 * 256u + (uint32_t)i5 - (uint32_t)K * 256u);
+  int64_t S = (int64_t)p45 * 256 + i6;
+  S += (int64_t)p23 * (1 << 24);
+  return S + (int64_t)((uint64_t)(uint32_t)((b1 - K) * 256) << 32);
+}
+
+// Steps of a CTA in order: brick, row tile r0, window c0 >= r0.
+struct StepIter : BrickIter {
+  int r0, c0;
+  __device__ __forceinline__ void begin(const F64Bricks& B) {
+    r0 = c0 = 0;
+    start(B);
+  }
+  __device__ __forceinline__ void step(const F64Bricks& B) {
+    c0 += kWin;
+    if (c0 < R()) return;
+    r0 += 128;
+    c0 = r0;
+    if (r0 < R()) return;
+    r0 = c0 = 0;
+    next(B);
+  }
+};
+
+struct F64HamArgs {
+  F64Bricks b;
+  F64HamWork w;
+  int64_t hsize;
+  int* status;
+};
+
+// V of every slot in brick order as a multiple of 2^-62 of the brick's bound
+// (zero past the grid), and the bounds.
+__global__ void __launch_bounds__(kHP) f64_vprep_kernel(F64Bricks b, const double* __restrict__ vpot,
+                                                        int64_t* __restrict__ vb, int32_t* __restrict__ vexp) {
+  __shared__ uint32_t s[2];
+  const int p = threadIdx.x;
+  for (int64_t k = blockIdx.x; k < b.nbricks; k += gridDim.x) {
+    const int64_t gi = p < b.npts ? brick_point_index(k, p, b.bdim, b.nb, b.ngrid) : -1;
+    const double v = gi >= 0 ? vpot[gi] : 0.0;
+    const uint32_t h = __reduce_max_sync(0xffffffffu, (uint32_t)__double2hiint(v) & 0x7fffffffu);
+    if ((p & 31) == 0) s[p >> 5] = h;
+    __syncthreads();
+    const int E = exp_bound(max(s[0], s[1]));
+    int e;
+    const uint64_t m = mantissa(v, e) << 10;
+    const int64_t t = (int64_t)(m >> min((uint32_t)(E - e), 63u));
+    vb[k * kHP + p] = E >= kBadExp ? 0 : (v < 0.0 ? -t : t);
+    if (p == 0) vexp[k] = E;
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __grid_constant__ F64HamArgs args) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ uint64_t afree_bar, bready_bar[2], bempty_bar[2], tfull_bar[2], tempty_bar[2], drain_bar;
+  __shared__ uint64_t rawfull_bar[kHRaw], rawempty_bar[kHRaw];
+  __shared__ uint32_t tslot;
+  __shared__ volatile int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int sched = warp & 3, rank = warp >> 2;
+  const int nepi = sched == 0 ? 4 : (sched == 1 ? 3 : 2);  // epilogue warps on this scheduler
+  const bool is_mma = warp == 16;
+  const F64Bricks& B = args.b;
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + kDig * kHADigit;
+  if (is_mma) tc::tmem_alloc(&tslot, 512);
+  if (tid == 0) {
+    tc::mbar_init(&afree_bar, 1);
+    for (int s = 0; s < kHRaw; ++s) {
+      tc::mbar_init(&rawfull_bar[s], 1);
+      tc::mbar_init(&rawempty_bar[s], kHConv);
+    }
+    for (int s = 0; s < 2; ++s) {
+      tc::mbar_init(&bready_bar[s], kHConv);
+      tc::mbar_init(&bempty_bar[s], 1);
+      tc::mbar_init(&tfull_bar[s], 1);
+      tc::mbar_init(&tempty_bar[s], kHEpi);
+    }
+    tc::mbar_init(&drain_bar, 1);
+    tc::fence_mbar_init();
+    abort_flag = 0;
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tslot;
+  auto give_up = [&]() {
+    if (!abort_flag) atomicExch(args.status, LCP_ETIMEDOUT);
+    abort_flag = 1;
+  };
+
+  if (rank < nepi) {
+    // ------------------------------------------------------------ epilogue
+    const uint32_t quarter = (uint32_t)sched;
+    uint32_t it = 0;
+    BrickIter x;
+    for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
+      const int R = x.R(), m = x.m();
+      const F64Row* rows = B.rows + x.b.row;
+      const int32_t* tab = B.tab + x.b.tab;
+      const int ve = __ldg(args.w.vexp + x.k);
+      const bool bad = ve >= kBadExp;
+      double* acc0 = args.w.acc + (x.k & (kF64Copies - 1)) * args.hsize;
+      for (int r0 = 0; r0 < R && !abort_flag; r0 += 128) {
+        const int rq = r0 + (int)quarter * 32, r = rq + lane;
+        F64Row mr{};
+        if (r < R) mr = load_meta(rows + r);
+        const int s_img = (int)(mr.img_orb >> 8), a = (int)(mr.img_orb & 255u), noi = row_no(mr.info);
+        const int r_eff = r < R ? r : 1 << 30;
+        const int ea = row_exp(mr.info) + ve - 1023 - 54 - 2046;
+        // scales beyond these take scalbn below (phi outside 2^-423 .. 2^177, V
+        // above 2^377, V phi below 2^-446); rows of zeros have S = 0
+        const auto odd_exp = [](int e) { return e > 1 && (e < 600 || e > 1200); };
+        const bool slow_r = __any_sync(0xffffffffu, bad || ve > 1400 ||
+                                                        (r < R && (odd_exp(row_exp(mr.info)) ||
+                                                                   (row_exp(mr.info) > 1 && row_exp(mr.info) + ve < 1600))));
+        double* acc = acc0 + a;
+        for (int c0 = r0; c0 < R && !abort_flag; c0 += kWin, ++it) {
+          const uint32_t buf = it & 1;
+          // the window's columns: lane l keeps column c0 + l for the shuffles below
+          F64Row mc{};
+          if (c0 + lane < R) mc = load_meta(rows + c0 + lane);
+          const bool slow = slow_r || __any_sync(0xffffffffu, c0 + lane < R && odd_exp(row_exp(mc.info)));
+          if (!tc::mbar_wait_warp(&tfull_bar[buf], (it >> 1) & 1, &abort_flag)) {
+            give_up();
+            break;
+          }
+          tc::fence_after_sync();
+          if (rq < R && rq <= c0) {  // rows of this warp that count in this window
+#pragma unroll 1
+            for (int cb = rank * 4; cb < kWin; cb += nepi * 4) {
+              if (c0 + cb >= R) break;
+              int32_t offs[4];  // every load in flight together (columns past R: entry t = 0)
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                offs[j] = __ldg(tab + (int64_t)s_img * m + (__shfl_sync(0xffffffffu, mc.img_orb, cb + j) >> 8));
+              uint32_t y[kDig][4];
+              load_acc(tmem, quarter, buf * kBufCols + cb, y);
+              // no branch before the adds: the four columns' chains interleave
+              // (with one, each column took 550 clocks of its own latency); one
+              // conversion on the FP64 pipe costs less than the dozen integer
+              // instructions that normalise S
+              double v[4];
+              int64_t S[4];
+              int ex[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint32_t io = __shfl_sync(0xffffffffu, mc.img_orb, cb + j);
+                ex[j] = ea + row_exp(__shfl_sync(0xffffffffu, mc.info, cb + j));
+                S[j] = assemble_bounded(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
+                // columns past R have S = 0
+                const bool counts = r_eff <= c0 + cb + j && offs[j] >= 0 && (S[j] != 0 || (bad && c0 + cb + j < R));
+                offs[j] = counts ? offs[j] + (int)(io & 255u) * noi : -1;
+                v[j] = (double)S[j];
+              }
+              if (!slow) {  // S 2^-54 2^(ea - 1023) 2^(eb - 1023): no under- or overflow
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                  v[j] = __hiloint2double(__double2hiint(v[j]) + (ex[j] << 20), __double2loint(v[j]));
+              } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                  v[j] = bad ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(v[j], ex[j]);
+              }
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                if (offs[j] >= 0 && bounds_ok((int64_t)offs[j] + a, args.hsize, 20)) atomicAdd(acc + offs[j], v[j]);
+            }
+          }
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&tempty_bar[buf]);
+        }
+      }
+    }
+  } else if (is_mma) {
+    // ------------------------------------------------------------ MMA issuer
+    uint32_t it = 0;
+    BrickIter x;
+    for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
+      const int R = x.R();
+      for (int r0 = 0; r0 < R && !abort_flag; r0 += 128) {
+        for (int c0 = r0; c0 < R; c0 += kWin, ++it) {
+          const uint32_t buf = it & 1, use = it >> 1;
+          if (use > 0 && !tc::mbar_wait_warp(&tempty_bar[buf], (use - 1) & 1, &abort_flag)) {
+            give_up();
+            break;
+          }
+          if (!tc::mbar_wait_warp(&bready_bar[buf], use & 1, &abort_flag)) {
+            give_up();
+            break;
+          }
+          tc::fence_after_sync();
+          const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sB + buf * kHBStage), d0 = tmem + buf * kBufCols;
+#pragma unroll
+          for (int ks = 0; ks < kHP / 16; ++ks) {
+            const uint64_t db = tc::smem_desc(b0 + ks * 2 * kHBLbo, kHBLbo, 128);
+#pragma unroll
+            for (int i = 0; i < kDig; ++i) {
+              const uint64_t da = tc::smem_desc(a0 + i * kHADigit + ks * 4096, 2048, 128);
+              // digit 0 writes all seven accumulators first
+              if (tc::elect_one())
+                tc::mma_bf16(d0 + kWin * i, da, db, idesc_f16_f32(128, kWin * (kDig - i), 0, 0),
+                             (ks > 0 || i > 0) ? 1u : 0u);
+            }
+          }
+          if (tc::elect_one()) {
+            tc::mma_commit(&bempty_bar[buf]);
+            tc::mma_commit(&tfull_bar[buf]);
+            if (c0 + kWin >= R) tc::mma_commit(&afree_bar);  // the tile's A may be overwritten
+          }
+          __syncwarp();
+        }
+      }
+    }
+    if (tc::elect_one()) {
+      tc::mma_commit(&drain_bar);
+      if (!tc::mbar_wait(&drain_bar, 0, 1u << 24)) give_up();
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ split
+    const int kg = sched == 1 ? rank - 3 : (sched == 2 ? rank : rank + 3);  // 0..7
+    uint32_t it = 0, tile = 0, rslot = 0, rpar = 0;
+    uint8_t* raw = smem + kDig * kHADigit + 2 * kHBStage;
+    StepIter x, ahead;  // warp kg 0 fetches kHRaw - 1 steps ahead
+    x.begin(B);
+    ahead = x;
+    RawRing<kHRaw> ring{raw, rawfull_bar, rawempty_bar};
+    auto fetch = [&]() {
+      if (!ahead.valid()) return true;
+      const bool ok = ring.issue(reinterpret_cast<const uint8_t*>(B.table + (int64_t)(ahead.b.chunk + ahead.c0 / 32) * 32 * kHP),
+                                 &abort_flag);
+      ahead.step(B);
+      return ok;
+    };
+    if (kg == 0)
+      for (int i = 0; i < kHRaw - 1; ++i) fetch();
+    while (x.valid() && !abort_flag) {
+      if (kg == 0 && !fetch()) {
+        give_up();
+        break;
+      }
+      const int k = x.k;
+      const int r0 = x.r0, c0 = x.c0;
+      x.step(B);
+      longlong2 v[4];
+      if (c0 < r0 + 128) {
+        const longlong2* vb = reinterpret_cast<const longlong2*>(args.w.vb + (int64_t)k * kHP + kg * 8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = __ldg(vb + i);
+      }
+      uint64_t t[8];
+      if (!tc::mbar_wait_warp(&rawfull_bar[rslot], rpar, &abort_flag)) {
+        give_up();
+        break;
+      }
+      read_piece(raw + rslot * kRawBytes + kg * 2048, lane, t);
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&rawempty_bar[rslot]);
+      if (++rslot == kHRaw) {
+        rslot = 0;
+        rpar ^= 1;
+      }
+      const uint32_t buf = it & 1, use = it >> 1;
+      if (use > 0 && !tc::mbar_wait_warp(&bempty_bar[buf], (use - 1) & 1, &abort_flag)) {
+        give_up();
+        break;
+      }
+      store_digits(sB + buf * kHBStage + kg * kHBLbo + lane * 16, kWin * 16, t);
+      if (c0 < r0 + 128) {  // also row block (c0 - r0) / 32 of A
+        if (c0 == r0) {
+          if (tile > 0 && !tc::mbar_wait_warp(&afree_bar, (tile - 1) & 1, &abort_flag)) {
+            give_up();
+            break;
+          }
+          ++tile;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          // t V 2^-62, rounded: V is a multiple of 2^-62 of its bound
+          t[2 * i] = (uint64_t)((__mul64hi((int64_t)(t[2 * i] - kF64Bias) * 8, v[i].x) + 1) >> 1) + kF64Bias;
+          t[2 * i + 1] = (uint64_t)((__mul64hi((int64_t)(t[2 * i + 1] - kF64Bias) * 8, v[i].y) + 1) >> 1) + kF64Bias;
+        }
+        store_digits(sA + kg * 2048 + (c0 - r0 + lane) * 16, kHADigit, t);
+      }
+      tc::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&bready_bar[buf]);
+      __syncwarp();
+      ++it;
+    }
+    if (kg == 0) ring.drain();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  if (is_mma) tc::tmem_dealloc(tmem, 512);
+}
+
+// The accumulated blocks (the later of a pair's two blocks, [b][a]), their
+// copies added in a fixed order, times gridvol, in both orientations; a self
+// pair holds a <= b only.
+__global__ void f64_finish_kernel(DevPairs pr, const int32_t* __restrict__ numorbs, const double* __restrict__ acc,
+                                  int64_t hsize, double gridvol, double* __restrict__ H) {
+  for (int64_t q = blockIdx.x; q < pr.nu; q += gridDim.x) {
+    const int noi = numorbs[pr.atom[q]], noj = numorbs[pr.jatom[q]];
+    const int64_t bp = pr.boff_p[q], bq = pr.boff_q[q];
+    const bool self = pr.self[q] != 0;
+    for (int e = threadIdx.x; e < noi * noj; e += blockDim.x) {
+      const int b = e / noi, a = e - b * noi;
+      if (self && a > b) continue;
+      double c[kF64Copies];
+#pragma unroll
+      for (int i = 0; i < kF64Copies; ++i) c[i] = acc[i * hsize + bq + e];
+#pragma unroll
+      for (int w = kF64Copies / 2; w > 0; w /= 2)
+#pragma unroll
+        for (int i = 0; i < w; ++i) c[i] += c[i + w];
+      const double v = c[0] * gridvol;
+      H[bq + e] = v;
+      H[bp + (int64_t)a * noj + b] = v;
+    }
+  }
+}
+
+}  // namespace
+
+// ==========================================================================
+// Density.  Per brick of 128 points, over its R packed rows,
+//
+//   rho(p) = sum_c phi_c(p) X[p][c],  X[p][c] = sum_{r <= c} phi_r(p) Ds[r][c],
+//   Ds[r][c] = D_rc + D_cr (r < c),  D_rr (r = c),
+//
+// M = the points, windows of 32 columns, K the packed rows in chunks of 32
+// (only the rows up to the window).  A (phi, scaled per point) is MN-major,
+// so that a lane splits one row at eight points; B (Ds, scaled per column) is
+// K-major.
+//
+// Roles (672 threads, one CTA per SM, persistent over bricks):
+//   warps 0-7    epilogue: lane = point, half a window each: X assembled in 64
+//                bits, times phi_c(p) into a 128-bit sum (FP64 products took
+//                128 clocks per column and warp of this GPU's FP64 pipe);
+//   warp 8       MMA issuer: per chunk 2 K steps x 7 MMAs;
+//   warps 9-16   split A: two of a chunk's sixteen pieces (8 points x 32 rows) each;
+//   warps 17-20  split B: one of its four pieces (8 rows x 32 columns) each; the
+//                entries' addresses come from the pair tables, two chunks ahead.
+// Every split warp has its next chunk's loads in flight while it splits one:
+// without that a chunk took 5,000 clocks, whatever the arithmetic.
+// ==========================================================================
+namespace {
+
+constexpr int kDP = 128;
+constexpr int kDEpi = 8, kDConvA = 8, kDConvB = 4, kDConv = kDConvA + kDConvB;
+constexpr int kDThreads = 32 * (kDEpi + 1 + kDConv);
+constexpr int kDChunk = 32;
+constexpr uint32_t kDStages = 2;
+constexpr int kDRaw = 5;                                      // half chunks of the table in shared memory
+constexpr uint32_t kDADigit = kDP * kDChunk * 2;             // 8 KB: [point group][32 rows][16 B]
+constexpr uint32_t kDBLbo = kDig * kWin * 16;
+constexpr uint32_t kDBBytes = (kDChunk / 8) * kDBLbo;        // 14 KB
+constexpr uint32_t kDStageBytes = kDig * kDADigit + kDBBytes;  // 70 KB
+constexpr size_t kDSmemBytes = kDStages * (size_t)kDStageBytes + kDRaw * (size_t)kRawBytes;  // 220 KB
+static_assert(2 * kRawBytes == 32 * kDP * 8, "a raw slot is half a chunk");
+
+// sum a_d 256^(7-d) / 256, rounded, for |a_d| <= 2^24 (d <= 5; a_6 and a_7 may
+// round in their last places, 2^-54 of the result's scale and below).
+__device__ __forceinline__ int64_t assemble(uint32_t u1, uint32_t u2, uint32_t u3, uint32_t u4, uint32_t u5, uint32_t u6,
+                                            uint32_t u7) {
+  constexpr float M = 12582912.0f;
+  const float f7 = __fadd_rn(__fmaf_rn(__uint_as_float(u7), 0.00390625f, M), -M);
+  const int i6 = __float2int_rn(__fadd_rn(__uint_as_float(u6), f7));
+  const int a1 = __float2int_rn(__uint_as_float(u1)), a2 = __float2int_rn(__uint_as_float(u2)),
+            a3 = __float2int_rn(__uint_as_float(u3)), a4 = __float2int_rn(__uint_as_float(u4)),
+            a5 = __float2int_rn(__uint_as_float(u5));
+  int64_t S = (int64_t)a5 * 256 + i6;
+  S += (int64_t)a4 * 65536;
+  S += (int64_t)a3 * (1 << 24);
+  return S + (int64_t)((uint64_t)(uint32_t)(a1 * 256 + a2) << 32);
+}
+
+struct F64DensArgs {
+  F64Bricks b;
+  const uint64_t* dfix;
+  const uint32_t* cmax;  // [natom * 32] high word of max |Ds| of a column, raised by the grid's slack
+  const int32_t* btop;   // [nbricks] exponent bound of the largest finite column of a brick
+  double* rho;
+  int* status;
+};
+
+// Ds per ordered pair and the largest magnitude of each column (orbital b of
+// the neighbour atom), one block per pair.
+__global__ void __launch_bounds__(128) f64_dsym_kernel(F64Pairs pr, const double* __restrict__ dm,
+                                                       double* __restrict__ dsym, uint32_t* __restrict__ cmax,
+                                                       int slack) {
+  __shared__ uint32_t mx[32];
+  for (int64_t p = blockIdx.x; p < pr.npairs; p += gridDim.x) {
+    const int i = pr.atom[p], j = pr.jatom[p];
+    const int noi = pr.numorbs[i], noj = pr.numorbs[j];
+    const int q = pr.partner[p];
+    const int64_t bp = pr.boff[p], bq = pr.boff[q];
+    if (threadIdx.x < 32) mx[threadIdx.x] = 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < noi * noj; e += blockDim.x) {
+      const int a = e / noj, b = e - a * noj;
+      double v = dm[bp + e];
+      if (q != p || a != b) v += dm[bq + (int64_t)b * noi + a];
+      dsym[bp + e] = v;
+      atomicMax(&mx[b], (uint32_t)__double2hiint(v) & 0x7fffffffu);
+    }
+    __syncthreads();
+    if (threadIdx.x < noj) {
+      const uint32_t h = mx[threadIdx.x];
+      atomicMax(cmax + (int64_t)j * 32 + threadIdx.x, h < 0x7fe00000u ? h + ((uint32_t)slack << 20) : h);
+    }
+    __syncthreads();
+  }
+}
+
+// Exponent bound of the largest finite column scale among a brick's rows (one warp per brick).
+__global__ void __launch_bounds__(256) f64_btop_kernel(F64Bricks b, const uint32_t* __restrict__ cmax,
+                                                       int32_t* __restrict__ btop) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < b.nbricks;
+       k += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const F64Brick br = load_brick(b.bricks + k);
+    int e = 1;
+    for (int r = lane; r < (int)(br.size & 0xffffu); r += 32) {
+      const int x = exp_bound(__ldg(cmax + row_col(load_meta(b.rows + br.row + r).info)));
+      if (x < kBadExp) e = max(e, x);
+    }
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) btop[k] = e;
+  }
+}
+
+// Ds on the grids of its columns' scales.
+__global__ void __launch_bounds__(128) f64_dfix_kernel(F64Pairs pr, const double* __restrict__ dsym,
+                                                       const uint32_t* __restrict__ cmax, uint64_t* __restrict__ dfix) {
+  for (int64_t p = blockIdx.x; p < pr.npairs; p += gridDim.x) {
+    const int j = pr.jatom[p], noj = pr.numorbs[j], n = pr.numorbs[pr.atom[p]] * noj;
+    const int64_t bp = pr.boff[p];
+    for (int e = threadIdx.x; e < n; e += blockDim.x)
+      dfix[bp + e] = fx_biased(dsym[bp + e], exp_bound(__ldg(cmax + (int64_t)j * 32 + e % noj)));
+  }
+}
+
+// Chunks of a CTA in order: brick, window c0, row chunk r0 <= c0.
+template <bool AHEAD>
+struct ChunkIter : BrickIterT<AHEAD> {
+  int c0, r0;
+  __device__ __forceinline__ void begin(const F64Bricks& B) {
+    c0 = r0 = 0;
+    this->start(B);
+  }
+  __device__ __forceinline__ void step(const F64Bricks& B) {
+    r0 += kDChunk;
+    if (r0 <= c0) return;
+    r0 = 0;
+    c0 += kWin;
+    if (c0 < this->R()) return;
+    c0 = 0;
+    this->next(B);
+  }
+};
+
+// Eight rows of a chunk's B for one column per lane, in three steps whose
+// loads depend on one another, each a chunk ahead of the next: the rows and
+// the column (ask_b), the pair tables' block offsets (locate_b), the entries
+// (gather_b).  The L1 that the shared memory leaves is too small to hold any
+// of them, so every load takes its time in L2.  No branches around the loads
+// (entry 0 where there is nothing), so that they are in flight together.
+struct BAsk {
+  F64Row col;
+  uint32_t rio, mask;  // img_orb of row lane % 8; rows that count: on or above the diagonal, inside R
+  uint32_t tab;
+  int m;
+  bool ok;
+};
+struct BPiece {
+  uint32_t rio, mask;
+  int b, noj;  // the column's orbital and its atom's orbitals
+  int32_t off[8];
+  bool ok;
+};
+__device__ __forceinline__ void ask_b(const F64Bricks& B, const ChunkIter<false>& x, int g, int lane, BAsk& q) {
+  q.ok = x.valid();
+  if (!q.ok) return;
+  const int c = x.c0 + lane, rh = x.r0 + 8 * g, R = x.R();
+  q.tab = x.b.tab;
+  q.m = x.m();
+  q.col = load_meta(B.rows + x.b.row + min(c, R - 1));
+  q.rio = load_meta(B.rows + x.b.row + min(rh + (lane & 7), R - 1)).img_orb;
+  q.mask = c < R && c >= rh ? (c - rh >= 7 ? 255u : (2u << (c - rh)) - 1u) : 0u;
+}
+__device__ __forceinline__ void locate_b(const F64Bricks& B, const BAsk& a, BPiece& q) {
+  q.ok = a.ok;
+  if (!a.ok) return;
+  q.rio = a.rio;
+  q.mask = a.mask;
+  q.b = (int)(a.col.img_orb & 255u);
+  q.noj = row_no(a.col.info);
+  const int32_t* tab = B.tab + a.tab + (a.col.img_orb >> 8);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q.off[i] = __ldg(tab + (int)(__shfl_sync(0xffffffffu, a.rio, i) >> 8) * a.m);
+}
+__device__ __forceinline__ void gather_b(const uint64_t* __restrict__ dfix, const BPiece& q, uint64_t* t) {
+  if (!q.ok) return;
+  uint32_t ok = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int a = (int)(__shfl_sync(0xffffffffu, q.rio, i) & 255u);
+    const bool y = ((q.mask >> i) & 1u) && q.off[i] >= 0;
+    ok |= (y ? 1u : 0u) << i;
+    t[i] = __ldg(dfix + (y ? q.off[i] + a * q.noj + q.b : 0));
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) t[i] = (ok >> i) & 1u ? t[i] : kF64Bias;
+}
+
+__global__ void __launch_bounds__(kDThreads, 1) f64_density_kernel(const __grid_constant__ F64DensArgs args) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ uint64_t full_bar[kDStages], empty_bar[kDStages], tfull_bar[2], tempty_bar[2], drain_bar;
+  __shared__ uint64_t rawfull_bar[kDRaw], rawempty_bar[kDRaw];
+  __shared__ uint32_t tslot;
+  __shared__ volatile int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const F64Bricks& B = args.b;
+  if (warp == kDEpi) tc::tmem_alloc(&tslot, 512);
+  if (tid == 0) {
+    for (int s = 0; s < kDRaw; ++s) {
+      tc::mbar_init(&rawfull_bar[s], 1);
+      tc::mbar_init(&rawempty_bar[s], kDConvA);
+    }
+    for (uint32_t s = 0; s < kDStages; ++s) {
+      tc::mbar_init(&full_bar[s], kDConv);
+      tc::mbar_init(&empty_bar[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      tc::mbar_init(&tfull_bar[s], 1);
+      tc::mbar_init(&tempty_bar[s], kDEpi);
+    }
+    tc::mbar_init(&drain_bar, 1);
+    tc::fence_mbar_init();
+    abort_flag = 0;
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tslot;
+  auto give_up = [&]() {
+    if (!abort_flag) atomicExch(args.status, LCP_ETIMEDOUT);
+    abort_flag = 1;
+  };
+
+  if (warp < kDEpi) {
+    // ------------------------------------------------------------ epilogue
+    const uint32_t quarter = warp & 3, half = warp >> 2;
+    const int p = (int)quarter * 32 + lane;
+    uint32_t win = 0;
+    BrickIter x;
+    for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
+      const int R = x.R();
+      const uint64_t* mine = B.table + (int64_t)x.b.chunk * 32 * kDP + (p >> 3) * 256 + ((p & 7) >> 1) * 64 + (p & 1);
+      // S, a multiple of 2^-54 of the scales' product, stays below 2^63 for R < 512
+      // (|X| <= R); with more rows Ds is split on a grid one bit coarser.  The sum
+      // of X phi is a 128-bit integer in units 2^-54 2^-62 of the scales' product
+      // with the brick's largest column scale (phi shifted up by what the column's
+      // scale lies below it, at most seven bits, beyond that S down)
+      uint64_t slo = 0;
+      int64_t shi = 0;
+      bool nan = false;
+      const int etop = __ldg(args.btop + x.k);
+      for (int c0 = 0; c0 < R && !abort_flag; c0 += kWin, ++win) {
+        const uint32_t buf = win & 1;
+        // lane l keeps how far column c0 + l's scale lies below the brick's
+        // largest, for the shuffles below
+        int ce = 0;
+        if (c0 + lane < R)
+          ce = etop - exp_bound(__ldg(args.cmax + row_col(load_meta(B.rows + x.b.row + c0 + lane).info)));
+        const bool odd = __any_sync(0xffffffffu, ce < 0 || ce > 7);
+        const uint32_t up = 128u >> min(max(ce, 0), 7);
+        const uint64_t* phi = mine + (int64_t)(c0 / 32) * 32 * kDP;
+        uint64_t ph[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ph[j] = __ldg(phi + (half * 16 + j) * 2);  // rows past R are zero in the table
+        if (!tc::mbar_wait_warp(&tfull_bar[buf], (win >> 1) & 1, &abort_flag)) {
+          give_up();
+          break;
+        }
+        tc::fence_after_sync();
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          const int cb = (int)half * 16 + q * 4;
+          if (c0 + cb >= R) break;
+          uint32_t y[kDig][4];
+          load_acc(tmem, quarter, buf * kBufCols + cb, y);
+          // no branches: the four columns' chains interleave (with them, each
+          // column took 650 clocks of its own latency), and multiplications for
+          // shifts: the integer pipe is the busiest one
+          int64_t S[4], tp[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int64_t t = (int64_t)(ph[j] - kF64Bias);
+            const uint32_t m = __shfl_sync(0xffffffffu, up, cb + j);
+            tp[j] = (int64_t)((uint64_t)(uint32_t)t * m + ((uint64_t)((uint32_t)(t >> 32) * m) << 32));
+            S[j] = assemble(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
+          }
+          if (odd) {  // columns far below the brick's largest, or with Inf or NaN
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int d = __shfl_sync(0xffffffffu, ce, cb + j);
+              nan = nan || (d < 0 && ph[j] != kF64Bias);
+              if (d < 0) S[j] = 0;
+              S[j] >>= min(max(d - 7, 0), 63);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint64_t lo = (uint64_t)S[j] * (uint64_t)tp[j];
+            slo += lo;
+            shi += __mul64hi(S[j], tp[j]) + (slo < lo ? 1 : 0);
+          }
+          if (q < 3) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) ph[j] = __ldg(phi + (cb + 4 + j) * 2);
+          }
+        }
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&tempty_bar[buf]);
+      }
+      if (abort_flag) break;
+      const int64_t gi = p < B.npts ? brick_point_index(x.k, p, B.bdim, B.nb, B.ngrid) : -1;
+      const bool neg = shi < 0;
+      if (neg) {
+        slo = ~slo + 1;
+        shi = ~shi + (slo == 0 ? 1 : 0);
+      }
+      double acc = fma((double)shi, 0x1p64, (double)slo);
+      if (neg) acc = -acc;
+      if (nan) acc = __longlong_as_double(0x7ff8000000000000ll);
+      // two halves onto a zeroed point: the same sum in either order
+      if (gi >= 0 && bounds_ok(gi, (int64_t)B.ngrid[0] * B.ngrid[1] * B.ngrid[2], 21))
+        atomicAdd(args.rho + gi, scalbn(acc, 2 * (B.ptexp[(int64_t)x.k * kDP + p] - 1023) + etop - 1023 - 116));
+    }
+  } else if (warp == kDEpi) {
+    // ------------------------------------------------------------ MMA issuer
+    uint32_t st = 0, par = 0, win = 0;
+    BrickIter x;
+    for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
+      const int R = x.R();
+      for (int c0 = 0; c0 < R && !abort_flag; c0 += kWin, ++win) {
+        const uint32_t buf = win & 1;
+        if (win >= 2 && !tc::mbar_wait_warp(&tempty_bar[buf], ((win >> 1) - 1) & 1, &abort_flag)) {
+          give_up();
+          break;
+        }
+        const uint32_t d0 = tmem + buf * kBufCols;
+        for (int r0 = 0; r0 <= c0; r0 += kDChunk) {
+          if (!tc::mbar_wait_warp(&full_bar[st], par, &abort_flag)) {
+            give_up();
+            break;
+          }
+          tc::fence_after_sync();
+          const uint32_t a0 = tc::smem_u32(smem + st * kDStageBytes), b0 = a0 + kDig * kDADigit;
+#pragma unroll
+          for (int ks = 0; ks < kDChunk / 16; ++ks) {
+            const uint64_t db = tc::smem_desc(b0 + ks * 2 * kDBLbo, kDBLbo, 128);
+#pragma unroll
+            for (int i = 0; i < kDig; ++i) {
+              const uint64_t da = tc::smem_desc(a0 + i * kDADigit + ks * 256, 128, 512);
+              if (tc::elect_one())
+                tc::mma_bf16(d0 + kWin * i, da, db, idesc_f16_f32(128, kWin * (kDig - i), 1, 0),
+                             (r0 > 0 || ks > 0 || i > 0) ? 1u : 0u);
+            }
+          }
+          if (tc::elect_one()) {
+            tc::mma_commit(&empty_bar[st]);
+            if (r0 == c0) tc::mma_commit(&tfull_bar[buf]);
+          }
+          __syncwarp();
+          if (++st == kDStages) {
+            st = 0;
+            par ^= 1;
+          }
+        }
+      }
+    }
+    if (tc::elect_one()) {
+      tc::mma_commit(&drain_bar);
+      if (!tc::mbar_wait(&drain_bar, 0, 1u << 24)) give_up();
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ split
+    const int cw = warp - kDEpi - 1;
+    uint32_t st = 0, par = 1, round = 0;  // par: parity of the stage's last release
+    if (cw < kDConvA) {
+      ChunkIter<true> x, ahead;  // warp 0 fetches up to kDRaw half chunks ahead
+      x.begin(B);
+      ahead = x;
+      uint8_t* raw = smem + kDStages * kDStageBytes;
+      RawRing<kDRaw> ring{raw, rawfull_bar, rawempty_bar};
+      uint32_t half = 0, rslot = 0, rpar = 0;
+      auto fetch = [&]() {
+        if (!ahead.valid()) return true;
+        const bool ok = ring.issue(reinterpret_cast<const uint8_t*>(B.table + (int64_t)(ahead.b.chunk + ahead.r0 / 32) * 32 * kDP) +
+                                       half * kRawBytes,
+                                   &abort_flag);
+        half ^= 1;
+        if (half == 0) ahead.step(B);
+        return ok;
+      };
+      if (cw == 0)
+        for (int i = 0; i < kDRaw - 2; ++i) fetch();
+      while (x.valid() && !abort_flag) {
+        if (cw == 0 && !(fetch() && fetch())) {
+          give_up();
+          break;
+        }
+        x.step(B);
+        bool ok = round == 0 || tc::mbar_wait_warp(&empty_bar[st], par, &abort_flag);
+        uint8_t* sA = smem + st * kDStageBytes;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          ok = ok && tc::mbar_wait_warp(&rawfull_bar[rslot], rpar, &abort_flag);
+          if (ok) {
+            uint64_t t[8];
+            read_piece(raw + rslot * kRawBytes + cw * 2048, lane, t);
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&rawempty_bar[rslot]);
+            if (++rslot == kDRaw) {
+              rslot = 0;
+              rpar ^= 1;
+            }
+            store_digits(sA + (cw + 8 * h) * 512 + lane * 16, kDADigit, t);
+          }
+        }
+        if (!ok) {
+          give_up();
+          break;
+        }
+        tc::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&full_bar[st]);
+        __syncwarp();
+        if (++st == kDStages) {
+          st = 0;
+          par ^= 1;
+          round = 1;
+        }
+      }
+      if (cw == 0) ring.drain();
+    } else {
+      const int g = cw - kDConvA;
+      ChunkIter<false> x;
+      x.begin(B);
+      uint64_t t[8];
+      BAsk ask;
+      BPiece q;
+      bool now = x.valid();  // there is a chunk in t
+      ask_b(B, x, g, lane, ask);
+      locate_b(B, ask, q);
+      if (x.valid()) x.step(B);
+      ask_b(B, x, g, lane, ask);
+      gather_b(args.dfix, q, t);
+      locate_b(B, ask, q);
+      if (x.valid()) x.step(B);
+      ask_b(B, x, g, lane, ask);
+      while (now && !abort_flag) {
+        if (round > 0 && !tc::mbar_wait_warp(&empty_bar[st], par, &abort_flag)) {
+          give_up();
+          break;
+        }
+        store_digits(smem + st * kDStageBytes + kDig * kDADigit + g * kDBLbo + lane * 16, kWin * 16, t);
+        tc::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&full_bar[st]);
+        __syncwarp();
+        now = q.ok;
+        gather_b(args.dfix, q, t);
+        locate_b(B, ask, q);
+        if (x.valid()) x.step(B);
+        ask_b(B, x, g, lane, ask);
+        if (++st == kDStages) {
+          st = 0;
+          par ^= 1;
+          round = 1;
+        }
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  if (warp == kDEpi) tc::tmem_dealloc(tmem, 512);
+}
+
+}  // namespace
+
+cudaError_t launch_f64_table(const F64Bricks& b, const F64Build& f, F64Row* rows, int32_t* ptexp, uint64_t* table,
+                             cudaStream_t st) {
+  const unsigned blocks = (unsigned)std::min<int64_t>(b.nbricks, 152 * 32);
+  f64_scales_kernel<<<blocks, 256, 0, st>>>(b, f, rows, ptexp);
+  LCP_CUDA_TRY(cudaGetLastError());
+  f64_table_kernel<<<blocks, 256, 0, st>>>(b, f, table);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_f64_density(const F64Bricks& b, const F64Pairs& pr, const double* dm, const F64DensWork& w,
+                               double* rho, int* status, cudaStream_t st) {
+  const int64_t nn = (int64_t)b.ngrid[0] * b.ngrid[1] * b.ngrid[2];
+  LCP_CUDA_TRY(cudaMemsetAsync(rho, 0, (size_t)nn * sizeof(double), st));
+  if (b.nrows == 0 || pr.npairs == 0) return cudaSuccess;
+  LCP_CUDA_TRY(cudaMemsetAsync(w.cmax, 0, (size_t)pr.natom * 32 * sizeof(uint32_t), st));
+  const unsigned blocks = (unsigned)std::min<int64_t>(pr.npairs, 152 * 16);
+  f64_dsym_kernel<<<blocks, 128, 0, st>>>(pr, dm, w.dsym, w.cmax, b.max_rows >= 512 ? 1 : 0);
+  LCP_CUDA_TRY(cudaGetLastError());
+  f64_dfix_kernel<<<blocks, 128, 0, st>>>(pr, w.dsym, w.cmax, w.dfix);
+  LCP_CUDA_TRY(cudaGetLastError());
+  f64_btop_kernel<<<(unsigned)std::min<int64_t>((b.nbricks + 7) / 8, 152 * 8), 256, 0, st>>>(b, w.cmax, w.btop);
+  LCP_CUDA_TRY(cudaGetLastError());
+  F64DensArgs a{b, w.dfix, w.cmax, w.btop, rho, status};
+  LCP_CUDA_TRY(raise_smem(f64_density_kernel, kDSmemBytes));
+  f64_density_kernel<<<(unsigned)std::min<int64_t>(b.nbricks, device_sms()), kDThreads, kDSmemBytes, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_f64_hamiltonian(const F64Bricks& b, const DevPairs& folded, const int32_t* numorbs,
+                                   const double* vpot, const F64HamWork& w, double gridvol, double* hks, int64_t hsize,
+                                   int* status, cudaStream_t st) {
+  if (b.nrows == 0 || folded.nu == 0) return cudaMemsetAsync(hks, 0, (size_t)hsize * sizeof(double), st);
+  LCP_CUDA_TRY(cudaMemsetAsync(w.acc, 0, (size_t)hsize * kF64Copies * sizeof(double), st));
+  f64_vprep_kernel<<<(unsigned)std::min<int64_t>(b.nbricks, 152 * 32), kHP, 0, st>>>(b, vpot, w.vb, w.vexp);
+  LCP_CUDA_TRY(cudaGetLastError());
+  F64HamArgs a{b, w, hsize, status};
+  LCP_CUDA_TRY(raise_smem(f64_hamiltonian_kernel, kHSmemBytes));
+  f64_hamiltonian_kernel<<<(unsigned)std::min<int64_t>(b.nbricks, device_sms()), kHThreads, kHSmemBytes, st>>>(a);
+  LCP_CUDA_TRY(cudaGetLastError());
+  f64_finish_kernel<<<(unsigned)std::min<int64_t>(folded.nu, 152 * 16), 128, 0, st>>>(folded, numorbs, w.acc, hsize,
+                                                                                       gridvol, hks);
+  return cudaGetLastError();
+}
+
+}  // namespace lcp

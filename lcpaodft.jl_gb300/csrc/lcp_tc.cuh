@@ -244,4 +244,16 @@ __device__ __forceinline__ uint32_t mnmajor_off(uint32_t mn, uint32_t k, uint32_
 
 
 }  // namespace tc
+
+// Grid index of slot p of home brick hb, or -1 for a slot of a ragged brick
+// that lies past the grid.
+__device__ __forceinline__ int64_t brick_point_index(int64_t hb, int p, const int32_t* bdim, const int32_t* nb,
+                                                     const int32_t* ngrid) {
+  const int l2 = p % bdim[2], l1 = (p / bdim[2]) % bdim[1], l0 = p / (bdim[1] * bdim[2]);
+  const int64_t h2 = hb % nb[2], h1 = (hb / nb[2]) % nb[1], h0 = hb / ((int64_t)nb[1] * nb[2]);
+  const int64_t x = h0 * bdim[0] + l0, y = h1 * bdim[1] + l1, z = h2 * bdim[2] + l2;
+  if (x >= ngrid[0] || y >= ngrid[1] || z >= ngrid[2]) return -1;
+  return (x * ngrid[1] + y) * ngrid[2] + z;
+}
+
 }  // namespace lcp

@@ -114,11 +114,93 @@ lcp_status ensure_phi32(lcp_ctx* ctx, lcp_orbs* o) {
   return LCP_OK;
 }
 
+// The overlap lists and work items of the pair kernels (FP32, the force term,
+// the FP64 cells beyond the tensor-core kernels' limits and FP64 steps whose
+// first run is inside a stream capture).
+static lcp_status make_lens(lcp_ctx* ctx, lcp_orbs* o) {
+  cudaStream_t st = ctx->stream;
+  const lcp::UCell& u = o->ucell->u;
+  // 512-entry work items: items of pairs with at most 16 orbitals per atom
+  // first, then the others (e.g. the 13-orbital pairs of a cell with some
+  // 18-orbital atoms get exact 13-orbital tiles instead of 18)
+  const int64_t nu = (int64_t)u.uniq_pair.size();
+  const int64_t chunk = 512;
+  std::vector<int64_t> ip, is, ip_l, is_l;
+  std::vector<int32_t> ic, ic_l;
+  for (int64_t q = 0; q < nu; ++q) {
+    const int p = u.uniq_pair[q];
+    const int ni = u.numorbs[u.pair_atom[p]], nj = u.numorbs[u.pair_jatom[p]];
+    if (ni == 0 || nj == 0) continue;
+    const int no = std::max(ni, nj);
+    const bool small = no <= 16;
+    if (small) o->max_no_small = std::max(o->max_no_small, no);
+    else o->max_no_large = std::max(o->max_no_large, no);
+    for (int64_t s0 = u.uniq_off[q]; s0 < u.uniq_off[q + 1]; s0 += chunk) {
+      (small ? ip : ip_l).push_back(q);
+      (small ? is : is_l).push_back(s0);
+      (small ? ic : ic_l).push_back((int32_t)std::min<int64_t>(chunk, u.uniq_off[q + 1] - s0));
+    }
+  }
+  o->nitems_small = (int64_t)ip.size();
+  ip.insert(ip.end(), ip_l.begin(), ip_l.end());
+  is.insert(is.end(), is_l.begin(), is_l.end());
+  ic.insert(ic.end(), ic_l.begin(), ic_l.end());
+  API_CUDA(upload(o->p_lensoff, u.uniq_off, st), "upload");
+  if (o->ucell->host_lens) {
+    API_CUDA(upload(o->p_g1, u.uniq_g1, st), "upload");
+    API_CUDA(upload(o->p_g2, u.uniq_g2, st), "upload");
+  } else if (o->ucell->device != ctx->device) {
+    const lcp_status s = ucell_device_lens(ctx, o->ucell, &o->p_g1, &o->p_g2);
+    if (s) return s;
+  }
+  API_CUDA(upload(o->it_pair, ip, st), "upload");
+  API_CUDA(upload(o->it_start, is, st), "upload");
+  API_CUDA(upload(o->it_count, ic, st), "upload");
+  if (o->grad) {
+    // the force term's per-atom entries: item k's kept orientation goes to
+    // its pair's atom, the partner orientation to the neighbour atom
+    std::vector<int64_t> cnt(u.natom + 1, 0), code;
+    auto ends = [&](size_t k, int& i, int& j) {
+      const int p = u.uniq_pair[ip[k]];
+      i = u.pair_atom[p];
+      j = u.partner[p] == p ? -1 : u.pair_jatom[p];
+    };
+    int i, j;
+    for (size_t k = 0; k < ip.size(); ++k) {
+      ends(k, i, j);
+      cnt[i + 1]++;
+      if (j >= 0) cnt[j + 1]++;
+    }
+    for (int a = 0; a < u.natom; ++a) cnt[a + 1] += cnt[a];
+    std::vector<int64_t> fill(cnt.begin(), cnt.end() - 1);
+    code.resize(cnt[u.natom]);
+    for (size_t k = 0; k < ip.size(); ++k) {
+      ends(k, i, j);
+      code[fill[i]++] = (int64_t)k * 2;
+      if (j >= 0) code[fill[j]++] = (int64_t)k * 2 + 1;
+    }
+    API_CUDA(upload(o->f_off, cnt, st), "upload");
+    API_CUDA(upload(o->f_code, code, st), "upload");
+  }
+  DevPairs& pr = o->pairs;
+  pr.lens_off = o->p_lensoff.as<int64_t>();
+  const bool shared = !o->ucell->host_lens && o->ucell->device == ctx->device;
+  pr.g1 = shared ? o->ucell->g1.as<int32_t>() : o->p_g1.as<int32_t>();
+  pr.g2 = shared ? o->ucell->g2.as<int32_t>() : o->p_g2.as<int32_t>();
+  pr.nitems = (int64_t)ip.size();
+  pr.item_pair = o->it_pair.as<int64_t>();
+  pr.item_start = o->it_start.as<int64_t>();
+  pr.item_count = o->it_count.as<int32_t>();
+  return LCP_OK;
+}
+
 // Brick tiling, split-BF16 orbital tables and the ordered pair list of the
 // tensor-core path, built once per tabulation.
 lcp_status ensure_bricks(lcp_ctx* ctx, lcp_orbs* o) {
   if (o->bricks_ready) return LCP_OK;
   if (o->phi_released) return fail(LCP_ESTATE, "the FP64 orbital tables were released");
+  const lcp_status ls = ucell_host_lists(o->ucell);
+  if (ls) return ls;
   const lcp::UCell& u = o->ucell->u;
   lcp::Bricks& b = o->bricks;
   std::string err = lcp::build_bricks(u, b, o->brick_shape[0] > 0 ? o->brick_shape : nullptr);
@@ -490,6 +572,10 @@ lcp_status lcp_ucell_get_info(const lcp_ucell* ucell, lcp_ucell_info* info) {
 lcp_status lcp_ucell_get_int(const lcp_ucell* ucell, int32_t field, int64_t index, int32_t* dst, int64_t count) {
   if (!ucell || (!dst && count > 0)) return fail(LCP_EINVAL, "NULL argument");
   const lcp::UCell& u = ucell->u;
+  if (field == LCP_F_GRIDLIST || field == LCP_F_CELLLIST || field == LCP_F_GLIST1 || field == LCP_F_GLIST2) {
+    const lcp_status s = ucell_host_lists(ucell);
+    if (s) return s;
+  }
   std::vector<int32_t> tmp;
   const int32_t* src = nullptr;
   int64_t n = 0;
@@ -537,6 +623,8 @@ lcp_status lcp_ucell_get_int(const lcp_ucell* ucell, int32_t field, int64_t inde
 
 lcp_status lcp_ucell_get_bricks(const lcp_ucell* ucell, int64_t* info) {
   if (!ucell || !info) return fail(LCP_EINVAL, "NULL argument");
+  const lcp_status ls = ucell_host_lists(ucell);
+  if (ls) return ls;
   lcp::Bricks b;
   std::string err = lcp::build_bricks(ucell->u, b);
   if (!err.empty()) return fail(LCP_EINVAL, err);
@@ -720,8 +808,12 @@ lcp_status lcp_set_orbitals_grid(lcp_ctx* ctx, const lcp_ucell* ucell, int32_t n
   API_CUDA(upload(o->gxyz, u.gxyz, st), "upload");
   API_CUDA(upload(o->spe, spe0, st), "upload");
   API_CUDA(upload(o->sph_off, u.sphere_off, st), "upload");
-  API_CUDA(upload(o->glist, u.glist, st), "upload");
-  API_CUDA(upload(o->clist, u.clist, st), "upload");
+  const bool shared = ucell->device == ctx->device;  // the cell's own lists on this device
+  if (!shared) {
+    if ((s = ucell_host_lists(ucell))) return s;
+    API_CUDA(upload(o->glist, u.glist, st), "upload");
+    API_CUDA(upload(o->clist, u.clist, st), "upload");
+  }
   API_CUDA(upload(o->phi_off, phi_off, st), "upload");
   API_CUDA(upload(o->numorbs, u.numorbs, st), "upload");
   API_CUDA(upload(o->species, sp, st), "upload");
@@ -739,23 +831,15 @@ lcp_status lcp_set_orbitals_grid(lcp_ctx* ctx, const lcp_ucell* ucell, int32_t n
   g.gxyz = o->gxyz.as<double>();
   g.spe = o->spe.as<int32_t>();
   g.sph_off = o->sph_off.as<int64_t>();
-  g.glist = o->glist.as<int32_t>();
-  g.clist = o->clist.as<int32_t>();
+  g.glist = shared ? ucell->glist.as<int32_t>() : o->glist.as<int32_t>();
+  g.clist = shared ? ucell->clist.as<int32_t>() : o->clist.as<int32_t>();
   g.phi_off = o->phi_off.as<int64_t>();
   g.numorbs = o->numorbs.as<int32_t>();
 
-  // folded pair lists and 512-entry work items
+  // folded pair lists
   const int64_t nu = (int64_t)u.uniq_pair.size();
   std::vector<int32_t> pa(nu), pj(nu), pself(nu);
   std::vector<int64_t> bp(nu), bq(nu);
-  std::vector<int64_t> ip, is;
-  std::vector<int32_t> ic;
-  const int64_t chunk = 512;
-  // items of pairs with at most 16 orbitals per atom first, then the others
-  // (e.g. the 13-orbital pairs of a cell with some 18-orbital atoms get exact
-  // 13-orbital tiles instead of 18)
-  std::vector<int64_t> ip_l, is_l;
-  std::vector<int32_t> ic_l;
   for (int64_t q = 0; q < nu; ++q) {
     int p = u.uniq_pair[q];
     pa[q] = u.pair_atom[p];
@@ -763,50 +847,12 @@ lcp_status lcp_set_orbitals_grid(lcp_ctx* ctx, const lcp_ucell* ucell, int32_t n
     bp[q] = u.block_off[p];
     bq[q] = u.block_off[u.partner[p]];
     pself[q] = u.partner[p] == p;
-    if (u.numorbs[pa[q]] == 0 || u.numorbs[pj[q]] == 0) continue;
-    const int no = std::max(u.numorbs[pa[q]], u.numorbs[pj[q]]);
-    const bool small = no <= 16;
-    if (small) o->max_no_small = std::max(o->max_no_small, no);
-    else o->max_no_large = std::max(o->max_no_large, no);
-    for (int64_t s0 = u.uniq_off[q]; s0 < u.uniq_off[q + 1]; s0 += chunk) {
-      (small ? ip : ip_l).push_back(q);
-      (small ? is : is_l).push_back(s0);
-      (small ? ic : ic_l).push_back((int32_t)std::min<int64_t>(chunk, u.uniq_off[q + 1] - s0));
-    }
   }
-  o->nitems_small = (int64_t)ip.size();
-  ip.insert(ip.end(), ip_l.begin(), ip_l.end());
-  is.insert(is.end(), is_l.begin(), is_l.end());
-  ic.insert(ic.end(), ic_l.begin(), ic_l.end());
   API_CUDA(upload(o->p_atom, pa, st), "upload");
   API_CUDA(upload(o->p_jatom, pj, st), "upload");
   API_CUDA(upload(o->p_boffp, bp, st), "upload");
   API_CUDA(upload(o->p_boffq, bq, st), "upload");
   API_CUDA(upload(o->p_self, pself, st), "upload");
-  API_CUDA(upload(o->p_lensoff, u.uniq_off, st), "upload");
-  API_CUDA(upload(o->p_g1, u.uniq_g1, st), "upload");
-  API_CUDA(upload(o->p_g2, u.uniq_g2, st), "upload");
-  API_CUDA(upload(o->it_pair, ip, st), "upload");
-  API_CUDA(upload(o->it_start, is, st), "upload");
-  API_CUDA(upload(o->it_count, ic, st), "upload");
-  if (o->grad) {
-    // the force term's per-atom entries: item k's kept orientation goes to
-    // its pair's atom, the partner orientation to the neighbour atom
-    std::vector<int64_t> cnt(u.natom + 1, 0), code;
-    for (size_t k = 0; k < ip.size(); ++k) {
-      cnt[pa[ip[k]] + 1]++;
-      if (!pself[ip[k]]) cnt[pj[ip[k]] + 1]++;
-    }
-    for (int a = 0; a < u.natom; ++a) cnt[a + 1] += cnt[a];
-    std::vector<int64_t> fill(cnt.begin(), cnt.end() - 1);
-    code.resize(cnt[u.natom]);
-    for (size_t k = 0; k < ip.size(); ++k) {
-      code[fill[pa[ip[k]]]++] = (int64_t)k * 2;
-      if (!pself[ip[k]]) code[fill[pj[ip[k]]]++] = (int64_t)k * 2 + 1;
-    }
-    API_CUDA(upload(o->f_off, cnt, st), "upload");
-    API_CUDA(upload(o->f_code, code, st), "upload");
-  }
   DevPairs& pr = o->pairs;
   pr.nu = nu;
   pr.atom = o->p_atom.as<int32_t>();
@@ -814,14 +860,7 @@ lcp_status lcp_set_orbitals_grid(lcp_ctx* ctx, const lcp_ucell* ucell, int32_t n
   pr.boff_p = o->p_boffp.as<int64_t>();
   pr.boff_q = o->p_boffq.as<int64_t>();
   pr.self = o->p_self.as<int32_t>();
-  pr.lens_off = o->p_lensoff.as<int64_t>();
-  pr.g1 = o->p_g1.as<int32_t>();
-  pr.g2 = o->p_g2.as<int32_t>();
   pr.hsize = u.total_hsize;
-  pr.nitems = (int64_t)ip.size();
-  pr.item_pair = o->it_pair.as<int64_t>();
-  pr.item_start = o->it_start.as<int64_t>();
-  pr.item_count = o->it_count.as<int32_t>();
 
   // tabulation
   API_CUDA(o->phi.ensure(o->table_elems * sizeof(double)), "phi alloc");
@@ -856,6 +895,7 @@ lcp_status lcp_set_orbitals_grid(lcp_ctx* ctx, const lcp_ucell* ucell, int32_t n
   cudaEventElapsedTime(&o->tab_ms, te[0], te[1]);
   cudaEventDestroy(te[0]);
   cudaEventDestroy(te[1]);
+  if ((s = make_lens(ctx, o.get()))) return s;
   *out = o.release();
   return LCP_OK;
 }
@@ -1824,6 +1864,8 @@ lcp_status lcp_job_footprint(const lcp_job* job, int64_t* bytes) {
   for (const F64Set* f : {&o->f64_density, &o->f64_elements})
     for (const DBuf* d : {&f->bricks, &f->rows, &f->table, &f->ptexp, &f->tab}) add(*d);
   for (const DBuf& d : o->f64_pair_buf) add(d);
+  if (o->ucell->device == o->device)  // the cell's lists that the tables read
+    for (const DBuf* d : {&o->ucell->glist, &o->ucell->clist, &o->ucell->g1, &o->ucell->g2}) add(*d);
   *bytes = b;
   return LCP_OK;
 }
@@ -1839,7 +1881,7 @@ int64_t job_footprint_estimate(lcp_job* job, int32_t precision) {
   const lcp_orbs* o = job->orbs;
   if (precision == LCP_PREC_BF16X3 && !o->bricks_ready) {
     lcp::Bricks b;
-    if (!lcp::build_bricks(o->ucell->u, b, o->brick_shape[0] > 0 ? o->brick_shape : nullptr).empty()) return -1;
+    if (ucell_host_lists(o->ucell) != LCP_OK || !lcp::build_bricks(o->ucell->u, b, o->brick_shape[0] > 0 ? o->brick_shape : nullptr).empty()) return -1;
     fp += b.nblocks * 6144 * 2 + (int64_t)b.point_code.size() * 4 + (int64_t)b.tab_pair.size() * 8 +
           (int64_t)(b.img_off.size() + b.slot_base.size() + b.red_off.size() + b.red_slot.size()) * 8 +
           (int64_t)(b.img_block.size() + b.sub_pair.size() + b.sub_chunks.size() + b.sb_fold.size() +

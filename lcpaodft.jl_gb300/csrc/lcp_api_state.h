@@ -72,6 +72,10 @@ struct DBuf {
     p = nullptr;
     bytes = 0;
   }
+  void swap(DBuf& o) {
+    std::swap(p, o.p);
+    std::swap(bytes, o.bytes);
+  }
   template <class T>
   T* as() const {
     return reinterpret_cast<T*>(p);
@@ -92,6 +96,12 @@ static inline int channels(int32_t spinpol) { return spinpol == LCP_SPIN_OFF ? 1
 
 struct lcp_ucell {
   lcp::UCell u;
+  // a cell built on the device: its sphere and overlap lists there, in u.glist
+  // / u.clist only once ucell_host_lists copied them, never in u.uniq_g1/2
+  int device = -1;
+  DBuf glist, clist, g1, g2;
+  bool host_lists = true, host_lens = true;
+  mutable std::mutex mutex;
 };
 
 // The hand-written FFT's plan of one grid shape: radices and roots of unity.
@@ -226,6 +236,8 @@ lcp_status make_fft_plan(const int32_t* ng, FftPlans* p);
 lcp_status check_ctx(lcp_ctx* ctx);
 lcp_status check_pair(const lcp_ucell* ucell, const lcp_orbs* orbs);
 lcp_status ensure_bricks(lcp_ctx* ctx, lcp_orbs* o);
+lcp_status ucell_host_lists(const lcp_ucell* c);
+lcp_status ucell_device_lens(lcp_ctx* ctx, const lcp_ucell* c, DBuf* g1, DBuf* g2);
 lcp_status device_status(lcp_ctx* ctx);
 lcp_status ensure_f64(lcp_ctx* ctx, lcp_orbs* o);
 int64_t f64_footprint_estimate(const lcp_orbs* o);

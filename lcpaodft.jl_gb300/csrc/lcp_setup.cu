@@ -590,14 +590,21 @@ struct SetupBuffers {
 
 }  // namespace
 
-// Calc_AtomsGrid and Calc_AtomOverlap_Grid on the device for a UCell whose
-// head (image cells, neighbour and pair lists) is built; fills the sphere and
-// overlap lists of u exactly as build_spheres_host / build_overlaps_host.
-lcp_status build_ucell_device(lcp_ctx* ctx, UCell& u) {
+namespace {
+
+struct DeviceLists {
+  SetupBuffers B;
+  SetupGeom G{};
+};
+
+// Calc_AtomsGrid on the device: the sphere lists and the box tables of a UCell
+// whose head (image cells, neighbour and pair lists) is built, in d.B; fills
+// u.sphere_off.
+lcp_status device_spheres(lcp_ctx* ctx, UCell& u, DeviceLists& d) {
   cudaStream_t st = ctx->stream;
   const int natom = u.natom;
   const int C = u.cpycell;
-  SetupBuffers B;
+  SetupBuffers& B = d.B;
   std::vector<SphereAtom> atoms(natom);
   std::vector<int32_t> tabs;
   std::vector<int64_t> cand_off(natom + 1, 0);
@@ -637,7 +644,7 @@ lcp_status build_ucell_device(lcp_ctx* ctx, UCell& u) {
   }
   const int64_t total = cand_off[natom];
   if (total >= ((int64_t)1 << 31)) return fail(LCP_ENOTSUP, "grid boxes too large for the device build");
-  SetupGeom G{};
+  SetupGeom& G = d.G;
   for (int d = 0; d < 3; ++d) {
     G.ng[d] = u.ngrid[d];
     G.origin[d] = u.origin[d];
@@ -683,14 +690,17 @@ lcp_status build_ucell_device(lcp_ctx* ctx, UCell& u) {
                                                               B.lut.as<int32_t>());
   API_CUDA(cudaGetLastError(), "sphere write");
   ctx->launches += 6;
-  u.glist.resize(nent);
-  u.clist.resize(nent);
-  if (nent) {
-    API_CUDA(cudaMemcpyAsync(u.glist.data(), B.glist.p, nent * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "D2H");
-    API_CUDA(cudaMemcpyAsync(u.clist.data(), B.clist.p, nent * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "D2H");
-  }
+  API_CUDA(cudaStreamSynchronize(st), "sphere lists");  // before the host tables above go
+  return LCP_OK;
+}
 
-  // overlap lists of the folded pairs
+// Calc_AtomOverlap_Grid on the device after device_spheres: the overlap lists
+// of the folded pairs (g1, g2) and their counts (u.uniq_off, u.numolg).
+lcp_status device_overlaps(lcp_ctx* ctx, UCell& u, DeviceLists& d, DBuf* g1, DBuf* g2) {
+  cudaStream_t st = ctx->stream;
+  SetupBuffers& B = d.B;
+  const SetupGeom& G = d.G;
+  const SphereAtom* dA = B.atoms.as<SphereAtom>();
   const int64_t nu = (int64_t)u.uniq_pair.size();
   std::vector<OvPair> pairs(nu);
   std::vector<int32_t> bpair;
@@ -729,25 +739,20 @@ lcp_status build_ucell_device(lcp_ctx* ctx, UCell& u) {
   API_CUDA(cudaMemcpyAsync(boff.data(), B.boff.p, (nblk + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st), "D2H");
   API_CUDA(cudaStreamSynchronize(st), "overlap counts");
   const int64_t nhit = boff[nblk];
-  API_CUDA(B.g1.ensure(std::max<int64_t>(nhit, 1) * sizeof(int32_t)), "alloc");
-  API_CUDA(B.g2.ensure(std::max<int64_t>(nhit, 1) * sizeof(int32_t)), "alloc");
+  ctx->launches += 4;
+  API_CUDA(g1->ensure(std::max<int64_t>(nhit, 1) * sizeof(int32_t)), "alloc");
+  API_CUDA(g2->ensure(std::max<int64_t>(nhit, 1) * sizeof(int32_t)), "alloc");
   if (nblk > 0) {
     overlap_kernel<true><<<(unsigned)nblk, kOvThreads, 0, st>>>(
         G, dA, B.pairs.as<OvPair>(), B.bpair.as<int32_t>(), B.bk0.as<int64_t>(), B.offs.as<int64_t>(),
         B.glist.as<int32_t>(), B.clist.as<int32_t>(), B.lut.as<int32_t>(), nullptr, B.boff.as<int64_t>(),
-        B.g1.as<int32_t>(), B.g2.as<int32_t>());
+        g1->as<int32_t>(), g2->as<int32_t>());
     API_CUDA(cudaGetLastError(), "overlap write");
   }
-  ctx->launches += 5;
+  ctx->launches++;
+  API_CUDA(cudaStreamSynchronize(st), "overlap lists");  // before the host tables above go
   u.uniq_off.assign(nu + 1, 0);
   for (int64_t q = 0; q <= nu; ++q) u.uniq_off[q] = boff[qfirst[q]];
-  u.uniq_g1.resize(nhit);
-  u.uniq_g2.resize(nhit);
-  if (nhit) {
-    API_CUDA(cudaMemcpyAsync(u.uniq_g1.data(), B.g1.p, nhit * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "D2H");
-    API_CUDA(cudaMemcpyAsync(u.uniq_g2.data(), B.g2.p, nhit * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "D2H");
-  }
-  API_CUDA(cudaStreamSynchronize(st), "overlap lists");
   u.numolg.assign(u.nloop, 0);
   for (int64_t q = 0; q < nu; ++q) {
     const int p = u.uniq_pair[q];
@@ -757,6 +762,64 @@ lcp_status build_ucell_device(lcp_ctx* ctx, UCell& u) {
   return LCP_OK;
 }
 
+}  // namespace
+
+// A UCell built on the device keeps its sphere lists (c.glist, c.clist) and
+// overlap lists (c.g1, c.g2) there, where the orbital tables made for it read
+// them: copying them to the host and back took most of a new geometry's time
+// (32-atom Si cell: 200 MB of overlap lists, 38 MB of sphere lists; UCell 10.9
+// ms, of which the kernels 2.1).
+lcp_status build_ucell_device(lcp_ctx* ctx, lcp_ucell& c) {
+  DeviceLists d;
+  lcp_status s = device_spheres(ctx, c.u, d);
+  if (s) return s;
+  if ((s = device_overlaps(ctx, c.u, d, &c.g1, &c.g2))) return s;
+  c.glist.swap(d.B.glist);
+  c.clist.swap(d.B.clist);
+  c.device = ctx->device;
+  c.host_lists = false;
+  c.host_lens = false;
+  return LCP_OK;
+}
+
+}  // namespace lcp
+
+// The overlap lists of a UCell built on another device than the context's.
+lcp_status ucell_device_lens(lcp_ctx* ctx, const lcp_ucell* c, DBuf* g1, DBuf* g2) {
+  lcp::DeviceLists d;
+  lcp::UCell u = c->u;
+  lcp_status s = lcp::device_spheres(ctx, u, d);
+  if (s) return s;
+  return lcp::device_overlaps(ctx, u, d, g1, g2);
+}
+
+// The sphere lists in host memory, copied there once for the calls that read them.
+lcp_status ucell_host_lists(const lcp_ucell* c) {
+  std::lock_guard<std::mutex> lock(c->mutex);
+  if (c->host_lists) return LCP_OK;
+  lcp_ucell* m = const_cast<lcp_ucell*>(c);
+  lcp::UCell& u = m->u;
+  const int64_t n = u.sphere_off.back();
+  int dev = 0;
+  API_CUDA(cudaGetDevice(&dev), "device");
+  API_CUDA(cudaSetDevice(c->device), "device");
+  try {
+    u.glist.resize(n);
+    u.clist.resize(n);
+  } catch (const std::bad_alloc&) {
+    cudaSetDevice(dev);
+    return fail(LCP_ENOMEM, "out of host memory for the sphere lists");
+  }
+  cudaError_t e = cudaSuccess;
+  if (n) e = cudaMemcpy(u.glist.data(), c->glist.p, n * sizeof(int32_t), cudaMemcpyDeviceToHost);
+  if (n && e == cudaSuccess) e = cudaMemcpy(u.clist.data(), c->clist.p, n * sizeof(int32_t), cudaMemcpyDeviceToHost);
+  cudaSetDevice(dev);
+  API_CUDA(e, "sphere lists");
+  m->host_lists = true;
+  return LCP_OK;
+}
+
+namespace lcp {
 }  // namespace lcp
 
 extern "C" {
@@ -775,7 +838,7 @@ lcp_status lcp_ucell_create_device(lcp_ctx* ctx, int32_t nspin, const double* la
     std::string err = lcp::build_ucell_head(u->u, nspin, latvecs, natom, atom2spe, gxyz, atoms_cut1, ngrid,
                                             grid_origin, total_numorbs);
     if (!err.empty()) return fail(LCP_EINVAL, err);
-    if ((s = lcp::build_ucell_device(ctx, u->u))) return s;
+    if ((s = lcp::build_ucell_device(ctx, *u))) return s;
   } catch (const std::bad_alloc&) {
     return fail(LCP_ENOMEM, "out of host memory building UCell");
   }
@@ -847,19 +910,25 @@ lcp_status lcp_set_adenpcc_grid(lcp_ctx* ctx, const lcp_ucell* ucell, int32_t sp
   API_CUDA(to_device(d_den, den, st), "H2D");
   API_CUDA(to_device(d_pcc, pcc, st), "H2D");
   API_CUDA(to_device(d_off, u.sphere_off, st), "H2D");
-  API_CUDA(to_device(d_gl, u.glist, st), "H2D");
-  API_CUDA(to_device(d_cl, u.clist, st), "H2D");
+  const int32_t *gl = ucell->glist.as<int32_t>(), *cl = ucell->clist.as<int32_t>();
+  if (ucell->device != ctx->device) {
+    if ((s = ucell_host_lists(ucell))) return s;
+    API_CUDA(to_device(d_gl, u.glist, st), "H2D");
+    API_CUDA(to_device(d_cl, u.clist, st), "H2D");
+    gl = d_gl.as<int32_t>();
+    cl = d_cl.as<int32_t>();
+  }
   API_CUDA(to_device(d_atv, u.atv, st), "H2D");
   API_CUDA(d_cnt.ensure(nn * sizeof(int32_t)), "alloc");
   API_CUDA(d_start.ensure((nn + 1) * sizeof(int64_t)), "alloc");
   API_CUDA(d_scan.ensure((scan_blocks(nn) + 1) * sizeof(int64_t)), "alloc");
   API_CUDA(d_idx.ensure(std::max<int64_t>(nent, 1) * sizeof(int32_t)), "alloc");
   API_CUDA(cudaMemsetAsync(d_cnt.p, 0, nn * sizeof(int32_t), st), "memset");
-  entry_count_kernel<<<grid_for(nent, 256), 256, 0, st>>>(d_gl.as<int32_t>(), nent, d_cnt.as<int32_t>());
+  entry_count_kernel<<<grid_for(nent, 256), 256, 0, st>>>(gl, nent, d_cnt.as<int32_t>());
   API_CUDA(cudaGetLastError(), "entry count");
   API_CUDA(exclusive_scan_i32(d_cnt.as<int32_t>(), nn, d_start.as<int64_t>(), d_scan.as<int64_t>(), st), "scan");
   API_CUDA(cudaMemsetAsync(d_cnt.p, 0, nn * sizeof(int32_t), st), "memset");
-  entry_fill_kernel<<<grid_for(nent, 256), 256, 0, st>>>(d_gl.as<int32_t>(), nent, d_start.as<int64_t>(),
+  entry_fill_kernel<<<grid_for(nent, 256), 256, 0, st>>>(gl, nent, d_start.as<int64_t>(),
                                                           d_cnt.as<int32_t>(), d_idx.as<int32_t>());
   API_CUDA(cudaGetLastError(), "entry fill");
   AdenArgs a{};
@@ -876,8 +945,8 @@ lcp_status lcp_set_adenpcc_grid(lcp_ctx* ctx, const lcp_ucell* ucell, int32_t sp
   a.den = d_den.as<Radial>();
   a.pcc = d_pcc.as<Radial>();
   a.sphere_off = d_off.as<int64_t>();
-  a.glist = d_gl.as<int32_t>();
-  a.clist = d_cl.as<int32_t>();
+  a.glist = gl;
+  a.clist = cl;
   a.start = d_start.as<int64_t>();
   a.idx = d_idx.as<int32_t>();
   for (int k = 0; k < 2 + nch; ++k) API_CUDA(d_out[k].ensure(nn * sizeof(double)), "alloc");

@@ -352,27 +352,43 @@ cudaError_t for_item_classes(const lcp_orbs* o, int* launches, F launch) {
   return cudaSuccess;
 }
 
+// Makes the tilings of `which` and their workspace; tc: whether there is room
+// for them and the cell is within the kernels' limits.
+static lcp_status f64_made(lcp_ctx* ctx, lcp_orbs* o, int which, bool* tc) {
+  *tc = false;
+  lcp_status s = ensure_f64(ctx, o, which);
+  if (s) return s;
+  if (((which & kF64Density) && o->f64_density.state != 1) || ((which & kF64Elements) && o->f64_elements.state != 1))
+    return LCP_OK;
+  s = ensure_f64_workspace(ctx, o);
+  if (s == LCP_ENOMEM) {
+    (void)cudaGetLastError();
+    return LCP_OK;
+  }
+  *tc = s == LCP_OK;
+  return s;
+}
+
 // Whether an FP64 contraction takes the tensor-core kernels, with their brick
 // lists and workspaces made if need be.  Always, except for cells beyond the
-// kernels' limits and inside a caller's stream capture before anything was
+// kernels' limits, without the memory for them, and inside a caller's stream capture before anything was
 // made (allocating and synchronising there would break the capture): those
 // take the pair kernels (64-atom 96^3 cell: 36.8 ms for density and matrix
 // elements, against 3.3 ms; 2-atom 24^3 cell: 0.62 ms against 0.15).
-static lcp_status f64_ready(lcp_ctx* ctx, const lcp_orbs* orbs, bool* tc) {
+static lcp_status f64_ready(lcp_ctx* ctx, const lcp_orbs* orbs, int which, bool* tc) {
   *tc = false;
   if (ctx->precision != LCP_PREC_FP64) return LCP_OK;
   lcp_orbs* o = const_cast<lcp_orbs*>(orbs);
+  auto built = [&]() {
+    return (!(which & kF64Density) || o->f64_density.state == 1) && (!(which & kF64Elements) || o->f64_elements.state == 1);
+  };
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   API_CUDA(cudaStreamIsCapturing(ctx->stream, &cap), "capture status");
   if (cap != cudaStreamCaptureStatusNone) {
-    if (o->f64_state == 1) return ensure_f64_workspace(ctx, o, tc);
+    if (built()) return ensure_f64_workspace(ctx, o, tc);
     return LCP_OK;
   }
-  lcp_status s = ensure_f64(ctx, o);
-  if (s || o->f64_state != 1) return s;
-  if ((s = ensure_f64_workspace(ctx, o))) return s;
-  *tc = true;
-  return LCP_OK;
+  return f64_made(ctx, o, which, tc);
 }
 
 lcp_status density_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nspin, const double* const* dm, double* const* rho,
@@ -381,7 +397,7 @@ lcp_status density_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nspin, const d
   if (prec == LCP_PREC_BF16X3) return density_tc_device(ctx, orbs, nspin, dm, rho);
   if (orbs->phi_released) return fail(LCP_ESTATE, "the FP64 orbital tables were released (split-BF16 only)");
   bool tc = false;
-  lcp_status fs = f64_ready(ctx, orbs, &tc);
+  lcp_status fs = f64_ready(ctx, orbs, kF64Density, &tc);
   if (fs) return fs;
   if (tc) {
     const lcp::F64DensWork w{ctx->w_f64d.as<double>() + orbs->ucell->u.total_hsize, ctx->w_f64d.as<uint64_t>(),
@@ -455,7 +471,7 @@ lcp_status hamiltonian_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nch, const
   if (prec == LCP_PREC_BF16X3) return hamiltonian_tc_device(ctx, orbs, nch, vpot, hks);
   if (orbs->phi_released) return fail(LCP_ESTATE, "the FP64 orbital tables were released (split-BF16 only)");
   bool tc = false;
-  lcp_status fs = f64_ready(ctx, orbs, &tc);
+  lcp_status fs = f64_ready(ctx, orbs, kF64Elements, &tc);
   if (fs) return fs;
   if (tc) {
     const lcp::F64HamWork w{ctx->w_f64v.as<int64_t>(), ctx->w_f64e.as<int32_t>(),
@@ -1123,10 +1139,32 @@ lcp_status lcp_calc_force3(lcp_ctx* ctx, const lcp_ucell* ucell, const lcp_orbs*
     dv[c] = ctx->w_in[c].as<double>();
     dd[c] = ctx->w_aux[c].as<double>();
   }
-  const int64_t nitems = orbs->pairs.nitems;
-  API_CUDA(ctx->w_part.ensure((size_t)std::max<int64_t>(nitems, 1) * 6 * sizeof(double)), "alloc");
   API_CUDA(ctx->w_out[0].ensure((size_t)std::max(u.natom, 1) * 3 * sizeof(double)), "alloc");
   const double* dphi[3] = {orbs->dphi[0].as<double>(), orbs->dphi[1].as<double>(), orbs->dphi[2].as<double>()};
+  // FP64 whatever the context's precision
+  lcp_orbs* o = const_cast<lcp_orbs*>(orbs);
+  bool tc = false;
+  if ((s = f64_made(ctx, o, kF64Density, &tc))) return s;
+  if (tc) {
+    const F64Set& set = o->f64_density;
+    API_CUDA(ctx->w_part.ensure(((size_t)set.g.nimg * lcp::kF64ForceParts +
+                                 (size_t)u.natom * 3 * lcp::kF64ForceSlices + 1) * sizeof(double)), "alloc");
+    const lcp::F64Force f{{dphi[0], dphi[1], dphi[2]}, o->geom.phi_off, set.img_off.as<int64_t>(),
+                          set.img_atom.as<int32_t>(), set.slot.as<int32_t>(), ctx->w_part.as<double>(), nullptr, 0.0};
+    const lcp::F64DensWork work{ctx->w_f64d.as<double>() + hs, ctx->w_f64d.as<uint64_t>(), ctx->w_f64c.as<uint32_t>(),
+                                ctx->w_f64e.as<int32_t>()};
+    API_CUDA(lcp::launch_f64_force(set.g, o->f64_pairs, nch, dv, dd, w, f, work, u.gridvol, ctx->w_out[0].as<double>(),
+                                   ctx->w_status.as<int>(), ctx->stream),
+             "force3");
+    ctx->launches += 5 * nch;
+    API_CUDA(cudaMemcpyAsync(force, ctx->w_out[0].p, (size_t)u.natom * 3 * sizeof(double), cudaMemcpyDeviceToHost,
+                             ctx->stream),
+             "D2H");
+    API_CUDA(cudaStreamSynchronize(ctx->stream), "force3");
+    return device_status(ctx);
+  }
+  const int64_t nitems = orbs->pairs.nitems;
+  API_CUDA(ctx->w_part.ensure((size_t)std::max<int64_t>(nitems, 1) * 6 * sizeof(double)), "alloc");
   int nl = 0;
   API_CUDA(for_item_classes(orbs, &nl,
                             [&](const lcp::DevPairs& pr, int max_no, int64_t first) {
@@ -1862,7 +1900,8 @@ lcp_status lcp_job_footprint(const lcp_job* job, int64_t* bytes) {
                         &o->o_jatom, &o->o_boff, &o->o_partner, &o->b_scale, &o->b_tmp})
     add(*d);
   for (const F64Set* f : {&o->f64_density, &o->f64_elements})
-    for (const DBuf* d : {&f->bricks, &f->rows, &f->table, &f->ptexp, &f->tab}) add(*d);
+    for (const DBuf* d : {&f->bricks, &f->rows, &f->table, &f->ptexp, &f->tab, &f->img_off, &f->img_atom, &f->slot})
+      add(*d);
   for (const DBuf& d : o->f64_pair_buf) add(d);
   if (o->ucell->device == o->device)  // the cell's lists that the tables read
     for (const DBuf* d : {&o->ucell->glist, &o->ucell->clist, &o->ucell->g1, &o->ucell->g2}) add(*d);
@@ -1888,7 +1927,7 @@ int64_t job_footprint_estimate(lcp_job* job, int32_t precision) {
                     b.sb_chunks.size()) * 4;
   } else if (precision == LCP_PREC_FP32 && !o->phi32.p) {
     fp += o->table_elems * 4;
-  } else if (precision == LCP_PREC_FP64 && o->f64_state == 0 && !o->phi_released) {
+  } else if (precision == LCP_PREC_FP64 && o->f64_density.state == 0 && o->f64_elements.state == 0 && !o->phi_released) {
     fp += f64_footprint_estimate(o);
   }
   return fp;
@@ -1904,7 +1943,7 @@ lcp_status lcp_job_prepare(lcp_ctx* ctx, lcp_job* job) {
   if (ctx->precision == LCP_PREC_BF16X3) return ensure_bricks(ctx, o);
   if (ctx->precision == LCP_PREC_FP64 && !o->phi_released) {
     bool tc = false;
-    if ((s = f64_ready(ctx, o, &tc))) return s;
+    if ((s = f64_ready(ctx, o, kF64Density | kF64Elements, &tc))) return s;
   }
   if (ctx->precision == LCP_PREC_FP32) {
     if ((s = ensure_phi32(ctx, o))) return s;

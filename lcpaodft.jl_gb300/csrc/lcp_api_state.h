@@ -149,9 +149,11 @@ struct lcp_ctx {
 // One brick tiling of the FP64 tensor-core contractions (lcp_f64bricks.cu).
 struct F64Set {
   lcp::F64Bricks g{};
+  int state = 0;  // 0 not built, 1 built, -1 beyond the kernels' limits
   DBuf bricks, rows, table, ptexp, tab;
+  DBuf img_off, img_atom, slot;  // density tiling of tables with gradients, for the force term
   void release() {
-    for (DBuf* d : {&bricks, &rows, &table, &ptexp, &tab}) d->release();
+    for (DBuf* d : {&bricks, &rows, &table, &ptexp, &tab, &img_off, &img_atom, &slot}) d->release();
     g = lcp::F64Bricks{};
   }
 };
@@ -185,9 +187,9 @@ struct lcp_orbs {
   DBuf o_atom, o_jatom, o_boff, o_partner;  // ordered pair list
   DBuf b_scale, b_tmp;                       // fixed-point scale of the tables: [S_phi, 1/S_phi]
   double phi_scale = 1.0;
-  // brick tilings of the FP64 contractions (ensure_f64: 0 not built, 1 built, -1 beyond the kernels' limits)
+  // brick tilings of the FP64 contractions (ensure_f64)
   std::mutex f64_mutex;
-  int f64_state = 0;
+  bool f64_pairs_ready = false;
   F64Set f64_density, f64_elements;
   lcp::F64Pairs f64_pairs{};
   DBuf f64_pair_buf[8];
@@ -239,7 +241,8 @@ lcp_status ensure_bricks(lcp_ctx* ctx, lcp_orbs* o);
 lcp_status ucell_host_lists(const lcp_ucell* c);
 lcp_status ucell_device_lens(lcp_ctx* ctx, const lcp_ucell* c, DBuf* g1, DBuf* g2);
 lcp_status device_status(lcp_ctx* ctx);
-lcp_status ensure_f64(lcp_ctx* ctx, lcp_orbs* o);
+constexpr int kF64Density = 1, kF64Elements = 2;
+lcp_status ensure_f64(lcp_ctx* ctx, lcp_orbs* o, int which);
 int64_t f64_footprint_estimate(const lcp_orbs* o);
 lcp_status ensure_f64_workspace(lcp_ctx* ctx, const lcp_orbs* o, bool* ready = nullptr);
 lcp_status density_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nspin, const double* const* dm, double* const* rho,

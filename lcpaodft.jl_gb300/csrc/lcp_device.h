@@ -376,8 +376,8 @@ struct F64Bricks {
   const F64Row* rows;          // [nrows]
   const uint64_t* table;       // [nchunks * 32 * P]
   const int32_t* ptexp;        // density: [nbricks * P] E of a point
-  const int32_t* tab;          // m x m per brick: offset of the block of the ordered pair (s, t) (density) or of
-                               // its partner (t, s), where the matrix elements are accumulated; -1: no pair
+  const int32_t* tab;          // m x m per brick: offset of the block of the ordered pair (s, t), or for matrix
+                               // elements of its partner (t, s), where they are accumulated (s <= t); -1: no pair
 };
 constexpr int kF64MaxRows = 1000;  // packed rows of a brick the kernels take
 // Ordered pair list of the cell (device pointers) for the brick pair tables and the symmetrised D.
@@ -406,6 +406,24 @@ struct F64DensWork {
 };
 cudaError_t launch_f64_density(const F64Bricks& b, const F64Pairs& pr, const double* dm, const F64DensWork& w,
                                double* rho, int* status, cudaStream_t st);
+// Force term: what its epilogue reads, and its partial sums (part: nimg *
+// kF64ForceParts doubles, three per image and epilogue warp, then natom * 3 *
+// kF64ForceSlices).
+constexpr int kF64ForceParts = 24, kF64ForceSlices = 32;
+struct F64Force {
+  const double* dphi[3];    // gradient tables
+  const int64_t* phi_off;
+  const int64_t* img_off;   // [nbricks+1]
+  const int32_t* img_atom;  // [nimg]
+  const int32_t* slot;      // [nimg * 128]
+  double* part;
+  const double* vpot;       // of one channel, with its weight (set by the launcher)
+  double w;
+};
+// force[natom][3] from the channels' V and D (src/Force.jl:405-566), on the density's tiling.
+cudaError_t launch_f64_force(const F64Bricks& b, const F64Pairs& pr, int nch, const double* const* vpot,
+                             const double* const* dm, const double* coef, const F64Force& f, const F64DensWork& w,
+                             double gridvol, double* force, int* status, cudaStream_t st);
 // H (one channel) from V, in both orientations, times gridvol.  Workspace: vb
 // (nbricks * 64 words: V by brick), vexp (nbricks ints: its scales) and acc
 // (kF64Copies * hsize doubles: the sums).

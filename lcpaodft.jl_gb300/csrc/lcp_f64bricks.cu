@@ -182,8 +182,8 @@ __global__ void __launch_bounds__(256) f64_slot_kernel(BuildGeom g, const BoxDev
   }
 }
 
-// Pair tables: the ordered pair (atom_s, atom_t, R_s - R_t) of images s <= t
-// by binary search in atom_s's list (the self pair first, then by neighbour
+// Pair tables: the ordered pair (atom_s, atom_t, R_s - R_t) of images s and t
+// (matrix elements: s <= t only) by binary search in atom_s's list (the self pair first, then by neighbour
 // and cell).
 __global__ void __launch_bounds__(256) f64_tab_kernel(F64Pairs pr, int64_t nbricks,
                                                       const int64_t* __restrict__ img_off,
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) f64_tab_kernel(F64Pairs pr, int64_t nbric
     for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
       const int s = e / m, t = e - s * m;
       int32_t out = -1;
-      if (s <= t) {
+      if (s <= t || !elements) {
         const int as = img_atom[i0 + s], at = img_atom[i0 + t];
         const int4 rs = img_per[i0 + s], rt = img_per[i0 + t];
         const int d0 = rs.x - rt.x, d1 = rs.y - rt.y, d2 = rs.z - rt.z;
@@ -216,10 +216,8 @@ __global__ void __launch_bounds__(256) f64_tab_kernel(F64Pairs pr, int64_t nbric
           }
           if (lo < pr.first[as + 1] && (int64_t)pr.jatom[lo] * pr.ncell + pr.cell[lo] == want) p = lo;
         }
-        if (p >= 0) {
-          // images are sorted by (atom, period), so the pair is the kept one of the two (or its own partner)
-          out = (int32_t)pr.boff[elements ? pr.partner[p] : p];
-        }
+        // images are sorted by (atom, period), so for s <= t the pair is the kept one of the two (or its own partner)
+        if (p >= 0) out = (int32_t)pr.boff[elements ? pr.partner[p] : p];
       }
       tab[tab_off[hb] + e] = out;
     }
@@ -395,13 +393,7 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   if (!*fits) return LCP_OK;
   API_CUDA(S.rows.ensure(std::max<int64_t>(g.nrows, 1) * sizeof(F64Row)), "alloc");
   API_CUDA(S.tab.ensure(std::max<int64_t>(ntab, 1) * sizeof(int32_t)), "alloc");
-  const cudaError_t te = S.table.ensure(std::max<int64_t>(g.nchunks, 1) * 32 * P * sizeof(uint64_t));
-  if (te == cudaErrorMemoryAllocation) {  // no room for the table: the pair kernels need none
-    (void)cudaGetLastError();
-    *fits = false;
-    return LCP_OK;
-  }
-  API_CUDA(te, "alloc");
+  API_CUDA(S.table.ensure(std::max<int64_t>(g.nchunks, 1) * 32 * P * sizeof(uint64_t)), "alloc");
   API_CUDA(S.bricks.ensure(g.nbricks * sizeof(F64Brick)), "alloc");
   f64_bricks_kernel<<<blocks_for(g.nbricks), 256, 0, st>>>(g.nbricks, d_img_off.as<int64_t>(), d_row_off.as<int64_t>(),
                                                            d_chunk_off.as<int64_t>(), d_tab_off.as<int64_t>(),
@@ -425,6 +417,11 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
       d_tab_off.as<int64_t>(), P == 64 ? 1 : 0, S.tab.as<int32_t>());
   API_CUDA(cudaGetLastError(), "brick pairs");
   API_CUDA(cudaStreamSynchronize(st), "brick tables");  // before the scratch above is freed
+  if (P == 128 && o->grad) {  // the force term's epilogue reads the gradient tables by image and point
+    S.img_off.swap(d_img_off);
+    S.img_atom.swap(d_img_atom);
+    S.slot.swap(d_slot);
+  }
   ctx->launches += 20;
   return LCP_OK;
 }
@@ -446,18 +443,15 @@ int64_t f64_footprint_estimate(const lcp_orbs* o) {
   return (int64_t)bytes;
 }
 
-// Builds both tilings once per orbital set.  Afterwards o->f64_state is 1, or
-// -1 for a cell beyond the kernels' limits (block offsets of 30 bits, bricks
-// of kF64MaxRows rows), which keeps the pair kernels.
-lcp_status ensure_f64(lcp_ctx* ctx, lcp_orbs* o) {
-  std::lock_guard<std::mutex> lock(o->f64_mutex);
-  if (o->f64_state != 0) return LCP_OK;
+// ensure_f64 builds the tilings it is asked for (kF64Density, kF64Elements)
+// once per orbital set.  Afterwards a tiling's state is 1, or -1 for a cell
+// beyond the kernels' limits (block offsets of 30 bits, bricks of kF64MaxRows
+// rows) or without room for its tables, which keeps the pair kernels.
+namespace {
+lcp_status pair_tables(lcp_ctx* ctx, lcp_orbs* o) {
+  if (o->f64_pairs_ready) return LCP_OK;
   const lcp::UCell& u = o->ucell->u;
   cudaStream_t st = ctx->stream;
-  if (u.total_hsize >= ((int64_t)1 << 30) || u.natom > 65535 || u.nloop == 0) {
-    o->f64_state = -1;
-    return LCP_OK;
-  }
   std::vector<int64_t> boff(u.block_off.begin(), u.block_off.end()), first(u.natom + 1, 0);
   for (int32_t a : u.pair_atom) first[a + 1]++;
   for (int a = 0; a < u.natom; ++a) first[a + 1] += first[a];
@@ -484,13 +478,31 @@ lcp_status ensure_f64(lcp_ctx* ctx, lcp_orbs* o) {
   p.ijk = q[6].as<int32_t>();
   p.ratv = q[7].as<int32_t>();
   p.numorbs = o->geom.numorbs;
-  bool fits = true;
-  lcp_status s = lcp::build_set(ctx, o, q[6], o->f64_density, 128, &fits);
-  if (s == LCP_OK && fits) s = lcp::build_set(ctx, o, q[6], o->f64_elements, 64, &fits);
-  if (s) return s;
-  if (!fits)
-    for (F64Set* x : {&o->f64_density, &o->f64_elements}) x->release();
-  o->f64_state = fits ? 1 : -1;
+  o->f64_pairs_ready = true;
+  return LCP_OK;
+}
+}  // namespace
+
+lcp_status ensure_f64(lcp_ctx* ctx, lcp_orbs* o, int which) {
+  std::lock_guard<std::mutex> lock(o->f64_mutex);
+  int* state[2] = {&o->f64_density.state, &o->f64_elements.state};
+  for (int k = 0; k < 2; ++k) {
+    if (!(which & (1 << k)) || *state[k] != 0) continue;
+    const lcp::UCell& u = o->ucell->u;
+    bool fits = u.total_hsize < ((int64_t)1 << 30) && u.natom <= 65535 && u.nloop > 0;
+    if (fits) {
+      lcp_status s = pair_tables(ctx, o);
+      if (s == LCP_OK) s = lcp::build_set(ctx, o, o->f64_pair_buf[6], k ? o->f64_elements : o->f64_density, k ? 64 : 128, &fits);
+      if (s == LCP_ENOMEM) {  // the pair kernels need none of it
+        (void)cudaGetLastError();
+        fits = false;
+      } else if (s) {
+        return s;
+      }
+    }
+    if (!fits) (k ? o->f64_elements : o->f64_density).release();
+    *state[k] = fits ? 1 : -1;
+  }
   return LCP_OK;
 }
 
@@ -502,8 +514,8 @@ lcp_status ensure_f64_workspace(lcp_ctx* ctx, const lcp_orbs* o, bool* ready) {
   const std::pair<DBuf*, size_t> need[] = {
       {&ctx->w_f64d, hs * lcp::kF64Copies * sizeof(double)},  // symmetrised D, twice (density); the sums of H
       {&ctx->w_f64c, (size_t)u.natom * 32 * sizeof(uint32_t)},  // D's column maxima
-      {&ctx->w_f64v, nb * 64 * sizeof(int64_t)},             // V by brick
-      {&ctx->w_f64e, std::max(nb, nd) * sizeof(int32_t)}};   // its scales; D's by brick (density)
+      {&ctx->w_f64v, std::max<size_t>(nb, 1) * 64 * sizeof(int64_t)},  // V by brick
+      {&ctx->w_f64e, std::max<size_t>(std::max(nb, nd), 1) * sizeof(int32_t)}};   // its scales; D's by brick (density)
   if (ready) {
     *ready = true;
     for (const auto& n : need) *ready = *ready && n.first->p && n.first->bytes >= n.second;

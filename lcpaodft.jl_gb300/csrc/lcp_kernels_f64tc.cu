@@ -687,13 +687,18 @@ __global__ void f64_finish_kernel(DevPairs pr, const int32_t* __restrict__ numor
 }  // namespace
 
 // ==========================================================================
-// Density.  Per brick of 128 points, over its R packed rows,
+// Density and force term.  Per brick of 128 points, over its R packed rows,
 //
 //   rho(p) = sum_c phi_c(p) X[p][c],  X[p][c] = sum_{r <= c} phi_r(p) Ds[r][c],
 //   Ds[r][c] = D_rc + D_cr (r < c),  D_rr (r = c),
 //
+// (src/Matrix/Set_Density_Grid.jl:268-304), and for the force term
+// (src/Force.jl:405-566, 3344-3394) over the rows of all images,
+//
+//   F[image of c] += w V(p) grad phi_c(p) Y[p][c],  Y[p][c] = sum_r phi_r(p) D_cr.
+//
 // M = the points, windows of 32 columns, K the packed rows in chunks of 32
-// (only the rows up to the window).  A (phi, scaled per point) is MN-major,
+// (density: only the rows up to the window).  A (phi, scaled per point) is MN-major,
 // so that a lane splits one row at eight points; B (Ds, scaled per column) is
 // K-major.
 //
@@ -707,12 +712,20 @@ __global__ void f64_finish_kernel(DevPairs pr, const int32_t* __restrict__ numor
 //                entries' addresses come from the pair tables, two chunks ahead.
 // Every split warp has its next chunk's loads in flight while it splits one:
 // without that a chunk took 5,000 clocks, whatever the arithmetic.
+//
+// The force term's epilogue holds Y's column as one FP64 value times the
+// gradients at its point, read from the point-major tables through the
+// brick's slots; the three sums of an image are kept over its columns, and
+// reduced over the points when the columns pass to the next image.  The sums
+// are added in a fixed order (no atomics).  A random 16-atom 13-orbital cell
+// took 5.30 ms with the pair kernel, bound by the FP64 pipe, and takes 1.13 ms.
 // ==========================================================================
 namespace {
 
 constexpr int kDP = 128;
 constexpr int kDEpi = 8, kDConvA = 8, kDConvB = 4, kDConv = kDConvA + kDConvB;
 constexpr int kDThreads = 32 * (kDEpi + 1 + kDConv);
+static_assert(kF64ForceParts == kDEpi * 3, "three sums per image and epilogue warp");
 constexpr int kDChunk = 32;
 constexpr uint32_t kDStages = 2;
 constexpr int kDRaw = 5;                                      // half chunks of the table in shared memory
@@ -745,6 +758,7 @@ struct F64DensArgs {
   const uint32_t* cmax;  // [natom * 32] high word of max |Ds| of a column, raised by the grid's slack
   const int32_t* btop;   // [nbricks] exponent bound of the largest finite column of a brick
   double* rho;
+  F64Force f;            // force term only
   int* status;
 };
 
@@ -794,6 +808,69 @@ __global__ void __launch_bounds__(256) f64_btop_kernel(F64Bricks b, const uint32
   }
 }
 
+// Force term: the largest magnitude of every row of D over its pairs (the
+// columns of the product: orbital a of the pair's first atom), one block per pair.
+__global__ void __launch_bounds__(128) f64_drow_kernel(F64Pairs pr, const double* __restrict__ dm,
+                                                       uint32_t* __restrict__ cmax, int slack) {
+  __shared__ uint32_t mx[32];
+  for (int64_t p = blockIdx.x; p < pr.npairs; p += gridDim.x) {
+    const int i = pr.atom[p], noi = pr.numorbs[i], noj = pr.numorbs[pr.jatom[p]];
+    const int64_t bp = pr.boff[p];
+    if (threadIdx.x < 32) mx[threadIdx.x] = 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < noi * noj; e += blockDim.x)
+      atomicMax(&mx[e / noj], (uint32_t)__double2hiint(dm[bp + e]) & 0x7fffffffu);
+    __syncthreads();
+    if (threadIdx.x < noi) {
+      const uint32_t h = mx[threadIdx.x];
+      atomicMax(cmax + (int64_t)i * 32 + threadIdx.x, h < 0x7fe00000u ? h + ((uint32_t)slack << 20) : h);
+    }
+    __syncthreads();
+  }
+}
+__global__ void __launch_bounds__(128) f64_drowfix_kernel(F64Pairs pr, const double* __restrict__ dm,
+                                                          const uint32_t* __restrict__ cmax,
+                                                          uint64_t* __restrict__ dfix) {
+  for (int64_t p = blockIdx.x; p < pr.npairs; p += gridDim.x) {
+    const int i = pr.atom[p], noj = pr.numorbs[pr.jatom[p]], n = pr.numorbs[i] * noj;
+    const int64_t bp = pr.boff[p];
+    for (int e = threadIdx.x; e < n; e += blockDim.x)
+      dfix[bp + e] = fx_biased(dm[bp + e], exp_bound(__ldg(cmax + (int64_t)i * 32 + e / noj)));
+  }
+}
+
+// The images' partial sums by atom: block (atom, slice) adds its slice of the
+// images in a fixed order, then force[atom] (+)= gridvol times the slices' sum.
+// (One block per atom over all images took 111 us for 16 atoms and 21,000 images.)
+__global__ void __launch_bounds__(256) f64_force_slices_kernel(int64_t nimg, const int32_t* __restrict__ img_atom,
+                                                               const double* __restrict__ part,
+                                                               double* __restrict__ slices) {
+  __shared__ double red[3][256];
+  const int atom = blockIdx.x;
+  const int64_t per = (nimg + kF64ForceSlices - 1) / kF64ForceSlices, i0 = blockIdx.y * per, i1 = min(i0 + per, nimg);
+  double v[3] = {0, 0, 0};
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x)
+    if (img_atom[i] == atom)
+      for (int w = 0; w < kDEpi; ++w)
+        for (int e = 0; e < 3; ++e) v[e] += part[(i * kDEpi + w) * 3 + e];
+  for (int e = 0; e < 3; ++e) red[e][threadIdx.x] = v[e];
+  __syncthreads();
+  for (int s = 128; s > 0; s >>= 1) {
+    if (threadIdx.x < s)
+      for (int e = 0; e < 3; ++e) red[e][threadIdx.x] += red[e][threadIdx.x + s];
+    __syncthreads();
+  }
+  if (threadIdx.x < 3) slices[((int64_t)blockIdx.y * gridDim.x + atom) * 3 + threadIdx.x] = red[threadIdx.x][0];
+}
+__global__ void f64_force_sum_kernel(int n, const double* __restrict__ slices, double gridvol, int add,
+                                     double* __restrict__ force) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  double v = 0.0;
+  for (int s = 0; s < kF64ForceSlices; ++s) v += slices[(int64_t)s * n + k];
+  force[k] = v * gridvol + (add ? force[k] : 0.0);
+}
+
 // Ds on the grids of its columns' scales.
 __global__ void __launch_bounds__(128) f64_dfix_kernel(F64Pairs pr, const double* __restrict__ dsym,
                                                        const uint32_t* __restrict__ cmax, uint64_t* __restrict__ dfix) {
@@ -805,8 +882,12 @@ __global__ void __launch_bounds__(128) f64_dfix_kernel(F64Pairs pr, const double
   }
 }
 
-// Chunks of a CTA in order: brick, window c0, row chunk r0 <= c0.
-template <bool AHEAD>
+// Chunks of a CTA in order: brick, window c0, row chunk r0 (density: r0 <= c0; force: every chunk).
+template <bool FORCE>
+__device__ __forceinline__ int last_chunk(int c0, int R) {
+  return FORCE ? (R - 1) & ~(kDChunk - 1) : c0;
+}
+template <bool FORCE, bool AHEAD>
 struct ChunkIter : BrickIterT<AHEAD> {
   int c0, r0;
   __device__ __forceinline__ void begin(const F64Bricks& B) {
@@ -815,7 +896,7 @@ struct ChunkIter : BrickIterT<AHEAD> {
   }
   __device__ __forceinline__ void step(const F64Bricks& B) {
     r0 += kDChunk;
-    if (r0 <= c0) return;
+    if (r0 <= last_chunk<FORCE>(c0, this->R())) return;
     r0 = 0;
     c0 += kWin;
     if (c0 < this->R()) return;
@@ -830,9 +911,11 @@ struct ChunkIter : BrickIterT<AHEAD> {
 // (gather_b).  The L1 that the shared memory leaves is too small to hold any
 // of them, so every load takes its time in L2.  No branches around the loads
 // (entry 0 where there is nothing), so that they are in flight together.
+// Density: Ds of row and column at tab[s][t] + a_row noj + b_col, rows up to the
+// column; force: D of (column's atom, row's atom) at tab[t][s] + a_col noj + b_row.
 struct BAsk {
   F64Row col;
-  uint32_t rio, mask;  // img_orb of row lane % 8; rows that count: on or above the diagonal, inside R
+  uint32_t rio, mask;  // img_orb (and orbital count << 24) of row lane % 8; rows that count
   uint32_t tab;
   int m;
   bool ok;
@@ -843,16 +926,20 @@ struct BPiece {
   int32_t off[8];
   bool ok;
 };
-__device__ __forceinline__ void ask_b(const F64Bricks& B, const ChunkIter<false>& x, int g, int lane, BAsk& q) {
+template <bool FORCE>
+__device__ __forceinline__ void ask_b(const F64Bricks& B, const ChunkIter<FORCE, false>& x, int g, int lane, BAsk& q) {
   q.ok = x.valid();
   if (!q.ok) return;
   const int c = x.c0 + lane, rh = x.r0 + 8 * g, R = x.R();
   q.tab = x.b.tab;
   q.m = x.m();
   q.col = load_meta(B.rows + x.b.row + min(c, R - 1));
-  q.rio = load_meta(B.rows + x.b.row + min(rh + (lane & 7), R - 1)).img_orb;
-  q.mask = c < R && c >= rh ? (c - rh >= 7 ? 255u : (2u << (c - rh)) - 1u) : 0u;
+  const F64Row row = load_meta(B.rows + x.b.row + min(rh + (lane & 7), R - 1));
+  q.rio = row.img_orb | ((uint32_t)row_no(row.info) << 24);
+  const int n = (FORCE ? R : c + 1) - rh;  // rows of this piece that count
+  q.mask = c < R && n > 0 ? (n >= 8 ? 255u : (1u << n) - 1u) : 0u;
 }
+template <bool FORCE>
 __device__ __forceinline__ void locate_b(const F64Bricks& B, const BAsk& a, BPiece& q) {
   q.ok = a.ok;
   if (!a.ok) return;
@@ -860,25 +947,42 @@ __device__ __forceinline__ void locate_b(const F64Bricks& B, const BAsk& a, BPie
   q.mask = a.mask;
   q.b = (int)(a.col.img_orb & 255u);
   q.noj = row_no(a.col.info);
-  const int32_t* tab = B.tab + a.tab + (a.col.img_orb >> 8);
+  const int t = (int)(a.col.img_orb >> 8);
+  const int32_t* tab = B.tab + a.tab + (FORCE ? t * a.m : t);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) q.off[i] = __ldg(tab + (int)(__shfl_sync(0xffffffffu, a.rio, i) >> 8) * a.m);
+  for (int i = 0; i < 8; ++i)
+    q.off[i] = __ldg(tab + (int)((__shfl_sync(0xffffffffu, a.rio, i) >> 8) & 0xffffu) * (FORCE ? 1 : a.m));
 }
+template <bool FORCE>
 __device__ __forceinline__ void gather_b(const uint64_t* __restrict__ dfix, const BPiece& q, uint64_t* t) {
   if (!q.ok) return;
   uint32_t ok = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int a = (int)(__shfl_sync(0xffffffffu, q.rio, i) & 255u);
+    const uint32_t io = __shfl_sync(0xffffffffu, q.rio, i);
+    const int a = (int)(io & 255u);
     const bool y = ((q.mask >> i) & 1u) && q.off[i] >= 0;
     ok |= (y ? 1u : 0u) << i;
-    t[i] = __ldg(dfix + (y ? q.off[i] + a * q.noj + q.b : 0));
+    t[i] = __ldg(dfix + (y ? q.off[i] + (FORCE ? q.b * (int)(io >> 24) + a : a * q.noj + q.b) : 0));
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) t[i] = (ok >> i) & 1u ? t[i] : kF64Bias;
 }
 
-__global__ void __launch_bounds__(kDThreads, 1) f64_density_kernel(const __grid_constant__ F64DensArgs args) {
+// The sums of three values over the warp: of the first in lane 0, of the
+// second in lane 8, of the third in lane 16 (six additions, not fifteen).
+__device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int lane) {
+  const bool up = lane & 16, odd = lane & 8;
+  const double x = __shfl_xor_sync(0xffffffffu, up ? v0 : v2, 16), y = __shfl_xor_sync(0xffffffffu, v1, 16);
+  const double a = (up ? v2 : v0) + x, b = v1 + y;
+  double t = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o /= 2) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+template <bool FORCE>
+__global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_constant__ F64DensArgs args) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[kDStages], empty_bar[kDStages], tfull_bar[2], tempty_bar[2], drain_bar;
   __shared__ uint64_t rawfull_bar[kDRaw], rawempty_bar[kDRaw];
@@ -918,91 +1022,187 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_density_kernel(const __grid_
     const uint32_t quarter = warp & 3, half = warp >> 2;
     const int p = (int)quarter * 32 + lane;
     uint32_t win = 0;
-    BrickIter x;
-    for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
-      const int R = x.R();
-      const uint64_t* mine = B.table + (int64_t)x.b.chunk * 32 * kDP + (p >> 3) * 256 + ((p & 7) >> 1) * 64 + (p & 1);
-      // S, a multiple of 2^-54 of the scales' product, stays below 2^63 for R < 512
-      // (|X| <= R); with more rows Ds is split on a grid one bit coarser.  The sum
-      // of X phi is a 128-bit integer in units 2^-54 2^-62 of the scales' product
-      // with the brick's largest column scale (phi shifted up by what the column's
-      // scale lies below it, at most seven bits, beyond that S down)
-      uint64_t slo = 0;
-      int64_t shi = 0;
-      bool nan = false;
-      const int etop = __ldg(args.btop + x.k);
-      for (int c0 = 0; c0 < R && !abort_flag; c0 += kWin, ++win) {
-        const uint32_t buf = win & 1;
-        // lane l keeps how far column c0 + l's scale lies below the brick's
-        // largest, for the shuffles below
-        int ce = 0;
-        if (c0 + lane < R)
-          ce = etop - exp_bound(__ldg(args.cmax + row_col(load_meta(B.rows + x.b.row + c0 + lane).info)));
-        const bool odd = __any_sync(0xffffffffu, ce < 0 || ce > 7);
-        const uint32_t up = 128u >> min(max(ce, 0), 7);
-        const uint64_t* phi = mine + (int64_t)(c0 / 32) * 32 * kDP;
-        uint64_t ph[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) ph[j] = __ldg(phi + (half * 16 + j) * 2);  // rows past R are zero in the table
-        if (!tc::mbar_wait_warp(&tfull_bar[buf], (win >> 1) & 1, &abort_flag)) {
-          give_up();
-          break;
-        }
-        tc::fence_after_sync();
-#pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
-          const int cb = (int)half * 16 + q * 4;
-          if (c0 + cb >= R) break;
-          uint32_t y[kDig][4];
-          load_acc(tmem, quarter, buf * kBufCols + cb, y);
-          // no branches: the four columns' chains interleave (with them, each
-          // column took 650 clocks of its own latency), and multiplications for
-          // shifts: the integer pipe is the busiest one
-          int64_t S[4], tp[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int64_t t = (int64_t)(ph[j] - kF64Bias);
-            const uint32_t m = __shfl_sync(0xffffffffu, up, cb + j);
-            tp[j] = (int64_t)((uint64_t)(uint32_t)t * m + ((uint64_t)((uint32_t)(t >> 32) * m) << 32));
-            S[j] = assemble(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
+    if constexpr (FORCE) {
+      const F64Force& F = args.f;
+      BrickIter x;
+      for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
+        const int R = x.R();
+        const int64_t i0 = __ldg(F.img_off + x.k);
+        const int64_t gi = p < B.npts ? brick_point_index(x.k, p, B.bdim, B.nb, B.ngrid) : -1;
+        const double vp = gi >= 0 ? F.w * __ldg(F.vpot + gi) : 0.0;
+        const int ep = __ldg(B.ptexp + (int64_t)x.k * kDP + p) - 2 * 1023 - 54;
+        int cur = -1, asked = -1, k = -1;  // image of the sums, image whose point is k
+        int64_t base = 0;
+        double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+        bool in = false;  // the point lies in the sphere of cur
+        auto flush = [&]() {  // this warp's sums of image cur, added in the order of its windows
+          const double s = in ? vp : 0.0;  // outside, whatever V holds there
+          const double t = warp_sum3(f0 * s, f1 * s, f2 * s, lane);
+          if ((lane & 7) == 0 && lane < 24) F.part[((i0 + cur) * kDEpi + warp) * 3 + (lane >> 3)] += t;
+          f0 = f1 = f2 = 0.0;
+          in = false;
+        };
+        for (int c0 = 0; c0 < R && !abort_flag; c0 += kWin, ++win) {
+          const uint32_t buf = win & 1;
+          F64Row mc{};
+          int ce = 1;
+          if (c0 + lane < R) {
+            mc = load_meta(B.rows + x.b.row + c0 + lane);
+            ce = exp_bound(__ldg(args.cmax + row_col(mc.info)));
           }
-          if (odd) {  // columns far below the brick's largest, or with Inf or NaN
+          if (!tc::mbar_wait_warp(&tfull_bar[buf], (win >> 1) & 1, &abort_flag)) {
+            give_up();
+            break;
+          }
+          tc::fence_after_sync();
+#pragma unroll 1
+          for (int q = 0; q < 4; ++q) {
+            const int cb = (int)half * 16 + q * 4;
+            if (c0 + cb >= R) break;
+            double d[4][3];
+            bool has[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {  // the gradients of the four columns
+              const uint32_t io = __shfl_sync(0xffffffffu, mc.img_orb, cb + j);
+              const int no = row_no(__shfl_sync(0xffffffffu, mc.info, cb + j)), img = (int)(io >> 8);
+              d[j][0] = d[j][1] = d[j][2] = 0.0;
+              has[j] = false;
+              if (c0 + cb + j < R) {  // uniform over the warp
+                if (img != asked) {
+                  asked = img;
+                  k = __ldg(F.slot + (i0 + img) * kDP + p);
+                  base = __ldg(F.phi_off + __ldg(F.img_atom + i0 + img));
+                }
+                has[j] = k >= 0;
+                if (has[j]) {
+                  const int64_t at = base + (int64_t)k * no + (int)(io & 255u);
+#pragma unroll
+                  for (int e = 0; e < 3; ++e) d[j][e] = __ldg(F.dphi[e] + at);
+                }
+              }
+            }
+            uint32_t y[kDig][4];
+            load_acc(tmem, quarter, buf * kBufCols + cb, y);
+            double v[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const int d = __shfl_sync(0xffffffffu, ce, cb + j);
-              nan = nan || (d < 0 && ph[j] != kF64Bias);
-              if (d < 0) S[j] = 0;
-              S[j] >>= min(max(d - 7, 0), 63);
+              const int ec = __shfl_sync(0xffffffffu, ce, cb + j), e = ec + ep;
+              const int64_t S = assemble(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
+              v[j] = (double)S;  // times 2^e
+              if (ec >= kBadExp) v[j] = has[j] ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+              else if (e > -800 && e < 800 && S != 0)
+                v[j] = __hiloint2double(__double2hiint(v[j]) + (e << 20), __double2loint(v[j]));
+              else v[j] = scalbn(v[j], e);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int img = (int)(__shfl_sync(0xffffffffu, mc.img_orb, cb + j) >> 8);
+              if (c0 + cb + j < R) {
+                if (img != cur) {
+                  if (cur >= 0) flush();
+                  cur = img;
+                }
+                in |= has[j];
+                f0 = fma(v[j], d[j][0], f0);
+                f1 = fma(v[j], d[j][1], f1);
+                f2 = fma(v[j], d[j][2], f2);
+              }
             }
           }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint64_t lo = (uint64_t)S[j] * (uint64_t)tp[j];
-            slo += lo;
-            shi += __mul64hi(S[j], tp[j]) + (slo < lo ? 1 : 0);
-          }
-          if (q < 3) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) ph[j] = __ldg(phi + (cb + 4 + j) * 2);
-          }
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&tempty_bar[buf]);
         }
-        tc::fence_before_sync();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&tempty_bar[buf]);
+        if (abort_flag) break;
+        if (cur >= 0) flush();
       }
-      if (abort_flag) break;
-      const int64_t gi = p < B.npts ? brick_point_index(x.k, p, B.bdim, B.nb, B.ngrid) : -1;
-      const bool neg = shi < 0;
-      if (neg) {
-        slo = ~slo + 1;
-        shi = ~shi + (slo == 0 ? 1 : 0);
+    } else {
+      BrickIter x;
+      for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
+        const int R = x.R();
+        const uint64_t* mine = B.table + (int64_t)x.b.chunk * 32 * kDP + (p >> 3) * 256 + ((p & 7) >> 1) * 64 + (p & 1);
+        // S, a multiple of 2^-54 of the scales' product, stays below 2^63 for R < 512
+        // (|X| <= R); with more rows Ds is split on a grid one bit coarser.  The sum
+        // of X phi is a 128-bit integer in units 2^-54 2^-62 of the scales' product
+        // with the brick's largest column scale (phi shifted up by what the column's
+        // scale lies below it, at most seven bits, beyond that S down)
+        uint64_t slo = 0;
+        int64_t shi = 0;
+        bool nan = false;
+        const int etop = __ldg(args.btop + x.k);
+        for (int c0 = 0; c0 < R && !abort_flag; c0 += kWin, ++win) {
+          const uint32_t buf = win & 1;
+          // lane l keeps how far column c0 + l's scale lies below the brick's
+          // largest, for the shuffles below
+          int ce = 0;
+          if (c0 + lane < R)
+            ce = etop - exp_bound(__ldg(args.cmax + row_col(load_meta(B.rows + x.b.row + c0 + lane).info)));
+          const bool odd = __any_sync(0xffffffffu, ce < 0 || ce > 7);
+          const uint32_t up = 128u >> min(max(ce, 0), 7);
+          const uint64_t* phi = mine + (int64_t)(c0 / 32) * 32 * kDP;
+          uint64_t ph[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) ph[j] = __ldg(phi + (half * 16 + j) * 2);  // rows past R are zero in the table
+          if (!tc::mbar_wait_warp(&tfull_bar[buf], (win >> 1) & 1, &abort_flag)) {
+            give_up();
+            break;
+          }
+          tc::fence_after_sync();
+#pragma unroll 1
+          for (int q = 0; q < 4; ++q) {
+            const int cb = (int)half * 16 + q * 4;
+            if (c0 + cb >= R) break;
+            uint32_t y[kDig][4];
+            load_acc(tmem, quarter, buf * kBufCols + cb, y);
+            // no branches: the four columns' chains interleave (with them, each
+            // column took 650 clocks of its own latency), and multiplications for
+            // shifts: the integer pipe is the busiest one
+            int64_t S[4], tp[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int64_t t = (int64_t)(ph[j] - kF64Bias);
+              const uint32_t m = __shfl_sync(0xffffffffu, up, cb + j);
+              tp[j] = (int64_t)((uint64_t)(uint32_t)t * m + ((uint64_t)((uint32_t)(t >> 32) * m) << 32));
+              S[j] = assemble(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
+            }
+            if (odd) {  // columns far below the brick's largest, or with Inf or NaN
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const int d = __shfl_sync(0xffffffffu, ce, cb + j);
+                nan = nan || (d < 0 && ph[j] != kF64Bias);
+                if (d < 0) S[j] = 0;
+                S[j] >>= min(max(d - 7, 0), 63);
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint64_t lo = (uint64_t)S[j] * (uint64_t)tp[j];
+              slo += lo;
+              shi += __mul64hi(S[j], tp[j]) + (slo < lo ? 1 : 0);
+            }
+            if (q < 3) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) ph[j] = __ldg(phi + (cb + 4 + j) * 2);
+            }
+          }
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&tempty_bar[buf]);
+        }
+        if (abort_flag) break;
+        const int64_t gi = p < B.npts ? brick_point_index(x.k, p, B.bdim, B.nb, B.ngrid) : -1;
+        const bool neg = shi < 0;
+        if (neg) {
+          slo = ~slo + 1;
+          shi = ~shi + (slo == 0 ? 1 : 0);
+        }
+        double acc = fma((double)shi, 0x1p64, (double)slo);
+        if (neg) acc = -acc;
+        if (nan) acc = __longlong_as_double(0x7ff8000000000000ll);
+        // two halves onto a zeroed point: the same sum in either order
+        if (gi >= 0 && bounds_ok(gi, (int64_t)B.ngrid[0] * B.ngrid[1] * B.ngrid[2], 21))
+          atomicAdd(args.rho + gi, scalbn(acc, 2 * (B.ptexp[(int64_t)x.k * kDP + p] - 1023) + etop - 1023 - 116));
       }
-      double acc = fma((double)shi, 0x1p64, (double)slo);
-      if (neg) acc = -acc;
-      if (nan) acc = __longlong_as_double(0x7ff8000000000000ll);
-      // two halves onto a zeroed point: the same sum in either order
-      if (gi >= 0 && bounds_ok(gi, (int64_t)B.ngrid[0] * B.ngrid[1] * B.ngrid[2], 21))
-        atomicAdd(args.rho + gi, scalbn(acc, 2 * (B.ptexp[(int64_t)x.k * kDP + p] - 1023) + etop - 1023 - 116));
     }
   } else if (warp == kDEpi) {
     // ------------------------------------------------------------ MMA issuer
@@ -1017,7 +1217,8 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_density_kernel(const __grid_
           break;
         }
         const uint32_t d0 = tmem + buf * kBufCols;
-        for (int r0 = 0; r0 <= c0; r0 += kDChunk) {
+        const int last = last_chunk<FORCE>(c0, R);
+        for (int r0 = 0; r0 <= last; r0 += kDChunk) {
           if (!tc::mbar_wait_warp(&full_bar[st], par, &abort_flag)) {
             give_up();
             break;
@@ -1037,7 +1238,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_density_kernel(const __grid_
           }
           if (tc::elect_one()) {
             tc::mma_commit(&empty_bar[st]);
-            if (r0 == c0) tc::mma_commit(&tfull_bar[buf]);
+            if (r0 == last) tc::mma_commit(&tfull_bar[buf]);
           }
           __syncwarp();
           if (++st == kDStages) {
@@ -1057,7 +1258,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_density_kernel(const __grid_
     const int cw = warp - kDEpi - 1;
     uint32_t st = 0, par = 1, round = 0;  // par: parity of the stage's last release
     if (cw < kDConvA) {
-      ChunkIter<true> x, ahead;  // warp 0 fetches up to kDRaw half chunks ahead
+      ChunkIter<FORCE, true> x, ahead;  // warp 0 fetches up to kDRaw half chunks ahead
       x.begin(B);
       ahead = x;
       uint8_t* raw = smem + kDStages * kDStageBytes;
@@ -1114,20 +1315,20 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_density_kernel(const __grid_
       if (cw == 0) ring.drain();
     } else {
       const int g = cw - kDConvA;
-      ChunkIter<false> x;
+      ChunkIter<FORCE, false> x;
       x.begin(B);
       uint64_t t[8];
       BAsk ask;
       BPiece q;
       bool now = x.valid();  // there is a chunk in t
-      ask_b(B, x, g, lane, ask);
-      locate_b(B, ask, q);
+      ask_b<FORCE>(B, x, g, lane, ask);
+      locate_b<FORCE>(B, ask, q);
       if (x.valid()) x.step(B);
-      ask_b(B, x, g, lane, ask);
-      gather_b(args.dfix, q, t);
-      locate_b(B, ask, q);
+      ask_b<FORCE>(B, x, g, lane, ask);
+      gather_b<FORCE>(args.dfix, q, t);
+      locate_b<FORCE>(B, ask, q);
       if (x.valid()) x.step(B);
-      ask_b(B, x, g, lane, ask);
+      ask_b<FORCE>(B, x, g, lane, ask);
       while (now && !abort_flag) {
         if (round > 0 && !tc::mbar_wait_warp(&empty_bar[st], par, &abort_flag)) {
           give_up();
@@ -1139,10 +1340,10 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_density_kernel(const __grid_
         if (lane == 0) tc::mbar_arrive(&full_bar[st]);
         __syncwarp();
         now = q.ok;
-        gather_b(args.dfix, q, t);
-        locate_b(B, ask, q);
+        gather_b<FORCE>(args.dfix, q, t);
+        locate_b<FORCE>(B, ask, q);
         if (x.valid()) x.step(B);
-        ask_b(B, x, g, lane, ask);
+        ask_b<FORCE>(B, x, g, lane, ask);
         if (++st == kDStages) {
           st = 0;
           par ^= 1;
@@ -1181,10 +1382,37 @@ cudaError_t launch_f64_density(const F64Bricks& b, const F64Pairs& pr, const dou
   LCP_CUDA_TRY(cudaGetLastError());
   f64_btop_kernel<<<(unsigned)std::min<int64_t>((b.nbricks + 7) / 8, 152 * 8), 256, 0, st>>>(b, w.cmax, w.btop);
   LCP_CUDA_TRY(cudaGetLastError());
-  F64DensArgs a{b, w.dfix, w.cmax, w.btop, rho, status};
-  LCP_CUDA_TRY(raise_smem(f64_density_kernel, kDSmemBytes));
-  f64_density_kernel<<<(unsigned)std::min<int64_t>(b.nbricks, device_sms()), kDThreads, kDSmemBytes, st>>>(a);
+  F64DensArgs a{b, w.dfix, w.cmax, w.btop, rho, F64Force{}, status};
+  LCP_CUDA_TRY(raise_smem(f64_points_kernel<false>, kDSmemBytes));
+  f64_points_kernel<false><<<(unsigned)std::min<int64_t>(b.nbricks, device_sms()), kDThreads, kDSmemBytes, st>>>(a);
   return cudaGetLastError();
+}
+
+cudaError_t launch_f64_force(const F64Bricks& b, const F64Pairs& pr, int nch, const double* const* vpot,
+                             const double* const* dm, const double* coef, const F64Force& f, const F64DensWork& w,
+                             double gridvol, double* force, int* status, cudaStream_t st) {
+  if (b.nrows == 0 || pr.npairs == 0) return cudaMemsetAsync(force, 0, (size_t)pr.natom * 3 * sizeof(double), st);
+  const unsigned blocks = (unsigned)std::min<int64_t>(pr.npairs, 152 * 16);
+  LCP_CUDA_TRY(raise_smem(f64_points_kernel<true>, kDSmemBytes));
+  for (int c = 0; c < nch; ++c) {
+    LCP_CUDA_TRY(cudaMemsetAsync(w.cmax, 0, (size_t)pr.natom * 32 * sizeof(uint32_t), st));
+    LCP_CUDA_TRY(cudaMemsetAsync(f.part, 0, (size_t)b.nimg * kF64ForceParts * sizeof(double), st));
+    f64_drow_kernel<<<blocks, 128, 0, st>>>(pr, dm[c], w.cmax, b.max_rows >= 512 ? 1 : 0);
+    LCP_CUDA_TRY(cudaGetLastError());
+    f64_drowfix_kernel<<<blocks, 128, 0, st>>>(pr, dm[c], w.cmax, w.dfix);
+    LCP_CUDA_TRY(cudaGetLastError());
+    F64DensArgs a{b, w.dfix, w.cmax, nullptr, nullptr, f, status};
+    a.f.vpot = vpot[c];
+    a.f.w = coef[c];
+    f64_points_kernel<true><<<(unsigned)std::min<int64_t>(b.nbricks, device_sms()), kDThreads, kDSmemBytes, st>>>(a);
+    LCP_CUDA_TRY(cudaGetLastError());
+    double* slices = f.part + b.nimg * kF64ForceParts;
+    f64_force_slices_kernel<<<dim3((unsigned)pr.natom, kF64ForceSlices), 256, 0, st>>>(b.nimg, f.img_atom, f.part, slices);
+    LCP_CUDA_TRY(cudaGetLastError());
+    f64_force_sum_kernel<<<(unsigned)(pr.natom * 3 + 127) / 128, 128, 0, st>>>(pr.natom * 3, slices, gridvol, c > 0, force);
+    LCP_CUDA_TRY(cudaGetLastError());
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_f64_hamiltonian(const F64Bricks& b, const DevPairs& folded, const int32_t* numorbs,

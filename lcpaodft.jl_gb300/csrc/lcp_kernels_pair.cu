@@ -1,5 +1,8 @@
 // Exact-lens pair contractions on CUDA cores: density assembly and grid
-// matrix elements in FP64 (the drop-in) or FP32 (comparison form).
+// matrix elements in FP32 (comparison form), and in FP64 with the force term
+// for what the FP64 tensor-core kernels do not take: cells beyond their limits
+// (kF64MaxRows orbitals at a brick, block offsets of 30 bits, no room for
+// their tables) and captures that begin before their tables are made.
 //
 // The reference walks every ordered pair (i, j, R) of the neighbour list over
 // the pair's overlap ("lens") points in 512-point blocks, with a small dgemm

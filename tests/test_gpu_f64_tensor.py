@@ -87,3 +87,35 @@ def test_f64_tensor_non_finite():
     inside[u.GridListAtom[0]] = True
     assert not np.isfinite(rho[0][inside]).all()
     assert np.isfinite(rho[0][~inside]).all()
+
+
+@pytest.mark.parametrize("name", list(CELLS))
+def test_f64_tensor_force_against_oracle(name):
+    """The force term on the same tilings, rows of every image.  1e-10 of the
+    largest component, as the oracle's gradient tables agree to 1e-12."""
+    from lcpgrid.workloads import synthetic_species
+    from oracle import lcp_oracle as O
+    natom, _, _, orbitals, rc = CELLS[name]
+    u, uo, orbs, phi, rng = _cell(*CELLS[name])
+    paos = [synthetic_species(70 + k, max_l=2 if BASES[no][2] else 1, num_basis=BASES[no][:3 if BASES[no][2] else 2], rc=r)
+            for k, (no, r) in enumerate(zip(orbitals, rc))]
+    dm = [rng.normal(size=u.Total_Hsize) for _ in range(2)]
+    v = [rng.normal(size=u.NN) for _ in range(2)]
+    dorbs = L.Set_dOrbitals_Grid(paos, u, ctx=L.Context(0))
+    grad = [[dorbs.data(a, k + 1) for a in range(natom)] for k in range(3)]
+    ref = O.calc_force3("on", uo, phi, grad, v, dm)
+    f = L.Force3_spin(paos, dorbs, v, dm, u)
+    assert np.max(np.abs(f - ref)) <= 1e-10 * np.max(np.abs(ref))
+    # a potential and a D that are not finite reach the atoms that have them, and no others
+    bad = v[0].copy()
+    outside = np.ones(u.NN, bool)
+    outside[u.GridListAtom[0]] = False
+    bad[outside] = np.nan
+    ref = O.calc_force3("on", uo, phi, grad, [bad, v[1]], dm)
+    f = L.Force3_spin(paos, dorbs, [bad, v[1]], dm, u)
+    assert (np.isfinite(f) == np.isfinite(ref)).all()
+    onsite = next(p for p in range(u.Nloop) if u.MPI_atom[p] == 1 and u.MPI_natn[p] == 1 and u.MPI_ncn[p] == 0)
+    d = dm[0].copy()
+    d[u.block_offset[onsite]] = np.inf
+    f = L.Force3_spin(paos, dorbs, v, [d, dm[1]], u)
+    assert not np.isfinite(f[0]).any() and np.isfinite(f[1:]).all()

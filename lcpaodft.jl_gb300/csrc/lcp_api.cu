@@ -796,8 +796,6 @@ lcp_status lcp_set_orbitals_grid(lcp_ctx* ctx, const lcp_ucell* ucell, int32_t n
     if (d.no > 64) return fail(LCP_ENOTSUP, "more than 64 orbitals per atom");
     d.rv_off = (int64_t)radial.size();
     radial.insert(radial.end(), p.rv, p.rv + p.num_mesh);
-    d.rwf_off = (int64_t)radial.size();
-    radial.insert(radial.end(), p.rwf, p.rwf + (size_t)d.nrad * p.num_mesh);
     lcp::append_spline_tables(p.rv, p.rwf, p.num_mesh, p.num_basis, p.max_l, d, radial, buckets);
     sp[k] = d;
   }

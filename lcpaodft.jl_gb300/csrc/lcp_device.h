@@ -39,9 +39,9 @@ struct DevSpecies {
   int32_t nrad;      // number of radial functions = sum_l nb[l]
   int32_t no;        // orbitals = sum_l nb[l]*(2l+1)
   int64_t rv_off;    // offset of RV in the packed radial array
-  int64_t rwf_off;   // offset of RWF[(l,p)][mesh] in the packed radial array
-  // value tables' spline, precomputed per mesh interval (append_spline_tables):
-  int64_t iv_off;    // per interval m: RV[m-1], 1/(RV[m]-RV[m-1]), then per radial c0..c3
+  // the tables' spline, precomputed per mesh interval (append_spline_tables):
+  int64_t iv_off;    // per interval m: RV[m-1], 1/(RV[m]-RV[m-1]), then per radial c0..c3 (the last
+                     // interval twice: values, gradients)
   int64_t ex_off;    // per radial: a, b, c, d of the extrapolation below RV[0]
   int64_t bk_off;    // bucket table (int32 array): first mesh index of each log2(R) bucket
   float bk_lo, bk_inv;  // bucket of R: (log2(R) - bk_lo) * bk_inv

@@ -11,21 +11,30 @@
 // m order, and the reference's derivative chain rule with the 1e-13 shift of
 // points that sit on the atom.
 //
-// The angles enter only through sin/cos, which are taken from the Cartesian
-// components (sin(theta) = r_xy/r, cos(phi) = x/r_xy, ...) instead of
-// acos/asin followed by sin/cos; the edge conventions of
-// src/utils/xyz_to_spherical.jl (r < 1e-14: theta = pi/2, phi = 0;
-// r_xy < 1e-14: phi = 0) are kept.
+// Both kernels take the spline from per-interval cubic coefficients computed
+// once per species on the host (the same Hermite interpolant: value and slope
+// at both mesh nodes of the interval, written as c0 + c1 u + c2 u^2 + c3 u^3
+// in u = (R - RV[m-1]) / (RV[m] - RV[m-1])), find the interval from a table of
+// log2(R) buckets and a short forward scan instead of a binary search, and
+// form Y_lm from the unit vector (x, y, z)/R (the edge convention of
+// src/utils/xyz_to_spherical.jl, theta = pi/2 and phi = 0 at R < 1e-14, is
+// kept).  That takes the FP64 work per point from the spline's divisions and
+// the per-function Hermite set-up to one Horner evaluation per radial function.
 //
-// The value tables (tabulate_values_kernel) take the spline from per-interval
-// cubic coefficients computed once per species on the host (the same Hermite
-// interpolant: value and slope at both mesh nodes of the interval, written as
-// c0 + c1 u + c2 u^2 + c3 u^3 in u = (R - RV[m-1]) / (RV[m] - RV[m-1])), find
-// the interval from a table of log2(R) buckets and a short forward scan
-// instead of a binary search, and form Y_lm from the unit vector (x, y, z)/R.
-// That takes the FP64 work per point from the spline's divisions and the
-// per-function Hermite set-up to one Horner evaluation per radial function.
-// The gradient tables keep the reference's per-point evaluation.
+// The gradients are taken in Cartesian form.  With Y = P(x, y, z) of degree l
+// on the unit sphere, G = grad P there, and q = R_lp / r,
+//
+//   grad phi = (R_lp' - l q) Y u + q G,   u = (x, y, z)/r,
+//
+// seven FP64 operations per function on top of its value (G is shared by the
+// functions of one l), where the reference's chain rule over r, theta and phi
+// (the same derivative, src/Matrix/Set_dOrbitals_Grid.jl:257-300) needs twenty
+// and the angles' sines and cosines.  Both kernels are bound by the FP64 pipe
+// (two operations a clock and SM): values and gradients of a random 16-atom
+// 13-orbital cell took 1.90 ms by the chain rule and 0.49 ms this way.  The
+// code of one l at a time, with compile-time loops over m, keeps Y and G in
+// registers: the same cell's values alone took 0.33 ms with a loop over l
+// that indexed them in local memory, and 0.22 ms.
 //
 // One thread per sphere point; a block stages its points x NO values per
 // table in shared memory and writes them back as contiguous, 16-byte
@@ -41,241 +50,8 @@ namespace lcp {
 
 namespace {
 
-constexpr int kTabPoints = 64;
+constexpr int kTabPoints = 64;  // points of a gradient block: four tables of staging
 constexpr double kPi = 3.14159265358979323846;
-
-// Real spherical harmonics of one l in the orbital order of
-// src/Matrix/Set_Orbitals_Grid.jl:242-268 (src/utils/Ylm_real.jl:1-53) and
-// their theta / phi derivatives (src/utils/Ylm_real.jl:56-162).
-template <bool GRAD>
-__device__ __forceinline__ void ylm_l(int l, double siQ, double coQ, double siP, double coP, double* Y,
-                                      double* dQ, double* dP) {
-  const double pi = kPi;
-  if (l == 0) {
-    Y[0] = 0.5 * sqrt(1 / pi);
-    if (GRAD) {
-      dQ[0] = 0.0;
-      dP[0] = 0.0;
-    }
-  } else if (l == 1) {
-    const double c = sqrt(3 / 4.0 / pi);
-    Y[0] = c * siQ * coP;  // px (m = 1)
-    Y[1] = c * siQ * siP;  // py (m = -1)
-    Y[2] = c * coQ;        // pz (m = 0)
-    if (GRAD) {
-      dQ[0] = c * coQ * coP;
-      dQ[1] = c * coQ * siP;
-      dQ[2] = -c * siQ;
-      dP[0] = -c * siP;
-      dP[1] = c * coP;
-      dP[2] = 0.0;
-    }
-  } else if (l == 2) {
-    const double s = sqrt(15 / pi);
-    Y[0] = 0.25 * sqrt(5 / pi) * (3 * coQ * coQ - 1);          // m = 0
-    Y[1] = 0.25 * s * siQ * siQ * (1 - 2 * siP * siP);         // m = 2
-    Y[2] = 0.5 * s * siQ * siQ * siP * coP;                    // m = -2
-    Y[3] = 0.5 * s * siQ * coQ * coP;                          // m = 1
-    Y[4] = 0.5 * s * siQ * coQ * siP;                          // m = -1
-    if (GRAD) {
-      dQ[0] = -1.5 * sqrt(5 / pi) * siQ * coQ;
-      dQ[1] = 0.5 * s * siQ * coQ * (1 - 2 * siP * siP);
-      dQ[2] = s * siQ * coQ * siP * coP;
-      dQ[3] = 0.5 * s * (1 - 2 * siQ * siQ) * coP;
-      dQ[4] = 0.5 * s * (1 - 2 * siQ * siQ) * siP;
-      dP[0] = 0.0;
-      dP[1] = -s * siQ * siP * coP;
-      dP[2] = 0.5 * s * siQ * (1 - 2 * siP * siP);
-      dP[3] = -0.5 * s * coQ * siP;
-      dP[4] = 0.5 * s * coQ * coP;
-    }
-  } else {
-    const double a = sqrt(35 / 2.0 / pi), b = sqrt(105 / pi), c = sqrt(21 / 2.0 / pi), d = sqrt(7 / pi);
-    Y[0] = 0.25 * d * (5 * coQ * coQ * coQ - 3 * coQ);                          // m = 0
-    Y[1] = 0.25 * c * siQ * (5 * coQ * coQ - 1) * coP;                          // m = 1
-    Y[2] = 0.25 * c * siQ * (5 * coQ * coQ - 1) * siP;                          // m = -1
-    Y[3] = 0.25 * b * siQ * siQ * coQ * (coP * coP - siP * siP);                // m = 2
-    Y[4] = 0.5 * b * siQ * siQ * coQ * siP * coP;                               // m = -2
-    Y[5] = 0.25 * a * siQ * siQ * siQ * (4 * coP * coP * coP - 3 * coP);        // m = 3
-    Y[6] = 0.25 * a * siQ * siQ * siQ * (3 * siP - 4 * siP * siP * siP);        // m = -3
-    if (GRAD) {
-      dQ[0] = 0.25 * d * siQ * (-15 * coQ * coQ + 3);
-      dQ[1] = 0.25 * c * coP * coQ * (15 * coQ * coQ - 11);
-      dQ[2] = 0.25 * c * siP * coQ * (15 * coQ * coQ - 11);
-      dQ[3] = 0.25 * b * (coP * coP - siP * siP) * siQ * (2 * coQ * coQ - siQ * siQ);
-      dQ[4] = 0.5 * b * coP * siP * siQ * (2 * coQ * coQ - siQ * siQ);
-      dQ[5] = 0.75 * a * coP * coQ * siQ * siQ * (-3 + 4 * coP * coP);
-      dQ[6] = 0.75 * a * siQ * siQ * coQ * siP * (3 - 4 * siP * siP);
-      dP[0] = 0.0;
-      dP[1] = 0.25 * c * siP * (-5 * coQ * coQ + 1);
-      dP[2] = 0.25 * c * coP * (5 * coQ * coQ - 1);
-      dP[3] = -b * coP * coQ * siP * siQ;
-      dP[4] = 0.5 * b * coQ * siQ * (coP * coP - siP * siP);
-      dP[5] = 0.75 * a * siP * siQ * siQ * (1 - 4 * coP * coP);
-      dP[6] = 0.75 * a * coP * siQ * siQ * (1 - 4 * siP * siP);
-    }
-  }
-}
-
-// xyz_to_spherical (src/utils/xyz_to_spherical.jl:1-31) expressed through
-// sin/cos of the angles.
-__device__ __forceinline__ void spherical_trig(double x, double y, double z, double& r, double& siQ,
-                                               double& coQ, double& siP, double& coP) {
-  const double min_r = 1e-14;
-  double dum = x * x + y * y;
-  r = sqrt(dum + z * z);
-  double r1 = sqrt(dum);
-  if (min_r <= r) {
-    coQ = (r < fabs(z)) ? copysign(1.0, z) : z / r;
-    siQ = (r < fabs(z)) ? 0.0 : r1 / r;
-    if (min_r <= r1) {
-      siP = (r1 < fabs(y)) ? copysign(1.0, y) : y / r1;
-      coP = (r1 < fabs(y)) ? 0.0 : x / r1;
-    } else {
-      siP = 0.0;
-      coP = 1.0;
-    }
-  } else {
-    // theta = pi/2, phi = 0
-    siQ = 1.0;
-    coQ = 6.123233995736766e-17;  // cos(pi/2) in double precision
-    siP = 0.0;
-    coP = 1.0;
-  }
-}
-
-// Values (WPHI) and/or gradients (WGRAD) of one point's orbitals, written to
-// the staging rows.  (R, siQ, coQ, siP, coP) describe the point relative to
-// the atom.
-template <bool WPHI, bool WGRAD>
-__device__ __forceinline__ void eval_point(const DevSpecies& sp, const double* __restrict__ rv,
-                                           const double* __restrict__ rwf, double R, double siQ, double coQ,
-                                           double siP, double coP, double* srow, double* sx, double* sy,
-                                           double* sz) {
-  const int n = sp.nmesh;
-  const bool outside = rv[n - 1] < R;
-  const bool inner = R < rv[0];
-
-  // spline geometry (src/Matrix/Set_Orbitals_Grid.jl:187-214); below RV[1]
-  // the geometry of 0-based mesh point 4 (:126-145)
-  int m = 0;
-  double h1 = 0, h2 = 1, h3 = 0, y1 = 0, y2 = 0, dum1 = 0, dum2 = 0, dum3 = 0, dum4 = 0;
-  const int me = 4;
-  const double rm = rv[me];
-  if (!outside) {
-    if (inner) {
-      m = me;
-    } else {
-      int lo = 1, hi = n - 1;  // first index >= 1 with rv[idx] >= R
-      while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        if (rv[mid] < R) lo = mid + 1;
-        else hi = mid;
-      }
-      m = min(max(lo, 2), n - 2);
-    }
-    h1 = rv[m - 1] - rv[m - 2];
-    h2 = rv[m] - rv[m - 1];
-    h3 = rv[m + 1] - rv[m];
-    const double xr = inner ? rm : R;
-    y1 = (xr - rv[m - 1]) / h2;
-    y2 = (xr - rv[m]) / h2;
-    double dum = h1 + h2;
-    dum1 = h1 / h2 / dum;
-    dum2 = h2 / h1 / dum;
-    dum = h2 + h3;
-    dum3 = h2 / h3 / dum;
-    dum4 = h3 / h2 / dum;
-  }
-  const double y12 = y1 * y1, y22 = y2 * y2;
-
-  double dRx = 0, dRy = 0, dRz = 0, dQx = 0, dQy = 0, dQz = 0, dPx = 0, dPy = 0;
-  if (WGRAD && !outside) {  // src/Matrix/Set_dOrbitals_Grid.jl:257-280
-    dRx = siQ * coP;
-    dRy = siQ * siP;
-    dRz = coQ;
-    if (R > 1.0e-13) {
-      dQx = coQ * coP / R;
-      dQy = coQ * siP / R;
-      dQz = -siQ / R;
-      dPx = -siP / R;
-      dPy = coP / R;
-    }
-  }
-
-  int ist = 0;
-  int rad = 0;
-  for (int l = 0; l <= sp.max_l; ++l) {
-    double Y[7], dQ[7], dP[7];
-    ylm_l<WGRAD>(l, siQ, coQ, siP, coP, Y, dQ, dP);
-    for (int p = 0; p < sp.nb[l]; ++p, ++rad) {
-      const double* w = rwf + (size_t)rad * n;
-      double rf = 0.0, drf = 0.0, rfd = 0.0;
-      if (!outside) {
-        const double f1 = w[m - 2], f2 = w[m - 1], f3 = w[m];
-        double f4 = w[m + 1];
-        const double dum = f3 - f2;
-        const double g1 = dum * dum1 + (f2 - f1) * dum2;
-        double g2 = (f4 - f3) * dum3 + dum * dum4;
-        const double A = 3 * f2 + h2 * g1, B = 2 * f2 + h2 * g1;
-        double C = 3 * f3 - h2 * g2, D = 2 * f3 - h2 * g2;
-        const double E = A + B * y2;
-        double F = C - D * y1;
-        const double f = y22 * E + y12 * F;
-        if (inner) {
-          // Set_Orbitals_Grid's derivative expression (:165) and
-          // Set_dOrbitals_Grid's (:168) round differently; each table uses its own
-          for (int which = 0; which < 2; ++which) {
-            if ((which == 0 && !WPHI) || (which == 1 && !WGRAD)) continue;
-            const double df = which == 0
-                                  ? (2 * y2 / h2) * E + y22 * B / h2 + (2 * y1 / h2) * F - y12 * D / h2
-                                  : (2 * y2 * E + y22 * B + 2.0 * y1 * F - y12 * D) / h2;
-            double a, b, c, d;
-            if (l == 0) {
-              a = 0.0; b = 0.5 * df / rm; c = 0.0; d = f - b * (rm * rm);
-            } else if (l == 1) {
-              a = (rm * df - f) / (2 * (rm * rm * rm)); b = 0.0; c = df - 3 * a * (rm * rm); d = 0.0;
-            } else {
-              b = (3 * f - rm * df) / (rm * rm); a = (f - b * (rm * rm)) / (rm * rm * rm); c = 0.0; d = 0.0;
-            }
-            const double val = a * (R * R * R) + b * (R * R) + c * R + d;
-            if (which == 0) {
-              rf = val;
-            } else {
-              rfd = val;
-              drf = 3 * a * (R * R) + 2 * b * R + c;
-            }
-          }
-        } else {
-          rfd = f;
-          if (WGRAD) drf = (2 * y2 * E + y22 * B + 2.0 * y1 * F - y12 * D) / h2;
-          if (WPHI && m == n - 2) {
-            // Set_Orbitals_Grid substitutes f4 = f1 here (:226-229)
-            f4 = f1;
-            g2 = (f4 - f3) * dum3 + dum * dum4;
-            C = 3 * f3 - h2 * g2;
-            D = 2 * f3 - h2 * g2;
-            F = C - D * y1;
-            rf = y22 * E + y12 * F;
-          } else {
-            rf = f;
-          }
-        }
-      }
-      for (int mm = 0; mm < 2 * l + 1; ++mm, ++ist) {
-        if (WPHI) srow[ist] = outside ? 0.0 : rf * Y[mm];
-        if (WGRAD) {
-          const double dchidr = drf * Y[mm];
-          const double dchidt = rfd * dQ[mm];
-          const double dchidp = rfd * dP[mm];
-          sx[ist] = outside ? 0.0 : -dRx * dchidr - dQx * dchidt - dPx * dchidp;
-          sy[ist] = outside ? 0.0 : -dRy * dchidr - dQy * dchidt - dPy * dchidp;
-          sz[ist] = outside ? 0.0 : -dRz * dchidr - dQz * dchidt;
-        }
-      }
-    }
-  }
-}
 
 // Real Y_lm of one l in the orbital order of src/Matrix/Set_Orbitals_Grid.jl:242-268
 // (src/utils/Ylm_real.jl:1-53), from the unit vector u = (x, y, z) / R:
@@ -309,6 +85,148 @@ __device__ __forceinline__ void ylm_unit(int l, double ux, double uy, double uz,
   }
 }
 
+// Gradients of the Y_lm's homogeneous polynomials at the unit vector.
+template <int l>
+__device__ __forceinline__ void ylm_grad(double ux, double uy, double uz, double (*G)[3]) {
+  const double pi = kPi;
+  if (l == 0) {
+    G[0][0] = G[0][1] = G[0][2] = 0.0;
+  } else if (l == 1) {
+    const double c = sqrt(3 / 4.0 / pi);
+    for (int m = 0; m < 3; ++m)
+      for (int d = 0; d < 3; ++d) G[m][d] = m == d ? c : 0.0;
+  } else if (l == 2) {
+    const double s = 0.5 * sqrt(15 / pi), k = 0.5 * sqrt(5 / pi);
+    G[0][0] = -k * ux, G[0][1] = -k * uy, G[0][2] = 2 * k * uz;  // k/2 (2 z^2 - x^2 - y^2)
+    G[1][0] = s * ux, G[1][1] = -s * uy, G[1][2] = 0.0;          // s/2 (x^2 - y^2)
+    G[2][0] = s * uy, G[2][1] = s * ux, G[2][2] = 0.0;           // s x y
+    G[3][0] = s * uz, G[3][1] = 0.0, G[3][2] = s * ux;           // s x z
+    G[4][0] = 0.0, G[4][1] = s * uz, G[4][2] = s * uy;           // s y z
+  } else {
+    const double a = 0.75 * sqrt(35 / 2.0 / pi), b = 0.5 * sqrt(105 / pi), c = 0.25 * sqrt(21 / 2.0 / pi),
+                 d = 0.75 * sqrt(7 / pi);
+    const double xx = ux * ux, yy = uy * uy, zz = uz * uz, xy = ux * uy, xz = ux * uz, yz = uy * uz;
+    G[0][0] = -2 * d * xz, G[0][1] = -2 * d * yz, G[0][2] = d * (2 * zz - xx - yy);             // d/3 (2 z^3 - 3 z (x^2 + y^2))
+    G[1][0] = c * (4 * zz - 3 * xx - yy), G[1][1] = -2 * c * xy, G[1][2] = 8 * c * xz;          // c x (4 z^2 - x^2 - y^2)
+    G[2][0] = -2 * c * xy, G[2][1] = c * (4 * zz - xx - 3 * yy), G[2][2] = 8 * c * yz;          // c y (4 z^2 - x^2 - y^2)
+    G[3][0] = b * xz, G[3][1] = -b * yz, G[3][2] = 0.5 * b * (xx - yy);                         // b/2 z (x^2 - y^2)
+    G[4][0] = b * yz, G[4][1] = b * xz, G[4][2] = b * xy;                                       // b x y z
+    G[5][0] = a * (xx - yy), G[5][1] = -2 * a * xy, G[5][2] = 0.0;                              // a/3 (x^3 - 3 x y^2)
+    G[6][0] = 2 * a * xy, G[6][1] = a * (xx - yy), G[6][2] = 0.0;                               // a/3 (3 x^2 y - y^3)
+  }
+}
+
+// A sphere point relative to its atom.
+__device__ __forceinline__ void point_xyz(const DevGeom& g, int atom, int64_t k, double* xyz) {
+  const int gn = g.glist[k];
+  const int cell = g.clist[k];
+  const int N2 = g.ngrid[1], N3 = g.ngrid[2];
+  const int n1 = gn / (N2 * N3);
+  const int n2 = (gn - n1 * N2 * N3) / N3;
+  const int n3 = gn - n1 * N2 * N3 - n2 * N3;
+  for (int d = 0; d < 3; ++d) {
+    double c = n1 * g.glat[0 * 3 + d] + n2 * g.glat[1 * 3 + d] + n3 * g.glat[2 * 3 + d] + g.origin[d];
+    xyz[d] = c + g.atv[cell * 3 + d] - g.gxyz[atom * 3 + d];
+  }
+}
+
+// Where a point lies on a species' radial mesh: its distance, unit vector and
+// interval record (none beyond RV[n-1] and, with inner, below RV[0]).
+struct TabPoint {
+  double R, ir, ux, uy, uz, u;
+  const double* rec;
+  int m;
+  bool inner;
+};
+__device__ __forceinline__ TabPoint locate(const DevSpecies& sp, const double* __restrict__ radial,
+                                           const int32_t* __restrict__ buckets, const double* xyz) {
+  TabPoint q;
+  const double r2 = xyz[0] * xyz[0] + xyz[1] * xyz[1] + xyz[2] * xyz[2];
+  if (r2 < 1e-28) {
+    // R < 1e-14: theta = pi/2, phi = 0 (src/utils/xyz_to_spherical.jl)
+    q.R = sqrt(r2);
+    q.ir = 0.0;
+    q.ux = 1.0;
+    q.uy = 0.0;
+    q.uz = 6.123233995736766e-17;  // cos(pi/2) in double precision
+  } else {
+    q.ir = rsqrt(r2);
+    q.R = r2 * q.ir;
+    q.ux = xyz[0] * q.ir;
+    q.uy = xyz[1] * q.ir;
+    q.uz = xyz[2] * q.ir;
+  }
+  const int n = sp.nmesh;
+  const double* rv = radial + sp.rv_off;
+  const bool outside = rv[n - 1] < q.R;
+  q.inner = q.R < rv[0];
+  q.rec = nullptr;
+  q.m = 0;
+  q.u = 0.0;
+  if (!outside && !q.inner) {
+    // the interval: first mesh index >= 1 with RV >= R, from one bucket down
+    int b = (int)((__log2f((float)q.R) - sp.bk_lo) * sp.bk_inv) - 1;
+    b = min(max(b, 0), kSplineBuckets - 1);
+    int i = buckets[sp.bk_off + b];
+    while (i < n - 1 && rv[i] < q.R) ++i;
+    q.m = min(max(i, 2), n - 2);
+    q.rec = radial + sp.iv_off + (size_t)q.m * (2 + 4 * sp.nrad);
+    q.u = (q.R - q.rec[0]) * q.rec[1];
+  }
+  return q;
+}
+
+// The functions of one l at a point: values (WPHI), and the gradients with
+// respect to the atom's position (WGRAD: -grad phi, as the reference's tables).
+template <int l, bool WPHI, bool WGRAD>
+__device__ __forceinline__ void eval_l(const DevSpecies& sp, const double* __restrict__ radial, const TabPoint& q,
+                                       int& rad, int& ist, double* srow, double* sx, double* sy, double* sz) {
+  double Y[2 * l + 1], G[2 * l + 1][3];
+  ylm_unit(l, q.ux, q.uy, q.uz, Y);
+  if (WGRAD) ylm_grad<l>(q.ux, q.uy, q.uz, G);
+  // the last interval's values have f4 = f1, its gradients have not (record nmesh - 1)
+  const bool last = q.rec && q.m == sp.nmesh - 2;
+  const double* grec = last ? q.rec + 2 + 4 * sp.nrad : q.rec;
+  for (int p = 0; p < sp.nb[l]; ++p, ++rad) {
+    double rf = 0.0, rg = 0.0, dr = 0.0;  // of the values; of the gradients, and its derivative
+    if (q.rec) {
+      const double* c = grec + 2 + 4 * rad;
+      rg = ((c[3] * q.u + c[2]) * q.u + c[1]) * q.u + c[0];
+      dr = ((3 * c[3] * q.u + 2 * c[2]) * q.u + c[1]) * q.rec[1];
+      rf = rg;
+      if (WPHI && last) {
+        const double* v = q.rec + 2 + 4 * rad;
+        rf = ((v[3] * q.u + v[2]) * q.u + v[1]) * q.u + v[0];
+      }
+    } else if (q.inner) {
+      const double* e = radial + sp.ex_off + 4 * rad;
+      rg = rf = ((e[0] * q.R + e[1]) * q.R + e[2]) * q.R + e[3];
+      dr = (3 * e[0] * q.R + 2 * e[1]) * q.R + e[2];
+    }
+    const double w = q.R > 1.0e-13 ? -rg * q.ir : 0.0;  // no angular part there
+    const double v = -dr - l * w;
+#pragma unroll
+    for (int m = 0; m < 2 * l + 1; ++m, ++ist) {
+      if (WPHI) srow[ist] = rf * Y[m];
+      if (WGRAD) {
+        const double t = v * Y[m];
+        sx[ist] = t * q.ux + w * G[m][0];
+        sy[ist] = t * q.uy + w * G[m][1];
+        sz[ist] = t * q.uz + w * G[m][2];
+      }
+    }
+  }
+}
+template <bool WPHI, bool WGRAD>
+__device__ __forceinline__ void eval_point(const DevSpecies& sp, const double* __restrict__ radial, const TabPoint& q,
+                                           double* srow, double* sx, double* sy, double* sz) {
+  int rad = 0, ist = 0;
+  eval_l<0, WPHI, WGRAD>(sp, radial, q, rad, ist, srow, sx, sy, sz);
+  if (sp.max_l >= 1) eval_l<1, WPHI, WGRAD>(sp, radial, q, rad, ist, srow, sx, sy, sz);
+  if (sp.max_l >= 2) eval_l<2, WPHI, WGRAD>(sp, radial, q, rad, ist, srow, sx, sy, sz);
+  if (sp.max_l >= 3) eval_l<3, WPHI, WGRAD>(sp, radial, q, rad, ist, srow, sx, sy, sz);
+}
+
 // Value tables: one thread per sphere point, kTabBlock points per block.
 __global__ void __launch_bounds__(kTabBlock) tabulate_values_kernel(DevGeom g, const DevSpecies* __restrict__ spes,
                                                                      const double* __restrict__ radial,
@@ -325,66 +243,11 @@ __global__ void __launch_bounds__(kTabBlock) tabulate_values_kernel(DevGeom g, c
   const int NO = sp.no;
   const int t = threadIdx.x;
   if (t < npts) {
-    const int64_t k = first + t;
-    const int gn = g.glist[k];
-    const int cell = g.clist[k];
-    const int N2 = g.ngrid[1], N3 = g.ngrid[2];
-    const int n1 = gn / (N2 * N3);
-    const int n2 = (gn - n1 * N2 * N3) / N3;
-    const int n3 = gn - n1 * N2 * N3 - n2 * N3;
     double xyz[3];
-    for (int d = 0; d < 3; ++d) {
-      double c = n1 * g.glat[0 * 3 + d] + n2 * g.glat[1 * 3 + d] + n3 * g.glat[2 * 3 + d] + g.origin[d];
-      xyz[d] = c + g.atv[cell * 3 + d] - g.gxyz[atom * 3 + d];
-    }
-    const double r2 = xyz[0] * xyz[0] + xyz[1] * xyz[1] + xyz[2] * xyz[2];
-    double R, ux, uy, uz;
-    if (r2 < 1e-28) {
-      // R < 1e-14: theta = pi/2, phi = 0 (src/utils/xyz_to_spherical.jl)
-      R = sqrt(r2);
-      ux = 1.0;
-      uy = 0.0;
-      uz = 6.123233995736766e-17;  // cos(pi/2) in double precision
-    } else {
-      const double ir = rsqrt(r2);
-      R = r2 * ir;
-      ux = xyz[0] * ir;
-      uy = xyz[1] * ir;
-      uz = xyz[2] * ir;
-    }
-    const int n = sp.nmesh;
-    const double* rv = radial + sp.rv_off;
+    point_xyz(g, atom, first + t, xyz);
+    const TabPoint q = locate(sp, radial, buckets, xyz);
     double* srow = stage + (size_t)t * NO;
-    const bool outside = rv[n - 1] < R;
-    const bool inner = R < rv[0];
-    const double* rec = nullptr;
-    double u = 0.0;
-    if (!outside && !inner) {
-      // the interval: first mesh index >= 1 with RV >= R, from one bucket down
-      int b = (int)((__log2f((float)R) - sp.bk_lo) * sp.bk_inv) - 1;
-      b = min(max(b, 0), kSplineBuckets - 1);
-      int i = buckets[sp.bk_off + b];
-      while (i < n - 1 && rv[i] < R) ++i;
-      const int m = min(max(i, 2), n - 2);
-      rec = radial + sp.iv_off + (size_t)m * (2 + 4 * sp.nrad);
-      u = (R - rec[0]) * rec[1];
-    }
-    int ist = 0, rad = 0;
-    for (int l = 0; l <= sp.max_l; ++l) {
-      double Y[7];
-      ylm_unit(l, ux, uy, uz, Y);
-      for (int p = 0; p < sp.nb[l]; ++p, ++rad) {
-        double rf = 0.0;
-        if (rec) {
-          const double* c = rec + 2 + 4 * rad;
-          rf = ((c[3] * u + c[2]) * u + c[1]) * u + c[0];
-        } else if (inner) {
-          const double* e = radial + sp.ex_off + 4 * rad;
-          rf = ((e[0] * R + e[1]) * R + e[2]) * R + e[3];
-        }
-        for (int mm = 0; mm < 2 * l + 1; ++mm, ++ist) srow[ist] = rf * Y[mm];
-      }
-    }
+    eval_point<true, false>(sp, radial, q, srow, nullptr, nullptr, nullptr);
   }
   __syncthreads();
   const int64_t base = g.phi_off[atom] + (first - s0) * NO;
@@ -399,12 +262,14 @@ __global__ void __launch_bounds__(kTabBlock) tabulate_values_kernel(DevGeom g, c
   if (t == 0 && tail < total) dst[tail] = stage[tail];
 }
 
-template <bool GRAD>
-__global__ void __launch_bounds__(kTabPoints) tabulate_kernel(DevGeom g, const DevSpecies* __restrict__ spes,
-                                                              const double* __restrict__ radial,
-                                                              const int32_t* __restrict__ block_atom,
-                                                              const int64_t* __restrict__ block_start, double* phi,
-                                                              double* dpx, double* dpy, double* dpz) {
+// Value and gradient tables: one thread per sphere point, kTabPoints per block.
+__global__ void __launch_bounds__(kTabPoints) tabulate_gradients_kernel(DevGeom g, const DevSpecies* __restrict__ spes,
+                                                                        const double* __restrict__ radial,
+                                                                        const int32_t* __restrict__ buckets,
+                                                                        const int32_t* __restrict__ block_atom,
+                                                                        const int64_t* __restrict__ block_start,
+                                                                        double* phi, double* dpx, double* dpy,
+                                                                        double* dpz) {
   extern __shared__ double stage[];
   const int atom = block_atom[blockIdx.x];
   const int64_t first = block_start[blockIdx.x];
@@ -412,39 +277,24 @@ __global__ void __launch_bounds__(kTabPoints) tabulate_kernel(DevGeom g, const D
   const int npts = (int)((s1 - first) < kTabPoints ? (s1 - first) : kTabPoints);
   const DevSpecies sp = spes[g.spe[atom]];
   const int NO = sp.no;
-  const double* rv = radial + sp.rv_off;
-  const double* rwf = radial + sp.rwf_off;
   const int t = threadIdx.x;
 
   if (t < npts) {
-    const int64_t k = first + t;
-    const int gn = g.glist[k];
-    const int cell = g.clist[k];
-    const int N2 = g.ngrid[1], N3 = g.ngrid[2];
-    const int n1 = gn / (N2 * N3);
-    const int n2 = (gn - n1 * N2 * N3) / N3;
-    const int n3 = gn - n1 * N2 * N3 - n2 * N3;
     double xyz[3];
-    for (int d = 0; d < 3; ++d) {
-      double c = n1 * g.glat[0 * 3 + d] + n2 * g.glat[1 * 3 + d] + n3 * g.glat[2 * 3 + d] + g.origin[d];
-      xyz[d] = c + g.atv[cell * 3 + d] - g.gxyz[atom * 3 + d];
-    }
+    point_xyz(g, atom, first + t, xyz);
     double* srow = stage + (size_t)t * NO;
     double* sx = stage + (size_t)kTabPoints * NO + (size_t)t * NO;
     double* sy = sx + (size_t)kTabPoints * NO;
     double* sz = sy + (size_t)kTabPoints * NO;
-    double R, siQ, coQ, siP, coP;
-    spherical_trig(xyz[0], xyz[1], xyz[2], R, siQ, coQ, siP, coP);
-    if (!GRAD) {
-      eval_point<true, false>(sp, rv, rwf, R, siQ, coQ, siP, coP, srow, sx, sy, sz);
-    } else if (R < 1.0e-13) {
+    const TabPoint q = locate(sp, radial, buckets, xyz);
+    if (q.R < 1.0e-13) {
       // the gradient tables shift points that sit on the atom
       // (src/Matrix/Set_dOrbitals_Grid.jl:107-112); the values do not
-      eval_point<true, false>(sp, rv, rwf, R, siQ, coQ, siP, coP, srow, sx, sy, sz);
-      spherical_trig(xyz[0] + 1.0e-13, xyz[1] + 1.0e-13, xyz[2] + 1.0e-13, R, siQ, coQ, siP, coP);
-      eval_point<false, true>(sp, rv, rwf, R, siQ, coQ, siP, coP, srow, sx, sy, sz);
+      eval_point<true, false>(sp, radial, q, srow, sx, sy, sz);
+      for (int d = 0; d < 3; ++d) xyz[d] += 1.0e-13;
+      eval_point<false, true>(sp, radial, locate(sp, radial, buckets, xyz), srow, sx, sy, sz);
     } else {
-      eval_point<true, true>(sp, rv, rwf, R, siQ, coQ, siP, coP, srow, sx, sy, sz);
+      eval_point<true, true>(sp, radial, q, srow, sx, sy, sz);
     }
   }
   __syncthreads();
@@ -452,9 +302,8 @@ __global__ void __launch_bounds__(kTabPoints) tabulate_kernel(DevGeom g, const D
   // contiguous write-back: the block's points occupy rows [first-s0, +npts)
   const int64_t base = g.phi_off[atom] + (first - s0) * NO;
   const int total = npts * NO;
-  const int ntab = GRAD ? 4 : 1;
   double* outs[4] = {phi, dpx, dpy, dpz};
-  for (int tab = 0; tab < ntab; ++tab) {
+  for (int tab = 0; tab < 4; ++tab) {
     const double* src = stage + (size_t)tab * kTabPoints * NO;
     double* dst = outs[tab] + base;
     // 16-byte stores where the destination is 16-byte aligned
@@ -489,21 +338,21 @@ cudaError_t launch_tabulate(const DevGeom& g, const DevSpecies* dspe, const doub
   }
   // the gradient kernel takes blocks of kTabPoints points
   const size_t smem = (size_t)kTabPoints * max_no * sizeof(double) * 4;
-  LCP_CUDA_TRY(raise_smem(tabulate_kernel<true>, smem));
-  tabulate_kernel<true><<<(unsigned)nblocks, kTabPoints, smem, st>>>(g, dspe, radial, block_atom, block_start, phi,
-                                                                     dphi_x, dphi_y, dphi_z);
+  LCP_CUDA_TRY(raise_smem(tabulate_gradients_kernel, smem));
+  tabulate_gradients_kernel<<<(unsigned)nblocks, kTabPoints, smem, st>>>(g, dspe, radial, buckets, block_atom,
+                                                                         block_start, phi, dphi_x, dphi_y, dphi_z);
   return cudaGetLastError();
 }
 
-// Per-interval cubic of the value tables' spline for interval m of one
+// Per-interval cubic of the tables' spline for interval m of one
 // radial function w (src/Matrix/Set_Orbitals_Grid.jl:187-238): the Hermite
 // interpolant through (RV[m-1], f2) and (RV[m], f3) with the slopes g1, g2 of
 // the reference, as coefficients of u = (R - RV[m-1]) / h2; at m = N-2 the
-// reference substitutes f4 = f1 (:226-229).
-static void interval_cubic(const double* rv, const double* w, int n, int m, double* c) {
+// reference's values (not its gradients) substitute f4 = f1 (:226-229).
+static void interval_cubic(const double* rv, const double* w, int n, int m, bool values, double* c) {
   const double h1 = rv[m - 1] - rv[m - 2], h2 = rv[m] - rv[m - 1], h3 = rv[m + 1] - rv[m];
   const double f1 = w[m - 2], f2 = w[m - 1], f3 = w[m];
-  const double f4 = m == n - 2 ? f1 : w[m + 1];
+  const double f4 = values && m == n - 2 ? f1 : w[m + 1];
   double dum = h1 + h2;
   const double dum1 = h1 / h2 / dum, dum2 = h2 / h1 / dum;
   dum = h2 + h3;
@@ -561,11 +410,12 @@ void append_spline_tables(const double* rv, const double* rwf, int n, const int*
   const int rec = 2 + 4 * nrad;
   d.iv_off = (int64_t)radial.size();
   radial.resize(radial.size() + (size_t)n * rec, 0.0);
-  for (int m = 2; m <= n - 2; ++m) {
-    double* r = radial.data() + d.iv_off + (size_t)m * rec;
+  for (int k = 2; k <= n - 1; ++k) {  // the last record: interval n - 2 of the gradients
+    const int m = std::min(k, n - 2);
+    double* r = radial.data() + d.iv_off + (size_t)k * rec;
     r[0] = rv[m - 1];
     r[1] = 1.0 / (rv[m] - rv[m - 1]);
-    for (int q = 0; q < nrad; ++q) interval_cubic(rv, rwf + (size_t)q * n, n, m, r + 2 + 4 * q);
+    for (int q = 0; q < nrad; ++q) interval_cubic(rv, rwf + (size_t)q * n, n, m, k == m, r + 2 + 4 * q);
   }
   d.ex_off = (int64_t)radial.size();
   radial.resize(radial.size() + (size_t)4 * nrad, 0.0);

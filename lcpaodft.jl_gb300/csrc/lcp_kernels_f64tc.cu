@@ -2,8 +2,8 @@
 //
 // GB300 issues 2 FP64 FMAs per clock and SM, and the pair kernels of
 // lcp_kernels_pair.cu keep that pipe 95 % busy: 16.9 ms (density) and 19.9 ms
-// (matrix elements) on the 64-atom 96^3 cell, where the kernels below take 1.75
-// and 1.5 ms.  The tensor cores do 4,096 FP16 multiply-adds per clock and SM
+// (matrix elements) on the 64-atom 96^3 cell, where the kernels below take 1.5
+// and 1.6 ms.  The tensor cores do 4,096 FP16 multiply-adds per clock and SM
 // with FP32 accumulation, which is exact for integers below 2^24.  So each FP64
 // operand is put on a fixed-point grid of 56 bits,
 //
@@ -136,27 +136,25 @@ __device__ __forceinline__ void read_piece(const uint8_t* piece, int row, uint64
 }
 
 // Table pieces of kRawBytes on their way into a ring of shared-memory slots
-// (bulk copies).  The issuing warp keeps the ring full; a slot is refilled
-// once every reading warp has arrived on its empty barrier.
+// (bulk copies), issued by the MMA warp: once the digits of a slot's piece have
+// arrived as operands, it holds the next one.  (A barrier on which the split
+// warps gave a slot back after loading from it let a refilled slot be read: an
+// arrival does not wait for loads whose values are only used after it.  Giving
+// it back after the digits had the issuing split warp wait for the others.)
 constexpr uint32_t kRawBytes = 16384;
 template <int SLOTS>
 struct RawRing {
   uint8_t* buf;
-  uint64_t *full, *empty;
-  uint32_t slot = 0, par = 1, issued = 0;  // par: parity of the slot's last release
-  __device__ __forceinline__ bool issue(const uint8_t* src, const volatile int* abort_flag) {  // the whole warp
-    if (issued >= SLOTS && !tc::mbar_wait_warp(&empty[slot], par, abort_flag)) return false;
+  uint64_t* full;
+  uint32_t slot = 0, issued = 0;
+  __device__ __forceinline__ void issue(const uint8_t* src) {  // the whole warp
     if (tc::elect_one()) {
       tc::mbar_arrive_expect_tx(&full[slot], kRawBytes);
       tc::bulk_g2s(buf + slot * kRawBytes, src, kRawBytes, &full[slot]);
     }
     __syncwarp();
     ++issued;
-    if (++slot == SLOTS) {
-      slot = 0;
-      par ^= 1;
-    }
-    return true;
+    if (++slot == SLOTS) slot = 0;
   }
   // the last copies have landed (before the shared memory goes away)
   __device__ __forceinline__ void drain() {
@@ -413,7 +411,7 @@ __global__ void __launch_bounds__(kHP) f64_vprep_kernel(F64Bricks b, const doubl
 __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __grid_constant__ F64HamArgs args) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t afree_bar, bready_bar[2], bempty_bar[2], tfull_bar[2], tempty_bar[2], drain_bar;
-  __shared__ uint64_t rawfull_bar[kHRaw], rawempty_bar[kHRaw];
+  __shared__ uint64_t rawfull_bar[kHRaw];
   __shared__ uint32_t tslot;
   __shared__ volatile int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -426,10 +424,7 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
   if (is_mma) tc::tmem_alloc(&tslot, 512);
   if (tid == 0) {
     tc::mbar_init(&afree_bar, 1);
-    for (int s = 0; s < kHRaw; ++s) {
-      tc::mbar_init(&rawfull_bar[s], 1);
-      tc::mbar_init(&rawempty_bar[s], kHConv);
-    }
+    for (int s = 0; s < kHRaw; ++s) tc::mbar_init(&rawfull_bar[s], 1);
     for (int s = 0; s < 2; ++s) {
       tc::mbar_init(&bready_bar[s], kHConv);
       tc::mbar_init(&bempty_bar[s], 1);
@@ -481,6 +476,14 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
           F64Row mc{};
           if (c0 + lane < R) mc = load_meta(rows + c0 + lane);
           const bool slow = slow_r || __any_sync(0xffffffffu, c0 + lane < R && odd_exp(row_exp(mc.info)));
+          // block offsets of a column group, loaded a group ahead (columns past R: entry t = 0)
+          const int32_t* trow = tab + (int64_t)s_img * m;
+          auto ask = [&](int cb, int32_t (&o)[4]) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[j] = __ldg(trow + (__shfl_sync(0xffffffffu, mc.img_orb, cb + j) >> 8));
+          };
+          int32_t next[4];
+          ask(rank * 4, next);
           if (!tc::mbar_wait_warp(&tfull_bar[buf], (it >> 1) & 1, &abort_flag)) {
             give_up();
             break;
@@ -490,10 +493,10 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
 #pragma unroll 1
             for (int cb = rank * 4; cb < kWin; cb += nepi * 4) {
               if (c0 + cb >= R) break;
-              int32_t offs[4];  // every load in flight together (columns past R: entry t = 0)
+              int32_t offs[4];
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
-                offs[j] = __ldg(tab + (int64_t)s_img * m + (__shfl_sync(0xffffffffu, mc.img_orb, cb + j) >> 8));
+              for (int j = 0; j < 4; ++j) offs[j] = next[j];
+              ask((cb + nepi * 4) & (kWin - 1), next);
               uint32_t y[kDig][4];
               load_acc(tmem, quarter, buf * kBufCols + cb, y);
               // no branch before the adds: the four columns' chains interleave
@@ -534,8 +537,17 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
       }
     }
   } else if (is_mma) {
-    // ------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------ MMA issuer, table producer
     uint32_t it = 0;
+    StepIter ahead;  // kHRaw steps ahead
+    ahead.begin(B);
+    RawRing<kHRaw> ring{smem + kDig * kHADigit + 2 * kHBStage, rawfull_bar};
+    auto fetch = [&]() {
+      if (!ahead.valid()) return;
+      ring.issue(reinterpret_cast<const uint8_t*>(B.table + (int64_t)(ahead.b.chunk + ahead.c0 / 32) * 32 * kHP));
+      ahead.step(B);
+    };
+    for (int i = 0; i < kHRaw; ++i) fetch();
     BrickIter x;
     for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
       const int R = x.R();
@@ -570,6 +582,7 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
             if (c0 + kWin >= R) tc::mma_commit(&afree_bar);  // the tile's A may be overwritten
           }
           __syncwarp();
+          fetch();  // into this step's slot: its B is split
         }
       }
     }
@@ -578,29 +591,15 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
       if (!tc::mbar_wait(&drain_bar, 0, 1u << 24)) give_up();
     }
     __syncwarp();
+    ring.drain();
   } else {
     // ------------------------------------------------------------ split
     const int kg = sched == 1 ? rank - 3 : (sched == 2 ? rank : rank + 3);  // 0..7
     uint32_t it = 0, tile = 0, rslot = 0, rpar = 0;
     uint8_t* raw = smem + kDig * kHADigit + 2 * kHBStage;
-    StepIter x, ahead;  // warp kg 0 fetches kHRaw - 1 steps ahead
+    StepIter x;
     x.begin(B);
-    ahead = x;
-    RawRing<kHRaw> ring{raw, rawfull_bar, rawempty_bar};
-    auto fetch = [&]() {
-      if (!ahead.valid()) return true;
-      const bool ok = ring.issue(reinterpret_cast<const uint8_t*>(B.table + (int64_t)(ahead.b.chunk + ahead.c0 / 32) * 32 * kHP),
-                                 &abort_flag);
-      ahead.step(B);
-      return ok;
-    };
-    if (kg == 0)
-      for (int i = 0; i < kHRaw - 1; ++i) fetch();
     while (x.valid() && !abort_flag) {
-      if (kg == 0 && !fetch()) {
-        give_up();
-        break;
-      }
       const int k = x.k;
       const int r0 = x.r0, c0 = x.c0;
       x.step(B);
@@ -616,8 +615,6 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
         break;
       }
       read_piece(raw + rslot * kRawBytes + kg * 2048, lane, t);
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&rawempty_bar[rslot]);
       if (++rslot == kHRaw) {
         rslot = 0;
         rpar ^= 1;
@@ -650,7 +647,6 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
       __syncwarp();
       ++it;
     }
-    if (kg == 0) ring.drain();
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -702,16 +698,21 @@ __global__ void f64_finish_kernel(DevPairs pr, const int32_t* __restrict__ numor
 // so that a lane splits one row at eight points; B (Ds, scaled per column) is
 // K-major.
 //
-// Roles (672 threads, one CTA per SM, persistent over bricks):
+// Roles (768 threads, one CTA per SM, persistent over bricks):
 //   warps 0-7    epilogue: lane = point, half a window each: X assembled in 64
 //                bits, times phi_c(p) into a 128-bit sum (FP64 products took
 //                128 clocks per column and warp of this GPU's FP64 pipe);
-//   warp 8       MMA issuer: per chunk 2 K steps x 7 MMAs;
+//   warp 8       MMA issuer: per chunk 2 K steps x 7 MMAs; then the bulk copies
+//                of the table's chunk after next;
 //   warps 9-16   split A: two of a chunk's sixteen pieces (8 points x 32 rows) each;
-//   warps 17-20  split B: one of its four pieces (8 rows x 32 columns) each; the
-//                entries' addresses come from the pair tables, two chunks ahead.
+//   warps 17-23  split B: its four pieces (8 rows x 32 columns) in turn; the
+//                entries' addresses come from the pair tables, two pieces ahead.
 // Every split warp has its next chunk's loads in flight while it splits one:
-// without that a chunk took 5,000 clocks, whatever the arithmetic.
+// without that a chunk took 5,000 clocks, whatever the arithmetic.  With four
+// warps on B, B set the pace (2,900 clocks a chunk); with one of the A warps
+// issuing the copies, that warp did.  Seven warps on B and the copies on the MMA
+// warp took the 64-atom 96^3 cell from 1.79 to 1.53 ms; the integer pipe is the
+// busiest unit now (2.5 of 4 instructions a clock issued).
 //
 // The force term's epilogue holds Y's column as one FP64 value times the
 // gradients at its point, read from the point-major tables through the
@@ -723,17 +724,20 @@ __global__ void f64_finish_kernel(DevPairs pr, const int32_t* __restrict__ numor
 namespace {
 
 constexpr int kDP = 128;
-constexpr int kDEpi = 8, kDConvA = 8, kDConvB = 4, kDConv = kDConvA + kDConvB;
+constexpr int kDEpi = 8, kDConvA = 8, kDConvB = 7, kDConv = kDConvA + kDConvB;
+constexpr int kDPiecesB = 4;  // of a chunk's B (8 rows each), taken in turn by the kDConvB warps
 constexpr int kDThreads = 32 * (kDEpi + 1 + kDConv);
 static_assert(kF64ForceParts == kDEpi * 3, "three sums per image and epilogue warp");
 constexpr int kDChunk = 32;
 constexpr uint32_t kDStages = 2;
-constexpr int kDRaw = 5;                                      // half chunks of the table in shared memory
+constexpr uint32_t kDEmpty = 4;  // barriers of the chunks' releases, chunk n's at n % 4
+static_assert(kDConvB <= 2 * kDPiecesB && kDEmpty >= 2 * kDStages, "a split warp passes over one chunk at most");
+constexpr int kDRaw = 4;                                      // half chunks of the table in shared memory
 constexpr uint32_t kDADigit = kDP * kDChunk * 2;             // 8 KB: [point group][32 rows][16 B]
 constexpr uint32_t kDBLbo = kDig * kWin * 16;
 constexpr uint32_t kDBBytes = (kDChunk / 8) * kDBLbo;        // 14 KB
 constexpr uint32_t kDStageBytes = kDig * kDADigit + kDBBytes;  // 70 KB
-constexpr size_t kDSmemBytes = kDStages * (size_t)kDStageBytes + kDRaw * (size_t)kRawBytes;  // 220 KB
+constexpr size_t kDSmemBytes = kDStages * (size_t)kDStageBytes + kDRaw * (size_t)kRawBytes;  // 204 KB
 static_assert(2 * kRawBytes == 32 * kDP * 8, "a raw slot is half a chunk");
 
 // sum a_d 256^(7-d) / 256, rounded, for |a_d| <= 2^24 (d <= 5; a_6 and a_7 may
@@ -913,16 +917,19 @@ struct ChunkIter : BrickIterT<AHEAD> {
 // (entry 0 where there is nothing), so that they are in flight together.
 // Density: Ds of row and column at tab[s][t] + a_row noj + b_col, rows up to the
 // column; force: D of (column's atom, row's atom) at tab[t][s] + a_col noj + b_row.
+// Nothing here uses a value that it has just loaded: loads of all three steps
+// are in flight together (with the entries' selection beside their loads a
+// piece took three latencies in turn).
 struct BAsk {
-  F64Row col;
-  uint32_t rio, mask;  // img_orb (and orbital count << 24) of row lane % 8; rows that count
+  F64Row col, row;  // the column's; of row lane % 8
+  uint32_t mask;    // rows that count
   uint32_t tab;
   int m;
   bool ok;
 };
 struct BPiece {
-  uint32_t rio, mask;
-  int b, noj;  // the column's orbital and its atom's orbitals
+  uint32_t rio, mask;  // img_orb (and orbital count << 24) of row lane % 8
+  int b, noj;          // the column's orbital and its atom's orbitals
   int32_t off[8];
   bool ok;
 };
@@ -934,8 +941,7 @@ __device__ __forceinline__ void ask_b(const F64Bricks& B, const ChunkIter<FORCE,
   q.tab = x.b.tab;
   q.m = x.m();
   q.col = load_meta(B.rows + x.b.row + min(c, R - 1));
-  const F64Row row = load_meta(B.rows + x.b.row + min(rh + (lane & 7), R - 1));
-  q.rio = row.img_orb | ((uint32_t)row_no(row.info) << 24);
+  q.row = load_meta(B.rows + x.b.row + min(rh + (lane & 7), R - 1));
   const int n = (FORCE ? R : c + 1) - rh;  // rows of this piece that count
   q.mask = c < R && n > 0 ? (n >= 8 ? 255u : (1u << n) - 1u) : 0u;
 }
@@ -943,7 +949,7 @@ template <bool FORCE>
 __device__ __forceinline__ void locate_b(const F64Bricks& B, const BAsk& a, BPiece& q) {
   q.ok = a.ok;
   if (!a.ok) return;
-  q.rio = a.rio;
+  q.rio = a.row.img_orb | ((uint32_t)row_no(a.row.info) << 24);
   q.mask = a.mask;
   q.b = (int)(a.col.img_orb & 255u);
   q.noj = row_no(a.col.info);
@@ -951,12 +957,12 @@ __device__ __forceinline__ void locate_b(const F64Bricks& B, const BAsk& a, BPie
   const int32_t* tab = B.tab + a.tab + (FORCE ? t * a.m : t);
 #pragma unroll
   for (int i = 0; i < 8; ++i)
-    q.off[i] = __ldg(tab + (int)((__shfl_sync(0xffffffffu, a.rio, i) >> 8) & 0xffffu) * (FORCE ? 1 : a.m));
+    q.off[i] = __ldg(tab + (int)((__shfl_sync(0xffffffffu, q.rio, i) >> 8) & 0xffffu) * (FORCE ? 1 : a.m));
 }
 template <bool FORCE>
-__device__ __forceinline__ void gather_b(const uint64_t* __restrict__ dfix, const BPiece& q, uint64_t* t) {
+__device__ __forceinline__ void gather_b(const uint64_t* __restrict__ dfix, const BPiece& q, uint64_t* t, uint32_t& ok) {
+  ok = 0;
   if (!q.ok) return;
-  uint32_t ok = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const uint32_t io = __shfl_sync(0xffffffffu, q.rio, i);
@@ -965,8 +971,6 @@ __device__ __forceinline__ void gather_b(const uint64_t* __restrict__ dfix, cons
     ok |= (y ? 1u : 0u) << i;
     t[i] = __ldg(dfix + (y ? q.off[i] + (FORCE ? q.b * (int)(io >> 24) + a : a * q.noj + q.b) : 0));
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) t[i] = (ok >> i) & 1u ? t[i] : kF64Bias;
 }
 
 // The sums of three values over the warp: of the first in lane 0, of the
@@ -984,22 +988,17 @@ __device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int
 template <bool FORCE>
 __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_constant__ F64DensArgs args) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ uint64_t full_bar[kDStages], empty_bar[kDStages], tfull_bar[2], tempty_bar[2], drain_bar;
-  __shared__ uint64_t rawfull_bar[kDRaw], rawempty_bar[kDRaw];
+  __shared__ uint64_t full_bar[kDStages], empty_bar[kDEmpty], tfull_bar[2], tempty_bar[2], drain_bar;
+  __shared__ uint64_t rawfull_bar[kDRaw];
   __shared__ uint32_t tslot;
   __shared__ volatile int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const F64Bricks& B = args.b;
   if (warp == kDEpi) tc::tmem_alloc(&tslot, 512);
   if (tid == 0) {
-    for (int s = 0; s < kDRaw; ++s) {
-      tc::mbar_init(&rawfull_bar[s], 1);
-      tc::mbar_init(&rawempty_bar[s], kDConvA);
-    }
-    for (uint32_t s = 0; s < kDStages; ++s) {
-      tc::mbar_init(&full_bar[s], kDConv);
-      tc::mbar_init(&empty_bar[s], 1);
-    }
+    for (int s = 0; s < kDRaw; ++s) tc::mbar_init(&rawfull_bar[s], 1);
+    for (uint32_t s = 0; s < kDStages; ++s) tc::mbar_init(&full_bar[s], kDConvA + kDPiecesB);
+    for (uint32_t s = 0; s < kDEmpty; ++s) tc::mbar_init(&empty_bar[s], 1);
     for (int s = 0; s < 2; ++s) {
       tc::mbar_init(&tfull_bar[s], 1);
       tc::mbar_init(&tempty_bar[s], kDEpi);
@@ -1205,8 +1204,19 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
       }
     }
   } else if (warp == kDEpi) {
-    // ------------------------------------------------------------ MMA issuer
-    uint32_t st = 0, par = 0, win = 0;
+    // ------------------------------------------------------------ MMA issuer, table producer
+    uint32_t st = 0, par = 0, win = 0, chunk = 0;
+    ChunkIter<FORCE, true> ahead;  // kDRaw / 2 chunks ahead
+    ahead.begin(B);
+    RawRing<kDRaw> ring{smem + kDStages * kDStageBytes, rawfull_bar};
+    auto fetch = [&]() {
+      if (!ahead.valid()) return;
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(B.table + (int64_t)(ahead.b.chunk + ahead.r0 / 32) * 32 * kDP);
+      ring.issue(src);
+      ring.issue(src + kRawBytes);
+      ahead.step(B);
+    };
+    for (int i = 0; i < kDRaw / 2; ++i) fetch();
     BrickIter x;
     for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
       const int R = x.R();
@@ -1237,10 +1247,12 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
             }
           }
           if (tc::elect_one()) {
-            tc::mma_commit(&empty_bar[st]);
+            tc::mma_commit(&empty_bar[chunk % kDEmpty]);
             if (r0 == last) tc::mma_commit(&tfull_bar[buf]);
           }
           __syncwarp();
+          fetch();  // into this chunk's slots: its A is split
+          ++chunk;
           if (++st == kDStages) {
             st = 0;
             par ^= 1;
@@ -1253,35 +1265,24 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
       if (!tc::mbar_wait(&drain_bar, 0, 1u << 24)) give_up();
     }
     __syncwarp();
+    ring.drain();
   } else {
     // ------------------------------------------------------------ split
     const int cw = warp - kDEpi - 1;
-    uint32_t st = 0, par = 1, round = 0;  // par: parity of the stage's last release
+    // chunk n's stage n % kDStages is free once chunk n - kDStages has been released
+    auto stage_free = [&](uint32_t n) {
+      const uint32_t u = n - kDStages;
+      return n < kDStages || tc::mbar_wait_warp(&empty_bar[u % kDEmpty], (u / kDEmpty) & 1, &abort_flag);
+    };
+    uint8_t* raw = smem + kDStages * kDStageBytes;
     if (cw < kDConvA) {
-      ChunkIter<FORCE, true> x, ahead;  // warp 0 fetches up to kDRaw half chunks ahead
+      ChunkIter<FORCE, true> x;
       x.begin(B);
-      ahead = x;
-      uint8_t* raw = smem + kDStages * kDStageBytes;
-      RawRing<kDRaw> ring{raw, rawfull_bar, rawempty_bar};
-      uint32_t half = 0, rslot = 0, rpar = 0;
-      auto fetch = [&]() {
-        if (!ahead.valid()) return true;
-        const bool ok = ring.issue(reinterpret_cast<const uint8_t*>(B.table + (int64_t)(ahead.b.chunk + ahead.r0 / 32) * 32 * kDP) +
-                                       half * kRawBytes,
-                                   &abort_flag);
-        half ^= 1;
-        if (half == 0) ahead.step(B);
-        return ok;
-      };
-      if (cw == 0)
-        for (int i = 0; i < kDRaw - 2; ++i) fetch();
-      while (x.valid() && !abort_flag) {
-        if (cw == 0 && !(fetch() && fetch())) {
-          give_up();
-          break;
-        }
+      uint32_t n = 0, rslot = 0, rpar = 0;
+      for (; x.valid() && !abort_flag; ++n) {
         x.step(B);
-        bool ok = round == 0 || tc::mbar_wait_warp(&empty_bar[st], par, &abort_flag);
+        const uint32_t st = n % kDStages;
+        bool ok = true;
         uint8_t* sA = smem + st * kDStageBytes;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -1289,13 +1290,12 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
           if (ok) {
             uint64_t t[8];
             read_piece(raw + rslot * kRawBytes + cw * 2048, lane, t);
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&rawempty_bar[rslot]);
             if (++rslot == kDRaw) {
               rslot = 0;
               rpar ^= 1;
             }
-            store_digits(sA + (cw + 8 * h) * 512 + lane * 16, kDADigit, t);
+            if (h == 0) ok = stage_free(n);
+            if (ok) store_digits(sA + (cw + 8 * h) * 512 + lane * 16, kDADigit, t);
           }
         }
         if (!ok) {
@@ -1306,49 +1306,51 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&full_bar[st]);
         __syncwarp();
-        if (++st == kDStages) {
-          st = 0;
-          par ^= 1;
-          round = 1;
-        }
       }
-      if (cw == 0) ring.drain();
     } else {
-      const int g = cw - kDConvA;
+      // Piece i of the CTA's sequence is piece i % 4 of chunk i / 4; this warp's are
+      // kDConvB apart.  It passes chunks over, and a barrier's parity tells a phase
+      // from its neighbours only: hence more release barriers than stages.  The
+      // warp's last piece waited for a release at most two chunks before the one
+      // it waits for next, so the phase before that is past.
+      int ga = cw - kDConvA;   // piece to ask for next, counted from x's chunk
+      uint32_t piece = ga;     // the piece in t
       ChunkIter<FORCE, false> x;
       x.begin(B);
+      auto ask_next = [&](BAsk& ask) {
+        for (; ga >= kDPiecesB; ga -= kDPiecesB)
+          if (x.valid()) x.step(B);
+        ask_b<FORCE>(B, x, ga, lane, ask);
+        ga += kDConvB;
+      };
       uint64_t t[8];
+      uint32_t rows;  // entries of t that there are
       BAsk ask;
       BPiece q;
-      bool now = x.valid();  // there is a chunk in t
-      ask_b<FORCE>(B, x, g, lane, ask);
+      ask_next(ask);
+      bool now = ask.ok;  // there is a piece in t
       locate_b<FORCE>(B, ask, q);
-      if (x.valid()) x.step(B);
-      ask_b<FORCE>(B, x, g, lane, ask);
-      gather_b<FORCE>(args.dfix, q, t);
+      ask_next(ask);
+      gather_b<FORCE>(args.dfix, q, t, rows);
       locate_b<FORCE>(B, ask, q);
-      if (x.valid()) x.step(B);
-      ask_b<FORCE>(B, x, g, lane, ask);
-      while (now && !abort_flag) {
-        if (round > 0 && !tc::mbar_wait_warp(&empty_bar[st], par, &abort_flag)) {
+      ask_next(ask);
+      for (; now && !abort_flag; piece += kDConvB) {
+        const uint32_t c = piece / kDPiecesB, st = c % kDStages;
+        if (!stage_free(c)) {
           give_up();
           break;
         }
-        store_digits(smem + st * kDStageBytes + kDig * kDADigit + g * kDBLbo + lane * 16, kWin * 16, t);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t[i] = (rows >> i) & 1u ? t[i] : kF64Bias;
+        store_digits(smem + st * kDStageBytes + kDig * kDADigit + piece % kDPiecesB * kDBLbo + lane * 16, kWin * 16, t);
         tc::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&full_bar[st]);
         __syncwarp();
         now = q.ok;
-        gather_b<FORCE>(args.dfix, q, t);
+        gather_b<FORCE>(args.dfix, q, t, rows);
         locate_b<FORCE>(B, ask, q);
-        if (x.valid()) x.step(B);
-        ask_b<FORCE>(B, x, g, lane, ask);
-        if (++st == kDStages) {
-          st = 0;
-          par ^= 1;
-          round = 1;
-        }
+        ask_next(ask);
       }
     }
   }

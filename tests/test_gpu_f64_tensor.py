@@ -106,6 +106,8 @@ def test_f64_tensor_force_against_oracle(name):
     ref = O.calc_force3("on", uo, phi, grad, v, dm)
     f = L.Force3_spin(paos, dorbs, v, dm, u)
     assert np.max(np.abs(f - ref)) <= 1e-10 * np.max(np.abs(ref))
+    for _ in range(10):  # every sum is taken in a fixed order
+        assert np.array_equal(f, L.Force3_spin(paos, dorbs, v, dm, u))
     # a potential and a D that are not finite reach the atoms that have them, and no others
     bad = v[0].copy()
     outside = np.ones(u.NN, bool)

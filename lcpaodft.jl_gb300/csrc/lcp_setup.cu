@@ -150,9 +150,9 @@ struct SetupGeom {
   int32_t ng[3];
   int32_t cpy, ncdim;  // CpyCell, 2 CpyCell + 1
   double glat[3][3];   // grid vectors (rows)
+  float glat32[3][3];
   double origin[3];
   const double* atv;       // [ncell][3]
-  const int32_t* atv_ijk;  // [ncell][3]
   const int32_t* ratv;     // [(2C+1)^3]
 };
 
@@ -162,6 +162,11 @@ struct SphereAtom {
   int32_t tab;   // offset of the tables: per axis rank[len], image[len]; then per axis count[nres], before[nres]
   int64_t cand;  // offset of the atom's box points among all atoms'
   double g[3], cut;
+  // FP32 bounds of the distance (box_side): the box's first point from the atom
+  // and the squares of the radii inside and outside of which a point surely is
+  float b[3], in2, out2;
+  // a box point packed as t0 << sh0 | t1 << sh1 | t2
+  int32_t sh0, sh1;
 };
 
 __device__ __forceinline__ int floor_div(int a, int n) {
@@ -181,23 +186,22 @@ __device__ __forceinline__ int atom_of(const int64_t* __restrict__ off, int nato
 }
 
 // Box point t (scan order) of atom A: its position in the atom's sorted list
-// order, its flat grid index, image cell and whether it is within the cutoff
-// (Calc_AtomsGrid, src/UCell.jl:365-400, with Find_CGrids!,
-// src/utils/Find_CGrid.jl:1-49).
+// order, its flat grid index and image cell (Calc_AtomsGrid,
+// src/UCell.jl:365-400, with Find_CGrids!, src/utils/Find_CGrid.jl:1-49).
 struct BoxPoint {
-  int64_t s;
-  int32_t g, rn;
-  bool keep;
+  int32_t s, g, rn;
+  int32_t tt[3], nn[3];
 };
 
 __device__ __forceinline__ BoxPoint box_point(const SetupGeom& G, const SphereAtom& A, const int32_t* __restrict__ tabs,
-                                              int64_t t) {
-  const int L1 = A.len[1], L2 = A.len[2];
-  const int t3 = (int)(t % L2);
-  const int64_t t12 = t / L2;
-  const int t2 = (int)(t12 % L1);
-  const int t1 = (int)(t12 / L1);
-  const int tt[3] = {t1, t2, t3};
+                                              uint32_t t) {  // all atoms' box points are fewer than 2^31
+  const uint32_t L1 = (uint32_t)A.len[1], L2 = (uint32_t)A.len[2];
+  const uint32_t t12 = t / L2, t1 = t12 / L1;
+  BoxPoint p;
+  p.tt[0] = (int)t1;
+  p.tt[1] = (int)(t12 - t1 * L1);
+  p.tt[2] = (int)(t - t12 * L2);
+  const int32_t* tt = p.tt;
   int rank[3], img[3], cnt[3], bef[3];
   int o = A.tab;
 #pragma unroll
@@ -212,33 +216,47 @@ __device__ __forceinline__ BoxPoint box_point(const SetupGeom& G, const SphereAt
     bef[d] = tabs[o + A.nres[d] + rank[d]];
     o += 2 * A.nres[d];
   }
-  BoxPoint p;
-  p.s = (int64_t)bef[0] * A.len[1] * A.len[2] +
-        (int64_t)cnt[0] * ((int64_t)bef[1] * A.len[2] + (int64_t)cnt[1] * bef[2]) +
-        ((int64_t)img[0] * cnt[1] + img[1]) * cnt[2] + img[2];
-  int nn[3], l[3];
+  p.s = bef[0] * A.len[1] * A.len[2] + cnt[0] * (bef[1] * A.len[2] + cnt[1] * bef[2]) +
+        (img[0] * cnt[1] + img[1]) * cnt[2] + img[2];
+  int l[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const int n = A.nmin[d] + tt[d];
     l[d] = floor_div(n, G.ng[d]);
-    nn[d] = n - l[d] * G.ng[d];
+    p.nn[d] = n - l[d] * G.ng[d];
   }
   const int C = G.cpy;
   p.rn = G.ratv[((C + l[0]) * G.ncdim + (C + l[1])) * G.ncdim + (C + l[2])];
-  p.g = (nn[0] * G.ng[1] + nn[1]) * G.ng[2] + nn[2];
+  p.g = (p.nn[0] * G.ng[1] + p.nn[1]) * G.ng[2] + p.nn[2];
+  return p;
+}
+
+// Whether a box point is within the cutoff.  The reference's distance takes 24
+// FP64 operations and a square root, and the FP64 pipe (two operations a clock
+// and SM) then bounds the pass (0.78 ms for the 32-atom Si cell, against 0.064).
+// In FP32, from the box's corner, the same distance is off by less than 2^-19
+// of the coordinates' bound (sphere_bounds): only points that near to the
+// cutoff take the FP64 test.
+__device__ __forceinline__ bool within_cutoff(const SetupGeom& G, const SphereAtom& A, const BoxPoint& p) {
+  float f[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    f[d] = A.b[d] + (float)p.tt[0] * G.glat32[0][d] + (float)p.tt[1] * G.glat32[1][d] + (float)p.tt[2] * G.glat32[2][d];
+  const float r2 = f[0] * f[0] + f[1] * f[1] + f[2] * f[2];
+  if (r2 < A.in2) return true;
+  if (r2 > A.out2) return false;
   double dd[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     double c = G.atv[p.rn * 3 + d];
-    c = __dadd_rn(c, __dmul_rn((double)nn[0], G.glat[0][d]));
-    c = __dadd_rn(c, __dmul_rn((double)nn[1], G.glat[1][d]));
-    c = __dadd_rn(c, __dmul_rn((double)nn[2], G.glat[2][d]));
+    c = __dadd_rn(c, __dmul_rn((double)p.nn[0], G.glat[0][d]));
+    c = __dadd_rn(c, __dmul_rn((double)p.nn[1], G.glat[1][d]));
+    c = __dadd_rn(c, __dmul_rn((double)p.nn[2], G.glat[2][d]));
     c = __dadd_rn(c, G.origin[d]);
     dd[d] = __dsub_rn(c, A.g[d]);
   }
   const double R = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(dd[0], dd[0]), __dmul_rn(dd[1], dd[1])), __dmul_rn(dd[2], dd[2])));
-  p.keep = R <= A.cut;
-  return p;
+  return R <= A.cut;
 }
 
 __global__ void sphere_flag_kernel(const __grid_constant__ SetupGeom G, const SphereAtom* __restrict__ atoms,
@@ -249,31 +267,32 @@ __global__ void sphere_flag_kernel(const __grid_constant__ SetupGeom G, const Sp
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int a = atom_of(cand_off, natom, idx);
     const SphereAtom& A = atoms[a];
-    const BoxPoint p = box_point(G, A, tabs, idx - A.cand);
-    flags[A.cand + p.s] = p.keep ? 1 : 0;
+    const BoxPoint p = box_point(G, A, tabs, (uint32_t)(idx - A.cand));
+    flags[A.cand + p.s] = within_cutoff(G, A, p) ? 1 : 0;
   }
 }
 
 // pos: exclusive scan of the flags (list position of every kept point among
 // all atoms'); lut[idx]: the box table, the point's index in its atom's list
-// or -1.
+// or -1; box[o]: the packed box point of list entry o.
 __global__ void sphere_write_kernel(const __grid_constant__ SetupGeom G, const SphereAtom* __restrict__ atoms,
                                     const int64_t* __restrict__ cand_off, int natom, const int32_t* __restrict__ tabs,
                                     const int32_t* __restrict__ flags, const int64_t* __restrict__ pos,
                                     int32_t* __restrict__ glist, int32_t* __restrict__ clist,
-                                    int32_t* __restrict__ lut) {
+                                    int32_t* __restrict__ lut, int64_t* __restrict__ box) {
   const int64_t total = cand_off[natom];
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int a = atom_of(cand_off, natom, idx);
     const SphereAtom& A = atoms[a];
-    const BoxPoint p = box_point(G, A, tabs, idx - A.cand);
+    const BoxPoint p = box_point(G, A, tabs, (uint32_t)(idx - A.cand));
     const int64_t f = A.cand + p.s;
     if (flags[f]) {
       const int64_t o = pos[f];
       glist[o] = p.g;
       clist[o] = p.rn;
       lut[idx] = (int32_t)(o - pos[A.cand]);
+      box[o] = ((int64_t)p.tt[0] << A.sh0) | ((int64_t)p.tt[1] << A.sh1) | p.tt[2];
     } else {
       lut[idx] = -1;
     }
@@ -295,39 +314,19 @@ struct OvPair {
   int32_t r[3];  // image cell R of the neighbour
 };
 
-// Index in atom i's list of the point at entry e of j's list seen through the
-// pair's cell R, or -1 (Calc_AtomOverlap_Grid, src/UCell.jl:439-512).
-__device__ __forceinline__ int32_t twin(const SetupGeom& G, const SphereAtom& Ai, const OvPair& P,
-                                        const int32_t* __restrict__ glist, const int32_t* __restrict__ clist,
-                                        const int32_t* __restrict__ lut, int64_t e) {
-  const int cell = clist[e];
-  const int C = G.cpy;
-  int l[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    l[d] = G.atv_ijk[cell * 3 + d] + P.r[d];
-    if (l[d] > C || l[d] < -C) return -1;
-  }
-  const int g = glist[e];
-  const int plane = G.ng[1] * G.ng[2];
-  const int nn0 = g / plane;
-  const int rem = g - nn0 * plane;
-  const int nn1 = rem / G.ng[2];
-  const int nn2 = rem - nn1 * G.ng[2];
-  const int nn[3] = {nn0, nn1, nn2};
-  int t[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    t[d] = nn[d] + l[d] * G.ng[d] - Ai.nmin[d];
-    if (t[d] < 0 || t[d] >= Ai.len[d]) return -1;
-  }
-  return lut[Ai.cand + ((int64_t)t[0] * Ai.len[1] + t[1]) * Ai.len[2] + t[2]];
-}
-
-// Block b covers entries [k0, k0 + kOvChunk) of pair q's j list; thread t its
-// entries k0 + t*kOvPer .. + kOvPer - 1, in order.  WRITE = false: the block's
-// number of hits into cnt[b]; WRITE = true: the hits (index in i's list, index
-// in j's list) at boff[b] + the hits before them in the block.
+// Block b covers entries [k0, k0 + kOvChunk) of pair q's j list, kOvThreads at
+// a time (consecutive entries on consecutive lanes, eight loads in flight).
+// WRITE = false: the block's number of hits into cnt[b]; WRITE = true: the hits
+// (index in i's list, index in j's list) at boff[b] + the hits before them in
+// the block.
+//
+// An entry's twin (Calc_AtomOverlap_Grid, src/UCell.jl:439-512) is the point
+// of i's box at j's box coordinate plus a shift that the whole pair shares;
+// i's box only holds cells within CpyCell, so being in the box is the whole
+// test.  The list keeps its box coordinates packed: taking them from the flat
+// grid index and the cell cost two integer divisions and four loads per entry
+// (count and write 0.56 and 0.66 ms for the 32-atom Si cell, now 0.16 and 0.18, bound by the
+// table's loads).
 template <bool WRITE>
 __global__ void __launch_bounds__(kOvThreads) overlap_kernel(const __grid_constant__ SetupGeom G,
                                                              const SphereAtom* __restrict__ atoms,
@@ -335,36 +334,74 @@ __global__ void __launch_bounds__(kOvThreads) overlap_kernel(const __grid_consta
                                                              const int32_t* __restrict__ blk_pair,
                                                              const int64_t* __restrict__ blk_k0,
                                                              const int64_t* __restrict__ sphere_off,
-                                                             const int32_t* __restrict__ glist,
-                                                             const int32_t* __restrict__ clist,
+                                                             const int64_t* __restrict__ box,
                                                              const int32_t* __restrict__ lut, int32_t* __restrict__ cnt,
                                                              const int64_t* __restrict__ boff, int32_t* __restrict__ g1,
                                                              int32_t* __restrict__ g2) {
+  constexpr int kWarps = kOvThreads / 32;
+  __shared__ int32_t s_cnt[kOvPer * kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const OvPair P = pairs[blk_pair[blockIdx.x]];
   const SphereAtom& Ai = atoms[P.i];
+  const SphereAtom& Aj = atoms[P.j];
   const int64_t base = sphere_off[P.j];
-  const int64_t nj = sphere_off[P.j + 1] - base;
-  const int64_t k0 = blk_k0[blockIdx.x] + (int64_t)threadIdx.x * kOvPer;
+  const int64_t k0 = blk_k0[blockIdx.x];
+  const int n = (int)min((int64_t)kOvChunk, sphere_off[P.j + 1] - base - k0);
+  int d[3], len[3];
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    d[e] = Aj.nmin[e] + P.r[e] * G.ng[e] - Ai.nmin[e];
+    len[e] = Ai.len[e];
+  }
+  const int sh0 = Aj.sh0, sh1 = Aj.sh1;
+  const int m1 = (int)((1u << (sh0 - sh1)) - 1u), m2 = (int)((1u << sh1) - 1u);
+  const int32_t* table = lut + Ai.cand;
   int32_t hit[kOvPer];
-  int64_t mine = 0;
+  int64_t t[kOvPer];
 #pragma unroll
   for (int m = 0; m < kOvPer; ++m) {
-    hit[m] = k0 + m < nj ? twin(G, Ai, P, glist, clist, lut, base + k0 + m) : -1;
-    mine += hit[m] >= 0 ? 1 : 0;
+    const int k = m * kOvThreads + (int)threadIdx.x;
+    t[m] = k < n ? __ldg(box + base + k0 + k) : -1;
   }
-  int64_t tot;
-  const int64_t before = block_exclusive_scan(mine, &tot);
-  if (!WRITE) {
-    if (threadIdx.x == 0) cnt[blockIdx.x] = (int32_t)tot;
-    return;
+#pragma unroll
+  for (int m = 0; m < kOvPer; ++m) {
+    const int t0 = (int)(t[m] >> sh0) + d[0], t1 = ((int)(t[m] >> sh1) & m1) + d[1], t2 = ((int)t[m] & m2) + d[2];
+    const bool in = t[m] >= 0 && (uint32_t)t0 < (uint32_t)len[0] && (uint32_t)t1 < (uint32_t)len[1] &&
+                    (uint32_t)t2 < (uint32_t)len[2];
+    hit[m] = in ? __ldg(table + ((uint32_t)t0 * (uint32_t)len[1] + (uint32_t)t1) * (uint32_t)len[2] + (uint32_t)t2) : -1;
   }
-  int64_t o = boff[blockIdx.x] + before;
+  uint32_t mask[kOvPer];
+#pragma unroll
+  for (int m = 0; m < kOvPer; ++m) {
+    mask[m] = __ballot_sync(0xffffffffu, hit[m] >= 0);
+    if (lane == 0) s_cnt[m * kWarps + warp] = __popc(mask[m]);
+  }
+  __syncthreads();
+  static_assert(kOvPer * kWarps == 64, "two counts per lane below");
+  if (warp == 0) {  // exclusive scan of the 64 counts, in list order
+    const int a = s_cnt[2 * lane], b = s_cnt[2 * lane + 1];
+    int x = a + b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (!WRITE) {
+      if (lane == 31) cnt[blockIdx.x] = x;
+    } else {
+      s_cnt[2 * lane] = x - a - b;
+      s_cnt[2 * lane + 1] = x - b;
+    }
+  }
+  if (!WRITE) return;
+  __syncthreads();
+  const int64_t o = boff[blockIdx.x];
 #pragma unroll
   for (int m = 0; m < kOvPer; ++m)
     if (hit[m] >= 0) {
-      g1[o] = hit[m];
-      g2[o] = (int32_t)(k0 + m);
-      ++o;
+      const int64_t at = o + s_cnt[m * kWarps + warp] + __popc(mask[m] & ((1u << lane) - 1u));
+      g1[at] = hit[m];
+      g2[at] = (int32_t)(k0 + m * kOvThreads + (int)threadIdx.x);
     }
 }
 
@@ -583,8 +620,40 @@ void axis_tables(int nmin, int len, int n, std::vector<int32_t>& rank, std::vect
   for (size_t k = 1; k < distinct.size(); ++k) before[k] = before[k - 1] + cnt[k - 1];
 }
 
+// A's FP32 bounds and the packing of its box points.  S bounds every
+// coordinate and partial sum of a component of the distance in either
+// evaluation; FP32 rounds the corner, the three grid vectors' components and
+// five operations, 2^-24 each: 10 2^-24 S, and sqrt(3) times that plus a few
+// roundings of the square is below 2^-19 S.  Twice that, and 1e-6 for the
+// image cells' vectors against whole multiples of the grid vectors.
+void sphere_bounds(const UCell& u, SphereAtom& A) {
+  double S = 0;
+  for (int e = 0; e < 3; ++e) {
+    double b = u.origin[e] - A.g[e], s = std::fabs(u.origin[e]) + std::fabs(A.g[e]);
+    for (int d = 0; d < 3; ++d) {
+      const double n0 = A.nmin[d], n1 = A.nmin[d] + A.len[d] - 1;
+      b += n0 * u.glat[d][e];
+      s += (std::max(std::fabs(n0), std::fabs(n1)) + A.len[d]) * std::fabs(u.glat[d][e]);
+    }
+    A.b[e] = (float)b;
+    S = std::max(S, s);
+  }
+  const double margin = std::ldexp(S, -18) + 1e-6;
+  const double in = A.cut - margin, out = A.cut + margin;
+  // a squared radius beyond FP32, or not a number, leaves every point to the FP64 test
+  A.in2 = in > 1e-18 && in < 1e18 ? (float)(in * in * (1 - 1e-6)) : -1.0f;
+  A.out2 = out > 1e-18 && out < 1e18 ? (float)(out * out * (1 + 1e-6)) : INFINITY;
+  auto bits = [](int n) {
+    int k = 0;
+    while ((1 << k) < n && k < 31) ++k;
+    return k;
+  };
+  A.sh1 = bits(A.len[2]);
+  A.sh0 = A.sh1 + bits(A.len[1]);
+}
+
 struct SetupBuffers {
-  DBuf atoms, tabs, cand, atv, ijk, ratv, flags, pos, scan, offs, at, glist, clist, lut;
+  DBuf atoms, tabs, cand, atv, ratv, flags, pos, scan, offs, glist, clist, lut, box;
   DBuf pairs, bpair, bk0, bcnt, boff, g1, g2;
 };
 
@@ -641,6 +710,7 @@ lcp_status device_spheres(lcp_ctx* ctx, UCell& u, DeviceLists& d) {
     cand_off[a + 1] = cand_off[a] + vol;
     for (int d = 0; d < 3; ++d) A.g[d] = u.gxyz[a * 3 + d];
     A.cut = u.cut[a];
+    sphere_bounds(u, A);
   }
   const int64_t total = cand_off[natom];
   if (total >= ((int64_t)1 << 31)) return fail(LCP_ENOTSUP, "grid boxes too large for the device build");
@@ -648,7 +718,10 @@ lcp_status device_spheres(lcp_ctx* ctx, UCell& u, DeviceLists& d) {
   for (int d = 0; d < 3; ++d) {
     G.ng[d] = u.ngrid[d];
     G.origin[d] = u.origin[d];
-    for (int e = 0; e < 3; ++e) G.glat[d][e] = u.glat[d][e];
+    for (int e = 0; e < 3; ++e) {
+      G.glat[d][e] = u.glat[d][e];
+      G.glat32[d][e] = (float)u.glat[d][e];
+    }
   }
   G.cpy = C;
   G.ncdim = 2 * C + 1;
@@ -656,10 +729,8 @@ lcp_status device_spheres(lcp_ctx* ctx, UCell& u, DeviceLists& d) {
   API_CUDA(to_device(B.tabs, tabs, st), "H2D");
   API_CUDA(to_device(B.cand, cand_off, st), "H2D");
   API_CUDA(to_device(B.atv, u.atv, st), "H2D");
-  API_CUDA(to_device(B.ijk, u.atv_ijk, st), "H2D");
   API_CUDA(to_device(B.ratv, u.ratv, st), "H2D");
   G.atv = B.atv.as<double>();
-  G.atv_ijk = B.ijk.as<int32_t>();
   G.ratv = B.ratv.as<int32_t>();
   API_CUDA(B.flags.ensure(std::max<int64_t>(total, 1) * sizeof(int32_t)), "alloc");
   API_CUDA(B.pos.ensure((total + 1) * sizeof(int64_t)), "alloc");
@@ -684,10 +755,11 @@ lcp_status device_spheres(lcp_ctx* ctx, UCell& u, DeviceLists& d) {
   const int64_t nent = u.sphere_off[natom];
   API_CUDA(B.glist.ensure(std::max<int64_t>(nent, 1) * sizeof(int32_t)), "alloc");
   API_CUDA(B.clist.ensure(std::max<int64_t>(nent, 1) * sizeof(int32_t)), "alloc");
+  API_CUDA(B.box.ensure(std::max<int64_t>(nent, 1) * sizeof(int64_t)), "alloc");
   sphere_write_kernel<<<grid_for(total, 256), 256, 0, st>>>(G, dA, dC, natom, B.tabs.as<int32_t>(),
                                                               B.flags.as<int32_t>(), B.pos.as<int64_t>(),
                                                               B.glist.as<int32_t>(), B.clist.as<int32_t>(),
-                                                              B.lut.as<int32_t>());
+                                                              B.lut.as<int32_t>(), B.box.as<int64_t>());
   API_CUDA(cudaGetLastError(), "sphere write");
   ctx->launches += 6;
   API_CUDA(cudaStreamSynchronize(st), "sphere lists");  // before the host tables above go
@@ -729,7 +801,7 @@ lcp_status device_overlaps(lcp_ctx* ctx, UCell& u, DeviceLists& d, DBuf* g1, DBu
   if (nblk > 0) {
     overlap_kernel<false><<<(unsigned)nblk, kOvThreads, 0, st>>>(
         G, dA, B.pairs.as<OvPair>(), B.bpair.as<int32_t>(), B.bk0.as<int64_t>(), B.offs.as<int64_t>(),
-        B.glist.as<int32_t>(), B.clist.as<int32_t>(), B.lut.as<int32_t>(), B.bcnt.as<int32_t>(), nullptr, nullptr,
+        B.box.as<int64_t>(), B.lut.as<int32_t>(), B.bcnt.as<int32_t>(), nullptr, nullptr,
         nullptr);
     API_CUDA(cudaGetLastError(), "overlap count");
   }
@@ -745,7 +817,7 @@ lcp_status device_overlaps(lcp_ctx* ctx, UCell& u, DeviceLists& d, DBuf* g1, DBu
   if (nblk > 0) {
     overlap_kernel<true><<<(unsigned)nblk, kOvThreads, 0, st>>>(
         G, dA, B.pairs.as<OvPair>(), B.bpair.as<int32_t>(), B.bk0.as<int64_t>(), B.offs.as<int64_t>(),
-        B.glist.as<int32_t>(), B.clist.as<int32_t>(), B.lut.as<int32_t>(), nullptr, B.boff.as<int64_t>(),
+        B.box.as<int64_t>(), B.lut.as<int32_t>(), nullptr, B.boff.as<int64_t>(),
         g1->as<int32_t>(), g2->as<int32_t>());
     API_CUDA(cudaGetLastError(), "overlap write");
   }

@@ -196,11 +196,66 @@ static lcp_status make_lens(lcp_ctx* ctx, lcp_orbs* o) {
 
 // Brick tiling, split-BF16 orbital tables and the ordered pair list of the
 // tensor-core path, built once per tabulation.
+// Blocks of 16 rows that the bricks' rows fill when they are packed: the
+// orbitals of the images' 16-orbital chunks (widths), end to end.
+static std::vector<int64_t> packed_blocks(const lcp::UCell& u, const lcp::Bricks& b, std::vector<uint8_t>& width) {
+  width.resize(b.nblocks);
+  for (int64_t blk = 0; blk < b.nblocks;) {
+    const int no = u.numorbs[b.block_atom[blk]];
+    for (int c = 0; c * 16 < no; ++c) width[blk++] = (uint8_t)std::min(16, no - 16 * c);
+  }
+  std::vector<int64_t> off(b.nbricks + 1, 0);
+  for (int64_t k = 0; k < b.nbricks; ++k) {
+    int64_t rows = 0;
+    for (int64_t i = b.img_off[k]; i < b.img_off[k + 1]; ++i) rows += width[i];
+    off[k + 1] = off[k] + (rows + 15) / 16;
+  }
+  return off;
+}
+
+// The rows that the matrix elements read.  Chunks of 13, 9, 4 or 2 orbitals in
+// blocks of 16 leave rows empty on both sides of the product, so the rows are
+// packed into a second table where that saves a sixteenth of the blocks or
+// more (13-orbital atoms: 0.66 of the products; 18: 0.32), and the images'
+// own blocks serve otherwise, or when there is no room for it.  (The density
+// takes an image's chunk as one K step and keeps the images' blocks.)
+static lcp_status pack_rows(lcp_ctx* ctx, lcp_orbs* o) {
+  const lcp::Bricks& b = o->bricks;
+  lcp::TcBrickGeom& g = o->bgeom;
+  std::vector<uint8_t> width;
+  std::vector<int64_t> off = packed_blocks(o->ucell->u, b, width);
+  bool packed = off.back() * 16 <= b.nblocks * 15;
+  if (packed) {
+    const cudaError_t e = o->b_ptab.ensure((size_t)std::max<int64_t>(off.back(), 1) * 6144 * 2);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      packed = false;
+    } else {
+      API_CUDA(e, "packed table alloc");
+    }
+  }
+  if (!packed) off = b.img_off;
+  DBuf d_width;
+  API_CUDA(upload(d_width, width, ctx->stream), "upload");
+  API_CUDA(upload(o->b_pkoff, off, ctx->stream), "upload");
+  API_CUDA(o->b_pkrow.ensure((size_t)std::max<int64_t>(off.back(), 1) * 16 * sizeof(uint32_t)), "row list alloc");
+  g.npk = off.back();
+  g.pk_off = o->b_pkoff.as<int64_t>();
+  g.pk_row = o->b_pkrow.as<uint32_t>();
+  g.ptab = packed ? o->b_ptab.as<__nv_bfloat16>() : o->b_tab.as<__nv_bfloat16>();
+  API_CUDA(lcp::launch_brick_pack(g, d_width.as<uint8_t>(), packed, o->b_pkrow.as<uint32_t>(),
+                                  o->b_tab.as<__nv_bfloat16>(), o->b_ptab.as<__nv_bfloat16>(), ctx->stream),
+           "packed table");
+  API_CUDA(cudaStreamSynchronize(ctx->stream), "packed table");  // before the widths go
+  ctx->launches += packed ? 2 : 1;
+  return LCP_OK;
+}
+
 lcp_status ensure_bricks(lcp_ctx* ctx, lcp_orbs* o) {
   if (o->bricks_ready) return LCP_OK;
   if (o->phi_released) return fail(LCP_ESTATE, "the FP64 orbital tables were released");
-  const lcp_status ls = ucell_host_lists(o->ucell);
-  if (ls) return ls;
+  lcp_status s = ucell_host_lists(o->ucell);
+  if (s) return s;
   const lcp::UCell& u = o->ucell->u;
   lcp::Bricks& b = o->bricks;
   std::string err = lcp::build_bricks(u, b, o->brick_shape[0] > 0 ? o->brick_shape : nullptr);
@@ -275,6 +330,7 @@ lcp_status ensure_bricks(lcp_ctx* ctx, lcp_orbs* o) {
   g.img_block = o->b_imgblk.as<int32_t>();
   g.tab_off = o->b_taboff.as<int64_t>();
   g.tab_pair = o->b_tabpair.as<int32_t>();
+  if ((s = pack_rows(ctx, o))) return s;
   API_CUDA(cudaStreamSynchronize(st), "bricks");
   o->bricks_ready = true;
   return LCP_OK;
@@ -285,6 +341,7 @@ void drop_bricks(lcp_orbs* o) {
   o->bricks_ready = false;
   o->bricks = lcp::Bricks();
   for (DBuf* d : {&o->b_code, &o->b_imgoff, &o->b_imgblk, &o->b_taboff, &o->b_tabpair, &o->b_tab, &o->b_tabslot,
+                  &o->b_ptab, &o->b_pkoff, &o->b_pkrow,
                   &o->b_slotbase, &o->b_redoff, &o->b_redslot, &o->b_subpair, &o->b_subchunks, &o->b_sbfold,
                   &o->b_sbchunks})
     d->release();
@@ -1893,7 +1950,8 @@ lcp_status lcp_job_footprint(const lcp_job* job, int64_t* bytes) {
                         &o->species, &o->radial, &o->phi, &o->dphi[0], &o->dphi[1], &o->dphi[2], &o->phi32,
                         &o->p_atom, &o->p_jatom, &o->p_boffp, &o->p_boffq, &o->p_self, &o->p_lensoff, &o->p_g1,
                         &o->p_g2, &o->it_pair, &o->it_start, &o->it_count, &o->f_off, &o->f_code, &o->b_code, &o->b_imgoff, &o->b_imgblk,
-                        &o->b_taboff, &o->b_tabpair, &o->b_tab, &o->b_tabslot, &o->b_slotbase, &o->b_redoff,
+                        &o->b_taboff, &o->b_tabpair, &o->b_tab, &o->b_tabslot, &o->b_slotbase, &o->b_redoff, &o->b_ptab,
+                        &o->b_pkoff, &o->b_pkrow,
                         &o->b_redslot, &o->b_subpair, &o->b_subchunks, &o->b_sbfold, &o->b_sbchunks, &o->o_atom,
                         &o->o_jatom, &o->o_boff, &o->o_partner, &o->b_scale, &o->b_tmp})
     add(*d);
@@ -1919,6 +1977,10 @@ int64_t job_footprint_estimate(lcp_job* job, int32_t precision) {
   if (precision == LCP_PREC_BF16X3 && !o->bricks_ready) {
     lcp::Bricks b;
     if (ucell_host_lists(o->ucell) != LCP_OK || !lcp::build_bricks(o->ucell->u, b, o->brick_shape[0] > 0 ? o->brick_shape : nullptr).empty()) return -1;
+    std::vector<uint8_t> width;
+    const int64_t npk = packed_blocks(o->ucell->u, b, width).back();
+    const bool packed = npk * 16 <= b.nblocks * 15;
+    fp += (packed ? npk * (6144 * 2 + 64) : b.nblocks * 64) + (b.nbricks + 1) * 8;
     fp += b.nblocks * 6144 * 2 + (int64_t)b.point_code.size() * 4 + (int64_t)b.tab_pair.size() * 8 +
           (int64_t)(b.img_off.size() + b.slot_base.size() + b.red_off.size() + b.red_slot.size()) * 8 +
           (int64_t)(b.img_block.size() + b.sub_pair.size() + b.sub_chunks.size() + b.sb_fold.size() +

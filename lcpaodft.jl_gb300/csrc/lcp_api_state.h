@@ -183,6 +183,7 @@ struct lcp_orbs {
   lcp::Bricks bricks;
   lcp::TcBrickGeom bgeom{};
   DBuf b_code, b_imgoff, b_imgblk, b_taboff, b_tabpair, b_tab, b_tabslot, b_slotbase, b_redoff, b_redslot;
+  DBuf b_ptab, b_pkoff, b_pkrow;  // packed rows (TcBrickGeom)
   DBuf b_subpair, b_subchunks, b_sbfold, b_sbchunks;  // sub-pairs and H sub-blocks (orbital chunks)
   DBuf o_atom, o_jatom, o_boff, o_partner;  // ordered pair list
   DBuf b_scale, b_tmp;                       // fixed-point scale of the tables: [S_phi, 1/S_phi]

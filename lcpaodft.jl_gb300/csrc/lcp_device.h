@@ -243,7 +243,15 @@ struct TcBrickGeom {
   const int32_t* img_block;
   const int64_t* tab_off;
   const int32_t* tab_pair;
+  // the tables' rows for the matrix elements: brick hb's blocks of 16 rows are
+  // pk_off[hb] .. pk_off[hb+1]-1 (pk_row: image << 16 | its orbitals << 8 | orbital of
+  // each, kNoRow: empty)
+  int64_t npk;
+  const __nv_bfloat16* ptab;
+  const int64_t* pk_off;
+  const uint32_t* pk_row;
 };
+constexpr uint32_t kNoRow = 0xffffffffu;
 // One cell of a tensor-core launch: its brick tiling and tables, and where the
 // step reads and writes.  A batch launch covers the bricks of several cells.
 struct TcCell {
@@ -256,6 +264,10 @@ struct TcCell {
   const int32_t* tab_pair;     // sub-pair tables (density)
   const int32_t* tab_slot;     // slot tables (matrix elements)
   const int64_t* slot_base;    // [nbricks+1]
+  int64_t npk;                 // matrix elements: the rows' blocks (TcBrickGeom)
+  const __nv_bfloat16* ptab;
+  const int64_t* pk_off;
+  const uint32_t* pk_row;
   double phi_scale;            // S_phi of the tables
   const __nv_bfloat16* dsym;   // density: split D blocks, zero block at zero_pair
   int64_t zero_pair;
@@ -331,6 +343,10 @@ cudaError_t launch_brick_table(const double* phi, const int64_t* phi_off, const 
                                const int32_t* block_atom, const int32_t* first_block, int64_t nimg,
                                int32_t* slot_point, const double* scale, __nv_bfloat16* tab, int64_t nblocks,
                                cudaStream_t st);
+// The row lists of bg's blocks of 16 rows, from the images' orbital counts (width): end to
+// end, or each image's in a block of its own; and, packed, the rows' table from the images' blocks.
+cudaError_t launch_brick_pack(const TcBrickGeom& bg, const uint8_t* width, bool packed, uint32_t* row,
+                              const __nv_bfloat16* tab, __nv_bfloat16* ptab, cudaStream_t st);
 cudaError_t launch_dsym(int64_t nsub, const int32_t* sub_pair, const int32_t* sub_chunks, const int32_t* pair_atom,
                         const int32_t* pair_jatom, const int64_t* boff, const int32_t* partner, const int32_t* numorbs,
                         const double* dm, const double* scale, __nv_bfloat16* out, cudaStream_t st);

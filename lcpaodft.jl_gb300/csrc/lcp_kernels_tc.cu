@@ -153,6 +153,46 @@ __device__ __forceinline__ void fx_split_f(float p, float e, __nv_bfloat16& hi, 
   lo = __float2bfloat16_rn(l);
 }
 
+// Two floats per register pair (add.f32x2 and its like: each half as the scalar
+// operation rounds it, in one issue slot).
+typedef unsigned long long float_pair;
+__device__ __forceinline__ float_pair pair_of(float a, float b) {
+  float_pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float_pair pair_of(uint32_t a, uint32_t b) { return pair_of(__uint_as_float(a), __uint_as_float(b)); }
+__device__ __forceinline__ float_pair add2(float_pair a, float_pair b) {
+  float_pair r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float_pair mul2(float_pair a, float_pair b) {
+  float_pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float_pair fma2(float_pair a, float_pair b, float_pair c) {
+  float_pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// BF16s of two floats that are exact in BF16: their upper halves.
+__device__ __forceinline__ uint32_t bf16_pair(float_pair x) { return __byte_perm((uint32_t)x, (uint32_t)(x >> 32), 0x7632); }
+// fx_split_f of two values.
+__device__ __forceinline__ void fx_split_f2(float_pair p, float_pair e, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  constexpr float C8 = 49152.0f, C17 = 96.0f, C26 = 0.1875f;
+  const float_pair m1 = pair_of(-1.0f, -1.0f);
+  const float_pair h = add2(add2(p, pair_of(C8, C8)), pair_of(-C8, -C8));
+  const float_pair r1 = add2(fma2(h, m1, p), e);
+  const float_pair m = add2(add2(r1, pair_of(C17, C17)), pair_of(-C17, -C17));
+  const float_pair r2 = fma2(m, m1, r1);
+  const float_pair l = add2(add2(r2, pair_of(C26, C26)), pair_of(-C26, -C26));
+  hi = bf16_pair(h);
+  mid = bf16_pair(m);
+  lo = bf16_pair(l);
+}
+
 // +-q * p as a BF16, for |q| <= 256 and p a power of two, with the sign of
 // q flipped when sv is 1: |q| becomes an FP32 by the 2^23 magic add and the
 // product is exact with at most eight significant bits, so its BF16 is the
@@ -362,6 +402,66 @@ __global__ void __launch_bounds__(256) brick_table_kernel(const double* __restri
       const int64_t off = (b0 + c) * kPart + (int64_t)((h * 16 + g) * 64 + r * 8);
 #pragma unroll
       for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(tab + q * nblocks * kPart + off) = part[q];
+    }
+  }
+}
+
+// pk_row, one warp per brick: the images' rows from the running sum of their widths.
+__global__ void __launch_bounds__(256) brick_rows_kernel(const __grid_constant__ TcBrickGeom bg,
+                                                         const uint8_t* __restrict__ width, int packed,
+                                                         uint32_t* __restrict__ row) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t hb = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; hb < bg.nbricks; hb += nw) {
+    const int64_t i0 = bg.img_off[hb];
+    const int m = (int)(bg.img_off[hb + 1] - i0);
+    uint32_t* out = row + bg.pk_off[hb] * 16;
+    int done = 0;
+    for (int k = 0; k < m; k += 32) {
+      const int i = k + lane, w = i < m ? width[i0 + i] : 0, step = packed ? w : (i < m ? 16 : 0);
+      int x = step;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      for (int a = 0; a < step; ++a)
+        out[done + x - step + a] = a < w ? (uint32_t)(i << 16 | w << 8 | a) : kNoRow;
+      done += __shfl_sync(0xffffffffu, x, 31);
+    }
+    const int end = (int)(bg.pk_off[hb + 1] - bg.pk_off[hb]) * 16;
+    if (done + lane < end) out[done + lane] = kNoRow;  // at most 15
+  }
+}
+
+// The same parts of the rows of pk_row: per block of 16 rows the layout of an
+// image's block, thread (h, g, r) gathering its eight rows at one point.
+__global__ void __launch_bounds__(256) brick_pack_kernel(const __grid_constant__ TcBrickGeom bg,
+                                                         const __nv_bfloat16* __restrict__ tab,
+                                                         __nv_bfloat16* __restrict__ ptab) {
+  const int t = threadIdx.x, h = t >> 7, pt = ((t >> 3) & 15) * 64 + (t & 7) * 8;
+  const uint16_t* src = reinterpret_cast<const uint16_t*>(tab);
+  for (int64_t hb = blockIdx.x; hb < bg.nbricks; hb += gridDim.x) {
+    const int64_t i0 = bg.img_off[hb];
+    for (int64_t b = bg.pk_off[hb]; b < bg.pk_off[hb + 1]; ++b) {
+      union {
+        uint16_t e[8];
+        uint4 v;
+      } part[3];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t row = bg.pk_row[b * 16 + h * 8 + k], a = row & 15;
+        const bool on = row != kNoRow;
+        const int64_t at = on ? (i0 + (row >> 16)) * kPart + (a >> 3) * 1024 + pt + (a & 7) : 0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const uint16_t x = __ldg(src + q * bg.nblocks * kPart + at);
+          part[q].e[k] = on ? x : (uint16_t)0;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        *reinterpret_cast<uint4*>(ptab + (q * bg.npk + b) * kPart + h * 1024 + pt) = part[q].v;
     }
   }
 }
@@ -804,23 +904,31 @@ __global__ void __launch_bounds__(192 + 32 * kDGatherWarps, 1) density_tc_kernel
 //
 //   G_st[a][b] = sum_{p in brick} phi_s(p)_a V(p) phi_t(p)_b
 //
-// (src/Hamiltonian.jl:384-429 restricted to the brick).  M = 128 rows are the
-// orbitals of 8 images s (the brick tables as stored), N the orbitals of a
-// window of up to 4 images t (V-weighted in shared memory with a per-brick
-// scale of V), K the brick's 128 point slots.  Both operands are
-// MN-major: the table block [h][g][8 pt][8 orb] is that layout with
-// LBO = 128 B (point groups) and SBO = 2048 B (orbital halves; images 4096 B
-// apart).  Partial blocks go to a scratch array (FP32); h_reduce_kernel sums
-// them per folded pair in a fixed order and writes both orientations of H --
-// no atomics.
+// (src/Hamiltonian.jl:384-429 restricted to the brick).  The brick's rows, its
+// images' orbitals, come in blocks of 16 (pk_row): packed end to end, or an
+// image's chunk to a block.  M = 128 rows are eight blocks, N the rows of a
+// window of up to four (V-weighted in shared memory with a per-brick scale of
+// V), K the brick's 128 point slots.  Both operands are MN-major: the table
+// block [h][g][8 pt][8 orb] is that layout with LBO = 128 B (point groups) and
+// SBO = 2048 B (row halves; blocks 4096 B apart).  Partial blocks go to a
+// scratch array (FP32), [orbital of t][orbital of s] without gaps, so that the
+// lanes of the epilogue, rows of s, write consecutive words; h_reduce_kernel
+// sums them per folded pair in a fixed order and writes both orientations of H
+// -- no atomics.
+//
+// Packed, the 13-orbital cells take 0.66 of the products and the 13/18-orbital
+// one half; the epilogue and the V-weighting, which had time to spare, then set
+// the pace.  Two warps per TMEM quarter, the window's lists loaded ahead and
+// packed FP32 pairs in both brought the 64-atom Si cell's kernel from 0.57 to
+// 0.45 ms and the 108-atom 18/13-orbital one from 1.51 to 1.02 ms (a channel).
 // ==========================================================================
 
-// Roles (448 threads, one CTA per SM, persistent over bricks).  A tile is
-// (brick, s-group of kHGroup images, t-window of kHWin images t >= the
-// group's first image); V weights the t side:
-//   warp 0     producer: per s-group the plain tables of its images into the
-//              A region (after a_free) -- one bulk copy per part, the images
-//              of a brick being consecutive blocks;
+// Roles (576 threads, one CTA per SM, persistent over bricks).  A tile is
+// (brick, group of kHGroup blocks of rows, window of kHWin blocks from the
+// group's first on); V weights the window's side:
+//   warp 0     producer: per group the plain tables of its blocks into the
+//              A region (after a_free) -- one bulk copy per part, the blocks
+//              of a brick being consecutive;
 //   warps 6-13 per tile the raw t window from the tables into registers,
 //              then (after b_empty) its V-weighted fixed-point split into one
 //              of kHStages B stages (b_ready), with the brick's V / S_V
@@ -828,19 +936,21 @@ __global__ void __launch_bounds__(192 + 32 * kDGatherWarps, 1) density_tc_kernel
 //   warp 1     MMA issuer: 8 K steps x 4 MMAs per tile into one of two TMEM
 //              tile buffers (4 accumulators x 64 columns each); after the
 //              group's last tile it commits a_free;
-//   warps 2-5  epilogue: per tile the FP32 partial blocks, TMEM read four
-//              loads per wait, then the buffer is freed.
+//   warps 2-5, 14-17  epilogue: per tile the FP32 partial blocks, two warps
+//              to a quarter of the TMEM lanes taking every other image of the
+//              window, then the buffer is freed.
 // Every wait is bounded; a timeout sets *status and stops all roles.
-constexpr int kHGroup = 8;                 // s images per M tile (M = 128)
-constexpr int kHWin = 4;                   // t images per N tile (N <= 64)
+constexpr int kHGroup = 8;                 // blocks of rows per M tile (M = 128)
+constexpr int kHWin = 4;                   // blocks per window (N <= 64)
 constexpr int kHStages = 2;
 constexpr int kHXformWarps = 8;            // warps V-weighting the B stages
 constexpr int kImgBytes = 4096;            // one part of an image block
 constexpr int kHABytes = kHGroup * kImgBytes;   // one part of the A operand
 constexpr int kHBBytes = kHWin * kImgBytes;     // one part of a B stage
 constexpr size_t kHSmem = 3 * (size_t)kHABytes + (size_t)kHStages * 3 * kHBBytes;  // 192 KB
+constexpr int kHEpiWarps = 8;  // two per TMEM quarter
 // TMEM: two tile buffers of 256 columns; inside one, the four accumulators
-// (W = 16 x the tile's t images columns each, at most 64), one per quantum
+// (W = 16 x the window's blocks columns each, at most 64), one per quantum
 // of the products: hi*hi (2^-16), hi*mid + mid*hi (2^-25),
 // hi*lo + lo*hi + mid*mid (2^-34), mid*lo + lo*mid (2^-43).  Over the 128
 // points of a brick the first two sums stay within 2^24 of their quanta (128
@@ -895,7 +1005,15 @@ __global__ void __launch_bounds__(128) vweight_kernel(const __grid_constant__ Tc
   }
 }
 
-__global__ void __launch_bounds__(192 + 32 * kHXformWarps, 1) hamiltonian_tc_kernel(const __grid_constant__ TcHamArgs args) {
+// First block of the windows of the group from block s0 on: one earlier when
+// the group's first row is not its image's first, for the elements between the
+// image's rows in the group and those before it.
+__device__ __forceinline__ int first_window(const TcCell& cl, int64_t i0, int s0) {
+  return s0 > 0 && (cl.pk_row[(i0 + s0) * 16] & 15) != 0 ? s0 - 1 : s0;
+}
+
+constexpr int kHThreads = 64 + 32 * (kHEpiWarps + kHXformWarps);
+__global__ void __launch_bounds__(kHThreads, 1) hamiltonian_tc_kernel(const __grid_constant__ TcHamArgs args) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t bready_bar[kHStages], bempty_bar[kHStages], tfull_bar[2], tempty_bar[2];
   __shared__ uint64_t afull_bar, afree_bar, drain_bar;
@@ -912,7 +1030,7 @@ __global__ void __launch_bounds__(192 + 32 * kHXformWarps, 1) hamiltonian_tc_ker
     }
     for (int b = 0; b < 2; ++b) {
       tc::mbar_init(&tfull_bar[b], 1);
-      tc::mbar_init(&tempty_bar[b], 4);
+      tc::mbar_init(&tempty_bar[b], kHEpiWarps);
     }
     tc::mbar_init(&afull_bar, 1);
     tc::mbar_init(&afree_bar, 1);
@@ -941,8 +1059,8 @@ __global__ void __launch_bounds__(192 + 32 * kHXformWarps, 1) hamiltonian_tc_ker
       if (k < 0) continue;
       int64_t hb;
       const TcCell& cl = *tc_cell(&args.cell0, args.batch, k, hb);
-      const int64_t i0 = cl.img_off[hb];
-      const int m = (int)(cl.img_off[hb + 1] - i0);
+      const int64_t i0 = cl.pk_off[hb];
+      const int m = (int)(cl.pk_off[hb + 1] - i0);
       for (int s0 = 0; s0 < m && !abort_flag; s0 += kHGroup, ++grp) {
         // the refill waits for the previous group's MMAs
         if (grp > 0 && !tc::mbar_wait_abortable(&afree_bar, (grp - 1) & 1, &abort_flag)) {
@@ -953,9 +1071,9 @@ __global__ void __launch_bounds__(192 + 32 * kHXformWarps, 1) hamiltonian_tc_ker
         if (lane == 0) {
           tc::mbar_arrive_expect_tx(&afull_bar, na * 3 * kImgBytes);
           // check build: a group outside the tables is replaced by blocks 0.. (same bytes)
-          const int64_t blk = bounds_ok(i0 + s0 + na - 1, cl.nblocks, 11) ? i0 + s0 : 0;
+          const int64_t blk = bounds_ok(i0 + s0 + na - 1, cl.npk, 11) ? i0 + s0 : 0;
           for (int part = 0; part < 3; ++part)
-            tc::bulk_g2s(sA + part * kHABytes, cl.tab + ((int64_t)part * cl.nblocks + blk) * kPart,
+            tc::bulk_g2s(sA + part * kHABytes, cl.ptab + ((int64_t)part * cl.npk + blk) * kPart,
                          na * kImgBytes, &afull_bar);
         }
         __syncwarp();
@@ -970,14 +1088,14 @@ __global__ void __launch_bounds__(192 + 32 * kHXformWarps, 1) hamiltonian_tc_ker
       if (k < 0) continue;
       int64_t hb;
       const TcCell& cl = *tc_cell(&args.cell0, args.batch, k, hb);
-      const int64_t i0 = cl.img_off[hb];
-      const int m = (int)(cl.img_off[hb + 1] - i0);
+      const int64_t i0 = cl.pk_off[hb];
+      const int m = (int)(cl.pk_off[hb + 1] - i0);
       for (int s0 = 0; s0 < m && !abort_flag; s0 += kHGroup, ++grp) {
         if (!tc::mbar_wait_warp(&afull_bar, grp & 1, &abort_flag)) {
           give_up();
           break;
         }
-        for (int t0 = s0; t0 < m; t0 += kHWin, ++it) {
+        for (int t0 = first_window(cl, i0, s0); t0 < m; t0 += kHWin, ++it) {
           const int stage = (int)(it % kHStages);
           const uint32_t buf = it & 1, tuse = it >> 1;
           if (tuse > 0 && !tc::mbar_wait_warp(&tempty_bar[buf], (tuse - 1) & 1, &abort_flag)) {
@@ -1043,7 +1161,7 @@ __global__ void __launch_bounds__(192 + 32 * kHXformWarps, 1) hamiltonian_tc_ker
       if (!tc::mbar_wait(&drain_bar, 0, 1u << 24)) give_up();
     }
     __syncwarp();
-  } else if (warp >= 6) {
+  } else if (warp >= 6 && warp < 6 + kHXformWarps) {
     // ------------------------------------------------------------ B tiles: load and V-weight
     // Each thread owns chunk q = tt of every image of a tile: 8 orbitals of
     // one point slot, all three parts.  It loads the tile's raw parts from
@@ -1061,15 +1179,15 @@ __global__ void __launch_bounds__(192 + 32 * kHXformWarps, 1) hamiltonian_tc_ker
       if (k < 0) continue;
       int64_t hb;
       const TcCell& cl = *tc_cell(&args.cell0, args.batch, k, hb);
-      const int64_t i0 = cl.img_off[hb];
-      const int m = (int)(cl.img_off[hb + 1] - i0);
+      const int64_t i0 = cl.pk_off[hb];
+      const int m = (int)(cl.pk_off[hb + 1] - i0);
       if (m == 0) continue;
       const float2 w = cl.vw[hb * 128 + pt];
-      const float vh = w.x, vl = w.y;
-      const uint4* tab4 = reinterpret_cast<const uint4*>(cl.tab) + tt;  // 16-byte chunk tt of block 0, part 0
-      const int64_t pstride = cl.nblocks * (kPart / 8);                 // one part, in 16-byte chunks
+      const float_pair vh2 = pair_of(w.x, w.x), nvh2 = pair_of(-w.x, -w.x), vl2 = pair_of(w.y, w.y);
+      const uint4* tab4 = reinterpret_cast<const uint4*>(cl.ptab) + tt;  // 16-byte chunk tt of block 0, part 0
+      const int64_t pstride = cl.npk * (kPart / 8);                 // one part, in 16-byte chunks
       for (int s0 = 0; s0 < m && !abort_flag; s0 += kHGroup) {
-        for (int t0 = s0; t0 < m && !abort_flag; t0 += kHWin, ++it) {
+        for (int t0 = first_window(cl, i0, s0); t0 < m && !abort_flag; t0 += kHWin, ++it) {
           const int nt = min(kHWin, m - t0);
           const int stage = (int)(it % kHStages);
           const uint32_t use = it / kHStages;
@@ -1091,24 +1209,20 @@ __global__ void __launch_bounds__(192 + 32 * kHXformWarps, 1) hamiltonian_tc_ker
 #pragma unroll
           for (int j = 0; j < kHWin; ++j) {
             if (j < nt) {
-              const __nv_bfloat16* xb_h = reinterpret_cast<const __nv_bfloat16*>(&raw[j][0]);
-              const __nv_bfloat16* xb_m = reinterpret_cast<const __nv_bfloat16*>(&raw[j][1]);
-              const __nv_bfloat16* xb_l = reinterpret_cast<const __nv_bfloat16*>(&raw[j][2]);
-              uint4 oh, om, ol;
-              __nv_bfloat16* xh = reinterpret_cast<__nv_bfloat16*>(&oh);
-              __nv_bfloat16* xm = reinterpret_cast<__nv_bfloat16*>(&om);
-              __nv_bfloat16* xl = reinterpret_cast<__nv_bfloat16*>(&ol);
+              uint32_t oh[4], om[4], ol[4];
+              const uint32_t* xh = reinterpret_cast<const uint32_t*>(&raw[j][0]);
+              const uint32_t* xm = reinterpret_cast<const uint32_t*>(&raw[j][1]);
+              const uint32_t* xl = reinterpret_cast<const uint32_t*>(&raw[j][2]);
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const float u = (__bfloat162float(xb_h[e]) + __bfloat162float(xb_m[e])) + __bfloat162float(xb_l[e]);
+              for (int e = 0; e < 4; ++e) {  // two orbitals at a time
+                auto two = [](uint32_t x) { return pair_of(x << 16, x & 0xffff0000u); };
+                const float_pair u = add2(add2(two(xh[e]), two(xm[e])), two(xl[e]));
                 // u * (vh + vl) = pr + er exactly up to u*vl's rounding (~2^-48)
-                const float pr = u * vh;
-                const float er = fmaf(u, vh, -pr) + u * vl;
-                fx_split_f(pr, er, xh[e], xm[e], xl[e]);
+                fx_split_f2(mul2(u, vh2), fma2(u, vl2, fma2(u, vh2, mul2(u, nvh2))), oh[e], om[e], ol[e]);
               }
-              *reinterpret_cast<uint4*>(sB + j * kImgBytes) = oh;
-              *reinterpret_cast<uint4*>(sB + pbytes + j * kImgBytes) = om;
-              *reinterpret_cast<uint4*>(sB + 2 * pbytes + j * kImgBytes) = ol;
+              *reinterpret_cast<uint4*>(sB + j * kImgBytes) = make_uint4(oh[0], oh[1], oh[2], oh[3]);
+              *reinterpret_cast<uint4*>(sB + pbytes + j * kImgBytes) = make_uint4(om[0], om[1], om[2], om[3]);
+              *reinterpret_cast<uint4*>(sB + 2 * pbytes + j * kImgBytes) = make_uint4(ol[0], ol[1], ol[2], ol[3]);
             }
           }
           tc::fence_proxy_async_smem();
@@ -1117,61 +1231,118 @@ __global__ void __launch_bounds__(192 + 32 * kHXformWarps, 1) hamiltonian_tc_ker
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2-5)
+    // ------------------------------------------------------------ epilogue (warps 2-5 and 14-17)
     const uint32_t quarter = warp & 3;
-    const int row = (int)quarter * 32 + lane;  // TMEM lane = M row = (s image, orbital)
+    const int row = (int)quarter * 32 + lane;  // TMEM lane = M row
+    const int half = warp < 6 ? 0 : 1;  // takes the even or the odd images of a window
     uint32_t it = 0;
     for (int64_t j = 0; j * gridDim.x < ntotal && !abort_flag; ++j) {
       const int64_t k = round_brick(j, ntotal);
       if (k < 0) continue;
       int64_t hb;
       const TcCell& cl = *tc_cell(&args.cell0, args.batch, k, hb);
-      const int64_t i0 = cl.img_off[hb];
-      const int m = (int)(cl.img_off[hb + 1] - i0);
+      const int64_t i0 = cl.pk_off[hb];
+      const int m = (int)(cl.pk_off[hb + 1] - i0);
       if (m == 0) continue;
-      const int64_t tb = cl.tab_off[hb];
+      const int mi = (int)(cl.img_off[hb + 1] - cl.img_off[hb]);  // images: the slot table's side
+      const uint32_t* rows = cl.pk_row + i0 * 16;
+      const int32_t* slots = cl.tab_slot + cl.tab_off[hb];
       const int64_t sbase = cl.slot_base[hb];
+      const int64_t nslots = cl.slot_base[cl.nbricks] - sbase;
+      float* out = cl.scratch + sbase * 256;
       const float out_scale = cl.vscale[hb];  // S_V * S_phi^2, a power of two
       for (int s0 = 0; s0 < m && !abort_flag; s0 += kHGroup) {
-        const int s = s0 + (row >> 4), a = row & 15;
-        for (int t0 = s0; t0 < m && !abort_flag; t0 += kHWin, ++it) {
-          const int nt = min(kHWin, m - t0);
-          const uint32_t W = 16u * (uint32_t)nt;  // accumulator k at columns kW of the buffer
-          const uint32_t buf = it & 1;
-          int slot[kHWin];
+        const uint32_t er = s0 * 16 + row < m * 16 ? rows[s0 * 16 + row] : kNoRow;
+        const int s = (int)(er >> 16), a = (int)(er & 255u), ws = (int)((er >> 8) & 255u);
+        // A window's columns, on the lanes; their images are consecutive, every
+        // other one this warp's.  Columns are loaded two windows ahead and the
+        // partial blocks of (s, image) one ahead: both in turn at the window
+        // itself took longer than its products.
+        struct Columns {
+          uint32_t e0, e1;
+        };
+        auto columns = [&](int t0) {
+          const int n = (m - t0) * 16;
+          return Columns{lane < n ? __ldg(rows + t0 * 16 + lane) : kNoRow,
+                         32 + lane < n ? __ldg(rows + t0 * 16 + 32 + lane) : kNoRow};
+        };
+        auto first = [&](const Columns& c) { return (int)(__shfl_sync(0xffffffffu, c.e0, 0) >> 16) + half; };
+        auto slot_of = [&](int t) { return er != kNoRow && s <= t && t < mi ? __ldg(slots + s * mi + t) : -1; };
+        const int tf = first_window(cl, i0, s0);
+        Columns cur = columns(tf), next = columns(tf + kHWin);
+        int32_t o[4], on[4];
+        {
+          const int t1 = first(cur);
 #pragma unroll
-          for (int j = 0; j < kHWin; ++j)
-            slot[j] = (j < nt && s < m && s <= t0 + j) ? cl.tab_slot[tb + s * m + t0 + j] : -1;
-          if (!tc::mbar_wait_abortable(&tfull_bar[buf], (it >> 1) & 1, &abort_flag)) {
+          for (int k = 0; k < 4; ++k) o[k] = slot_of(t1 + 2 * k);
+        }
+        for (int t0 = tf; t0 < m && !abort_flag; t0 += kHWin, ++it) {
+          const int nt = min(kHWin, m - t0);
+          const int W = 16 * nt;  // accumulator k at columns kW of the buffer
+          const uint32_t buf = it & 1;
+          const Columns after = columns(t0 + 2 * kHWin);
+          if (t0 + kHWin < m) {
+            const int t1 = first(next);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) on[k] = slot_of(t1 + 2 * k);
+          }
+          if (!tc::mbar_wait_warp(&tfull_bar[buf], (it >> 1) & 1, &abort_flag)) {
             give_up();
             break;
           }
           tc::fence_after_sync();
+          auto image = [&](int t, int slot) {
+            // its columns c0 .. c1 - 1 of the window, from its orbital b0 on
+            const uint32_t in0 = __ballot_sync(0xffffffffu, (cur.e0 >> 16) == (uint32_t)t),
+                           in1 = __ballot_sync(0xffffffffu, (cur.e1 >> 16) == (uint32_t)t);
+            if (!(in0 | in1)) return false;  // past the window
+            if (!__any_sync(0xffffffffu, slot >= 0)) return true;
+            const int c0 = in0 ? __ffs(in0) - 1 : 31 + __ffs(in1), c1 = c0 + __popc(in0) + __popc(in1);
+            const int b0 = (int)(__shfl_sync(0xffffffffu, c0 < 32 ? cur.e0 : cur.e1, c0 & 31) & 255u);
+            const bool ok = slot >= 0 && bounds_ok(slot, nslots, 12);
 #pragma unroll
-          for (int j = 0; j < kHWin; ++j) {
-            if (j < nt) {
-              uint32_t y[4][16];
-              const uint32_t col = buf * kHBufCols + 16 * j;
+            for (int q = 0; q < 2; ++q) {  // eight columns at a time, inside the accumulators' width
+              const int lc = min(c0 + 8 * q, W - 8), from = c0 + 8 * q;
+              if (from >= c1) break;
+              uint32_t y[4][8];
 #pragma unroll
-              for (int k = 0; k < 4; ++k) tc::tmem_ld16_nowait(tc::tmem_addr(tmem, quarter * 32, col + k * W), y[k]);
+              for (int k = 0; k < 4; ++k)
+                tc::tmem_ld8_nowait(tc::tmem_addr(tmem, quarter * 32, buf * kHBufCols + (uint32_t)(lc + k * W)), y[k]);
               tc::tmem_wait_ld();
 #pragma unroll
-              for (int k = 0; k < 4; ++k) tc::tmem_regs_ready(y[k]);
-              if (slot[j] >= 0 && bounds_ok(sbase + slot[j], cl.slot_base[cl.nbricks], 12)) {
-                float o[16];
+              for (int k = 0; k < 4; ++k)
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
-                  o[c] = (__uint_as_float(y[0][c]) +
-                          (__uint_as_float(y[1][c]) + (__uint_as_float(y[2][c]) + __uint_as_float(y[3][c])))) *
-                         out_scale;
-                float4* dst = reinterpret_cast<float4*>(cl.scratch + (sbase + slot[j]) * 256 + a * 16);
-                dst[0] = make_float4(o[0], o[1], o[2], o[3]);
-                dst[1] = make_float4(o[4], o[5], o[6], o[7]);
-                dst[2] = make_float4(o[8], o[9], o[10], o[11]);
-                dst[3] = make_float4(o[12], o[13], o[14], o[15]);
+                for (int c = 0; c < 8; ++c) asm volatile("" : "+r"(y[k][c]));  // no use before the wait
+              float* dst = out + (ok ? (int64_t)slot * 256 + a + (b0 + lc - c0) * ws : 0);
+              float v[8];
+#pragma unroll
+              for (int c = 0; c < 8; c += 2) {
+                auto two = [&](int k) { return pair_of(y[k][c], y[k][c + 1]); };
+                const float_pair x = mul2(add2(two(0), add2(two(1), add2(two(2), two(3)))), pair_of(out_scale, out_scale));
+                v[c] = __uint_as_float((uint32_t)x);
+                v[c + 1] = __uint_as_float((uint32_t)(x >> 32));
+              }
+              if (lc == from && c1 - lc >= 8) {  // uniform
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                  if (ok) dst[c * ws] = v[c];
+              } else {
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                  if (ok && lc + c >= from && lc + c < c1) dst[c * ws] = v[c];
               }
             }
-          }
+            return true;
+          };
+          const int t1 = first(cur);
+          bool more = true;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) more = more && image(t1 + 2 * k, o[k]);
+          for (int t = t1 + 8; more; t += 2) more = image(t, slot_of(t));
+          cur = next;
+          next = after;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = on[k];
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(&tempty_bar[buf]);
@@ -1223,11 +1394,10 @@ __device__ __forceinline__ void h_reduce_block(int64_t u, const int64_t* __restr
   const int fq = sb_fold[u], ch = sb_chunks[u];
   const int ia = pr.atom[fq], ja = pr.jatom[fq];
   const int noi = numorbs[ia], noj = numorbs[ja];
-  // rows of a partial past its atom's orbitals are padding: lane pair
-  // (2r, 2r+1) holds row r, which a direct partial indexes by the i chunk's
-  // orbitals and a transposed one by the j chunk's
-  const int row = lane >> 1;
-  const bool row_d = row < noi - (ch >> 8) * 16, row_t = row < noj - (ch & 255) * 16;
+  // a partial is stored [column][row] without gaps: a direct one as [j chunk's
+  // orbital][i chunk's], one that enters transposed the other way round
+  const int wi = min(16, noi - (ch >> 8) * 16), wj = min(16, noj - (ch & 255) * 16);
+  const bool mine = lane * 8 < wi * wj;
   const int64_t k0 = red_off[u], k1 = red_off[u + 1];
   for (int64_t kb = k0; kb < k1; kb += kRedCodes) {
     const int n = (int)min((int64_t)kRedCodes, k1 - kb);
@@ -1241,7 +1411,7 @@ __device__ __forceinline__ void h_reduce_block(int64_t u, const int64_t* __restr
     const int cnt = warp < n ? (n - warp + 7) / 8 : 0;
     auto code_of = [&](int i) -> int64_t {
       const int64_t c = s_code[warp + 8 * i];
-      return ((c & 1) ? row_t : row_d) ? c : -1;  // padding row: nothing to add
+      return mine ? c : -1;
     };
     auto issue = [&](int i) {
       const int64_t c = code_of(i);
@@ -1281,11 +1451,12 @@ __device__ __forceinline__ void h_reduce_block(int64_t u, const int64_t* __restr
     s_part[3][warp][lane * 8 + i] = tl[i];
   }
   __syncthreads();
-  const int a = tid >> 4, b = tid & 15, et = b * 16 + a;
+  const int a = tid >> 4, b = tid & 15;
+  const int ed = min(b * wi + a, 255), et = min(a * wj + b, 255);  // entries past a chunk's orbitals are not written below
   float hi = 0.0f, lo = 0.0f;
   for (int w = 0; w < 8; ++w) {
-    ff_add(hi, lo, s_part[0][w][tid]);
-    lo += s_part[1][w][tid];
+    ff_add(hi, lo, s_part[0][w][ed]);
+    lo += s_part[1][w][ed];
     ff_add(hi, lo, s_part[2][w][et]);
     lo += s_part[3][w][et];
   }
@@ -1368,6 +1539,17 @@ cudaError_t launch_brick_table(const double* phi, const int64_t* phi_off, const 
   return cudaGetLastError();
 }
 
+cudaError_t launch_brick_pack(const TcBrickGeom& bg, const uint8_t* width, bool packed, uint32_t* row,
+                              const __nv_bfloat16* tab, __nv_bfloat16* ptab, cudaStream_t st) {
+  if (bg.npk == 0) return cudaSuccess;
+  const int blocks = (int)std::min<int64_t>(bg.nbricks, (int64_t)sm_count() * 8);
+  brick_rows_kernel<<<blocks, 256, 0, st>>>(bg, width, packed ? 1 : 0, row);
+  LCP_CUDA_TRY(cudaGetLastError());
+  if (!packed) return cudaSuccess;
+  brick_pack_kernel<<<blocks, 256, 0, st>>>(bg, tab, ptab);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_dsym(int64_t nsub, const int32_t* sub_pair, const int32_t* sub_chunks, const int32_t* pair_atom,
                         const int32_t* pair_jatom, const int64_t* boff, const int32_t* partner, const int32_t* numorbs,
                         const double* dm, const double* scale, __nv_bfloat16* out, cudaStream_t st) {
@@ -1422,6 +1604,10 @@ TcCell tc_cell_of(const TcBrickGeom& bg, const __nv_bfloat16* tab) {
   c.img_off = bg.img_off;
   c.tab_off = bg.tab_off;
   c.tab_pair = bg.tab_pair;
+  c.npk = bg.npk;
+  c.ptab = bg.ptab;
+  c.pk_off = bg.pk_off;
+  c.pk_row = bg.pk_row;
   return c;
 }
 
@@ -1470,7 +1656,7 @@ cudaError_t launch_hamiltonian_tc_batch(const TcCell& cell0, const TcBatch& batc
   LCP_CUDA_TRY(cudaFuncSetAttribute(hamiltonian_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHSmem));
   static_assert(kHSmem > 120 * 1024, "one CTA per SM");
   if (ev_begin) LCP_CUDA_TRY(cudaEventRecord(ev_begin, st));
-  LCP_CUDA_TRY(launch_pdl(hamiltonian_tc_kernel, tc_grid(cell0, batch), dim3(192 + 32 * kHXformWarps), kHSmem, st, a));
+  LCP_CUDA_TRY(launch_pdl(hamiltonian_tc_kernel, tc_grid(cell0, batch), dim3(kHThreads), kHSmem, st, a));
   if (ev_end) LCP_CUDA_TRY(cudaEventRecord(ev_end, st));
   return cudaSuccess;
 }

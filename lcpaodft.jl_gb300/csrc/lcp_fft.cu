@@ -16,10 +16,15 @@
 //   3. i:     forward along i, times S (FP64), inverse along i, in one pass;
 //   4. j:     inverse along j;
 //   5. rows:  the inverse real transform of two rows at once, written to dV_H.
-// Every pencil is transformed in shared memory by one warp: a mixed-radix
-// Stockham autosort FFT (radix 4, 2 and 3 butterflies in registers, any other
-// prime radix by its direct DFT), natural order in and out, with the
-// pencil length's roots of unity from a host-built table.
+// Every pencil is transformed in shared memory: a mixed-radix Stockham autosort
+// FFT (radix 4, 2, 3, 5 and 7 butterflies in registers, any other prime radix by
+// its direct DFT), natural order in and out, with the pencil length's roots of
+// unity from a host-built table.  A stage's butterflies of all the block's
+// pencils are dealt to its threads in one sequence: with a warp to a pencil,
+// length 98 kept 14 of 32 lanes busy in its radix-7 stages, and an FP64
+// instruction holds its pipe for as many clocks whatever its lanes do.  The FP64
+// solve is bound by that pipe: on a 105 x 98 x 126 grid its passes took 1.06 ms with
+// direct DFTs of radix 7 and a warp to a pencil, and take 0.34 ms.
 //
 // Arithmetic: FP64 for the FP64 drop-in form; double-float (pairs of FP32,
 // about 48 significant bits, on the FP32 pipe) for the precision forms, where
@@ -194,6 +199,42 @@ __device__ __forceinline__ void bfly5(const Cx<T>* a, Cx<T>* b, int j, int nb, i
   b[o + 3 * ns] = csub_l(a2, ib2);
 }
 
+// radix 7, as radix 5: t_k = v_k + v_7-k, d_k = v_k - v_7-k, y_s,7-s = a_s -+ i b_s
+// with a_s = v0 + sum_k c_sk t_k and b_s = sum_k s_sk d_k (indices mod 7, c even,
+// s odd): 18 FP64 operations a point with its twiddle, against 36 and the direct
+// DFT's loads.
+template <class T, bool INV>
+__device__ __forceinline__ void bfly7(const Cx<T>* a, Cx<T>* b, int j, int nb, int o, int ns, bool tw, int m,
+                                      const Cx<T>* w, int n) {
+  const Cx<T> v0 = a[j];
+  Cx<T> t[3], d[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    Cx<T> p = a[j + (k + 1) * nb], q = a[j + (6 - k) * nb];
+    if (tw) {
+      p = cmul(p, root<T, INV>(w, (k + 1) * m));
+      q = cmul(q, root<T, INV>(w, (6 - k) * m));
+    }
+    t[k] = cadd_l(p, q);
+    d[k] = csub_l(p, q);
+  }
+  const Cx<T> w1 = w[n / 7], w2 = w[2 * (n / 7)], w3 = w[3 * (n / 7)];
+  const T c[3] = {w1.x, w2.x, w3.x}, s[3] = {-w1.y, -w2.y, -w3.y};
+  b[o] = cadd_l(v0, cadd_l(cadd_l(t[0], t[1]), t[2]));
+  auto out = [&](int q, T c1, T c2, T c3, T s1, T s2, T s3) {
+    const Cx<T> x = cadd_l(v0, Cx<T>{add_lazy(dot2(c1, t[0].x, c2, t[1].x), c3 * t[2].x),
+                                     add_lazy(dot2(c1, t[0].y, c2, t[1].y), c3 * t[2].y)});
+    const Cx<T> y = {add_lazy(dot2(s1, d[0].x, s2, d[1].x), s3 * d[2].x),
+                     add_lazy(dot2(s1, d[0].y, s2, d[1].y), s3 * d[2].y)};
+    const Cx<T> iy = INV ? mul_pi(y) : mul_mi(y);
+    b[o + q * ns] = cadd_l(x, iy);
+    b[o + (7 - q) * ns] = csub_l(x, iy);
+  };
+  out(1, c[0], c[1], c[2], s[0], s[1], s[2]);
+  out(2, c[1], c[2], c[0], s[1], -s[2], -s[0]);
+  out(3, c[2], c[0], c[1], s[2], -s[0], s[1]);
+}
+
 // any other radix: the twiddles applied in place (the lane owns these
 // inputs), then the direct DFT with the inputs read from shared memory.
 template <class T, bool INV>
@@ -214,9 +255,9 @@ __device__ void bfly_dft(Cx<T>* a, Cx<T>* b, int j, int nb, int o, int ns, bool 
   }
 }
 
-// Stockham autosort FFT of length n on a (natural order), b scratch; returns
-// the buffer holding the result.  One warp per pencil (lane = 0..31); both
-// buffers may be overwritten.
+// Stockham autosort FFT of length n, double-float: one warp per pencil (lane =
+// 0..31), a (natural order) and b scratch, both may be overwritten; returns the
+// buffer holding the result.
 template <class T, bool INV>
 __device__ Cx<T>* fft_warp(Cx<T>* a, Cx<T>* b, int n, const int* fac, int nfac, const Cx<T>* w, int lane) {
   int ns = 1;
@@ -247,6 +288,74 @@ __device__ Cx<T>* fft_warp(Cx<T>* a, Cx<T>* b, int n, const int* fac, int nfac, 
     ns *= R;
   }
   return a;
+}
+
+// The same in FP64: all of the block's np pencils, pencil p in bufs + p S with n
+// elements of scratch behind it, called by the whole block and synchronised on
+// entry and return.  A stage's butterflies of all pencils form one sequence over
+// the block's threads.
+template <bool INV>
+__device__ void fft_block(Cx<double>* bufs, int S, int np, int n, const int* fac, int nfac, const Cx<double>* w,
+                          int& off) {
+  using T = double;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  int ns = 1;
+  for (int st = 0; st < nfac; ++st) {
+    const int R = fac[st];
+    const int nb = n / R;
+    const int tstep = n / (ns * R);
+    const bool tw = ns > 1;
+    // butterfly j of pencil p, nt apart in the sequence over both
+    const int dp = nt / nb, dj = nt - dp * nb;
+    int p = tid / nb, j = tid - p * nb;
+    while (p < np) {
+      Cx<T>*a = bufs + (size_t)p * S + off, *b = bufs + (size_t)p * S + (n - off);
+      const int k = j % ns;
+      const int o = (j - k) * R + k;
+      const int m = k * tstep;
+      if (R == 4)
+        bfly4<T, INV>(a, b, j, nb, o, ns, tw, m, w);
+      else if (R == 2)
+        bfly2<T, INV>(a, b, j, nb, o, ns, tw, m, w);
+      else if (R == 3)
+        bfly3<T, INV>(a, b, j, nb, o, ns, tw, m, w, n);
+      else if (R == 5)
+        bfly5<T, INV>(a, b, j, nb, o, ns, tw, m, w, n);
+      else if (R == 7)
+        bfly7<T, INV>(a, b, j, nb, o, ns, tw, m, w, n);
+      else
+        bfly_dft<T, INV>(a, b, j, nb, o, ns, tw, m, w, n, R);
+      p += dp;
+      j += dj;
+      if (j >= nb) {
+        j -= nb;
+        ++p;
+      }
+    }
+    __syncthreads();
+    off = n - off;
+    ns *= R;
+  }
+}
+
+// The block's pencils, each with its data at offset off (0 or n) of its buffer
+// pair, on return the result's.  A warp sees its own pencil's results (FP64:
+// the block all).  The double-float form is bound by instruction issue, and keeps
+// a warp to a pencil: there the sequence over the block cost more than idle
+// lanes (64-atom 96^3 cell: 0.089 ms against 0.082).
+template <class T, bool INV>
+__device__ __forceinline__ void fft_pencils(Cx<T>* bufs, int S, int np, int n, const int* fac, int nfac,
+                                            const Cx<T>* w, int& off) {
+  if constexpr (std::is_same<T, double>::value) {
+    __syncthreads();
+    fft_block<INV>(bufs, S, np, n, fac, nfac, w, off);
+  } else {
+    __syncwarp();
+    const int warp = threadIdx.x >> 5;
+    Cx<T>* p = bufs + (size_t)warp * S;
+    if (warp < np) fft_warp<T, INV>(p + off, p + (n - off), n, fac, nfac, w, threadIdx.x & 31);
+    if (nfac & 1) off = n - off;
+  }
 }
 
 // ------------------------------------------------------------ passes
@@ -297,7 +406,7 @@ constexpr int kRowWarps = 4;
 
 // Pass 1: the source rows (two per warp) to their half spectra.
 template <class T>
-__global__ void __launch_bounds__(32 * kRowWarps, 8) fft_rows_fwd_kernel(const __grid_constant__ FftArgs a) {
+__global__ void __launch_bounds__(32 * kRowWarps, std::is_same<T, double>::value ? 5 : 8) fft_rows_fwd_kernel(const __grid_constant__ FftArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const GridCell& c = fft_cell(a);
   const int n = a.g.n[2], h = n / 2 + 1;
@@ -308,20 +417,21 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) fft_rows_fwd_kernel(const _
   pdl_trigger();
   load_roots(w, roots_of<T>(a.g, 2), n);
   pdl_wait();
-  __syncthreads();
-  const int64_t pair = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-  const int64_t ra = 2 * pair, rb = ra + 1;
-  if (ra >= nrows) return;
-  const bool has_b = rb < nrows;
-  for (int k = lane; k < n; k += 32) {
+  __syncthreads();  // the roots
+  const int64_t first = (int64_t)blockIdx.x * kRowWarps;  // of the block's row pairs
+  const int np = (int)min((int64_t)kRowWarps, (nrows + 1) / 2 - first);
+  const int64_t ra = 2 * (first + warp), rb = ra + 1;
+  const bool live = ra < nrows, has_b = rb < nrows;
+  for (int k = live ? lane : n; k < n; k += 32) {
     const T va = source_at<T>(c, a.spinpol, ra * n + k);
     const T vb = has_b ? source_at<T>(c, a.spinpol, rb * n + k) : Num<T>::zero();
     buf[k] = {va, vb};
   }
-  __syncwarp();
-  const Cx<T>* z = fft_warp<T, false>(buf, buf + n, n, a.g.fac[2], a.g.nfac[2], w, lane);
+  int off = 0;
+  fft_pencils<T, false>(w + n, 2 * n, np, n, a.g.fac[2], a.g.nfac[2], w, off);
+  const Cx<T>* z = buf + off;
   Cx<T>* spec = reinterpret_cast<Cx<T>*>(c.spec);
-  for (int k = lane; k < h; k += 32) {
+  for (int k = live ? lane : h; k < h; k += 32) {
     const Cx<T> p = z[k], q = conj(z[k == 0 ? 0 : n - k]);
     const Cx<T> s = p + q, d = p - q;
     spec[ra * h + k] = {Num<T>::half(s.x), Num<T>::half(s.y)};  // (z + conj z(-k)) / 2
@@ -331,7 +441,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) fft_rows_fwd_kernel(const _
 
 // Pass 5: the half spectra of two rows to the real output rows.
 template <class T>
-__global__ void __launch_bounds__(32 * kRowWarps, 8) fft_rows_inv_kernel(const __grid_constant__ FftArgs a) {
+__global__ void __launch_bounds__(32 * kRowWarps, std::is_same<T, double>::value ? 5 : 8) fft_rows_inv_kernel(const __grid_constant__ FftArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const GridCell& c = fft_cell(a);
   const int n = a.g.n[2], h = n / 2 + 1;
@@ -342,13 +452,13 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) fft_rows_inv_kernel(const _
   pdl_trigger();
   load_roots(w, roots_of<T>(a.g, 2), n);
   pdl_wait();
-  __syncthreads();
-  const int64_t pair = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-  const int64_t ra = 2 * pair, rb = ra + 1;
-  if (ra >= nrows) return;
-  const bool has_b = rb < nrows;
+  __syncthreads();  // the roots
+  const int64_t first = (int64_t)blockIdx.x * kRowWarps;  // of the block's row pairs
+  const int np = (int)min((int64_t)kRowWarps, (nrows + 1) / 2 - first);
+  const int64_t ra = 2 * (first + warp), rb = ra + 1;
+  const bool live = ra < nrows, has_b = rb < nrows;
   const Cx<T>* spec = reinterpret_cast<const Cx<T>*>(c.spec);
-  for (int k = lane; k < n; k += 32) {
+  for (int k = live ? lane : n; k < n; k += 32) {
     const bool lower = k < h;
     const int kk = lower ? k : n - k;
     Cx<T> p = spec[ra * h + kk];
@@ -363,10 +473,11 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) fft_rows_inv_kernel(const _
     }
     buf[k] = p + mul_pi(q);  // row a + i row b
   }
-  __syncwarp();
-  const Cx<T>* z = fft_warp<T, true>(buf, buf + n, n, a.g.fac[2], a.g.nfac[2], w, lane);
+  int off = 0;
+  fft_pencils<T, true>(w + n, 2 * n, np, n, a.g.fac[2], a.g.nfac[2], w, off);
+  const Cx<T>* z = buf + off;
   double* out = const_cast<double*>(c.dvh);
-  for (int k = lane; k < n; k += 32) {
+  for (int k = live ? lane : n; k < n; k += 32) {
     const Cx<T> v = z[k];
     out[ra * n + k] = Num<T>::to(v.x);
     if (has_b) out[rb * n + k] = Num<T>::to(v.y);
@@ -375,13 +486,13 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) fft_rows_inv_kernel(const _
 
 // Passes 2-4: pencils along axis 1 (j) or 0 (i) of the half spectrum.  The
 // pencils are numbered c = outer * h + k' (outer = i for axis 1, j for axis
-// 0), and a block takes W consecutive ones, one warp each, so every block is
+// 0), and a block of W warps takes W consecutive ones, so every block is
 // full.  Thread t of the block stages column t mod W (consecutive addresses
 // for consecutive threads) into a shared-memory stride that is odd in 16-byte
 // elements, so these stores hit distinct banks.  MODE 0 forward, 1 inverse, 2
 // forward, times the FP64 factors, inverse.
 template <class T, int MODE>
-__global__ void __launch_bounds__(256, 4) fft_cols_kernel(const __grid_constant__ FftArgs a, int axis) {
+__global__ void __launch_bounds__(256, std::is_same<T, double>::value ? 3 : 4) fft_cols_kernel(const __grid_constant__ FftArgs a, int axis) {
   extern __shared__ __align__(16) unsigned char smem[];
   const GridCell& c = fft_cell(a);
   const int n2 = a.g.n[1], h = a.g.n[2] / 2 + 1;
@@ -411,26 +522,23 @@ __global__ void __launch_bounds__(256, 4) fft_cols_kernel(const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int* fac = a.g.fac[axis];
   const int nfac = a.g.nfac[axis];
-  if ((int64_t)blockIdx.x * W + warp < ncols) {
-    Cx<T>* p = bufs + (size_t)warp * S;
-    Cx<T>* q = p + n;
-    Cx<T>* r = fft_warp<T, MODE == 1>(p, q, n, fac, nfac, w, lane);
-    if (MODE == 2) {
+  const int np = (int)min((int64_t)W, ncols - (int64_t)blockIdx.x * W);
+  int off = 0;
+  fft_pencils<T, MODE == 1>(bufs, S, np, n, fac, nfac, w, off);
+  if (MODE == 2) {
+    if (warp < np) {
+      Cx<T>* r = bufs + (size_t)warp * S + off;
       const double* f = pf + (size_t)warp * a.pfstride;
       for (int e = lane; e < n; e += 32) {
         const Cx<T> v = r[e];
         r[e] = {Num<T>::from(Num<T>::to(v.x) * f[e]), Num<T>::from(Num<T>::to(v.y) * f[e])};
       }
-      __syncwarp();
-      fft_warp<T, true>(r, r == p ? q : p, n, fac, nfac, w, lane);
     }
+    fft_pencils<T, true>(bufs, S, np, n, fac, nfac, w, off);
   }
   __syncthreads();
-  // every warp's result sits in the same half of its buffer pair
-  const int passes = MODE == 2 ? 2 * nfac : nfac;
-  const size_t res = (passes & 1) ? (size_t)n : 0;
   if (live)
-    for (int e = threadIdx.x / W; e < n; e += rows) spec[base + e * estride] = norm(bufs[(size_t)col * S + res + e]);
+    for (int e = threadIdx.x / W; e < n; e += rows) spec[base + e * estride] = norm(bufs[(size_t)col * S + off + e]);
 }
 
 // Shared-memory budget of a pass 2-4 block: four blocks per SM.

@@ -1512,7 +1512,8 @@ static lcp_status energy_host(lcp_ctx* ctx, int32_t xc, int32_t spinpol, int64_t
   }
   API_CUDA(ctx->w_part.ensure((size_t)std::max<int64_t>(lcp::red_tiles(nn), 1) * 3 * sizeof(double)), "alloc");
   API_CUDA(ctx->w_scal.ensure(8 * sizeof(double)), "alloc");
-  API_CUDA(lcp::launch_energy_sums(xc, spinpol, nn, d_ad, d_pc, dr, d_vh, ctx->w_part.as<double>(),
+  // one caller reads the Hartree term (with dV_H), the other the xc terms
+  API_CUDA(lcp::launch_energy_sums(xc, dvhart == nullptr, spinpol, nn, d_ad, d_pc, dr, d_vh, ctx->w_part.as<double>(),
                                    ctx->w_scal.as<double>(), ctx->stream),
            "energy");
   ctx->launches += 2;

@@ -136,7 +136,7 @@ cudaError_t launch_vpot(int spinpol, int64_t nn, const double* dvh, const double
                         const double* vna, double* const* vpot, cudaStream_t st);
 // Deterministic FP64 energy sums: out[0] = sum dRho*dVH, out[1..2] = xc sums;
 // partials: 3 * red_tiles(nn) doubles.
-cudaError_t launch_energy_sums(int xc, int spinpol, int64_t nn, const double* aden,
+cudaError_t launch_energy_sums(int xc, bool with_xc, int spinpol, int64_t nn, const double* aden,
                                const double* pcc, const double* const* rho, const double* dvh,
                                double* partials, double* out, cudaStream_t st);
 // Reductions run over tiles of kRedTile elements, one block per tile.

@@ -123,6 +123,10 @@ __device__ __forceinline__ const GridCell& grid_cell(const GridCell& c0, const G
   return b.cells[lo];
 }
 
+__device__ __forceinline__ double density_change(int spinpol, double r0, double r1, double ad) {
+  return spinpol == LCP_SPIN_OFF ? 2 * (r0 - ad) : r0 + r1 - 2 * ad;
+}
+
 // Calc_EH1 (src/Energy.jl:655-666) and Calc_EXC1 (src/Energy.jl:669-700, with
 // Calc_Vxc_Grid switch 0 of src/XC/XC_Func.jl:164-189) terms of one point;
 // e is the xc energy density at the point's density (DF: the atomic
@@ -130,8 +134,7 @@ __device__ __forceinline__ const GridCell& grid_cell(const GridCell& c0, const G
 template <bool DF = false>
 __device__ __forceinline__ void energy_terms(int xc, int spinpol, double r0, double r1, double ad, double pc,
                                              double dvh, double e, double (&acc)[3]) {
-  const double drho = spinpol == LCP_SPIN_OFF ? 2 * (r0 - ad) : r0 + r1 - 2 * ad;
-  acc[0] += drho * dvh;
+  acc[0] += density_change(spinpol, r0, r1, ad) * dvh;
   const double temp = ad + pc;
   double eat, vat;
   lda_eval<DF>(2 * temp, eat, vat);

@@ -566,7 +566,9 @@ __device__ __forceinline__ void load_coef(const GridCell& c, double* dc) {
 // where t >= den_min ("off") / t > den_min ("on"), energy where t > den_min,
 // with t = 2 rho ("off") or rho_up + rho_down, before the PCC is added.
 // DF: the stencil and the functional in double-float (the precision forms).
-template <bool SYM, bool DF>
+// POT: the potential's outputs; without them (Calc_EXC1 alone) the functional's
+// derivatives go too (1.3 M points, FP64: 0.97 ms against 1.10).
+template <bool SYM, bool DF, bool POT>
 __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_constant__ GgaArgs a) {
   int64_t t;
   const GridCell& c = grid_cell(a.cell0, a.batch, blockIdx.x, t);
@@ -652,7 +654,7 @@ __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_c
       xc_pbe_point<SYM>(r0 + pc, r1 + pc, g, e, v, dg);
     }
 #pragma unroll
-    for (int s = 0; s < (SYM ? 1 : 2); ++s) {
+    for (int s = 0; s < (POT ? (SYM ? 1 : 2) : 0); ++s) {
       c.vpot[s][x] = v[s];
 #pragma unroll
       for (int q = 0; q < 3; ++q) c.dexc[(3 * s + q) * nn + x] = dg[3 * s + q];
@@ -741,9 +743,13 @@ __global__ void __launch_bounds__(kRedThreads) gga_div_g_kernel(const __grid_con
 
 template <bool SYM, bool DF>
 cudaError_t launch_gga_t(const GgaArgs& a, int64_t n, bool potential, cudaStream_t st) {
-  gga_point_g_kernel<SYM, DF><<<(unsigned)n, kRedThreads, 0, st>>>(a);
+  if (!potential) {
+    gga_point_g_kernel<SYM, DF, false><<<(unsigned)n, kRedThreads, 0, st>>>(a);
+    return cudaGetLastError();
+  }
+  gga_point_g_kernel<SYM, DF, true><<<(unsigned)n, kRedThreads, 0, st>>>(a);
   LCP_CUDA_TRY(cudaGetLastError());
-  if (potential) gga_div_g_kernel<SYM, DF><<<(unsigned)n, kRedThreads, 0, st>>>(a);
+  gga_div_g_kernel<SYM, DF><<<(unsigned)n, kRedThreads, 0, st>>>(a);
   return cudaGetLastError();
 }
 

@@ -557,6 +557,18 @@ __device__ __forceinline__ void load_coef(const GridCell& c, double* dc) {
   __syncthreads();
 }
 
+// The weights' odd part (they are odd but for the rounding of their inversion).
+__device__ __forceinline__ void odd_coef(double* dc) {
+  double w = 0.0;
+  if (threadIdx.x < 81) {
+    const int d = threadIdx.x / 27, q = threadIdx.x - 27 * d;
+    w = 0.5 * (dc[27 * d + q] - dc[27 * d + 26 - q]);
+  }
+  __syncthreads();
+  if (threadIdx.x < 81) dc[threadIdx.x] = w;
+  __syncthreads();
+}
+
 // Pass 1: Set_dDensity_Grid! (src/XC/GGA_PBE.jl:53-159) and the pointwise
 // part of Set_Vxc_GGA_PBE! (src/XC/GGA_PBE.jl:274-322, 358-420); where the
 // cell has tile partials, also Calc_EH1 / Calc_EXC1's terms (src/Energy.jl:
@@ -578,6 +590,8 @@ __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_c
   if (DF) {
     for (int q = threadIdx.x; q < 81; q += blockDim.x) dcf[q] = dfl_of(dc[q]);
     __syncthreads();
+  } else {
+    odd_coef(dc);
   }
   const int64_t nn = c.nn;
   const int64_t x0 = t * kRedTile, x1 = min(nn, x0 + kRedTile);
@@ -594,10 +608,34 @@ __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_c
     Dfl gd[6] = {};
     if (kDenMin < test) {
       const Stencil nb(x, c.ng);
+      // FP64: the weights are odd under inversion, so the 13 pairs of opposite
+      // neighbours enter with their differences: four FP64 operations a pair and
+      // spin (six with a partial core) where the 27 points take four each.
+      if (!DF) {
+        auto pair = [&](int64_t y, int64_t z, const double* w) {
+          const double dp = pcp ? pcp[y] - pcp[z] : 0.0;
+          double d = r0p[y] - r0p[z];
+          if (pcp) d += dp;
+          g[0] += d * w[0];
+          g[1] += d * w[27];
+          g[2] += d * w[54];
+          if (!SYM) {
+            d = r1p[y] - r1p[z];
+            if (pcp) d += dp;
+            g[3] += d * w[0];
+            g[4] += d * w[27];
+            g[5] += d * w[54];
+          }
+        };
+        const int64_t b0 = nb.plane_base(0), b1 = nb.plane_base(1), b2 = nb.plane_base(2);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) pair(nb.at(b2, q), nb.at(b0, 8 - q), dc + 18 + q);
+#pragma unroll
+        for (int q = 5; q < 9; ++q) pair(nb.at(b1, q), nb.at(b1, 8 - q), dc + 9 + q);
+      }
 #pragma unroll 1
-      for (int pa = 0; pa < 3; ++pa) {
+      for (int pa = 0; pa < (DF ? 3 : 0); ++pa) {
         const int64_t base = nb.plane_base(pa);
-        const double* w = dc + 9 * pa;
         const Dfl* wf = dcf + (DF ? 9 * pa : 0);
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
@@ -613,18 +651,6 @@ __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_c
               gd[3] = fma_acc(gd[3], fd, wf[q]);
               gd[4] = fma_acc(gd[4], fd, wf[27 + q]);
               gd[5] = fma_acc(gd[5], fd, wf[54 + q]);
-            }
-          } else {
-            const double py = pcp ? pcp[y] : 0.0;
-            const double fu = r0p[y] + py;
-            g[0] += fu * w[q];
-            g[1] += fu * w[27 + q];
-            g[2] += fu * w[54 + q];
-            if (!SYM) {
-              const double fd = r1p[y] + py;
-              g[3] += fd * w[q];
-              g[4] += fd * w[27 + q];
-              g[5] += fd * w[54 + q];
             }
           }
         }

@@ -217,16 +217,23 @@ static std::vector<int64_t> packed_blocks(const lcp::UCell& u, const lcp::Bricks
 // blocks of 16 leave rows empty on both sides of the product, so the rows are
 // packed into a second table where that saves a sixteenth of the blocks or
 // more (13-orbital atoms: 0.66 of the products; 18: 0.32), and the images'
-// own blocks serve otherwise, or when there is no room for it.  (The density
-// takes an image's chunk as one K step and keeps the images' blocks.)
+// own blocks serve otherwise, or unless seven eighths of the device's memory
+// stay free.  (The density takes an image's chunk as one K step and keeps the
+// images' blocks.)  That line: a batch of 256 cells fills most of the memory
+// with its image blocks and 48 GB of partial blocks.  With a second table for
+// every cell its tables ran out of memory, and with them while three quarters
+// were free (234 GB held) its partial blocks did; one large cell has room.
 static lcp_status pack_rows(lcp_ctx* ctx, lcp_orbs* o) {
   const lcp::Bricks& b = o->bricks;
   lcp::TcBrickGeom& g = o->bgeom;
   std::vector<uint8_t> width;
   std::vector<int64_t> off = packed_blocks(o->ucell->u, b, width);
-  bool packed = off.back() * 16 <= b.nblocks * 15;
+  const size_t bytes = (size_t)std::max<int64_t>(off.back(), 1) * 6144 * 2;
+  size_t mem_free = 0, mem_total = 0;
+  API_CUDA(cudaMemGetInfo(&mem_free, &mem_total), "memory");
+  bool packed = off.back() * 16 <= b.nblocks * 15 && mem_free >= bytes + mem_total / 8 * 7;
   if (packed) {
-    const cudaError_t e = o->b_ptab.ensure((size_t)std::max<int64_t>(off.back(), 1) * 6144 * 2);
+    const cudaError_t e = o->b_ptab.ensure(bytes);
     if (e == cudaErrorMemoryAllocation) {
       (void)cudaGetLastError();
       packed = false;
@@ -1014,6 +1021,15 @@ lcp_status lcp_orbs_release_fp64(lcp_ctx* ctx, lcp_orbs* orbs) {
   if ((s = ensure_bricks(ctx, orbs))) return s;
   API_CUDA(cudaStreamSynchronize(ctx->stream), "release");
   for (DBuf* d : {&orbs->phi, &orbs->dphi[0], &orbs->dphi[1], &orbs->dphi[2], &orbs->phi32}) d->release();
+  {
+    std::lock_guard<std::mutex> lock(orbs->f64_mutex);  // the FP64 kernels' tables go with the tables they came from
+    for (F64Set* x : {&orbs->f64_density, &orbs->f64_elements}) {
+      x->release();
+      x->state = 0;
+    }
+    for (DBuf& d : orbs->f64_pair_buf) d.release();
+    orbs->f64_pairs_ready = false;
+  }
   orbs->phi_released = true;
   return LCP_OK;
 }

@@ -121,3 +121,18 @@ def test_f64_tensor_force_against_oracle(name):
     d[u.block_offset[onsite]] = np.inf
     f = L.Force3_spin(paos, dorbs, v, [d, dm[1]], u)
     assert not np.isfinite(f[0]).any() and np.isfinite(f[1:]).all()
+
+
+def test_f64_tables_go_with_the_orbital_tables():
+    """release_fp64 frees the FP64 kernels' tables too: the same bytes whether they were made or not."""
+    held = []
+    for made in (True, False):
+        u, _, orbs, _, rng = _cell(*CELLS["mixed"])
+        job = L.GridStepJob(u, orbs, "off", "LDA", None, None, np.zeros(u.NN))
+        if made:
+            job.set_dm([rng.normal(size=u.Total_Hsize)])
+            job.step()
+        orbs.ctx.set_precision("bf16x3")
+        orbs.release_fp64()
+        held.append(job.footprint())
+    assert held[0] == held[1]

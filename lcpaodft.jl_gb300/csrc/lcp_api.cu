@@ -218,11 +218,13 @@ static std::vector<int64_t> packed_blocks(const lcp::UCell& u, const lcp::Bricks
 // packed into a second table where that saves a sixteenth of the blocks or
 // more (13-orbital atoms: 0.66 of the products; 18: 0.32), and the images'
 // own blocks serve otherwise, or unless seven eighths of the device's memory
-// stay free.  (The density takes an image's chunk as one K step and keeps the
-// images' blocks.)  That line: a batch of 256 cells fills most of the memory
-// with its image blocks and 48 GB of partial blocks.  With a second table for
-// every cell its tables ran out of memory, and with them while three quarters
-// were free (234 GB held) its partial blocks did; one large cell has room.
+// stay free, half of it for a table of a 64th of the memory or more.  (The
+// density takes an image's chunk as one K step and keeps the images' blocks.)
+// These lines: a batch of 256 cells fills most of the memory with its image
+// blocks and 48 GB of partial blocks.  With a second table for every cell its
+// tables ran out of memory, and with them while three quarters were free (234
+// GB held) its partial blocks did.  A cell whose table is that large does not
+// come by the hundred.
 static lcp_status pack_rows(lcp_ctx* ctx, lcp_orbs* o) {
   const lcp::Bricks& b = o->bricks;
   lcp::TcBrickGeom& g = o->bgeom;
@@ -231,7 +233,7 @@ static lcp_status pack_rows(lcp_ctx* ctx, lcp_orbs* o) {
   const size_t bytes = (size_t)std::max<int64_t>(off.back(), 1) * 6144 * 2;
   size_t mem_free = 0, mem_total = 0;
   API_CUDA(cudaMemGetInfo(&mem_free, &mem_total), "memory");
-  bool packed = off.back() * 16 <= b.nblocks * 15 && mem_free >= bytes + mem_total / 8 * 7;
+  bool packed = off.back() * 16 <= b.nblocks * 15 && mem_free >= bytes + (bytes >= mem_total / 64 ? mem_total / 2 : mem_total / 8 * 7);
   if (packed) {
     const cudaError_t e = o->b_ptab.ensure(bytes);
     if (e == cudaErrorMemoryAllocation) {

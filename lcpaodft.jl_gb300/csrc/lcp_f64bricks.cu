@@ -390,11 +390,12 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   for (int32_t r : rows) g.max_rows = std::max(g.max_rows, r);
   if (g.max_rows > kF64MaxRows) *fits = false;
   if (ntab >= ((int64_t)1 << 32)) *fits = false;
-  // half of the device's memory stays free for what a program allocates next
-  // (the pair kernels, which need no tables, left it that)
+  // a quarter of the device's memory stays free for what a program allocates
+  // next: hundreds of cells whose orbital tables fit beside each other still do
+  // (256 of them take 77 GB, and these tables would take 200)
   size_t mem_free = 0, mem_total = 0;
   API_CUDA(cudaMemGetInfo(&mem_free, &mem_total), "memory");
-  if (mem_free < (size_t)g.nchunks * 32 * P * sizeof(uint64_t) + mem_total / 2) *fits = false;
+  if (mem_free < (size_t)g.nchunks * 32 * P * sizeof(uint64_t) + mem_total / 4) *fits = false;
   if (!*fits) return LCP_OK;
   API_CUDA(S.rows.ensure(std::max<int64_t>(g.nrows, 1) * sizeof(F64Row)), "alloc");
   API_CUDA(S.tab.ensure(std::max<int64_t>(ntab, 1) * sizeof(int32_t)), "alloc");

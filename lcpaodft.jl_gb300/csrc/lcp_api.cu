@@ -440,7 +440,7 @@ static lcp_status f64_made(lcp_ctx* ctx, lcp_orbs* o, int which, bool* tc) {
 // kernels' limits, without the memory for them, and inside a caller's stream capture before anything was
 // made (allocating and synchronising there would break the capture): those
 // take the pair kernels (64-atom 96^3 cell: 36.8 ms for density and matrix
-// elements, against 3.3 ms; 2-atom 24^3 cell: 0.62 ms against 0.15).
+// elements, against 3.15 ms; 2-atom 24^3 cell: 0.62 ms against 0.145).
 static lcp_status f64_ready(lcp_ctx* ctx, const lcp_orbs* orbs, int which, bool* tc) {
   *tc = false;
   if (ctx->precision != LCP_PREC_FP64) return LCP_OK;

@@ -35,11 +35,11 @@ METRIC = "ms per SCF grid step & jobs/s (p50/p99) split-BF16 vs FP64, <=1uHa/ato
 # and h_reduce_kernel 93.6 + 3.2 MB, over 12076 blocks)
 # DRAM bytes (read + write) per table block of a stage's big kernels, from
 # one ncu capture of the 64-atom 96^3 cell (96,608 table blocks): the density
-# kernel 1,199.0 + 9.4 MB; the H kernel 1,199.9 + 702.5 MB and the
-# partial-block reduction 656.1 + 5.0 MB
+# kernel 1,198.9 + 9.4 MB; the H kernel (packed rows) 1,052.7 + 478.3 MB and the
+# partial-block reduction 563.1 + 4.7 MB
 TRAFFIC_BLOCKS = 96608
-TRAFFIC_PER_BLOCK = {"density": (1199.03e6 + 9.38e6) / TRAFFIC_BLOCKS,
-                     "hamiltonian": (1199.94e6 + 702.50e6 + 656.07e6 + 5.00e6) / TRAFFIC_BLOCKS}
+TRAFFIC_PER_BLOCK = {"density": (1198.94e6 + 9.37e6) / TRAFFIC_BLOCKS,
+                     "hamiltonian": (1052.73e6 + 478.30e6 + 563.13e6 + 4.68e6) / TRAFFIC_BLOCKS}
 UNIT = "grid steps/s"
 
 

@@ -595,6 +595,7 @@ lcp::GridCell job_grid_cell(lcp_job* job) {
   if (job->xc == LCP_XC_GGA_PBE) {
     c.dcoef = job->dcoef.as<double>();
     c.dexc = job->dexc.as<double>();
+    c.even_weights = job->even_weights;
   }
   return c;
 }
@@ -1385,6 +1386,24 @@ lcp_status lcp_calc_diff_coef(const double* glatvecs, double* diff_coef) {
   return LCP_OK;
 }
 
+// Whether stencil weights [3][27] have a part that is even under inversion,
+// beyond 2^-48 of a direction's largest weight.  Calc_Diff_Coef's are odd but
+// for the rounding of its inversion: 2^-50 on cells of moderate skew, up to
+// 2^-31 on nearly singular ones; a caller's own may be anything.
+static bool even_weights(const double* dc) {
+  for (int d = 0; d < 3; ++d) {
+    const double* w = dc + 27 * d;
+    double even = 0.0, most = 0.0;
+    for (int q = 0; q < 27; ++q) {
+      if (!std::isfinite(w[q])) return true;
+      even = std::max(even, std::fabs(w[q] + w[26 - q]));
+      most = std::max(most, std::fabs(w[q]));
+    }
+    if (even > std::ldexp(most, -48)) return true;
+  }
+  return false;
+}
+
 // Uploads the GGA inputs into the context's workspaces and fills the cell:
 // rho (1 or 2 spins; "nc" angles into w_in[2..3]), pcc, the stencil weights,
 // the dE/d(grad rho) scratch and, if wanted, the gradient output.
@@ -1415,6 +1434,7 @@ static lcp_status gga_cell_host(lcp_ctx* ctx, int32_t spinpol, const int32_t* ng
   API_CUDA(ctx->w_a.ensure(81 * sizeof(double)), "alloc");
   API_CUDA(cudaMemcpyAsync(ctx->w_a.p, dc, 81 * sizeof(double), cudaMemcpyHostToDevice, ctx->stream), "H2D");
   c.dcoef = ctx->w_a.as<double>();
+  c.even_weights = even_weights(dc);
   API_CUDA(ctx->w_aux[0].ensure((size_t)3 * ns * nn * sizeof(double)), "alloc");
   c.dexc = ctx->w_aux[0].as<double>();
   if (want_dden) {
@@ -1664,6 +1684,7 @@ lcp_status lcp_job_create(lcp_ctx* ctx, const lcp_ucell* ucell, const lcp_orbs* 
     double gtv[3][3], dc[81];
     grid_vectors(&u.lat[0][0], u.ngrid, gtv);
     if (!lcp::calc_diff_coef(gtv, dc)) return fail(LCP_EINVAL, "singular gradient stencil (check Latvecs)");
+    j->even_weights = even_weights(dc);
     API_CUDA(j->dcoef.ensure(81 * sizeof(double)), "alloc");
     API_CUDA(j->dexc.ensure((size_t)3 * j->nspin * nn * sizeof(double)), "alloc");
     API_CUDA(cudaMemcpyAsync(j->dcoef.p, dc, sizeof dc, cudaMemcpyHostToDevice, ctx->stream), "H2D");

@@ -209,6 +209,7 @@ struct lcp_job {
   DBuf aden, pcc, vna, dvh, real, spec, part, scal;
   DBuf pfac;  // Poisson factors of the half spectrum, tabulated at creation
   DBuf dcoef, dexc;  // GGA_PBE: stencil weights [3][27] and dE/d(grad rho) [spin][xyz][nn]
+  bool even_weights = false;  // GridCell::even_weights
   bool has_aden = false, has_pcc = false, has_vna = false;
   FftPlans* plans = nullptr;
   // lcp_job_step's CUDA graphs, one per context that steps the job: the

@@ -167,6 +167,7 @@ struct GridCell {
   double* sums;          // [0..2] grid sums, [3] sum <D,H>, [8..12] the step's energies
   // GGA-PBE only (nullptr otherwise)
   const double* dcoef;   // gradient stencil weights [3][27] (Calc_Diff_Coef)
+  bool even_weights;     // they are not odd under inversion
   double* dexc;          // dE/d(grad rho) scratch: [spin][xyz][nn]
   double* dden;          // optional output: grad(rho + pcc) as [spin][xyz][nn]
 };

@@ -580,7 +580,11 @@ __device__ __forceinline__ void odd_coef(double* dc) {
 // DF: the stencil and the functional in double-float (the precision forms).
 // POT: the potential's outputs; without them (Calc_EXC1 alone) the functional's
 // derivatives go too (1.3 M points, FP64: 0.97 ms against 1.10).
-template <bool SYM, bool DF, bool POT>
+// ODD: the weights are odd under inversion but for their rounding (FP64 only;
+// GridCell::even_weights tells), so the 13 pairs of opposite neighbours enter
+// with their differences: four FP64 operations a pair and spin (six with a
+// partial core) where the 27 points take four each.
+template <bool SYM, bool DF, bool POT, bool ODD>
 __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_constant__ GgaArgs a) {
   int64_t t;
   const GridCell& c = grid_cell(a.cell0, a.batch, blockIdx.x, t);
@@ -590,7 +594,7 @@ __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_c
   if (DF) {
     for (int q = threadIdx.x; q < 81; q += blockDim.x) dcf[q] = dfl_of(dc[q]);
     __syncthreads();
-  } else {
+  } else if (ODD) {
     odd_coef(dc);
   }
   const int64_t nn = c.nn;
@@ -608,10 +612,7 @@ __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_c
     Dfl gd[6] = {};
     if (kDenMin < test) {
       const Stencil nb(x, c.ng);
-      // FP64: the weights are odd under inversion, so the 13 pairs of opposite
-      // neighbours enter with their differences: four FP64 operations a pair and
-      // spin (six with a partial core) where the 27 points take four each.
-      if (!DF) {
+      if (ODD) {
         auto pair = [&](int64_t y, int64_t z, const double* w) {
           const double dp = pcp ? pcp[y] - pcp[z] : 0.0;
           double d = r0p[y] - r0p[z];
@@ -634,8 +635,9 @@ __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_c
         for (int q = 5; q < 9; ++q) pair(nb.at(b1, q), nb.at(b1, 8 - q), dc + 9 + q);
       }
 #pragma unroll 1
-      for (int pa = 0; pa < (DF ? 3 : 0); ++pa) {
+      for (int pa = 0; pa < (ODD ? 0 : 3); ++pa) {
         const int64_t base = nb.plane_base(pa);
+        const double* w = dc + 9 * pa;
         const Dfl* wf = dcf + (DF ? 9 * pa : 0);
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
@@ -651,6 +653,18 @@ __global__ void __launch_bounds__(kRedThreads) gga_point_g_kernel(const __grid_c
               gd[3] = fma_acc(gd[3], fd, wf[q]);
               gd[4] = fma_acc(gd[4], fd, wf[27 + q]);
               gd[5] = fma_acc(gd[5], fd, wf[54 + q]);
+            }
+          } else {
+            const double py = pcp ? pcp[y] : 0.0;
+            const double fu = r0p[y] + py;
+            g[0] += fu * w[q];
+            g[1] += fu * w[27 + q];
+            g[2] += fu * w[54 + q];
+            if (!SYM) {
+              const double fd = r1p[y] + py;
+              g[3] += fd * w[q];
+              g[4] += fd * w[27 + q];
+              g[5] += fd * w[54 + q];
             }
           }
         }
@@ -767,13 +781,13 @@ __global__ void __launch_bounds__(kRedThreads) gga_div_g_kernel(const __grid_con
 
 }  // namespace
 
-template <bool SYM, bool DF>
+template <bool SYM, bool DF, bool ODD>
 cudaError_t launch_gga_t(const GgaArgs& a, int64_t n, bool potential, cudaStream_t st) {
   if (!potential) {
-    gga_point_g_kernel<SYM, DF, false><<<(unsigned)n, kRedThreads, 0, st>>>(a);
+    gga_point_g_kernel<SYM, DF, false, ODD><<<(unsigned)n, kRedThreads, 0, st>>>(a);
     return cudaGetLastError();
   }
-  gga_point_g_kernel<SYM, DF, true><<<(unsigned)n, kRedThreads, 0, st>>>(a);
+  gga_point_g_kernel<SYM, DF, true, ODD><<<(unsigned)n, kRedThreads, 0, st>>>(a);
   LCP_CUDA_TRY(cudaGetLastError());
   gga_div_g_kernel<SYM, DF><<<(unsigned)n, kRedThreads, 0, st>>>(a);
   return cudaGetLastError();
@@ -787,9 +801,11 @@ cudaError_t launch_gga_g(int spinpol, const GridCell& c0, const GridBatch& b, bo
   a.cell0 = c0;
   a.batch = b;
   a.spinpol = spinpol == LCP_SPIN_OFF ? LCP_SPIN_OFF : LCP_SPIN_ON;
-  if (a.spinpol == LCP_SPIN_OFF)
-    return dfl ? launch_gga_t<true, true>(a, n, potential, st) : launch_gga_t<true, false>(a, n, potential, st);
-  return dfl ? launch_gga_t<false, true>(a, n, potential, st) : launch_gga_t<false, false>(a, n, potential, st);
+  const bool off = a.spinpol == LCP_SPIN_OFF;
+  if (dfl) return off ? launch_gga_t<true, true, false>(a, n, potential, st) : launch_gga_t<false, true, false>(a, n, potential, st);
+  if (b.cells || c0.even_weights)
+    return off ? launch_gga_t<true, false, false>(a, n, potential, st) : launch_gga_t<false, false, false>(a, n, potential, st);
+  return off ? launch_gga_t<true, false, true>(a, n, potential, st) : launch_gga_t<false, false, true>(a, n, potential, st);
 }
 
 }  // namespace lcp

@@ -540,11 +540,12 @@ lcp_status hamiltonian_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nch, const
   lcp_status fs = f64_ready(ctx, orbs, kF64Elements, &tc);
   if (fs) return fs;
   if (tc) {
+    const F64Set& set = orbs->f64_elements;
     const lcp::F64HamWork w{ctx->w_f64v.as<int64_t>(), ctx->w_f64e.as<int32_t>(),
-                            ctx->w_f64d.as<double>()};
+                            ctx->w_f64e.as<int32_t>() + set.g.nbricks, ctx->w_f64d.as<double>()};
     for (int c = 0; c < nch; ++c)
-      API_CUDA(lcp::launch_f64_hamiltonian(orbs->f64_elements.g, orbs->pairs, orbs->geom.numorbs, vpot[c], w,
-                                           orbs->ucell->u.gridvol, hks[c], hsize, ctx->w_status.as<int>(), ctx->stream),
+      API_CUDA(lcp::launch_f64_hamiltonian(set.g, set.src, orbs->pairs, vpot[c], w, orbs->ucell->u.gridvol, hks[c],
+                                           hsize, ctx->w_status.as<int>(), ctx->stream),
                "hamiltonian kernel");
     ctx->launches += 3 * nch;
     return LCP_OK;
@@ -1996,7 +1997,7 @@ lcp_status lcp_job_footprint(const lcp_job* job, int64_t* bytes) {
                         &o->o_jatom, &o->o_boff, &o->o_partner, &o->b_scale, &o->b_tmp})
     add(*d);
   for (const F64Set* f : {&o->f64_density, &o->f64_elements})
-    for (const DBuf* d : {&f->bricks, &f->rows, &f->table, &f->ptexp, &f->tab, &f->img_off, &f->img_atom, &f->slot})
+    for (const DBuf* d : {&f->bricks, &f->rows, &f->table, &f->ptexp, &f->cover, &f->tab, &f->img_off, &f->img_atom, &f->slot})
       add(*d);
   for (const DBuf& d : o->f64_pair_buf) add(d);
   if (o->ucell->device == o->device)  // the cell's lists that the tables read

@@ -150,11 +150,13 @@ struct lcp_ctx {
 struct F64Set {
   lcp::F64Bricks g{};
   int state = 0;  // 0 not built, 1 built, -1 beyond the kernels' limits
-  DBuf bricks, rows, table, ptexp, tab;
-  DBuf img_off, img_atom, slot;  // density tiling of tables with gradients, for the force term
+  lcp::F64Source src{};
+  DBuf bricks, rows, table, ptexp, cover, tab;
+  DBuf img_off, img_atom, slot;  // of src; the density tiling's also for the force term
   void release() {
-    for (DBuf* d : {&bricks, &rows, &table, &ptexp, &tab, &img_off, &img_atom, &slot}) d->release();
+    for (DBuf* d : {&bricks, &rows, &table, &ptexp, &cover, &tab, &img_off, &img_atom, &slot}) d->release();
     g = lcp::F64Bricks{};
+    src = lcp::F64Source{};
   }
 };
 

@@ -395,8 +395,18 @@ struct F64Bricks {
   const int32_t* ptexp;        // density: [nbricks * P] E of a point
   const int32_t* tab;          // m x m per brick: offset of the block of the ordered pair (s, t), or for matrix
                                // elements of its partner (t, s), where they are accumulated (s <= t); -1: no pair
+  const uint64_t* cover;       // matrix elements: [nbricks] slots that some image holds (0 beside rows: phi is not finite)
 };
 constexpr int kF64MaxRows = 1000;  // packed rows of a brick the kernels take
+// What a tiling is made from.
+struct F64Source {
+  const double* phi;
+  const int64_t* phi_off;
+  const int32_t* numorbs;
+  const int64_t* img_off;   // [nbricks+1]
+  const int32_t* img_atom;  // [nimg]
+  const int32_t* slot;      // [nimg * P] sphere point of the image's atom at each slot (-1: outside)
+};
 // Ordered pair list of the cell (device pointers) for the brick pair tables and the symmetrised D.
 struct F64Pairs {
   int32_t natom, ncell, cpy;
@@ -441,30 +451,25 @@ struct F64Force {
 cudaError_t launch_f64_force(const F64Bricks& b, const F64Pairs& pr, int nch, const double* const* vpot,
                              const double* const* dm, const double* coef, const F64Force& f, const F64DensWork& w,
                              double gridvol, double* force, int* status, cudaStream_t st);
-// H (one channel) from V, in both orientations, times gridvol.  Workspace: vb
-// (nbricks * 64 words: V by brick), vexp (nbricks ints: its scales) and acc
-// (kF64Copies * hsize doubles: the sums).
+// H (one channel) from V, in both orientations, times gridvol; f: what the
+// tiling was made from, for the bricks that are summed directly.  Workspace: vb
+// (nbricks * 64 words: V by brick), vexp (nbricks ints: its scales), odd
+// (nbricks ints: the bricks summed directly) and acc (kF64Copies * hsize doubles:
+// the sums, then two words: the number of odd, the next unit of their work).
 constexpr int kF64Copies = 8;
 struct F64HamWork {
   int64_t* vb;
   int32_t* vexp;
+  int32_t* odd;
   double* acc;
 };
-cudaError_t launch_f64_hamiltonian(const F64Bricks& b, const DevPairs& folded, const int32_t* numorbs,
-                                   const double* vpot, const F64HamWork& w, double gridvol, double* hks, int64_t hsize,
-                                   int* status, cudaStream_t st);
-// The rows, scales and table of a tiling from the FP64 orbital tables.
-struct F64Build {
-  const double* phi;
-  const int64_t* phi_off;
-  const int32_t* numorbs;
-  const int64_t* img_off;   // [nbricks+1]
-  const int32_t* img_atom;  // [nimg]
-  const int32_t* img_row0;  // [nimg] first row of an image within its brick
-  const int32_t* slot;      // [nimg * P] sphere point of the image's atom at each slot (-1: outside)
-};
-cudaError_t launch_f64_table(const F64Bricks& b, const F64Build& f, F64Row* rows, int32_t* ptexp, uint64_t* table,
-                             cudaStream_t st);
+cudaError_t launch_f64_hamiltonian(const F64Bricks& b, const F64Source& f, const DevPairs& folded, const double* vpot,
+                                   const F64HamWork& w, double gridvol, double* hks, int64_t hsize, int* status,
+                                   cudaStream_t st);
+// The rows, scales, cover and table of a tiling from the FP64 orbital tables
+// (row0: first row of each image within its brick).
+cudaError_t launch_f64_table(const F64Bricks& b, const F64Source& f, const int32_t* row0, F64Row* rows, int32_t* ptexp,
+                             uint64_t* cover, uint64_t* table, cudaStream_t st);
 // Exclusive scan of n int32 into n + 1 int64 (totals: scan_blocks(n) + 1 int64 of scratch).
 int64_t scan_blocks(int64_t n);
 cudaError_t exclusive_scan_i32(const int32_t* in, int64_t n, int64_t* out, int64_t* totals, cudaStream_t st);

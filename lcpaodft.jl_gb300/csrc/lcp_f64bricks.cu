@@ -309,8 +309,8 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   for (int a = 0; a < u.natom; ++a) most = std::max(most, u.sphere_off[a + 1] - u.sphere_off[a]);
   const dim3 pts((unsigned)std::min<int64_t>((most + 1023) / 1024, 256), (unsigned)u.natom);
   // boxes
-  DBuf d_img_off, d_img_atom, d_row_off, d_chunk_off, d_tab_off;
-  DBuf d_box, d_boxes, d_flag, d_cnt, d_key, d_scan, d_per, d_row0, d_slot, d_cc, d_tc;
+  DBuf d_row_off, d_chunk_off, d_tab_off;
+  DBuf d_box, d_boxes, d_flag, d_cnt, d_key, d_scan, d_per, d_row0, d_cc, d_tc;
   std::vector<int32_t> box(6 * (size_t)u.natom);
   for (size_t i = 0; i < box.size(); ++i) box[i] = i % 6 < 3 ? (1 << 30) : -(1 << 30);
   API_CUDA(upload(d_box, box, st), "upload");
@@ -338,7 +338,7 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   API_CUDA(cudaMemsetAsync(d_flag.p, 0, nflag * sizeof(int32_t), st), "memset");
   API_CUDA(d_cnt.ensure(g.nbricks * sizeof(int32_t)), "alloc");
   API_CUDA(cudaMemsetAsync(d_cnt.p, 0, g.nbricks * sizeof(int32_t), st), "memset");
-  API_CUDA(d_img_off.ensure((g.nbricks + 1) * sizeof(int64_t)), "alloc");
+  API_CUDA(S.img_off.ensure((g.nbricks + 1) * sizeof(int64_t)), "alloc");
   API_CUDA(d_row_off.ensure((g.nbricks + 1) * sizeof(int64_t)), "alloc");
   API_CUDA(d_chunk_off.ensure((g.nbricks + 1) * sizeof(int64_t)), "alloc");
   API_CUDA(d_tab_off.ensure((g.nbricks + 1) * sizeof(int64_t)), "alloc");
@@ -348,8 +348,8 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   API_CUDA(cudaGetLastError(), "brick marks");
   f64_images_kernel<false><<<bxs, 256, 0, st>>>(bg, dbx, no, d_flag.as<int32_t>(), d_cnt.as<int32_t>(), nullptr, nullptr);
   API_CUDA(cudaGetLastError(), "brick counts");
-  API_CUDA(exclusive_scan_i32(d_cnt.as<int32_t>(), g.nbricks, d_img_off.as<int64_t>(), d_scan.as<int64_t>(), st), "scan");
-  API_CUDA(cudaMemcpyAsync(&g.nimg, d_img_off.as<int64_t>() + g.nbricks, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "D2H");
+  API_CUDA(exclusive_scan_i32(d_cnt.as<int32_t>(), g.nbricks, S.img_off.as<int64_t>(), d_scan.as<int64_t>(), st), "scan");
+  API_CUDA(cudaMemcpyAsync(&g.nimg, S.img_off.as<int64_t>() + g.nbricks, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "D2H");
   API_CUDA(cudaStreamSynchronize(st), "brick counts");
   if (g.nimg * P >= ((int64_t)1 << 31)) {
     *fits = false;
@@ -358,18 +358,18 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   const int64_t ni = std::max<int64_t>(g.nimg, 1);
   API_CUDA(d_key.ensure(ni * sizeof(uint64_t)), "alloc");
   API_CUDA(d_per.ensure(ni * sizeof(int4)), "alloc");
-  API_CUDA(d_img_atom.ensure(ni * sizeof(int32_t)), "alloc");
-  API_CUDA(d_slot.ensure(ni * P * sizeof(int32_t)), "alloc");
+  API_CUDA(S.img_atom.ensure(ni * sizeof(int32_t)), "alloc");
+  API_CUDA(S.slot.ensure(ni * P * sizeof(int32_t)), "alloc");
   API_CUDA(d_row0.ensure(ni * sizeof(int32_t)), "alloc");
   API_CUDA(d_cc.ensure(g.nbricks * sizeof(int32_t)), "alloc");
   API_CUDA(cudaMemsetAsync(d_cnt.p, 0, g.nbricks * sizeof(int32_t), st), "memset");
   f64_images_kernel<true><<<bxs, 256, 0, st>>>(bg, dbx, no, d_flag.as<int32_t>(), d_cnt.as<int32_t>(),
-                                               d_img_off.as<int64_t>(), d_key.as<uint64_t>());
+                                               S.img_off.as<int64_t>(), d_key.as<uint64_t>());
   API_CUDA(cudaGetLastError(), "brick images");
   API_CUDA(d_tc.ensure(g.nbricks * sizeof(int32_t)), "alloc");
-  f64_sort_kernel<<<blocks_for(g.nbricks * 32), 256, 0, st>>>(bg, dbx, no, g.nbricks, d_img_off.as<int64_t>(),
+  f64_sort_kernel<<<blocks_for(g.nbricks * 32), 256, 0, st>>>(bg, dbx, no, g.nbricks, S.img_off.as<int64_t>(),
                                                               d_key.as<uint64_t>(), d_flag.as<int32_t>(),
-                                                              d_img_atom.as<int32_t>(), d_per.as<int4>(),
+                                                              S.img_atom.as<int32_t>(), d_per.as<int4>(),
                                                               d_row0.as<int32_t>(), d_cnt.as<int32_t>(),
                                                               d_cc.as<int32_t>(), d_tc.as<int32_t>());
   API_CUDA(cudaGetLastError(), "brick sort");
@@ -382,9 +382,9 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   API_CUDA(cudaMemcpyAsync(&g.nrows, d_row_off.as<int64_t>() + g.nbricks, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "D2H");
   API_CUDA(cudaMemcpyAsync(&g.nchunks, d_chunk_off.as<int64_t>() + g.nbricks, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "D2H");
   API_CUDA(cudaMemcpyAsync(rows.data(), d_cnt.p, g.nbricks * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "D2H");
-  f64_fill_kernel<<<blocks_for(ni * P), 256, 0, st>>>(d_slot.as<int32_t>(), g.nimg * P, -1);
+  f64_fill_kernel<<<blocks_for(ni * P), 256, 0, st>>>(S.slot.as<int32_t>(), g.nimg * P, -1);
   API_CUDA(cudaGetLastError(), "brick slots");
-  f64_slot_kernel<<<pts, 256, 0, st>>>(bg, dbx, no, d_flag.as<int32_t>(), d_slot.as<int32_t>());
+  f64_slot_kernel<<<pts, 256, 0, st>>>(bg, dbx, no, d_flag.as<int32_t>(), S.slot.as<int32_t>());
   API_CUDA(cudaGetLastError(), "brick slots");
   API_CUDA(cudaStreamSynchronize(st), "brick rows");
   for (int32_t r : rows) g.max_rows = std::max(g.max_rows, r);
@@ -401,7 +401,7 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   API_CUDA(S.tab.ensure(std::max<int64_t>(ntab, 1) * sizeof(int32_t)), "alloc");
   API_CUDA(S.table.ensure(std::max<int64_t>(g.nchunks, 1) * 32 * P * sizeof(uint64_t)), "alloc");
   API_CUDA(S.bricks.ensure(g.nbricks * sizeof(F64Brick)), "alloc");
-  f64_bricks_kernel<<<blocks_for(g.nbricks), 256, 0, st>>>(g.nbricks, d_img_off.as<int64_t>(), d_row_off.as<int64_t>(),
+  f64_bricks_kernel<<<blocks_for(g.nbricks), 256, 0, st>>>(g.nbricks, S.img_off.as<int64_t>(), d_row_off.as<int64_t>(),
                                                            d_chunk_off.as<int64_t>(), d_tab_off.as<int64_t>(),
                                                            S.bricks.as<F64Brick>());
   API_CUDA(cudaGetLastError(), "bricks");
@@ -414,20 +414,20 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
     f64_fill_kernel<<<blocks_for(g.nbricks * P), 256, 0, st>>>(S.ptexp.as<int32_t>(), g.nbricks * P, 1);
     API_CUDA(cudaGetLastError(), "brick scales");
     g.ptexp = S.ptexp.as<int32_t>();
+  } else {
+    API_CUDA(S.cover.ensure(g.nbricks * sizeof(uint64_t)), "alloc");
+    g.cover = S.cover.as<uint64_t>();
   }
-  const F64Build f{o->phi.as<double>(), o->geom.phi_off, no, d_img_off.as<int64_t>(), d_img_atom.as<int32_t>(),
-                   d_row0.as<int32_t>(), d_slot.as<int32_t>()};
-  API_CUDA(launch_f64_table(g, f, S.rows.as<F64Row>(), S.ptexp.as<int32_t>(), S.table.as<uint64_t>(), st), "brick table");
+  S.src = F64Source{o->phi.as<double>(), o->geom.phi_off, no, S.img_off.as<int64_t>(), S.img_atom.as<int32_t>(),
+                    S.slot.as<int32_t>()};
+  API_CUDA(launch_f64_table(g, S.src, d_row0.as<int32_t>(), S.rows.as<F64Row>(), S.ptexp.as<int32_t>(),
+                            S.cover.as<uint64_t>(), S.table.as<uint64_t>(), st),
+           "brick table");
   f64_tab_kernel<<<(unsigned)std::min<int64_t>(g.nbricks, 152 * 32), 256, 0, st>>>(
-      o->f64_pairs, g.nbricks, d_img_off.as<int64_t>(), d_img_atom.as<int32_t>(), d_per.as<int4>(),
+      o->f64_pairs, g.nbricks, S.img_off.as<int64_t>(), S.img_atom.as<int32_t>(), d_per.as<int4>(),
       d_tab_off.as<int64_t>(), P == 64 ? 1 : 0, S.tab.as<int32_t>());
   API_CUDA(cudaGetLastError(), "brick pairs");
   API_CUDA(cudaStreamSynchronize(st), "brick tables");  // before the scratch above is freed
-  if (P == 128 && o->grad) {  // the force term's epilogue reads the gradient tables by image and point
-    S.img_off.swap(d_img_off);
-    S.img_atom.swap(d_img_atom);
-    S.slot.swap(d_slot);
-  }
   ctx->launches += 20;
   return LCP_OK;
 }
@@ -444,7 +444,10 @@ int64_t f64_footprint_estimate(const lcp_orbs* o) {
     const double rows = lcp::choose_shape(u, P, bd);
     double nb = 1.0;
     for (int d = 0; d < 3; ++d) nb *= (double)((u.ngrid[d] + bd[d] - 1) / bd[d]);
-    bytes += nb * ((rows + 16.0) * (P * 8.0 + 8.0) + rows * rows / 9.0);
+    double no = 0.0;
+    for (int a = 0; a < u.natom; ++a) no += u.numorbs[a];
+    const double images = rows * u.natom / std::max(no, 1.0);
+    bytes += nb * ((rows + 16.0) * (P * 8.0 + 8.0) + images * (images + P + 1.0) * 4.0);
   }
   return (int64_t)bytes;
 }
@@ -518,10 +521,10 @@ lcp_status ensure_f64_workspace(lcp_ctx* ctx, const lcp_orbs* o, bool* ready) {
   const lcp::UCell& u = o->ucell->u;
   const size_t hs = (size_t)u.total_hsize, nb = (size_t)o->f64_elements.g.nbricks, nd = (size_t)o->f64_density.g.nbricks;
   const std::pair<DBuf*, size_t> need[] = {
-      {&ctx->w_f64d, hs * lcp::kF64Copies * sizeof(double)},  // symmetrised D, twice (density); the sums of H
+      {&ctx->w_f64d, (hs * lcp::kF64Copies + 2) * sizeof(double)},  // symmetrised D, twice (density); the sums of H
       {&ctx->w_f64c, (size_t)u.natom * 32 * sizeof(uint32_t)},  // D's column maxima
       {&ctx->w_f64v, std::max<size_t>(nb, 1) * 64 * sizeof(int64_t)},  // V by brick
-      {&ctx->w_f64e, std::max<size_t>(std::max(nb, nd), 1) * sizeof(int32_t)}};   // its scales; D's by brick (density)
+      {&ctx->w_f64e, std::max<size_t>(std::max(2 * nb, nd), 1) * sizeof(int32_t)}};  // its scales and odd bricks; D's by brick (density)
   if (ready) {
     *ready = true;
     for (const auto& n : need) *ready = *ready && n.first->p && n.first->bytes >= n.second;

@@ -222,13 +222,22 @@ int device_sms() {
 namespace {
 
 // Rows and scales, one warp per image (lane = orbital): each row's exponent
-// bound over the brick's points, or each point's over all rows.
-__global__ void __launch_bounds__(256) f64_scales_kernel(F64Bricks b, F64Build f, F64Row* __restrict__ rows,
-                                                         int32_t* __restrict__ ptexp) {
+// bound over the brick's points, or each point's over all rows; with cover, the
+// slots that the images hold, none of a brick where a phi is not finite.
+__global__ void __launch_bounds__(256) f64_scales_kernel(F64Bricks b, F64Source f, const int32_t* __restrict__ row0,
+                                                         F64Row* __restrict__ rows, int32_t* __restrict__ ptexp,
+                                                         uint64_t* __restrict__ cover) {
+  __shared__ uint32_t s_cover[2];
+  __shared__ int s_bad;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int64_t hb = blockIdx.x; hb < b.nbricks; hb += gridDim.x) {
     const int64_t i0 = f.img_off[hb];
     const int m = (int)(f.img_off[hb + 1] - i0);
+    if (cover) {
+      __syncthreads();
+      if (threadIdx.x == 0) s_cover[0] = s_cover[1] = 0, s_bad = 0;
+      __syncthreads();
+    }
     for (int i = warp; i < m; i += nw) {
       const int a = f.img_atom[i0 + i], no = f.numorbs[a];
       const double* src = f.phi + f.phi_off[a] + lane;
@@ -245,16 +254,27 @@ __global__ void __launch_bounds__(256) f64_scales_kernel(F64Bricks b, F64Build f
         }
       }
       if (lane < no)
-        rows[(int64_t)b.bricks[hb].row + f.img_row0[i0 + i] + lane] =
+        rows[(int64_t)b.bricks[hb].row + row0[i0 + i] + lane] =
             F64Row{(uint32_t)no | ((ptexp ? (uint32_t)(a * 32 + lane) : (uint32_t)exp_bound(mx)) << 6),
                    ((uint32_t)i << 8) | (uint32_t)lane};
+      if (cover) {
+        if (lane < no && exp_bound(mx) >= kBadExp) s_bad = 1;
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t in = __ballot_sync(0xffffffffu, sl[h * 32 + lane] >= 0);
+          if (lane == 0) atomicOr(&s_cover[h], in);
+        }
+      }
+    }
+    if (cover) {
+      __syncthreads();
+      if (threadIdx.x == 0) cover[hb] = s_bad ? 0 : ((uint64_t)s_cover[1] << 32) | s_cover[0];
     }
   }
 }
 
 // phi of every row at every slot on its scale's grid: lane = row of a chunk,
 // two slots per store (the phi rows of a point are contiguous over its lanes).
-__global__ void __launch_bounds__(256) f64_table_kernel(F64Bricks b, F64Build f, uint64_t* __restrict__ table) {
+__global__ void __launch_bounds__(256) f64_table_kernel(F64Bricks b, F64Source f, uint64_t* __restrict__ table) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int64_t hb = blockIdx.x; hb < b.nbricks; hb += gridDim.x) {
     const F64Brick br = load_brick(b.bricks + hb);
@@ -381,30 +401,140 @@ struct StepIter : BrickIter {
 
 struct F64HamArgs {
   F64Bricks b;
+  F64Source f;
   F64HamWork w;
+  const double* vpot;
+  const int32_t* nodd;
+  unsigned long long* next;  // unit of the odd bricks' elements
   int64_t hsize;
   int* status;
 };
 
-// V of every slot in brick order as a multiple of 2^-62 of the brick's bound
-// (zero past the grid), and the bounds.
+// V of every slot that an image holds, in brick order, as a multiple of 2^-62 of
+// the brick's bound (zero at the other slots, whatever V holds there), and the bounds.
+//
+// One scale serves all of a brick's pairs, and a pair may hold only those of its
+// points where V is small: what V spans, its elements lose.  So the bricks where
+// V spans more than the kernel should lose are listed as odd and summed directly
+// (their V is zero here): V is not finite; some V but zero lies 2^16 below the
+// largest; or an eighth of the points 2^8.  A sign change of a smooth V does
+// neither: the potentials of SCF steps on cells of 2 to 64 atoms, with and without
+// vacuum, list 0 to 0.06 % of the bricks (up to 0.4 % in the transverse channels
+// of non-collinear spin, which are all sign changes).  A line at 2^12 would list
+// 0.5 % (10 %), one at 2^8 of a single point 8 % (59 %).
 __global__ void __launch_bounds__(kHP) f64_vprep_kernel(F64Bricks b, const double* __restrict__ vpot,
-                                                        int64_t* __restrict__ vb, int32_t* __restrict__ vexp) {
+                                                        int64_t* __restrict__ vb, int32_t* __restrict__ vexp,
+                                                        int32_t* __restrict__ odd, int32_t* __restrict__ nodd) {
   __shared__ uint32_t s[2];
+  __shared__ int far[2];
   const int p = threadIdx.x;
   for (int64_t k = blockIdx.x; k < b.nbricks; k += gridDim.x) {
-    const int64_t gi = p < b.npts ? brick_point_index(k, p, b.bdim, b.nb, b.ngrid) : -1;
+    const uint64_t cover = __ldg(b.cover + k);
+    const int64_t gi = p < b.npts && ((cover >> p) & 1u) ? brick_point_index(k, p, b.bdim, b.nb, b.ngrid) : -1;
     const double v = gi >= 0 ? vpot[gi] : 0.0;
-    const uint32_t h = __reduce_max_sync(0xffffffffu, (uint32_t)__double2hiint(v) & 0x7fffffffu);
+    const uint32_t mine = (uint32_t)__double2hiint(v) & 0x7fffffffu, h = __reduce_max_sync(0xffffffffu, mine);
     if ((p & 31) == 0) s[p >> 5] = h;
     __syncthreads();
     const int E = exp_bound(max(s[0], s[1]));
+    const int below = v != 0.0 ? E - 1 - (int)(mine >> 20) : 0;
+    const int n = __popc(__ballot_sync(0xffffffffu, below > 8)), any = __any_sync(0xffffffffu, below > 16);
+    if ((p & 31) == 0) far[p >> 5] = any ? kHP : n;
+    __syncthreads();
+    const bool is_odd = E >= kBadExp || 8 * (far[0] + far[1]) > __popcll(cover) ||
+                        (cover == 0 && (load_brick(b.bricks + k).size & 0xffffu) > 0);
     int e;
     const uint64_t m = mantissa(v, e) << 10;
     const int64_t t = (int64_t)(m >> min((uint32_t)(E - e), 63u));
-    vb[k * kHP + p] = E >= kBadExp ? 0 : (v < 0.0 ? -t : t);
-    if (p == 0) vexp[k] = E;
-    __syncthreads();
+    vb[k * kHP + p] = is_odd ? 0 : (v < 0.0 ? -t : t);
+    if (p == 0) {
+      vexp[k] = is_odd ? 1 : E;
+      if (is_odd) odd[atomicAdd(nodd, 1)] = (int32_t)k;
+    }
+  }
+}
+
+// The odd bricks' elements as FP64 sums over the points that both images hold,
+// as the pair kernels take them.  A warp claims 32 elements of an image pair at a
+// time: the blocks that run out of bricks early do most of it.  One odd brick of
+// a 2-atom cell's 216 takes 16 us (20 with the units dealt evenly), one of a
+// 64-atom cell's 13,824 nothing that shows; if every one of those is odd, 45 ms
+// (pair kernels 20).
+__device__ __forceinline__ int64_t claim_unit(unsigned long long* next, int lane) {
+  unsigned long long u = 0;
+  if (lane == 0) u = atomicAdd(next, 1ull);
+  return (int64_t)__shfl_sync(0xffffffffu, u, 0);
+}
+__device__ __forceinline__ void odd_elements(const F64HamArgs& A, int nodd) {
+  constexpr int kParts = 8, kAhead = 8;  // units of an image pair; points whose loads are in flight
+  const F64Bricks& B = A.b;
+  const F64Source& f = A.f;
+  const int lane = threadIdx.x & 31;
+  int64_t unit = claim_unit(A.next, lane), base = 0;  // base: the first unit of a brick
+  for (int q0 = 0; q0 < nodd; q0 += 32) {
+    const int kl = q0 + lane < nodd ? A.w.odd[q0 + lane] : -1;
+    const int ml = kl >= 0 ? (int)(load_brick(B.bricks + kl).size >> 16) : 0;
+    for (int q = 0; q < min(32, nodd - q0); ++q) {
+      const int k = __shfl_sync(0xffffffffu, kl, q), m = __shfl_sync(0xffffffffu, ml, q);
+      const int64_t end = base + (int64_t)m * (m + 1) / 2 * kParts;
+      for (; unit < end; unit = claim_unit(A.next, lane)) {
+        // pair (s, t), s <= t, is number t (t + 1) / 2 + s
+        const int part = (int)((unit - base) % kParts), st = (int)((unit - base) / kParts);
+        int t = (int)((sqrtf(8.0f * (float)st + 1.0f) - 1.0f) * 0.5f);
+        while (t * (t + 1) / 2 > st) --t;
+        while ((t + 1) * (t + 2) / 2 <= st) ++t;
+        const int s = st - t * (t + 1) / 2;
+        const int32_t off = B.tab[(int64_t)load_brick(B.bricks + k).tab + s * m + t];
+        if (off < 0) continue;
+        const int64_t i0 = f.img_off[k];
+        const int as = f.img_atom[i0 + s], at = f.img_atom[i0 + t], noi = f.numorbs[as], noj = f.numorbs[at];
+        if (part * 32 >= noi * noj) continue;
+        const double *ps = f.phi + f.phi_off[as], *pt = f.phi + f.phi_off[at];
+        double* acc = A.w.acc + (k & (kF64Copies - 1)) * A.hsize + off;
+        int ks[2], kt[2];
+        double v[2];
+        uint32_t in[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int p = h * 32 + lane;
+          ks[h] = f.slot[(i0 + s) * kHP + p];
+          kt[h] = f.slot[(i0 + t) * kHP + p];
+          const bool both = ks[h] >= 0 && kt[h] >= 0;
+          v[h] = both ? A.vpot[brick_point_index(k, p, B.bdim, B.nb, B.ngrid)] : 0.0;
+          in[h] = __ballot_sync(0xffffffffu, both);
+        }
+        for (int e0 = part * 32; e0 < noi * noj; e0 += 32 * kParts) {
+          const int e = e0 + lane;
+          const bool on = e < noi * noj;
+          const int b = on ? e / noi : 0, a = on ? e - b * noi : 0;
+          double sum = 0.0;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            for (uint32_t left = in[h]; left;) {
+              double x[kAhead], y[kAhead];
+              int n = 0, p[kAhead];
+#pragma unroll
+              for (int j = 0; j < kAhead; ++j) {  // past the last point: that point again, not added
+                p[j] = j > 0 ? p[j - 1] : 0;
+                if (left) {
+                  p[j] = __ffs(left) - 1;
+                  left &= left - 1;
+                  ++n;
+                }
+                x[j] = __ldg(ps + (int64_t)__shfl_sync(0xffffffffu, ks[h], p[j]) * noi + a);
+                y[j] = __ldg(pt + (int64_t)__shfl_sync(0xffffffffu, kt[h], p[j]) * noj + b);
+              }
+#pragma unroll
+              for (int j = 0; j < kAhead; ++j) {
+                const double w = __shfl_sync(0xffffffffu, v[h], p[j]);
+                if (j < n) sum = fma(x[j] * w, y[j], sum);
+              }
+            }
+          }
+          if (on && (s < t || a <= b) && bounds_ok((int64_t)off + e, A.hsize, 20)) atomicAdd(acc + e, sum);
+        }
+      }
+      base = end;
+    }
   }
 }
 
@@ -413,6 +543,7 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
   __shared__ uint64_t afree_bar, bready_bar[2], bempty_bar[2], tfull_bar[2], tempty_bar[2], drain_bar;
   __shared__ uint64_t rawfull_bar[kHRaw];
   __shared__ uint32_t tslot;
+  __shared__ int nodd;
   __shared__ volatile int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int sched = warp & 3, rank = warp >> 2;
@@ -434,6 +565,7 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
     tc::mbar_init(&drain_bar, 1);
     tc::fence_mbar_init();
     abort_flag = 0;
+    nodd = *args.nodd;
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -454,7 +586,6 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
       const F64Row* rows = B.rows + x.b.row;
       const int32_t* tab = B.tab + x.b.tab;
       const int ve = __ldg(args.w.vexp + x.k);
-      const bool bad = ve >= kBadExp;
       double* acc0 = args.w.acc + (x.k & (kF64Copies - 1)) * args.hsize;
       for (int r0 = 0; r0 < R && !abort_flag; r0 += 128) {
         const int rq = r0 + (int)quarter * 32, r = rq + lane;
@@ -466,7 +597,7 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
         // scales beyond these take scalbn below (phi outside 2^-423 .. 2^177, V
         // above 2^377, V phi below 2^-446); rows of zeros have S = 0
         const auto odd_exp = [](int e) { return e > 1 && (e < 600 || e > 1200); };
-        const bool slow_r = __any_sync(0xffffffffu, bad || ve > 1400 ||
+        const bool slow_r = __any_sync(0xffffffffu, ve > 1400 ||
                                                         (r < R && (odd_exp(row_exp(mr.info)) ||
                                                                    (row_exp(mr.info) > 1 && row_exp(mr.info) + ve < 1600))));
         double* acc = acc0 + a;
@@ -512,7 +643,7 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
                 ex[j] = ea + row_exp(__shfl_sync(0xffffffffu, mc.info, cb + j));
                 S[j] = assemble_bounded(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
                 // columns past R have S = 0
-                const bool counts = r_eff <= c0 + cb + j && offs[j] >= 0 && (S[j] != 0 || (bad && c0 + cb + j < R));
+                const bool counts = r_eff <= c0 + cb + j && offs[j] >= 0 && S[j] != 0;
                 offs[j] = counts ? offs[j] + (int)(io & 255u) * noi : -1;
                 v[j] = (double)S[j];
               }
@@ -523,7 +654,7 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
               } else {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                  v[j] = bad ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(v[j], ex[j]);
+                  v[j] = scalbn(v[j], ex[j]);
               }
 #pragma unroll
               for (int j = 0; j < 4; ++j)
@@ -652,6 +783,7 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
   __syncthreads();
   tc::fence_after_sync();
   if (is_mma) tc::tmem_dealloc(tmem, 512);
+  if (nodd > 0) odd_elements(args, nodd);
 }
 
 // The accumulated blocks (the later of a pair's two blocks, [b][a]), their
@@ -1362,10 +1494,10 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
 
 }  // namespace
 
-cudaError_t launch_f64_table(const F64Bricks& b, const F64Build& f, F64Row* rows, int32_t* ptexp, uint64_t* table,
-                             cudaStream_t st) {
+cudaError_t launch_f64_table(const F64Bricks& b, const F64Source& f, const int32_t* row0, F64Row* rows, int32_t* ptexp,
+                             uint64_t* cover, uint64_t* table, cudaStream_t st) {
   const unsigned blocks = (unsigned)std::min<int64_t>(b.nbricks, 152 * 32);
-  f64_scales_kernel<<<blocks, 256, 0, st>>>(b, f, rows, ptexp);
+  f64_scales_kernel<<<blocks, 256, 0, st>>>(b, f, row0, rows, ptexp, cover);
   LCP_CUDA_TRY(cudaGetLastError());
   f64_table_kernel<<<blocks, 256, 0, st>>>(b, f, table);
   return cudaGetLastError();
@@ -1417,18 +1549,20 @@ cudaError_t launch_f64_force(const F64Bricks& b, const F64Pairs& pr, int nch, co
   return cudaSuccess;
 }
 
-cudaError_t launch_f64_hamiltonian(const F64Bricks& b, const DevPairs& folded, const int32_t* numorbs,
-                                   const double* vpot, const F64HamWork& w, double gridvol, double* hks, int64_t hsize,
-                                   int* status, cudaStream_t st) {
+cudaError_t launch_f64_hamiltonian(const F64Bricks& b, const F64Source& f, const DevPairs& folded, const double* vpot,
+                                   const F64HamWork& w, double gridvol, double* hks, int64_t hsize, int* status,
+                                   cudaStream_t st) {
   if (b.nrows == 0 || folded.nu == 0) return cudaMemsetAsync(hks, 0, (size_t)hsize * sizeof(double), st);
-  LCP_CUDA_TRY(cudaMemsetAsync(w.acc, 0, (size_t)hsize * kF64Copies * sizeof(double), st));
-  f64_vprep_kernel<<<(unsigned)std::min<int64_t>(b.nbricks, 152 * 32), kHP, 0, st>>>(b, vpot, w.vb, w.vexp);
+  int32_t* nodd = reinterpret_cast<int32_t*>(w.acc + hsize * kF64Copies);
+  unsigned long long* next = reinterpret_cast<unsigned long long*>(w.acc + hsize * kF64Copies + 1);
+  LCP_CUDA_TRY(cudaMemsetAsync(w.acc, 0, ((size_t)hsize * kF64Copies + 2) * sizeof(double), st));
+  f64_vprep_kernel<<<(unsigned)std::min<int64_t>(b.nbricks, 152 * 32), kHP, 0, st>>>(b, vpot, w.vb, w.vexp, w.odd, nodd);
   LCP_CUDA_TRY(cudaGetLastError());
-  F64HamArgs a{b, w, hsize, status};
+  F64HamArgs a{b, f, w, vpot, nodd, next, hsize, status};
   LCP_CUDA_TRY(raise_smem(f64_hamiltonian_kernel, kHSmemBytes));
   f64_hamiltonian_kernel<<<(unsigned)std::min<int64_t>(b.nbricks, device_sms()), kHThreads, kHSmemBytes, st>>>(a);
   LCP_CUDA_TRY(cudaGetLastError());
-  f64_finish_kernel<<<(unsigned)std::min<int64_t>(folded.nu, 152 * 16), 128, 0, st>>>(folded, numorbs, w.acc, hsize,
+  f64_finish_kernel<<<(unsigned)std::min<int64_t>(folded.nu, 152 * 16), 128, 0, st>>>(folded, f.numorbs, w.acc, hsize,
                                                                                        gridvol, hks);
   return cudaGetLastError();
 }

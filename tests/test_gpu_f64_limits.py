@@ -1,0 +1,98 @@
+"""FP64 density and matrix elements on the tensor cores where their fixed-point
+grids could tell: potentials whose size at points that a pair does not hold is
+out of proportion.
+
+Tolerance, as for the other FP64 comparisons: both sides round like FP64 sums
+of at most a few thousand terms, so they agree to a few hundred units of 2^-53
+of the largest value of the compared part: 1e-13."""
+import numpy as np
+import pytest
+
+import lcpgrid as L
+from lcpgrid.workloads import synthetic_species
+from oracle import lcp_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-13
+
+
+def _cell(lat, pos, spe, paos, ngrid, orbs_of=L.Set_Orbitals_Grid):
+    """Product and oracle cells and the orbital tables (the oracle reads the product's values)."""
+    cut = [paos[s - 1].Spe_Atom_Cut1 for s in spe]
+    no = [paos[s - 1].Spe_Total_NumOrbs for s in spe]
+    args = (1, np.asarray(lat, float), len(spe), spe, np.asarray(pos, float), cut, ngrid, [0, 0, 0])
+    u = L.UCell(*args, Total_NumOrbs=no)
+    orbs = orbs_of(paos, u, ctx=L.Context(0))
+    return u, O.UCell(*args, total_numorbs=no), orbs, [orbs.data(a) for a in range(len(spe))]
+
+
+def _sparse_cell():
+    """Two overlapping atoms (13 and 4 orbitals) and a third apart, in a box with empty corners."""
+    paos = [synthetic_species(81, rc=4.0), synthetic_species(82, max_l=1, num_basis=(1, 1), rc=4.5)]
+    return _cell(np.diag([15.0, 15.5, 16.0]), [[4.0, 4.1, 4.2], [9.0, 4.5, 5.0], [10.5, 10.8, 11.0]], [1, 2, 1], paos,
+                 (24, 25, 23))
+
+
+def _counts(u):
+    """Spheres (images included) that hold each grid point, and those of atom 1."""
+    n = np.zeros(u.NN, int)
+    for a in range(3):
+        np.add.at(n, u.GridListAtom[a], 1)
+    first = np.zeros(u.NN, int)
+    np.add.at(first, u.GridListAtom[0], 1)
+    return n, first
+
+
+def _pair(u, atom, jatom):
+    return [p for p in range(u.Nloop) if u.MPI_atom[p] == atom and u.MPI_natn[p] == jatom]
+
+
+def _block(u, p):
+    n = int(u.Total_NumOrbs[u.MPI_atom[p] - 1]) * int(u.Total_NumOrbs[u.MPI_natn[p] - 1])
+    return slice(int(u.block_offset[p]), int(u.block_offset[p]) + n)
+
+
+@pytest.mark.parametrize("value", [2.0 ** 6, 1e6, 1e12, 1e300, np.inf, np.nan])
+@pytest.mark.parametrize("where", ["no_sphere", "first_sphere"])
+def test_elements_do_not_see_v_outside_the_pair(where, value):
+    """A pair's elements depend on V at the points that both its spheres hold, and on no other."""
+    u, uo, orbs, phi = _sparse_cell()
+    n, first = _counts(u)
+    v = np.random.default_rng(7).normal(size=u.NN)
+    at = np.flatnonzero(n == 0 if where == "no_sphere" else (n == 1) & (first == 1))
+    if where == "first_sphere":
+        at = at[::5]
+    assert at.size > 100
+    bad = v.copy()
+    bad[at] = value
+    h = [np.zeros(u.Total_Hsize)]
+    L.Calc_MatrixElements_dVH_Vxc_off(u, orbs, [bad], h)
+    with np.errstate(invalid="ignore"):
+        ref = O.calc_matrix_elements(uo, phi, [bad], 1)[0]
+    same = O.calc_matrix_elements(uo, phi, [v], 1)[0]
+    own = _pair(u, 1, 1)[0]  # the self pair of the first atom comes first
+    for p in range(u.Nloop):
+        b = _block(u, p)
+        if where == "first_sphere" and p == own:
+            assert np.array_equal(np.isfinite(h[0][b]), np.isfinite(ref[b]))
+            if np.isfinite(value):
+                assert np.max(np.abs(h[0][b] - ref[b])) <= TOL * np.max(np.abs(ref[b]))
+            continue
+        assert np.max(np.abs(h[0][b] - same[b])) <= TOL * np.max(np.abs(same[b])) + 1e-300, (p, value)
+
+
+def test_elements_of_one_infinite_point():
+    """One infinite V inside two overlapping spheres: infinities of the oracle's signs, nothing elsewhere."""
+    u, uo, orbs, phi = _sparse_cell()
+    n, first = _counts(u)
+    v = np.random.default_rng(8).normal(size=u.NN)
+    v[np.flatnonzero((n == 2) & (first == 1))[3]] = -np.inf
+    h = [np.zeros(u.Total_Hsize)]
+    L.Calc_MatrixElements_dVH_Vxc_off(u, orbs, [v], h)
+    with np.errstate(invalid="ignore"):
+        ref = O.calc_matrix_elements(uo, phi, [v], 1)[0]
+    ok = np.isfinite(ref)
+    assert not ok.all() and np.array_equal(np.isfinite(h[0]), ok)
+    assert np.array_equal(h[0][np.isinf(ref)], ref[np.isinf(ref)])
+    assert np.max(np.abs(h[0][ok] - ref[ok])) <= TOL * np.max(np.abs(ref[ok]))

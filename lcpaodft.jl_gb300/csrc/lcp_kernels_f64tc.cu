@@ -1105,6 +1105,18 @@ __device__ __forceinline__ void gather_b(const uint64_t* __restrict__ dfix, cons
   }
 }
 
+// The 192-bit integer w2:w1:w0 >> n, 0 <= n < 192 (n the same in a warp).
+__device__ __forceinline__ void shift_down(uint64_t& w0, uint64_t& w1, int64_t& w2, int n) {
+  for (; n >= 64; n -= 64) {
+    w0 = w1;
+    w1 = (uint64_t)w2;
+    w2 >>= 63;
+  }
+  w0 = (w0 >> n) | (w1 << 1) << (63 - n);
+  w1 = (w1 >> n) | ((uint64_t)w2 << 1) << (63 - n);
+  w2 >>= n;
+}
+
 // The sums of three values over the warp: of the first in lane 0, of the
 // second in lane 8, of the third in lane 16 (six additions, not fifteen).
 __device__ __forceinline__ double warp_sum3(double v0, double v1, double v2, int lane) {
@@ -1255,9 +1267,10 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
         // S, a multiple of 2^-54 of the scales' product, stays below 2^63 for R < 512
         // (|X| <= R); with more rows Ds is split on a grid one bit coarser.  The sum
         // of X phi is a 128-bit integer in units 2^-54 2^-62 of the scales' product
-        // with the brick's largest column scale (phi shifted up by what the column's
-        // scale lies below it, at most seven bits, beyond that S down)
-        uint64_t slo = 0;
+        // with the brick's largest column scale (phi shifted up by seven bits less what
+        // the column's scale lies below it, beyond that the product down, into 64 more
+        // bits below: a column 2^-128 of the largest keeps 52 bits of its own)
+        uint64_t slo = 0, sx = 0;
         int64_t shi = 0;
         bool nan = false;
         const int etop = __ldg(args.btop + x.k);
@@ -1296,20 +1309,29 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
               tp[j] = (int64_t)((uint64_t)(uint32_t)t * m + ((uint64_t)((uint32_t)(t >> 32) * m) << 32));
               S[j] = assemble(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
             }
-            if (odd) {  // columns far below the brick's largest, or with Inf or NaN
+            if (!odd) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint64_t lo = (uint64_t)S[j] * (uint64_t)tp[j];
+                slo += lo;
+                shi += __mul64hi(S[j], tp[j]) + (slo < lo ? 1 : 0);
+              }
+            } else {  // columns far below the brick's largest, or with Inf or NaN
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 const int d = __shfl_sync(0xffffffffu, ce, cb + j);
                 nan = nan || (d < 0 && ph[j] != kF64Bias);
                 if (d < 0) S[j] = 0;
-                S[j] >>= min(max(d - 7, 0), 63);
+                uint64_t w0 = 0, w1 = (uint64_t)S[j] * (uint64_t)tp[j];
+                int64_t w2 = __mul64hi(S[j], tp[j]);
+                shift_down(w0, w1, w2, min(max(d - 7, 0), 191));
+                sx += w0;
+                const uint64_t c = sx < w0 ? 1 : 0;
+                slo += w1;
+                shi += w2 + (slo < w1 ? 1 : 0);
+                slo += c;
+                shi += slo < c ? 1 : 0;
               }
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint64_t lo = (uint64_t)S[j] * (uint64_t)tp[j];
-              slo += lo;
-              shi += __mul64hi(S[j], tp[j]) + (slo < lo ? 1 : 0);
             }
             if (q < 3) {
 #pragma unroll
@@ -1324,10 +1346,11 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
         const int64_t gi = p < B.npts ? brick_point_index(x.k, p, B.bdim, B.nb, B.ngrid) : -1;
         const bool neg = shi < 0;
         if (neg) {
-          slo = ~slo + 1;
-          shi = ~shi + (slo == 0 ? 1 : 0);
+          sx = ~sx + 1;
+          slo = ~slo + (sx == 0 ? 1 : 0);
+          shi = ~shi + (sx == 0 && slo == 0 ? 1 : 0);
         }
-        double acc = fma((double)shi, 0x1p64, (double)slo);
+        double acc = fma((double)shi, 0x1p64, fma((double)sx, 0x1p-64, (double)slo));
         if (neg) acc = -acc;
         if (nan) acc = __longlong_as_double(0x7ff8000000000000ll);
         // two halves onto a zeroed point: the same sum in either order

@@ -1,6 +1,6 @@
 """FP64 density and matrix elements on the tensor cores where their fixed-point
 grids could tell: potentials whose size at points that a pair does not hold is
-out of proportion.
+out of proportion, columns of D far below the others'.
 
 Tolerance, as for the other FP64 comparisons: both sides round like FP64 sums
 of at most a few thousand terms, so they agree to a few hundred units of 2^-53
@@ -96,3 +96,23 @@ def test_elements_of_one_infinite_point():
     assert not ok.all() and np.array_equal(np.isfinite(h[0]), ok)
     assert np.array_equal(h[0][np.isinf(ref)], ref[np.isinf(ref)])
     assert np.max(np.abs(h[0][ok] - ref[ok])) <= TOL * np.max(np.abs(ref[ok]))
+
+
+@pytest.mark.parametrize("shift", [6, 9, 40, 100])
+def test_density_of_an_atom_with_a_small_d(shift):
+    """An atom whose D is 2^-shift of its neighbour's keeps its own accuracy where it is alone."""
+    u, uo, orbs, phi = _sparse_cell()
+    rng = np.random.default_rng(shift)
+    dm = np.zeros(u.Total_Hsize)
+    for p in range(u.Nloop):
+        if u.MPI_atom[p] == u.MPI_natn[p]:
+            dm[_block(u, p)] = rng.normal(size=dm[_block(u, p)].size) * (2.0 ** -shift if u.MPI_atom[p] == 2 else 1.0)
+    rho = [np.zeros(u.NN)]
+    L.Set_Density_Grid("off", u, orbs, [dm], rho)
+    ref = O.set_density_grid("off", uo, phi, [dm])[0]
+    n, _ = _counts(u)
+    second = np.zeros(u.NN, bool)
+    second[u.GridListAtom[1]] = True
+    alone = second & (n == 1)
+    for part in (alone, ~second):
+        assert np.max(np.abs(rho[0] - ref)[part]) <= TOL * np.max(np.abs(ref[part]))

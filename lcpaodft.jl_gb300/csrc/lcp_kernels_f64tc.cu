@@ -1105,6 +1105,16 @@ __device__ __forceinline__ void gather_b(const uint64_t* __restrict__ dfix, cons
   }
 }
 
+// Bits by which a brick of R rows aligns its columns' products: the sum of X phi
+// over the columns is at most sum_c sum_{r <= c} |phi_r phi_c| < (R^2 + R) / 2 in
+// units of the scales' product, and the 128-bit sum holds 2^18-base of them.
+// (Seven for any R wrapped the sum from 90 to 130 rows of like size and sign on.)
+__device__ __forceinline__ int align_bits(int R) {
+  int base = 7;
+  while ((R * R + R) / 2 >= 1 << (18 - base)) --base;
+  return base;  // 7 to 63 rows, 3 at 200, -1 at 1,000
+}
+
 // The 192-bit integer w2:w1:w0 >> n, 0 <= n < 192 (n the same in a warp).
 __device__ __forceinline__ void shift_down(uint64_t& w0, uint64_t& w1, int64_t& w2, int n) {
   for (; n >= 64; n -= 64) {
@@ -1266,11 +1276,12 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
         const uint64_t* mine = B.table + (int64_t)x.b.chunk * 32 * kDP + (p >> 3) * 256 + ((p & 7) >> 1) * 64 + (p & 1);
         // S, a multiple of 2^-54 of the scales' product, stays below 2^63 for R < 512
         // (|X| <= R); with more rows Ds is split on a grid one bit coarser.  The sum
-        // of X phi is a 128-bit integer in units 2^-54 2^-62 of the scales' product
-        // with the brick's largest column scale (phi shifted up by seven bits less what
-        // the column's scale lies below it, beyond that the product down, into 64 more
-        // bits below: a column 2^-128 of the largest keeps 52 bits of its own)
+        // of X phi is a 128-bit integer in units 2^-54 2^-(55 + base) of the scales'
+        // product with the brick's largest column scale (phi shifted up by base less
+        // what the column's scale lies below it, beyond that the product down, into 64
+        // more bits below: a column 2^-120 of the largest keeps 52 bits of its own)
         uint64_t slo = 0, sx = 0;
+        const int base = align_bits(R);
         int64_t shi = 0;
         bool nan = false;
         const int etop = __ldg(args.btop + x.k);
@@ -1281,8 +1292,8 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
           int ce = 0;
           if (c0 + lane < R)
             ce = etop - exp_bound(__ldg(args.cmax + row_col(load_meta(B.rows + x.b.row + c0 + lane).info)));
-          const bool odd = __any_sync(0xffffffffu, ce < 0 || ce > 7);
-          const uint32_t up = 128u >> min(max(ce, 0), 7);
+          const bool odd = __any_sync(0xffffffffu, ce < 0 || ce > base);
+          const uint32_t up = 1u << min(max(base - ce, 0), 7);
           const uint64_t* phi = mine + (int64_t)(c0 / 32) * 32 * kDP;
           uint64_t ph[4];
 #pragma unroll
@@ -1324,7 +1335,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
                 if (d < 0) S[j] = 0;
                 uint64_t w0 = 0, w1 = (uint64_t)S[j] * (uint64_t)tp[j];
                 int64_t w2 = __mul64hi(S[j], tp[j]);
-                shift_down(w0, w1, w2, min(max(d - 7, 0), 191));
+                shift_down(w0, w1, w2, min(max(d - base, 0), 191));
                 sx += w0;
                 const uint64_t c = sx < w0 ? 1 : 0;
                 slo += w1;
@@ -1355,7 +1366,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
         if (nan) acc = __longlong_as_double(0x7ff8000000000000ll);
         // two halves onto a zeroed point: the same sum in either order
         if (gi >= 0 && bounds_ok(gi, (int64_t)B.ngrid[0] * B.ngrid[1] * B.ngrid[2], 21))
-          atomicAdd(args.rho + gi, scalbn(acc, 2 * (B.ptexp[(int64_t)x.k * kDP + p] - 1023) + etop - 1023 - 116));
+          atomicAdd(args.rho + gi, scalbn(acc, 2 * (B.ptexp[(int64_t)x.k * kDP + p] - 1023) + etop - 1023 - 109 - base));
       }
     }
   } else if (warp == kDEpi) {

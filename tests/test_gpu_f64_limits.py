@@ -1,6 +1,6 @@
 """FP64 density and matrix elements on the tensor cores where their fixed-point
 grids could tell: potentials whose size at points that a pair does not hold is
-out of proportion, columns of D far below the others'.
+out of proportion, many rows of like size and sign, columns of D far below the others'.
 
 Tolerance, as for the other FP64 comparisons: both sides round like FP64 sums
 of at most a few thousand terms, so they agree to a few hundred units of 2^-53
@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 import lcpgrid as L
+from lcpgrid.pao import PAO
 from lcpgrid.workloads import synthetic_species
 from oracle import lcp_oracle as O
 
@@ -116,3 +117,32 @@ def test_density_of_an_atom_with_a_small_d(shift):
     alone = second & (n == 1)
     for part in (alone, ~second):
         assert np.max(np.abs(rho[0] - ref)[part]) <= TOL * np.max(np.abs(ref[part]))
+
+
+def _flat(nfun, values):
+    """nfun s functions of constant value inside the cutoff."""
+    rv = np.exp(np.linspace(np.log(1e-4), np.log(7.0), 400))
+    return PAO(0, [nfun], rv, [[np.full(rv.size, float(x)) for x in values]], Spe_Atom_Cut1=6.0)
+
+
+def _flat_cell(nfun, values):
+    """At every point all orbitals of dozens of images count alike: 160 to 900 rows at a brick."""
+    return _cell(np.diag([5.0] * 3), [[0.1, 0.2, 0.3], [2.0, 2.6, 1.1]], [1, 1], [_flat(nfun, values)], (12, 12, 12))
+
+
+@pytest.mark.parametrize("nfun", [2, 8, 16, 32])
+def test_density_of_many_like_rows(nfun):
+    """Rows and D of one sign and nearly one size, up to the most rows that a brick
+    takes: the sums over rows and columns are as large as they can be."""
+    rng = np.random.default_rng(nfun)
+    u, uo, orbs, phi = _flat_cell(nfun, np.ones(nfun))
+    dm = np.ones(u.Total_Hsize)
+    rho = [np.zeros(u.NN)]
+    L.Set_Density_Grid("off", u, orbs, [dm], rho)
+    ref = O.set_density_grid("off", uo, phi, [dm])[0]
+    assert np.max(np.abs(rho[0] - ref) / ref) <= TOL
+    v = 1.0 + 0.1 * rng.uniform(size=u.NN)
+    h = [np.zeros(u.Total_Hsize)]
+    L.Calc_MatrixElements_dVH_Vxc_off(u, orbs, [v], h)
+    ref = O.calc_matrix_elements(uo, phi, [v], 1)[0]
+    assert np.max(np.abs(h[0] - ref)) <= TOL * np.max(np.abs(ref))

@@ -13,8 +13,8 @@
 // operands is the 28 digit products d_i d_j' with i + j <= 8, each group of
 // equal weight (i + j = d + 1) in its own FP32 accumulator a_d.  Over 64 terms
 // |a_d| <= d 2^20 < 2^24, so every sum is exact in the matrix elements; in the
-// density (up to R packed rows) the first R d <= 1024 groups are exact for any
-// values.  The dropped groups are below 2^-62 of the scales' product.  What is
+// density, over segments of 256 rows, a_1 to a_4 are, for any values (kDSeg).
+// The dropped groups are below 2^-62 of the scales' product.  What is
 // rounded: each operand once to 2^-56 of its row's (column's, point's) largest
 // value, the assembled sum once to 2^-55 of the scales' product, and the FP64
 // additions that follow.  An FP64 FMA chain rounds every partial sum to 2^-53
@@ -861,6 +861,24 @@ constexpr int kDPiecesB = 4;  // of a chunk's B (8 rows each), taken in turn by 
 constexpr int kDThreads = 32 * (kDEpi + 1 + kDConv);
 static_assert(kF64ForceParts == kDEpi * 3, "three sums per image and epilogue warp");
 constexpr int kDChunk = 32;
+// Rows that one accumulator sums.  |a_d| <= d 2^14 a row, and above 2^24 an MMA
+// step truncates; over 256 rows a_1 to a_4 are exact for any digits.  a_5 loses
+// 2^-46 of the scales' product a step only if its five digit products average more
+// than 0.8 of their largest over a segment; a_6 and a_7 2^-54 and less.  More rows
+// of a window are further segments, each with its own buffer and turn of the
+// epilogue, which adds up X phi anyway.  (Without segments a_2 is truncated from
+// 512 rows on: with 830 that count at a point and large leading digits rho was off
+// by 3e-10.)  192 rows would make a_5 exact for any digits too, at 3 % of a step;
+// 256 are all that most bricks of cells of 13-orbital atoms have (two segments take
+// 0.8 % of the step of a 20-atom 18-orbital cell, 330 rows).  The force term takes
+// 320: a_4 then loses 2^-38 a step only if its four products average 0.8 of their
+// largest, the leading digits among them, which takes phi of one size in all rows
+// (4- to 18-orbital cells: their sum is 11 to 53 times the largest).  A second segment
+// of a few rows repeats its epilogue with the gradients: at 256 rows the bricks of
+// 260 of a 16-atom cell made the kernel 12 % slower.
+template <bool FORCE>
+constexpr int kDSeg = FORCE ? 320 : 256;
+static_assert(kDSeg<false> % kDChunk == 0 && kDSeg<true> % kDChunk == 0, "segments are whole chunks");
 constexpr uint32_t kDStages = 2;
 constexpr uint32_t kDEmpty = 4;  // barriers of the chunks' releases, chunk n's at n % 4
 static_assert(kDConvB <= 2 * kDPiecesB && kDEmpty >= 2 * kDStages, "a split warp passes over one chunk at most");
@@ -872,8 +890,7 @@ constexpr uint32_t kDStageBytes = kDig * kDADigit + kDBBytes;  // 70 KB
 constexpr size_t kDSmemBytes = kDStages * (size_t)kDStageBytes + kDRaw * (size_t)kRawBytes;  // 204 KB
 static_assert(2 * kRawBytes == 32 * kDP * 8, "a raw slot is half a chunk");
 
-// sum a_d 256^(7-d) / 256, rounded, for |a_d| <= 2^24 (d <= 5; a_6 and a_7 may
-// round in their last places, 2^-54 of the result's scale and below).
+// sum a_d 256^(7-d) / 256, rounded, over a segment: the sum is below 2^63.
 __device__ __forceinline__ int64_t assemble(uint32_t u1, uint32_t u2, uint32_t u3, uint32_t u4, uint32_t u5, uint32_t u6,
                                             uint32_t u7) {
   constexpr float M = 12582912.0f;
@@ -891,7 +908,7 @@ __device__ __forceinline__ int64_t assemble(uint32_t u1, uint32_t u2, uint32_t u
 struct F64DensArgs {
   F64Bricks b;
   const uint64_t* dfix;
-  const uint32_t* cmax;  // [natom * 32] high word of max |Ds| of a column, raised by the grid's slack
+  const uint32_t* cmax;  // [natom * 32] high word of max |Ds| of a column
   const int32_t* btop;   // [nbricks] exponent bound of the largest finite column of a brick
   double* rho;
   F64Force f;            // force term only
@@ -901,8 +918,7 @@ struct F64DensArgs {
 // Ds per ordered pair and the largest magnitude of each column (orbital b of
 // the neighbour atom), one block per pair.
 __global__ void __launch_bounds__(128) f64_dsym_kernel(F64Pairs pr, const double* __restrict__ dm,
-                                                       double* __restrict__ dsym, uint32_t* __restrict__ cmax,
-                                                       int slack) {
+                                                       double* __restrict__ dsym, uint32_t* __restrict__ cmax) {
   __shared__ uint32_t mx[32];
   for (int64_t p = blockIdx.x; p < pr.npairs; p += gridDim.x) {
     const int i = pr.atom[p], j = pr.jatom[p];
@@ -919,10 +935,7 @@ __global__ void __launch_bounds__(128) f64_dsym_kernel(F64Pairs pr, const double
       atomicMax(&mx[b], (uint32_t)__double2hiint(v) & 0x7fffffffu);
     }
     __syncthreads();
-    if (threadIdx.x < noj) {
-      const uint32_t h = mx[threadIdx.x];
-      atomicMax(cmax + (int64_t)j * 32 + threadIdx.x, h < 0x7fe00000u ? h + ((uint32_t)slack << 20) : h);
-    }
+    if (threadIdx.x < noj) atomicMax(cmax + (int64_t)j * 32 + threadIdx.x, mx[threadIdx.x]);
     __syncthreads();
   }
 }
@@ -947,7 +960,7 @@ __global__ void __launch_bounds__(256) f64_btop_kernel(F64Bricks b, const uint32
 // Force term: the largest magnitude of every row of D over its pairs (the
 // columns of the product: orbital a of the pair's first atom), one block per pair.
 __global__ void __launch_bounds__(128) f64_drow_kernel(F64Pairs pr, const double* __restrict__ dm,
-                                                       uint32_t* __restrict__ cmax, int slack) {
+                                                       uint32_t* __restrict__ cmax) {
   __shared__ uint32_t mx[32];
   for (int64_t p = blockIdx.x; p < pr.npairs; p += gridDim.x) {
     const int i = pr.atom[p], noi = pr.numorbs[i], noj = pr.numorbs[pr.jatom[p]];
@@ -957,10 +970,7 @@ __global__ void __launch_bounds__(128) f64_drow_kernel(F64Pairs pr, const double
     for (int e = threadIdx.x; e < noi * noj; e += blockDim.x)
       atomicMax(&mx[e / noj], (uint32_t)__double2hiint(dm[bp + e]) & 0x7fffffffu);
     __syncthreads();
-    if (threadIdx.x < noi) {
-      const uint32_t h = mx[threadIdx.x];
-      atomicMax(cmax + (int64_t)i * 32 + threadIdx.x, h < 0x7fe00000u ? h + ((uint32_t)slack << 20) : h);
-    }
+    if (threadIdx.x < noi) atomicMax(cmax + (int64_t)i * 32 + threadIdx.x, mx[threadIdx.x]);
     __syncthreads();
   }
 }
@@ -1022,6 +1032,15 @@ __global__ void __launch_bounds__(128) f64_dfix_kernel(F64Pairs pr, const double
 template <bool FORCE>
 __device__ __forceinline__ int last_chunk(int c0, int R) {
   return FORCE ? (R - 1) & ~(kDChunk - 1) : c0;
+}
+// The segment of rows after r0 of window c0, or the next window's first.
+template <bool FORCE>
+__device__ __forceinline__ void next_segment(int& c0, int& r0, int R) {
+  r0 += kDSeg<FORCE>;
+  if (r0 > last_chunk<FORCE>(c0, R)) {
+    r0 = 0;
+    c0 += kWin;
+  }
 }
 template <bool FORCE, bool AHEAD>
 struct ChunkIter : BrickIterT<AHEAD> {
@@ -1144,6 +1163,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[kDStages], empty_bar[kDEmpty], tfull_bar[2], tempty_bar[2], drain_bar;
   __shared__ uint64_t rawfull_bar[kDRaw];
+  __shared__ uint64_t s_low[FORCE ? 1 : 32 * kDEpi];  // the low word of the points' sums
   __shared__ uint32_t tslot;
   __shared__ volatile int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1195,7 +1215,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
           f0 = f1 = f2 = 0.0;
           in = false;
         };
-        for (int c0 = 0; c0 < R && !abort_flag; c0 += kWin, ++win) {
+        for (int c0 = 0, r0 = 0; c0 < R && !abort_flag; ++win) {  // segment r0 of window c0
           const uint32_t buf = win & 1;
           F64Row mc{};
           int ce = 1;
@@ -1265,6 +1285,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(&tempty_bar[buf]);
+          next_segment<FORCE>(c0, r0, R);
         }
         if (abort_flag) break;
         if (cur >= 0) flush();
@@ -1274,18 +1295,18 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
       for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
         const int R = x.R();
         const uint64_t* mine = B.table + (int64_t)x.b.chunk * 32 * kDP + (p >> 3) * 256 + ((p & 7) >> 1) * 64 + (p & 1);
-        // S, a multiple of 2^-54 of the scales' product, stays below 2^63 for R < 512
-        // (|X| <= R); with more rows Ds is split on a grid one bit coarser.  The sum
+        // S, a multiple of 2^-54 of the scales' product, is a segment's part of X.  The sum
         // of X phi is a 128-bit integer in units 2^-54 2^-(55 + base) of the scales'
         // product with the brick's largest column scale (phi shifted up by base less
         // what the column's scale lies below it, beyond that the product down, into 64
         // more bits below: a column 2^-120 of the largest keeps 52 bits of its own)
-        uint64_t slo = 0, sx = 0;
+        uint64_t slo = 0;
+        s_low[tid] = 0;  // not in registers: the kernel has none left, and few windows need it
         const int base = align_bits(R);
         int64_t shi = 0;
         bool nan = false;
         const int etop = __ldg(args.btop + x.k);
-        for (int c0 = 0; c0 < R && !abort_flag; c0 += kWin, ++win) {
+        for (int c0 = 0, r0 = 0; c0 < R && !abort_flag; ++win) {  // segment r0 of window c0
           const uint32_t buf = win & 1;
           // lane l keeps how far column c0 + l's scale lies below the brick's
           // largest, for the shuffles below
@@ -1320,29 +1341,31 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
               tp[j] = (int64_t)((uint64_t)(uint32_t)t * m + ((uint64_t)((uint32_t)(t >> 32) * m) << 32));
               S[j] = assemble(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
             }
-            if (!odd) {
+            if (odd) {  // columns far below the brick's largest, or with Inf or NaN
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const uint64_t lo = (uint64_t)S[j] * (uint64_t)tp[j];
-                slo += lo;
-                shi += __mul64hi(S[j], tp[j]) + (slo < lo ? 1 : 0);
-              }
-            } else {  // columns far below the brick's largest, or with Inf or NaN
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const int d = __shfl_sync(0xffffffffu, ce, cb + j);
+                const int d = __shfl_sync(0xffffffffu, ce, cb + j), n = min(max(d - base, 0), 191);
                 nan = nan || (d < 0 && ph[j] != kF64Bias);
                 if (d < 0) S[j] = 0;
-                uint64_t w0 = 0, w1 = (uint64_t)S[j] * (uint64_t)tp[j];
-                int64_t w2 = __mul64hi(S[j], tp[j]);
-                shift_down(w0, w1, w2, min(max(d - base, 0), 191));
-                sx += w0;
-                const uint64_t c = sx < w0 ? 1 : 0;
+                // S tp >> n = (S >> n) tp + ((S mod 2^n) tp >> n): the second part here
+                const int64_t x = n < 64 ? S[j] & ((1ll << n) - 1) : S[j];
+                S[j] = n < 64 ? S[j] >> n : 0;
+                uint64_t w0 = 0, w1 = (uint64_t)x * (uint64_t)tp[j];
+                int64_t w2 = __mul64hi(x, tp[j]);
+                shift_down(w0, w1, w2, n);
+                const uint64_t low = s_low[tid] + w0, c = low < w0 ? 1 : 0;
+                s_low[tid] = low;
                 slo += w1;
                 shi += w2 + (slo < w1 ? 1 : 0);
                 slo += c;
                 shi += slo < c ? 1 : 0;
               }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint64_t lo = (uint64_t)S[j] * (uint64_t)tp[j];
+              slo += lo;
+              shi += __mul64hi(S[j], tp[j]) + (slo < lo ? 1 : 0);
             }
             if (q < 3) {
 #pragma unroll
@@ -1352,9 +1375,11 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(&tempty_bar[buf]);
+          next_segment<FORCE>(c0, r0, R);
         }
         if (abort_flag) break;
         const int64_t gi = p < B.npts ? brick_point_index(x.k, p, B.bdim, B.nb, B.ngrid) : -1;
+        uint64_t sx = s_low[tid];
         const bool neg = shi < 0;
         if (neg) {
           sx = ~sx + 1;
@@ -1386,42 +1411,45 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
     BrickIter x;
     for (x.start(B); x.valid() && !abort_flag; x.next(B)) {
       const int R = x.R();
-      for (int c0 = 0; c0 < R && !abort_flag; c0 += kWin, ++win) {
-        const uint32_t buf = win & 1;
-        if (win >= 2 && !tc::mbar_wait_warp(&tempty_bar[buf], ((win >> 1) - 1) & 1, &abort_flag)) {
-          give_up();
-          break;
-        }
-        const uint32_t d0 = tmem + buf * kBufCols;
+      for (int c0 = 0; c0 < R && !abort_flag; c0 += kWin) {
         const int last = last_chunk<FORCE>(c0, R);
-        for (int r0 = 0; r0 <= last; r0 += kDChunk) {
-          if (!tc::mbar_wait_warp(&full_bar[st], par, &abort_flag)) {
+        for (int s0 = 0; s0 <= last && !abort_flag; s0 += kDSeg<FORCE>, ++win) {
+          const uint32_t buf = win & 1;
+          if (win >= 2 && !tc::mbar_wait_warp(&tempty_bar[buf], ((win >> 1) - 1) & 1, &abort_flag)) {
             give_up();
             break;
           }
-          tc::fence_after_sync();
-          const uint32_t a0 = tc::smem_u32(smem + st * kDStageBytes), b0 = a0 + kDig * kDADigit;
-#pragma unroll
-          for (int ks = 0; ks < kDChunk / 16; ++ks) {
-            const uint64_t db = tc::smem_desc(b0 + ks * 2 * kDBLbo, kDBLbo, 128);
-#pragma unroll
-            for (int i = 0; i < kDig; ++i) {
-              const uint64_t da = tc::smem_desc(a0 + i * kDADigit + ks * 256, 128, 512);
-              if (tc::elect_one())
-                tc::mma_bf16(d0 + kWin * i, da, db, idesc_f16_f32(128, kWin * (kDig - i), 1, 0),
-                             (r0 > 0 || ks > 0 || i > 0) ? 1u : 0u);
+          const uint32_t d0 = tmem + buf * kBufCols;
+          const int end = min(s0 + kDSeg<FORCE> - kDChunk, last);
+          for (int r0 = s0; r0 <= end; r0 += kDChunk) {
+            if (!tc::mbar_wait_warp(&full_bar[st], par, &abort_flag)) {
+              give_up();
+              break;
             }
-          }
-          if (tc::elect_one()) {
-            tc::mma_commit(&empty_bar[chunk % kDEmpty]);
-            if (r0 == last) tc::mma_commit(&tfull_bar[buf]);
-          }
-          __syncwarp();
-          fetch();  // into this chunk's slots: its A is split
-          ++chunk;
-          if (++st == kDStages) {
-            st = 0;
-            par ^= 1;
+            tc::fence_after_sync();
+            const uint32_t a0 = tc::smem_u32(smem + st * kDStageBytes), b0 = a0 + kDig * kDADigit;
+#pragma unroll
+            for (int ks = 0; ks < kDChunk / 16; ++ks) {
+              const uint64_t db = tc::smem_desc(b0 + ks * 2 * kDBLbo, kDBLbo, 128);
+#pragma unroll
+              for (int i = 0; i < kDig; ++i) {
+                const uint64_t da = tc::smem_desc(a0 + i * kDADigit + ks * 256, 128, 512);
+                if (tc::elect_one())
+                  tc::mma_bf16(d0 + kWin * i, da, db, idesc_f16_f32(128, kWin * (kDig - i), 1, 0),
+                               (r0 > s0 || ks > 0 || i > 0) ? 1u : 0u);
+              }
+            }
+            if (tc::elect_one()) {
+              tc::mma_commit(&empty_bar[chunk % kDEmpty]);
+              if (r0 == end) tc::mma_commit(&tfull_bar[buf]);
+            }
+            __syncwarp();
+            fetch();  // into this chunk's slots: its A is split
+            ++chunk;
+            if (++st == kDStages) {
+              st = 0;
+              par ^= 1;
+            }
           }
         }
       }
@@ -1544,7 +1572,7 @@ cudaError_t launch_f64_density(const F64Bricks& b, const F64Pairs& pr, const dou
   if (b.nrows == 0 || pr.npairs == 0) return cudaSuccess;
   LCP_CUDA_TRY(cudaMemsetAsync(w.cmax, 0, (size_t)pr.natom * 32 * sizeof(uint32_t), st));
   const unsigned blocks = (unsigned)std::min<int64_t>(pr.npairs, 152 * 16);
-  f64_dsym_kernel<<<blocks, 128, 0, st>>>(pr, dm, w.dsym, w.cmax, b.max_rows >= 512 ? 1 : 0);
+  f64_dsym_kernel<<<blocks, 128, 0, st>>>(pr, dm, w.dsym, w.cmax);
   LCP_CUDA_TRY(cudaGetLastError());
   f64_dfix_kernel<<<blocks, 128, 0, st>>>(pr, w.dsym, w.cmax, w.dfix);
   LCP_CUDA_TRY(cudaGetLastError());
@@ -1565,7 +1593,7 @@ cudaError_t launch_f64_force(const F64Bricks& b, const F64Pairs& pr, int nch, co
   for (int c = 0; c < nch; ++c) {
     LCP_CUDA_TRY(cudaMemsetAsync(w.cmax, 0, (size_t)pr.natom * 32 * sizeof(uint32_t), st));
     LCP_CUDA_TRY(cudaMemsetAsync(f.part, 0, (size_t)b.nimg * kF64ForceParts * sizeof(double), st));
-    f64_drow_kernel<<<blocks, 128, 0, st>>>(pr, dm[c], w.cmax, b.max_rows >= 512 ? 1 : 0);
+    f64_drow_kernel<<<blocks, 128, 0, st>>>(pr, dm[c], w.cmax);
     LCP_CUDA_TRY(cudaGetLastError());
     f64_drowfix_kernel<<<blocks, 128, 0, st>>>(pr, dm[c], w.cmax, w.dfix);
     LCP_CUDA_TRY(cudaGetLastError());

@@ -125,9 +125,9 @@ def _flat(nfun, values):
     return PAO(0, [nfun], rv, [[np.full(rv.size, float(x)) for x in values]], Spe_Atom_Cut1=6.0)
 
 
-def _flat_cell(nfun, values):
+def _flat_cell(nfun, values, side=5.0, n=12):
     """At every point all orbitals of dozens of images count alike: 160 to 900 rows at a brick."""
-    return _cell(np.diag([5.0] * 3), [[0.1, 0.2, 0.3], [2.0, 2.6, 1.1]], [1, 1], [_flat(nfun, values)], (12, 12, 12))
+    return _cell(np.diag([side] * 3), [[0.1, 0.2, 0.3], [2.0, 2.6, 1.1]], [1, 1], [_flat(nfun, values)], (n, n, n))
 
 
 @pytest.mark.parametrize("nfun", [2, 8, 16, 32])
@@ -146,3 +146,22 @@ def test_density_of_many_like_rows(nfun):
     L.Calc_MatrixElements_dVH_Vxc_off(u, orbs, [v], h)
     ref = O.calc_matrix_elements(uo, phi, [v], 1)[0]
     assert np.max(np.abs(h[0] - ref)) <= TOL * np.max(np.abs(ref))
+
+
+def test_density_of_large_digits():
+    """Up to 830 rows that count at one point, with phi's and D's two leading base-256
+    digits large, odd and different from row to row: no sum of digit products may lose a unit."""
+    rng = np.random.default_rng(5)
+    phi0, d0 = 0.5 * (125 + 125 / 256) / 128, (63 + 120 / 256) / 128
+    values = phi0 * 2 * np.sqrt(np.pi) * (1 + 2e-5 * rng.uniform(-1, 1, 32))
+    u, uo, orbs, phi = _flat_cell(32, values, 4.4, 24)
+    dm = d0 * (1 + 2e-5 * rng.uniform(-1, 1, u.Total_Hsize))
+    l0 = orbs.ctx.launch_count
+    rho = [np.zeros(u.NN)]
+    L.Set_Density_Grid("off", u, orbs, [dm], rho)
+    assert orbs.ctx.launch_count > l0 + 1  # the tensor-core kernels
+    f = phi[0][:, 0]
+    ref = np.zeros(u.NN)
+    for p in range(u.Nloop):
+        np.add.at(ref, uo.GridListAtom[u.MPI_atom[p] - 1][uo.MPI_GListTAtoms1[p]], f @ dm[_block(u, p)].reshape(32, 32) @ f)
+    assert np.max(np.abs(rho[0] - ref) / ref) <= TOL

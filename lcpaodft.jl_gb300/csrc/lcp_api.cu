@@ -469,8 +469,8 @@ lcp_status density_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nspin, const d
     const lcp::F64DensWork w{ctx->w_f64d.as<double>() + orbs->ucell->u.total_hsize, ctx->w_f64d.as<uint64_t>(),
                              ctx->w_f64c.as<uint32_t>(), ctx->w_f64e.as<int32_t>()};
     for (int c = 0; c < nspin; ++c)
-      API_CUDA(lcp::launch_f64_density(orbs->f64_density.g, orbs->f64_pairs, dm[c], w, rho[c], ctx->w_status.as<int>(),
-                                       ctx->stream),
+      API_CUDA(lcp::launch_f64_density(orbs->f64_density.g, orbs->f64_density.src, orbs->f64_pairs, dm[c], w, rho[c],
+                                       ctx->w_status.as<int>(), ctx->stream),
                "density kernel");
     ctx->launches += 4 * nspin;
     return LCP_OK;

@@ -423,16 +423,19 @@ struct F64Pairs {
 };
 // rho (one channel) from D.  Workspace: dsym (hsize doubles) and dfix (hsize
 // words: D symmetrised per ordered pair, as FP64 and on the grids of its
-// columns' scales), cmax (natom * 32 words: the columns' largest magnitudes)
-// and btop (nbricks ints: the bricks' largest column scales).
+// columns' scales), cmax (natom * 32 words: the columns' largest magnitudes, then
+// the number of odd bricks and, two words on, 64 bits of the next unit of their
+// work) and btop (2 * nbricks ints: the bricks' largest column scales, -1 for odd
+// ones, and the list of those, which are summed directly from f).
 struct F64DensWork {
   double* dsym;
   uint64_t* dfix;
   uint32_t* cmax;
   int32_t* btop;
 };
-cudaError_t launch_f64_density(const F64Bricks& b, const F64Pairs& pr, const double* dm, const F64DensWork& w,
-                               double* rho, int* status, cudaStream_t st);
+constexpr int kF64CmaxTail = 4;  // words behind cmax
+cudaError_t launch_f64_density(const F64Bricks& b, const F64Source& f, const F64Pairs& pr, const double* dm,
+                               const F64DensWork& w, double* rho, int* status, cudaStream_t st);
 // Force term: what its epilogue reads, and its partial sums (part: nimg *
 // kF64ForceParts doubles, three per image and epilogue warp, then natom * 3 *
 // kF64ForceSlices).

@@ -207,6 +207,13 @@ struct BrickIterT {
 };
 using BrickIter = BrickIterT<true>;
 
+// The next of the units that warps take one by one.
+__device__ __forceinline__ int64_t claim_unit(unsigned long long* next, int lane) {
+  unsigned long long u = 0;
+  if (lane == 0) u = atomicAdd(next, 1ull);
+  return (int64_t)__shfl_sync(0xffffffffu, u, 0);
+}
+
 int device_sms() {
   int dev = 0, sms = 152;
   cudaGetDevice(&dev);
@@ -459,11 +466,6 @@ __global__ void __launch_bounds__(kHP) f64_vprep_kernel(F64Bricks b, const doubl
 // a 2-atom cell's 216 takes 16 us (20 with the units dealt evenly), one of a
 // 64-atom cell's 13,824 nothing that shows; if every one of those is odd, 45 ms
 // (pair kernels 20).
-__device__ __forceinline__ int64_t claim_unit(unsigned long long* next, int lane) {
-  unsigned long long u = 0;
-  if (lane == 0) u = atomicAdd(next, 1ull);
-  return (int64_t)__shfl_sync(0xffffffffu, u, 0);
-}
 __device__ __forceinline__ void odd_elements(const F64HamArgs& A, int nodd) {
   constexpr int kParts = 8, kAhead = 8;  // units of an image pair; points whose loads are in flight
   const F64Bricks& B = A.b;
@@ -909,8 +911,14 @@ struct F64DensArgs {
   F64Bricks b;
   const uint64_t* dfix;
   const uint32_t* cmax;  // [natom * 32] high word of max |Ds| of a column
-  const int32_t* btop;   // [nbricks] exponent bound of the largest finite column of a brick
+  const int32_t* btop;   // [nbricks] exponent bound of the largest column of a brick; -1: odd
   double* rho;
+  // density: of the odd bricks
+  F64Source src;
+  const double* dm;
+  const int32_t* odd;
+  const int32_t* nodd;
+  unsigned long long* next;
   F64Force f;            // force term only
   int* status;
 };
@@ -940,20 +948,67 @@ __global__ void __launch_bounds__(128) f64_dsym_kernel(F64Pairs pr, const double
   }
 }
 
-// Exponent bound of the largest finite column scale among a brick's rows (one warp per brick).
+// Exponent bound of the largest column scale among a brick's rows (one warp per
+// brick).  Odd, and summed directly: bricks where a column is not finite (an
+// element of D reaches only the points that its two atoms hold), or lies further
+// below the largest than the sum reaches (2^-120 and not zero).
 __global__ void __launch_bounds__(256) f64_btop_kernel(F64Bricks b, const uint32_t* __restrict__ cmax,
-                                                       int32_t* __restrict__ btop) {
+                                                       int32_t* __restrict__ btop, int32_t* __restrict__ odd,
+                                                       int32_t* __restrict__ nodd) {
   const int lane = threadIdx.x & 31;
   for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < b.nbricks;
        k += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     const F64Brick br = load_brick(b.bricks + k);
-    int e = 1;
+    int top = 1, low = kBadExp;
     for (int r = lane; r < (int)(br.size & 0xffffu); r += 32) {
-      const int x = exp_bound(__ldg(cmax + row_col(load_meta(b.rows + br.row + r).info)));
-      if (x < kBadExp) e = max(e, x);
+      const uint32_t h = __ldg(cmax + row_col(load_meta(b.rows + br.row + r).info));
+      top = max(top, exp_bound(h));
+      if (h > 0) low = min(low, exp_bound(h));
     }
-    e = __reduce_max_sync(0xffffffffu, e);
-    if (lane == 0) btop[k] = e;
+    top = __reduce_max_sync(0xffffffffu, top);
+    low = __reduce_min_sync(0xffffffffu, low);
+    if (lane == 0) {
+      const bool is_odd = top >= kBadExp || top - low > 120;
+      btop[k] = is_odd ? -1 : top;
+      if (is_odd) odd[atomicAdd(nodd, 1)] = (int32_t)k;
+    }
+  }
+}
+
+// The density at the odd bricks' points: the pairs of images that hold a point, a
+// warp to a point, as FP64 sums.
+__device__ __forceinline__ void odd_points(const F64DensArgs& A, int nodd) {
+  const F64Bricks& B = A.b;
+  const F64Source& f = A.src;
+  const int lane = threadIdx.x & 31;
+  for (int64_t unit = claim_unit(A.next, lane); unit < (int64_t)nodd * 128; unit = claim_unit(A.next, lane)) {
+    const int k = A.odd[unit >> 7], p = (int)(unit & 127);
+    const int64_t gi = p < B.npts ? brick_point_index(k, p, B.bdim, B.nb, B.ngrid) : -1;
+    if (gi < 0) continue;
+    const F64Brick br = load_brick(B.bricks + k);
+    const int m = (int)(br.size >> 16);
+    const int64_t i0 = f.img_off[k];
+    double sum = 0.0;
+    for (int s = 0; s < m; ++s) {
+      const int ks = f.slot[(i0 + s) * 128 + p];
+      if (ks < 0) continue;
+      const int as = f.img_atom[i0 + s], noi = f.numorbs[as];
+      const double* ps = f.phi + f.phi_off[as] + (int64_t)ks * noi;
+      for (int t = 0; t < m; ++t) {
+        const int kt = f.slot[(i0 + t) * 128 + p];
+        const int32_t off = kt >= 0 ? B.tab[(int64_t)br.tab + s * m + t] : -1;
+        if (off < 0) continue;
+        const int at = f.img_atom[i0 + t], noj = f.numorbs[at];
+        const double* pt = f.phi + f.phi_off[at] + (int64_t)kt * noj;
+        for (int e = lane; e < noi * noj; e += 32) {
+          const int a = e / noj, b = e - a * noj;
+          sum = fma(__ldg(ps + a) * __ldg(A.dm + off + e), __ldg(pt + b), sum);
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o /= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0 && bounds_ok(gi, (int64_t)B.ngrid[0] * B.ngrid[1] * B.ngrid[2], 21)) A.rho[gi] = sum;
   }
 }
 
@@ -1165,6 +1220,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
   __shared__ uint64_t rawfull_bar[kDRaw];
   __shared__ uint64_t s_low[FORCE ? 1 : 32 * kDEpi];  // the low word of the points' sums
   __shared__ uint32_t tslot;
+  __shared__ int nodd;
   __shared__ volatile int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const F64Bricks& B = args.b;
@@ -1180,6 +1236,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
     tc::mbar_init(&drain_bar, 1);
     tc::fence_mbar_init();
     abort_flag = 0;
+    nodd = FORCE ? 0 : *args.nodd;
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -1304,7 +1361,6 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
         s_low[tid] = 0;  // not in registers: the kernel has none left, and few windows need it
         const int base = align_bits(R);
         int64_t shi = 0;
-        bool nan = false;
         const int etop = __ldg(args.btop + x.k);
         for (int c0 = 0, r0 = 0; c0 < R && !abort_flag; ++win) {  // segment r0 of window c0
           const uint32_t buf = win & 1;
@@ -1313,7 +1369,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
           int ce = 0;
           if (c0 + lane < R)
             ce = etop - exp_bound(__ldg(args.cmax + row_col(load_meta(B.rows + x.b.row + c0 + lane).info)));
-          const bool odd = __any_sync(0xffffffffu, ce < 0 || ce > base);
+          const bool far = __any_sync(0xffffffffu, ce > base);
           const uint32_t up = 1u << min(max(base - ce, 0), 7);
           const uint64_t* phi = mine + (int64_t)(c0 / 32) * 32 * kDP;
           uint64_t ph[4];
@@ -1341,12 +1397,10 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
               tp[j] = (int64_t)((uint64_t)(uint32_t)t * m + ((uint64_t)((uint32_t)(t >> 32) * m) << 32));
               S[j] = assemble(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
             }
-            if (odd) {  // columns far below the brick's largest, or with Inf or NaN
+            if (far) {  // columns far below the brick's largest
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 const int d = __shfl_sync(0xffffffffu, ce, cb + j), n = min(max(d - base, 0), 191);
-                nan = nan || (d < 0 && ph[j] != kF64Bias);
-                if (d < 0) S[j] = 0;
                 // S tp >> n = (S >> n) tp + ((S mod 2^n) tp >> n): the second part here
                 const int64_t x = n < 64 ? S[j] & ((1ll << n) - 1) : S[j];
                 S[j] = n < 64 ? S[j] >> n : 0;
@@ -1388,9 +1442,8 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
         }
         double acc = fma((double)shi, 0x1p64, fma((double)sx, 0x1p-64, (double)slo));
         if (neg) acc = -acc;
-        if (nan) acc = __longlong_as_double(0x7ff8000000000000ll);
-        // two halves onto a zeroed point: the same sum in either order
-        if (gi >= 0 && bounds_ok(gi, (int64_t)B.ngrid[0] * B.ngrid[1] * B.ngrid[2], 21))
+        // two halves onto a zeroed point: the same sum in either order (odd bricks: odd_points)
+        if (gi >= 0 && etop >= 0 && bounds_ok(gi, (int64_t)B.ngrid[0] * B.ngrid[1] * B.ngrid[2], 21))
           atomicAdd(args.rho + gi, scalbn(acc, 2 * (B.ptexp[(int64_t)x.k * kDP + p] - 1023) + etop - 1023 - 109 - base));
       }
     }
@@ -1552,6 +1605,9 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
   __syncthreads();
   tc::fence_after_sync();
   if (warp == kDEpi) tc::tmem_dealloc(tmem, 512);
+  if constexpr (!FORCE) {
+    if (nodd > 0) odd_points(args, nodd);
+  }
 }
 
 }  // namespace
@@ -1565,20 +1621,23 @@ cudaError_t launch_f64_table(const F64Bricks& b, const F64Source& f, const int32
   return cudaGetLastError();
 }
 
-cudaError_t launch_f64_density(const F64Bricks& b, const F64Pairs& pr, const double* dm, const F64DensWork& w,
-                               double* rho, int* status, cudaStream_t st) {
+cudaError_t launch_f64_density(const F64Bricks& b, const F64Source& f, const F64Pairs& pr, const double* dm,
+                               const F64DensWork& w, double* rho, int* status, cudaStream_t st) {
   const int64_t nn = (int64_t)b.ngrid[0] * b.ngrid[1] * b.ngrid[2];
   LCP_CUDA_TRY(cudaMemsetAsync(rho, 0, (size_t)nn * sizeof(double), st));
   if (b.nrows == 0 || pr.npairs == 0) return cudaSuccess;
-  LCP_CUDA_TRY(cudaMemsetAsync(w.cmax, 0, (size_t)pr.natom * 32 * sizeof(uint32_t), st));
+  LCP_CUDA_TRY(cudaMemsetAsync(w.cmax, 0, ((size_t)pr.natom * 32 + kF64CmaxTail) * sizeof(uint32_t), st));
+  int32_t* nodd = reinterpret_cast<int32_t*>(w.cmax + (size_t)pr.natom * 32);
+  unsigned long long* next = reinterpret_cast<unsigned long long*>(nodd + 2);
+  int32_t* odd = w.btop + b.nbricks;
   const unsigned blocks = (unsigned)std::min<int64_t>(pr.npairs, 152 * 16);
   f64_dsym_kernel<<<blocks, 128, 0, st>>>(pr, dm, w.dsym, w.cmax);
   LCP_CUDA_TRY(cudaGetLastError());
   f64_dfix_kernel<<<blocks, 128, 0, st>>>(pr, w.dsym, w.cmax, w.dfix);
   LCP_CUDA_TRY(cudaGetLastError());
-  f64_btop_kernel<<<(unsigned)std::min<int64_t>((b.nbricks + 7) / 8, 152 * 8), 256, 0, st>>>(b, w.cmax, w.btop);
+  f64_btop_kernel<<<(unsigned)std::min<int64_t>((b.nbricks + 7) / 8, 152 * 8), 256, 0, st>>>(b, w.cmax, w.btop, odd, nodd);
   LCP_CUDA_TRY(cudaGetLastError());
-  F64DensArgs a{b, w.dfix, w.cmax, w.btop, rho, F64Force{}, status};
+  F64DensArgs a{b, w.dfix, w.cmax, w.btop, rho, f, dm, odd, nodd, next, F64Force{}, status};
   LCP_CUDA_TRY(raise_smem(f64_points_kernel<false>, kDSmemBytes));
   f64_points_kernel<false><<<(unsigned)std::min<int64_t>(b.nbricks, device_sms()), kDThreads, kDSmemBytes, st>>>(a);
   return cudaGetLastError();
@@ -1597,7 +1656,7 @@ cudaError_t launch_f64_force(const F64Bricks& b, const F64Pairs& pr, int nch, co
     LCP_CUDA_TRY(cudaGetLastError());
     f64_drowfix_kernel<<<blocks, 128, 0, st>>>(pr, dm[c], w.cmax, w.dfix);
     LCP_CUDA_TRY(cudaGetLastError());
-    F64DensArgs a{b, w.dfix, w.cmax, nullptr, nullptr, f, status};
+    F64DensArgs a{b, w.dfix, w.cmax, nullptr, nullptr, F64Source{}, nullptr, nullptr, nullptr, nullptr, f, status};
     a.f.vpot = vpot[c];
     a.f.w = coef[c];
     f64_points_kernel<true><<<(unsigned)std::min<int64_t>(b.nbricks, device_sms()), kDThreads, kDSmemBytes, st>>>(a);

@@ -99,7 +99,7 @@ def test_elements_of_one_infinite_point():
     assert np.max(np.abs(h[0][ok] - ref[ok])) <= TOL * np.max(np.abs(ref[ok]))
 
 
-@pytest.mark.parametrize("shift", [6, 9, 40, 100])
+@pytest.mark.parametrize("shift", [6, 9, 40, 100, 140])
 def test_density_of_an_atom_with_a_small_d(shift):
     """An atom whose D is 2^-shift of its neighbour's keeps its own accuracy where it is alone."""
     u, uo, orbs, phi = _sparse_cell()
@@ -165,3 +165,18 @@ def test_density_of_large_digits():
     for p in range(u.Nloop):
         np.add.at(ref, uo.GridListAtom[u.MPI_atom[p] - 1][uo.MPI_GListTAtoms1[p]], f @ dm[_block(u, p)].reshape(32, 32) @ f)
     assert np.max(np.abs(rho[0] - ref) / ref) <= TOL
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_density_of_a_d_that_is_not_finite(value):
+    """An element of D between two atoms reaches the points that both hold, and no other."""
+    u, uo, orbs, phi = _sparse_cell()
+    dm = np.random.default_rng(9).normal(size=u.Total_Hsize)
+    dm[_block(u, _pair(u, 1, 2)[0])][5:6] = value
+    rho = [np.zeros(u.NN)]
+    L.Set_Density_Grid("off", u, orbs, [dm], rho)
+    with np.errstate(invalid="ignore"):
+        ref = O.set_density_grid("off", uo, phi, [dm])[0]
+    ok = np.isfinite(ref)
+    assert not ok.all() and np.array_equal(np.isfinite(rho[0]), ok)
+    assert np.max(np.abs(rho[0][ok] - ref[ok])) <= TOL * np.max(np.abs(ref[ok]))

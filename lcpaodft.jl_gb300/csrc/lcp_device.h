@@ -393,6 +393,7 @@ struct F64Bricks {
   const F64Row* rows;          // [nrows]
   const uint64_t* table;       // [nchunks * 32 * P]
   const int32_t* ptexp;        // density: [nbricks * P] E of a point
+  const int32_t* bad;          // density: [nbricks] 1 where a phi is not finite
   const int32_t* tab;          // m x m per brick: offset of the block of the ordered pair (s, t), or for matrix
                                // elements of its partner (t, s), where they are accumulated (s <= t); -1: no pair
   const uint64_t* cover;       // matrix elements: [nbricks] slots that some image holds (0 beside rows: phi is not finite)

@@ -410,10 +410,12 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   g.table = S.table.as<uint64_t>();
   g.tab = S.tab.as<int32_t>();
   if (P == 128) {
-    API_CUDA(S.ptexp.ensure(g.nbricks * P * sizeof(int32_t)), "alloc");
+    API_CUDA(S.ptexp.ensure(g.nbricks * (P + 1) * sizeof(int32_t)), "alloc");  // and bad
     f64_fill_kernel<<<blocks_for(g.nbricks * P), 256, 0, st>>>(S.ptexp.as<int32_t>(), g.nbricks * P, 1);
     API_CUDA(cudaGetLastError(), "brick scales");
     g.ptexp = S.ptexp.as<int32_t>();
+    g.bad = g.ptexp + g.nbricks * P;
+    API_CUDA(cudaMemsetAsync(S.ptexp.as<int32_t>() + g.nbricks * P, 0, g.nbricks * sizeof(int32_t), st), "memset");
   } else {
     API_CUDA(S.cover.ensure(g.nbricks * sizeof(uint64_t)), "alloc");
     g.cover = S.cover.as<uint64_t>();

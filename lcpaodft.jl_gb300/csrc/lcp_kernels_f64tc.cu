@@ -229,8 +229,9 @@ int device_sms() {
 namespace {
 
 // Rows and scales, one warp per image (lane = orbital): each row's exponent
-// bound over the brick's points, or each point's over all rows; with cover, the
-// slots that the images hold, none of a brick where a phi is not finite.
+// bound over the brick's points, or each point's over all rows, and behind those
+// the bricks where a phi is not finite; with cover, the slots that the images hold,
+// none of such a brick.
 __global__ void __launch_bounds__(256) f64_scales_kernel(F64Bricks b, F64Source f, const int32_t* __restrict__ row0,
                                                          F64Row* __restrict__ rows, int32_t* __restrict__ ptexp,
                                                          uint64_t* __restrict__ cover) {
@@ -257,7 +258,10 @@ __global__ void __launch_bounds__(256) f64_scales_kernel(F64Bricks b, F64Source 
         mx = max(mx, h);
         if (k >= 0 && ptexp) {
           const uint32_t pm = __reduce_max_sync(0xffffffffu, h);
-          if (lane == 0) atomicMax(ptexp + hb * b.P + p, exp_bound(pm));
+          if (lane == 0) {
+            atomicMax(ptexp + hb * b.P + p, exp_bound(pm));
+            if (exp_bound(pm) >= kBadExp) ptexp[b.nbricks * b.P + hb] = 1;  // bad
+          }
         }
       }
       if (lane < no)
@@ -951,7 +955,8 @@ __global__ void __launch_bounds__(128) f64_dsym_kernel(F64Pairs pr, const double
 // Exponent bound of the largest column scale among a brick's rows (one warp per
 // brick).  Odd, and summed directly: bricks where a column is not finite (an
 // element of D reaches only the points that its two atoms hold), or lies further
-// below the largest than the sum reaches (2^-120 and not zero).
+// below the largest than the sum reaches (2^-120 and not zero), or where a phi is
+// not finite.
 __global__ void __launch_bounds__(256) f64_btop_kernel(F64Bricks b, const uint32_t* __restrict__ cmax,
                                                        int32_t* __restrict__ btop, int32_t* __restrict__ odd,
                                                        int32_t* __restrict__ nodd) {
@@ -968,7 +973,7 @@ __global__ void __launch_bounds__(256) f64_btop_kernel(F64Bricks b, const uint32
     top = __reduce_max_sync(0xffffffffu, top);
     low = __reduce_min_sync(0xffffffffu, low);
     if (lane == 0) {
-      const bool is_odd = top >= kBadExp || top - low > 120;
+      const bool is_odd = top >= kBadExp || top - low > 120 || __ldg(b.bad + k) != 0;
       btop[k] = is_odd ? -1 : top;
       if (is_odd) odd[atomicAdd(nodd, 1)] = (int32_t)k;
     }
@@ -1260,7 +1265,8 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
         const int64_t i0 = __ldg(F.img_off + x.k);
         const int64_t gi = p < B.npts ? brick_point_index(x.k, p, B.bdim, B.nb, B.ngrid) : -1;
         const double vp = gi >= 0 ? F.w * __ldg(F.vpot + gi) : 0.0;
-        const int ep = __ldg(B.ptexp + (int64_t)x.k * kDP + p) - 2 * 1023 - 54;
+        const int et = __ldg(B.ptexp + (int64_t)x.k * kDP + p);
+        const int ep = et >= kBadExp ? kBadExp : et - 2 * 1023 - 54;  // a phi there is not finite: no column is
         int cur = -1, asked = -1, k = -1;  // image of the sums, image whose point is k
         int64_t base = 0;
         double f0 = 0.0, f1 = 0.0, f2 = 0.0;
@@ -1319,7 +1325,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
               const int ec = __shfl_sync(0xffffffffu, ce, cb + j), e = ec + ep;
               const int64_t S = assemble(y[0][j], y[1][j], y[2][j], y[3][j], y[4][j], y[5][j], y[6][j]);
               v[j] = (double)S;  // times 2^e
-              if (ec >= kBadExp) v[j] = has[j] ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+              if (e >= kBadExp || ec >= kBadExp) v[j] = has[j] ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
               else if (e > -800 && e < 800 && S != 0)
                 v[j] = __hiloint2double(__double2hiint(v[j]) + (e << 20), __double2loint(v[j]));
               else v[j] = scalbn(v[j], e);

@@ -180,3 +180,26 @@ def test_density_of_a_d_that_is_not_finite(value):
     ok = np.isfinite(ref)
     assert not ok.all() and np.array_equal(np.isfinite(rho[0]), ok)
     assert np.max(np.abs(rho[0][ok] - ref[ok])) <= TOL * np.max(np.abs(ref[ok]))
+
+
+def test_radial_functions_that_are_not_finite():
+    """A radial function with a NaN marks the results of the points in that shell, as the oracle's are."""
+    paos = [synthetic_species(81, rc=4.0), synthetic_species(82, max_l=1, num_basis=(1, 1), rc=4.5)]
+    paos[1].Spe_PAO_RWF[1][0][int(np.searchsorted(paos[1].Spe_PAO_RV, 4.2))] = np.nan
+    lat, pos = np.diag([15.0, 15.5, 16.0]), [[4.0, 4.1, 4.2], [9.0, 4.5, 5.0], [10.5, 10.8, 11.0]]
+    u, uo, orbs, phi = _cell(lat, pos, [1, 2, 1], paos, (24, 25, 23), L.Set_dOrbitals_Grid)
+    assert not all(np.isfinite(x).all() for x in phi)
+    rng = np.random.default_rng(10)
+    dm, v = rng.normal(size=u.Total_Hsize), rng.normal(size=u.NN)
+    rho, h = [np.zeros(u.NN)], [np.zeros(u.Total_Hsize)]
+    L.Set_Density_Grid("off", u, orbs, [dm], rho)
+    L.Calc_MatrixElements_dVH_Vxc_off(u, orbs, [v], h)
+    f = L.Force3_nospin(paos, orbs, [v], [dm], u)
+    grad = [[orbs.data(a, k + 1) for a in range(3)] for k in range(3)]
+    with np.errstate(invalid="ignore"):
+        refs = [O.set_density_grid("off", uo, phi, [dm])[0], O.calc_matrix_elements(uo, phi, [v], 1)[0],
+                O.calc_force3("off", uo, phi, grad, [v], [dm])]
+    for got, ref, tol in zip((rho[0], h[0], f), refs, (TOL, TOL, 1e-10)):
+        ok = np.isfinite(ref)
+        assert not ok.all() and np.array_equal(np.isfinite(got), ok)
+        assert np.max(np.abs(got[ok] - ref[ok]), initial=0.0) <= tol * np.max(np.abs(ref[ok]), initial=1.0)

@@ -286,7 +286,13 @@ lcp_status lcp_job_set_dm(lcp_ctx* ctx, lcp_job* job, const double* const* dm);
 /* Launch one grid step on the context stream (asynchronous).  Any context of
  * the job's device may run it (its workspaces and FFT plans are used); steps
  * of one job must not overlap.  From a job's second step on a context the
- * launches are replayed as one CUDA graph (lcp_ctx_set_step_graphs). */
+ * launches are replayed as one CUDA graph (lcp_ctx_set_step_graphs).  While the
+ * caller captures the context's stream, the launches go into the caller's graph.
+ * That graph uses the context's workspaces: it must not run beside other work of
+ * the context, nor after the job, its orbitals (or lcp_orbs_release_fp64) or the
+ * context have gone.  An FP64 graph's workspaces stay until the context goes; a
+ * split-BF16 graph's are reallocated by the context's next call on a larger cell,
+ * after which it must not run. */
 lcp_status lcp_job_step(lcp_ctx* ctx, lcp_job* job);
 /* The same step with CUDA events between its stages (synchronises); stage_ms[6] =
  * density, Poisson, xc+potential (with the energy partial sums of the same

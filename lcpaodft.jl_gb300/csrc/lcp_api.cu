@@ -451,8 +451,10 @@ static lcp_status f64_ready(lcp_ctx* ctx, const lcp_orbs* orbs, int which, bool*
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   API_CUDA(cudaStreamIsCapturing(ctx->stream, &cap), "capture status");
   if (cap != cudaStreamCaptureStatusNone) {
-    if (built()) return ensure_f64_workspace(ctx, o, tc);
-    return LCP_OK;
+    if (!built()) return LCP_OK;
+    const lcp_status s = ensure_f64_workspace(ctx, o, tc);
+    if (*tc && !ctx->own_capture) ctx->f64_captured = ~0u;
+    return s;
   }
   return f64_made(ctx, o, which, tc);
 }
@@ -1866,7 +1868,9 @@ lcp_status lcp_job_step(lcp_ctx* ctx, lcp_job* job) {
   if (!G.off && G.have_prev && same(G.prev, sig)) {
     const int64_t l0 = ctx->launches;
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      ctx->own_capture = true;
       s = job_step_impl(ctx, job, nullptr);
+      ctx->own_capture = false;
       cudaGraph_t g = nullptr;
       const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
       int64_t after[8];

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -122,6 +123,12 @@ struct lcp_ctx {
   DBuf w_in[4], w_out[4], w_aux[4], w_real, w_spec, w_part, w_scal, w_a, w_b;
   DBuf w_dsym, w_status, w_hscratch, w_dscale, w_dtmp, w_vw, w_vscale, w_pfac;
   DBuf w_f64d, w_f64c, w_f64v, w_f64e;  // FP64 contractions (ensure_f64_workspace)
+  // A caller's own stream capture may hold their addresses (bit i: the i-th of
+  // them): a larger cell then gets a new buffer, and the old one is kept here, for
+  // the caller's graph, until the context goes.
+  uint32_t f64_captured = 0;
+  std::list<DBuf> kept;
+  bool own_capture = false;  // lcp_job_step's capture into the job's own graph, invalidated by any free
   // second stream of the step: the xc pass runs there beside the FFT Poisson solve
   cudaStream_t aux = nullptr;
   // device address of the no-allocation density's fixed scratch array, looked

@@ -532,6 +532,14 @@ lcp_status ensure_f64_workspace(lcp_ctx* ctx, const lcp_orbs* o, bool* ready) {
     for (const auto& n : need) *ready = *ready && n.first->p && n.first->bytes >= n.second;
     return LCP_OK;
   }
-  for (const auto& n : need) API_CUDA(n.first->ensure(n.second), "alloc");
+  for (size_t i = 0; i < 4; ++i) {
+    DBuf& b = *need[i].first;
+    if (((ctx->f64_captured >> i) & 1u) && b.p && b.bytes < need[i].second) {
+      ctx->kept.emplace_back();
+      ctx->kept.back().swap(b);
+      ctx->f64_captured &= ~(1u << i);
+    }
+    API_CUDA(b.ensure(need[i].second), "alloc");
+  }
   return LCP_OK;
 }

@@ -2032,7 +2032,8 @@ int64_t job_footprint_estimate(lcp_job* job, int32_t precision) {
                     b.sb_chunks.size()) * 4;
   } else if (precision == LCP_PREC_FP32 && !o->phi32.p) {
     fp += o->table_elems * 4;
-  } else if (precision == LCP_PREC_FP64 && o->f64_density.state == 0 && o->f64_elements.state == 0 && !o->phi_released) {
+  } else if (precision == LCP_PREC_FP64 && o->f64_density.state == 0 && o->f64_elements.state == 0 &&
+             !o->f64_density.need && !o->f64_elements.need && !o->phi_released) {
     fp += f64_footprint_estimate(o);
   }
   return fp;

@@ -156,7 +156,8 @@ struct lcp_ctx {
 // One brick tiling of the FP64 tensor-core contractions (lcp_f64bricks.cu).
 struct F64Set {
   lcp::F64Bricks g{};
-  int state = 0;  // 0 not built, 1 built, -1 beyond the kernels' limits
+  int state = 0;    // 0 not built, 1 built, -1 beyond the kernels' limits
+  size_t need = 0;  // not built for lack of room: the free bytes that it takes to try again
   lcp::F64Source src{};
   DBuf bricks, rows, table, ptexp, cover, tab;
   DBuf img_off, img_atom, slot;  // of src; the density tiling's also for the force term
@@ -164,6 +165,7 @@ struct F64Set {
     for (DBuf* d : {&bricks, &rows, &table, &ptexp, &cover, &tab, &img_off, &img_atom, &slot}) d->release();
     g = lcp::F64Bricks{};
     src = lcp::F64Source{};
+    need = 0;
   }
 };
 

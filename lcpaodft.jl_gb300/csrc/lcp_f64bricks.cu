@@ -281,6 +281,7 @@ double choose_shape(const UCell& u, int P, int32_t* bd) {
 int blocks_for(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 8)); }
 
 // One tiling; *fits = false when a brick or a table is beyond the kernels' limits.
+// Without the room for it, S.need is set and S holds nothing.
 lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int P, bool* fits) {
   const UCell& u = o->ucell->u;
   cudaStream_t st = ctx->stream;
@@ -395,8 +396,12 @@ lcp_status build_set(lcp_ctx* ctx, lcp_orbs* o, const DBuf& ijk, F64Set& S, int 
   // (256 of them take 77 GB, and these tables would take 200)
   size_t mem_free = 0, mem_total = 0;
   API_CUDA(cudaMemGetInfo(&mem_free, &mem_total), "memory");
-  if (mem_free < (size_t)g.nchunks * 32 * P * sizeof(uint64_t) + mem_total / 4) *fits = false;
-  if (!*fits) return LCP_OK;
+  const size_t need = (size_t)g.nchunks * 32 * P * sizeof(uint64_t) + mem_total / 4;
+  if (*fits && mem_free < need) {
+    S.release();
+    S.need = need;
+  }
+  if (!*fits || S.need) return LCP_OK;
   API_CUDA(S.rows.ensure(std::max<int64_t>(g.nrows, 1) * sizeof(F64Row)), "alloc");
   API_CUDA(S.tab.ensure(std::max<int64_t>(ntab, 1) * sizeof(int32_t)), "alloc");
   API_CUDA(S.table.ensure(std::max<int64_t>(g.nchunks, 1) * 32 * P * sizeof(uint64_t)), "alloc");
@@ -457,7 +462,9 @@ int64_t f64_footprint_estimate(const lcp_orbs* o) {
 // ensure_f64 builds the tilings it is asked for (kF64Density, kF64Elements)
 // once per orbital set.  Afterwards a tiling's state is 1, or -1 for a cell
 // beyond the kernels' limits (block offsets of 30 bits, bricks of kF64MaxRows
-// rows) or without room for its tables, which keeps the pair kernels.
+// rows), which keeps the pair kernels.  Without room for its tables it stays 0, on
+// the pair kernels, and is tried again once enough memory is free (asking for that
+// takes 0.1 ms at most, a step with the pair kernels of such a cell ten or more).
 namespace {
 lcp_status pair_tables(lcp_ctx* ctx, lcp_orbs* o) {
   if (o->f64_pairs_ready) return LCP_OK;
@@ -496,23 +503,31 @@ lcp_status pair_tables(lcp_ctx* ctx, lcp_orbs* o) {
 
 lcp_status ensure_f64(lcp_ctx* ctx, lcp_orbs* o, int which) {
   std::lock_guard<std::mutex> lock(o->f64_mutex);
-  int* state[2] = {&o->f64_density.state, &o->f64_elements.state};
   for (int k = 0; k < 2; ++k) {
-    if (!(which & (1 << k)) || *state[k] != 0) continue;
+    F64Set& S = k ? o->f64_elements : o->f64_density;
+    if (!(which & (1 << k)) || S.state != 0) continue;
+    size_t mem_free = 0, mem_total = 0;
+    if (S.need) {
+      API_CUDA(cudaMemGetInfo(&mem_free, &mem_total), "memory");
+      if (mem_free < S.need) continue;
+      S.need = 0;
+    }
     const lcp::UCell& u = o->ucell->u;
     bool fits = u.total_hsize < ((int64_t)1 << 30) && u.natom <= 65535 && u.nloop > 0;
     if (fits) {
       lcp_status s = pair_tables(ctx, o);
-      if (s == LCP_OK) s = lcp::build_set(ctx, o, o->f64_pair_buf[6], k ? o->f64_elements : o->f64_density, k ? 64 : 128, &fits);
+      if (s == LCP_OK) s = lcp::build_set(ctx, o, o->f64_pair_buf[6], S, k ? 64 : 128, &fits);
       if (s == LCP_ENOMEM) {  // the pair kernels need none of it
         (void)cudaGetLastError();
-        fits = false;
+        S.release();
+        API_CUDA(cudaMemGetInfo(&mem_free, &mem_total), "memory");
+        S.need = mem_free + ((size_t)1 << 28);
       } else if (s) {
         return s;
       }
     }
-    if (!fits) (k ? o->f64_elements : o->f64_density).release();
-    *state[k] = fits ? 1 : -1;
+    if (!fits) S.release();
+    if (!S.need) S.state = fits ? 1 : -1;
   }
   return LCP_OK;
 }

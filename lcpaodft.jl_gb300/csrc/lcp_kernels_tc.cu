@@ -877,6 +877,10 @@ __global__ void __launch_bounds__(192 + 32 * kDGatherWarps, 1) density_tc_kernel
           for (int c = 0; c < 16; ++c) d = fmaf(u[c], ym[c] + yc[c], d);
           ff_add(acc_hi, acc_lo, d);
           tc::fence_before_sync();
+          // the loads of phi above come before the copy that the release lets into
+          // the stage: an arrival alone orders them against later reads and writes of
+          // threads, not against the bulk copy, which is another proxy
+          tc::fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0 && !withhold) tc::mbar_arrive(&empty_bar[stage]);
         }

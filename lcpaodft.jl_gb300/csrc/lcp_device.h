@@ -426,7 +426,7 @@ struct F64Pairs {
 // words: D symmetrised per ordered pair, as FP64 and on the grids of its
 // columns' scales), cmax (natom * 32 words: the columns' largest magnitudes, then
 // the number of odd bricks and, two words on, 64 bits of the next unit of their
-// work) and btop (2 * nbricks ints: the bricks' largest column scales, -1 for odd
+// work, then natom words: the largest of each atom's own block) and btop (2 * nbricks ints: the bricks' largest column scales, -1 for odd
 // ones, and the list of those, which are summed directly from f).
 struct F64DensWork {
   double* dsym;
@@ -434,7 +434,7 @@ struct F64DensWork {
   uint32_t* cmax;
   int32_t* btop;
 };
-constexpr int kF64CmaxTail = 4;  // words behind cmax
+constexpr int kF64CmaxTail = 4;  // words of the odd bricks behind the columns'
 cudaError_t launch_f64_density(const F64Bricks& b, const F64Source& f, const F64Pairs& pr, const double* dm,
                                const F64DensWork& w, double* rho, int* status, cudaStream_t st);
 // Force term: what its epilogue reads, and its partial sums (part: nimg *

@@ -539,7 +539,7 @@ lcp_status ensure_f64_workspace(lcp_ctx* ctx, const lcp_orbs* o, bool* ready) {
   const size_t hs = (size_t)u.total_hsize, nb = (size_t)o->f64_elements.g.nbricks, nd = (size_t)o->f64_density.g.nbricks;
   const std::pair<DBuf*, size_t> need[] = {
       {&ctx->w_f64d, (hs * lcp::kF64Copies + 2) * sizeof(double)},  // symmetrised D, twice (density); the sums of H
-      {&ctx->w_f64c, ((size_t)u.natom * 32 + lcp::kF64CmaxTail) * sizeof(uint32_t)},  // D's column maxima
+      {&ctx->w_f64c, ((size_t)u.natom * 33 + lcp::kF64CmaxTail) * sizeof(uint32_t)},  // D's column maxima
       {&ctx->w_f64v, std::max<size_t>(nb, 1) * 64 * sizeof(int64_t)},  // V by brick
       {&ctx->w_f64e, std::max<size_t>(2 * std::max(nb, nd), 1) * sizeof(int32_t)}};  // its scales, or D's by brick (density), and odd bricks
   if (ready) {

@@ -928,9 +928,10 @@ struct F64DensArgs {
 };
 
 // Ds per ordered pair and the largest magnitude of each column (orbital b of
-// the neighbour atom), one block per pair.
+// the neighbour atom) and of each atom's own block (smax), one block per pair.
 __global__ void __launch_bounds__(128) f64_dsym_kernel(F64Pairs pr, const double* __restrict__ dm,
-                                                       double* __restrict__ dsym, uint32_t* __restrict__ cmax) {
+                                                       double* __restrict__ dsym, uint32_t* __restrict__ cmax,
+                                                       uint32_t* __restrict__ smax) {
   __shared__ uint32_t mx[32];
   for (int64_t p = blockIdx.x; p < pr.npairs; p += gridDim.x) {
     const int i = pr.atom[p], j = pr.jatom[p];
@@ -948,6 +949,10 @@ __global__ void __launch_bounds__(128) f64_dsym_kernel(F64Pairs pr, const double
     }
     __syncthreads();
     if (threadIdx.x < noj) atomicMax(cmax + (int64_t)j * 32 + threadIdx.x, mx[threadIdx.x]);
+    if (threadIdx.x < 32 && p == pr.first[i]) {  // the self pair
+      const uint32_t h = __reduce_max_sync(0xffffffffu, mx[threadIdx.x]);
+      if (threadIdx.x == 0) smax[i] = h;
+    }
     __syncthreads();
   }
 }
@@ -956,24 +961,55 @@ __global__ void __launch_bounds__(128) f64_dsym_kernel(F64Pairs pr, const double
 // brick).  Odd, and summed directly: bricks where a column is not finite (an
 // element of D reaches only the points that its two atoms hold), or lies further
 // below the largest than the sum reaches (2^-120 and not zero), or where a phi is
-// not finite.
-__global__ void __launch_bounds__(256) f64_btop_kernel(F64Bricks b, const uint32_t* __restrict__ cmax,
-                                                       int32_t* __restrict__ btop, int32_t* __restrict__ odd,
-                                                       int32_t* __restrict__ nodd) {
+// not finite; and bricks whose pairs hold only entries more than 2^12 below their
+// column's scale, which is the largest of all pairs.  The last is looked into only
+// for columns that far above their atom's own block, whose pair is in every brick
+// of the atom: for a D of occupied orbitals, |D_rc|^2 <= D_rr D_cc, that takes an
+// atom 2^24 emptier than its neighbour.
+__global__ void __launch_bounds__(256) f64_btop_kernel(F64Bricks b, const double* __restrict__ dsym,
+                                                       const uint32_t* __restrict__ cmax,
+                                                       const uint32_t* __restrict__ smax, int32_t* __restrict__ btop,
+                                                       int32_t* __restrict__ odd, int32_t* __restrict__ nodd) {
+  constexpr int kSpan = 12;
   const int lane = threadIdx.x & 31;
   for (int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; k < b.nbricks;
        k += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     const F64Brick br = load_brick(b.bricks + k);
+    const int R = (int)(br.size & 0xffffu), m = (int)(br.size >> 16);
+    const F64Row* rows = b.rows + br.row;
+    auto above = [&](int r, uint32_t& h) {  // the row's column lies far above its atom's own block
+      const int c = row_col(load_meta(rows + r).info);
+      h = __ldg(cmax + c);
+      return exp_bound(h) > exp_bound(__ldg(smax + (c >> 5))) + kSpan;
+    };
     int top = 1, low = kBadExp;
-    for (int r = lane; r < (int)(br.size & 0xffffu); r += 32) {
-      const uint32_t h = __ldg(cmax + row_col(load_meta(b.rows + br.row + r).info));
+    bool any = false;
+    for (int r = lane; r < R; r += 32) {
+      uint32_t h;
+      any |= above(r, h);
       top = max(top, exp_bound(h));
       if (h > 0) low = min(low, exp_bound(h));
     }
     top = __reduce_max_sync(0xffffffffu, top);
     low = __reduce_min_sync(0xffffffffu, low);
+    bool is_odd = top >= kBadExp || top - low > 120 || __ldg(b.bad + k) != 0;
+    if (!is_odd && __any_sync(0xffffffffu, any)) {
+      for (int c = 0; c < R && !is_odd; ++c) {
+        uint32_t h, most = 0;
+        if (!above(c, h)) continue;
+        const F64Row mc = load_meta(rows + c);
+        const int t = (int)(mc.img_orb >> 8), noj = row_no(mc.info);
+        for (int r = lane; r <= c; r += 32) {  // the entries of the column
+          const uint32_t io = load_meta(rows + r).img_orb;
+          const int32_t off = __ldg(b.tab + br.tab + (int64_t)(io >> 8) * m + t);
+          if (off >= 0)
+            most = max(most, (uint32_t)__double2hiint(__ldg(dsym + off + (int)(io & 255u) * noj + (int)(mc.img_orb & 255u))) & 0x7fffffffu);
+        }
+        most = __reduce_max_sync(0xffffffffu, most);
+        is_odd = most > 0 && exp_bound(h) > exp_bound(most) + kSpan;
+      }
+    }
     if (lane == 0) {
-      const bool is_odd = top >= kBadExp || top - low > 120 || __ldg(b.bad + k) != 0;
       btop[k] = is_odd ? -1 : top;
       if (is_odd) odd[atomicAdd(nodd, 1)] = (int32_t)k;
     }
@@ -1634,14 +1670,15 @@ cudaError_t launch_f64_density(const F64Bricks& b, const F64Source& f, const F64
   if (b.nrows == 0 || pr.npairs == 0) return cudaSuccess;
   LCP_CUDA_TRY(cudaMemsetAsync(w.cmax, 0, ((size_t)pr.natom * 32 + kF64CmaxTail) * sizeof(uint32_t), st));
   int32_t* nodd = reinterpret_cast<int32_t*>(w.cmax + (size_t)pr.natom * 32);
+  uint32_t* smax = w.cmax + (size_t)pr.natom * 32 + kF64CmaxTail;
   unsigned long long* next = reinterpret_cast<unsigned long long*>(nodd + 2);
   int32_t* odd = w.btop + b.nbricks;
   const unsigned blocks = (unsigned)std::min<int64_t>(pr.npairs, 152 * 16);
-  f64_dsym_kernel<<<blocks, 128, 0, st>>>(pr, dm, w.dsym, w.cmax);
+  f64_dsym_kernel<<<blocks, 128, 0, st>>>(pr, dm, w.dsym, w.cmax, smax);
   LCP_CUDA_TRY(cudaGetLastError());
   f64_dfix_kernel<<<blocks, 128, 0, st>>>(pr, w.dsym, w.cmax, w.dfix);
   LCP_CUDA_TRY(cudaGetLastError());
-  f64_btop_kernel<<<(unsigned)std::min<int64_t>((b.nbricks + 7) / 8, 152 * 8), 256, 0, st>>>(b, w.cmax, w.btop, odd, nodd);
+  f64_btop_kernel<<<(unsigned)std::min<int64_t>((b.nbricks + 7) / 8, 152 * 8), 256, 0, st>>>(b, w.dsym, w.cmax, smax, w.btop, odd, nodd);
   LCP_CUDA_TRY(cudaGetLastError());
   F64DensArgs a{b, w.dfix, w.cmax, w.btop, rho, f, dm, odd, nodd, next, F64Force{}, status};
   LCP_CUDA_TRY(raise_smem(f64_points_kernel<false>, kDSmemBytes));

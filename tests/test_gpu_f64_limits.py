@@ -167,6 +167,21 @@ def test_density_of_large_digits():
     assert np.max(np.abs(rho[0] - ref) / ref) <= TOL
 
 
+@pytest.mark.parametrize("value", [2.0 ** 6, 1e6, 1e12, 1e100])
+def test_density_of_one_large_element_of_d(value):
+    """An element of D between two atoms counts at the points that both hold, and
+    takes no digits from the others."""
+    u, uo, orbs, phi = _sparse_cell()
+    dm = np.random.default_rng(11).normal(size=u.Total_Hsize)
+    dm[_block(u, _pair(u, 1, 2)[0])][7:8] = value
+    rho = [np.zeros(u.NN)]
+    L.Set_Density_Grid("off", u, orbs, [dm], rho)
+    ref = O.set_density_grid("off", uo, phi, [dm])[0]
+    n, _ = _counts(u)
+    for part in (n == 1, n > 1):
+        assert np.max(np.abs(rho[0] - ref)[part]) <= TOL * np.max(np.abs(ref[part]))
+
+
 @pytest.mark.parametrize("value", [np.inf, np.nan])
 def test_density_of_a_d_that_is_not_finite(value):
     """An element of D between two atoms reaches the points that both hold, and no other."""

@@ -362,8 +362,13 @@ void lcp_server_destroy(lcp_server* srv);
  * by the caller, who keeps ownership): admitted now if its footprint (with
  * the precision's tables) fits the free budget, else queued for admission
  * with its requests until removals free the budget (lcp_server_state);
- * LCP_ENOMEM only when it exceeds the whole budget.  nspin / hsize: channels
- * and Total_Hsize of its D. */
+ * LCP_ENOMEM only when it exceeds the whole budget.  Tables that the precision
+ * can do without (FP64: the tensor-core kernels', a multiple of the rest;
+ * split-BF16: the packed rows) keep no structure out: they are made while the
+ * budget has room for them too, and the FP64 ones are freed when another
+ * structure needs it (a caller's own graph of a job's step must not run after
+ * the job was added to a server).  nspin / hsize: channels and Total_Hsize of
+ * its D. */
 lcp_status lcp_server_add(lcp_server* srv, lcp_job* job, int32_t nspin, int64_t hsize, int32_t* id);
 /* Releases a structure's budget (LCP_ESTATE while it has requests queued)
  * and admits queued structures that now fit, in order. */

@@ -233,7 +233,7 @@ static lcp_status pack_rows(lcp_ctx* ctx, lcp_orbs* o) {
   const size_t bytes = (size_t)std::max<int64_t>(off.back(), 1) * 6144 * 2;
   size_t mem_free = 0, mem_total = 0;
   API_CUDA(cudaMemGetInfo(&mem_free, &mem_total), "memory");
-  bool packed = off.back() * 16 <= b.nblocks * 15 && mem_free >= bytes + (bytes >= mem_total / 64 ? mem_total / 2 : mem_total / 8 * 7);
+  bool packed = !ctx->no_optional && off.back() * 16 <= b.nblocks * 15 && mem_free >= bytes + (bytes >= mem_total / 64 ? mem_total / 2 : mem_total / 8 * 7);
   if (packed) {
     const cudaError_t e = o->b_ptab.ensure(bytes);
     if (e == cudaErrorMemoryAllocation) {
@@ -1027,15 +1027,7 @@ lcp_status lcp_orbs_release_fp64(lcp_ctx* ctx, lcp_orbs* orbs) {
   if ((s = ensure_bricks(ctx, orbs))) return s;
   API_CUDA(cudaStreamSynchronize(ctx->stream), "release");
   for (DBuf* d : {&orbs->phi, &orbs->dphi[0], &orbs->dphi[1], &orbs->dphi[2], &orbs->phi32}) d->release();
-  {
-    std::lock_guard<std::mutex> lock(orbs->f64_mutex);  // the FP64 kernels' tables go with the tables they came from
-    for (F64Set* x : {&orbs->f64_density, &orbs->f64_elements}) {
-      x->release();
-      x->state = 0;
-    }
-    for (DBuf& d : orbs->f64_pair_buf) d.release();
-    orbs->f64_pairs_ready = false;
-  }
+  drop_f64(orbs);  // the FP64 kernels' tables go with the tables they came from
   orbs->phi_released = true;
   return LCP_OK;
 }
@@ -2012,11 +2004,35 @@ lcp_status lcp_job_footprint(const lcp_job* job, int64_t* bytes) {
 
 }  // extern "C"
 
+// Frees the FP64 kernels' tables; the next call that would use them makes them again.
+void drop_f64(lcp_orbs* o) {
+  std::lock_guard<std::mutex> lock(o->f64_mutex);
+  for (F64Set* x : {&o->f64_density, &o->f64_elements}) {
+    x->release();
+    x->state = 0;
+  }
+  for (DBuf& d : o->f64_pair_buf) d.release();
+  o->f64_pairs_ready = false;
+}
+
+// Device bytes of the tables that the orbitals' forms can do without: the FP64
+// tensor-core kernels', and split-BF16's packed rows.
+int64_t orbs_optional_bytes(const lcp_orbs* o) {
+  int64_t b = (int64_t)o->b_ptab.bytes;
+  for (const F64Set* f : {&o->f64_density, &o->f64_elements})
+    for (const DBuf* d : {&f->bricks, &f->rows, &f->table, &f->ptexp, &f->tab, &f->img_off, &f->img_atom, &f->slot})
+      b += (int64_t)d->bytes;
+  for (const DBuf& d : o->f64_pair_buf) b += (int64_t)d.bytes;
+  return b;
+}
+
 // Device bytes the job will hold once its tables for `precision` exist: its
 // footprint now plus, when not built yet, the split-BF16 brick tables (from
-// the host brick geometry), the FP32 orbital copy or the FP64 kernels' tables.
-int64_t job_footprint_estimate(lcp_job* job, int32_t precision) {
+// the host brick geometry) or the FP32 orbital copy; in *optional those of the
+// tables that it can do without (orbs_optional_bytes).
+int64_t job_footprint_estimate(lcp_job* job, int32_t precision, int64_t* optional) {
   int64_t fp = 0;
+  *optional = 0;
   if (lcp_job_footprint(job, &fp) != LCP_OK) return -1;
   const lcp_orbs* o = job->orbs;
   if (precision == LCP_PREC_BF16X3 && !o->bricks_ready) {
@@ -2025,7 +2041,8 @@ int64_t job_footprint_estimate(lcp_job* job, int32_t precision) {
     std::vector<uint8_t> width;
     const int64_t npk = packed_blocks(o->ucell->u, b, width).back();
     const bool packed = npk * 16 <= b.nblocks * 15;
-    fp += (packed ? npk * (6144 * 2 + 64) : b.nblocks * 64) + (b.nbricks + 1) * 8;
+    if (packed) *optional = npk * 6144 * 2;
+    fp += b.nblocks * 64 + (b.nbricks + 1) * 8;
     fp += b.nblocks * 6144 * 2 + (int64_t)b.point_code.size() * 4 + (int64_t)b.tab_pair.size() * 8 +
           (int64_t)(b.img_off.size() + b.slot_base.size() + b.red_off.size() + b.red_slot.size()) * 8 +
           (int64_t)(b.img_block.size() + b.sub_pair.size() + b.sub_chunks.size() + b.sb_fold.size() +
@@ -2034,7 +2051,7 @@ int64_t job_footprint_estimate(lcp_job* job, int32_t precision) {
     fp += o->table_elems * 4;
   } else if (precision == LCP_PREC_FP64 && o->f64_density.state == 0 && o->f64_elements.state == 0 &&
              !o->f64_density.need && !o->f64_elements.need && !o->phi_released) {
-    fp += f64_footprint_estimate(o);
+    *optional = f64_footprint_estimate(o);
   }
   return fp;
 }

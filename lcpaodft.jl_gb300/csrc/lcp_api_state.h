@@ -128,6 +128,7 @@ struct lcp_ctx {
   // the caller's graph, until the context goes.
   uint32_t f64_captured = 0;
   std::list<DBuf> kept;
+  bool no_optional = false;  // a server's: makes no table that a form can do without
   bool own_capture = false;  // lcp_job_step's capture into the job's own graph, invalidated by any free
   // second stream of the step: the xc pass runs there beside the FFT Poisson solve
   cudaStream_t aux = nullptr;
@@ -264,7 +265,9 @@ lcp_status hamiltonian_device(lcp_ctx* ctx, const lcp_orbs* orbs, int nch, const
                               double* const* hks, int64_t hsize);
 lcp::GridCell job_grid_cell(lcp_job* job);
 
-int64_t job_footprint_estimate(lcp_job* job, int32_t precision);
+int64_t job_footprint_estimate(lcp_job* job, int32_t precision, int64_t* optional);
+int64_t orbs_optional_bytes(const lcp_orbs* o);
+void drop_f64(lcp_orbs* o);
 
 // batches re-assembled over changing sets of jobs (lcp_batch.cu), for the serving engine
 lcp_batch* batch_new(int device);

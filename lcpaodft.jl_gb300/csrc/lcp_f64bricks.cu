@@ -505,7 +505,7 @@ lcp_status ensure_f64(lcp_ctx* ctx, lcp_orbs* o, int which) {
   std::lock_guard<std::mutex> lock(o->f64_mutex);
   for (int k = 0; k < 2; ++k) {
     F64Set& S = k ? o->f64_elements : o->f64_density;
-    if (!(which & (1 << k)) || S.state != 0) continue;
+    if (!(which & (1 << k)) || S.state != 0 || ctx->no_optional) continue;
     size_t mem_free = 0, mem_total = 0;
     if (S.need) {
       API_CUDA(cudaMemGetInfo(&mem_free, &mem_total), "memory");

@@ -5,7 +5,10 @@
 // needs) is charged against a byte budget.  A structure that does not fit
 // the free budget waits in an admission queue, with its requests, until
 // removals free enough of the budget (first come, first admitted); only a
-// structure larger than the whole budget is refused.
+// structure larger than the whole budget is refused.  Tables that a precision
+// can do without (the FP64 tensor-core kernels', the packed rows of split-BF16)
+// are made while the budget has room for them too, and keep no other structure
+// out: the FP64 ones are freed again when one needs their room.
 //
 // Continuous batching: each of `nslots` execution slots -- a context of its
 // own (stream and workspaces) with a worker thread -- repeatedly takes the
@@ -59,6 +62,7 @@ struct Structure {
   int nspin = 1;
   int64_t hsize = 0;
   int64_t footprint = 0;  // charged against the budget (an estimate while not admitted)
+  int64_t extra = 0;      // bytes of optional tables that this server had made
   int state = kAdmitted;
   bool busy = false;
   int64_t queued = 0;          // requests submitted and not yet completed
@@ -71,7 +75,7 @@ struct lcp_server {
   int device = 0;
   int32_t precision = LCP_PREC_BF16X3;
   int32_t max_batch = 1;  // requests per batched step
-  int64_t budget = 0, resident = 0;
+  int64_t budget = 0, resident = 0, extras = 0;  // resident: footprints; extras: optional tables beside them
   std::vector<lcp_ctx*> slots;
   std::vector<lcp_batch*> runners;  // per slot, re-assembled for every batch
   std::deque<int32_t> waiting;      // structures in the admission queue, in order
@@ -211,10 +215,57 @@ struct lcp_server {
           r->t_done = now;
           finish(r);
         }
+        if (resident + extras > budget) shed();
       }
       cv_done.notify_all();
       cv_work.notify_all();  // these structures may have more requests waiting
     }
+  }
+
+  // Frees FP64 structures' optional tables, of those that no worker is stepping,
+  // until everything fits the budget (under mu).
+  void shed() {
+    for (auto& kv : structs) {
+      if (resident + extras <= budget) return;
+      Structure& st = kv.second;
+      if (precision != LCP_PREC_FP64 || st.extra == 0 || st.state != kAdmitted) continue;
+      bool busy = false;
+      for (auto& other : structs) busy = busy || (other.second.busy && other.second.job->orbs == st.job->orbs);
+      if (busy) continue;  // when its step is done
+      drop_f64(const_cast<lcp_orbs*>(st.job->orbs));
+      extras -= st.extra;
+      st.extra = 0;
+    }
+  }
+
+  // Makes an admitted structure's tables on the admission context (caller's
+  // thread): the optional ones if there is room for them.
+  lcp_status make_tables(int32_t id, int64_t optional) {
+    lcp_job* job = nullptr;
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      shed();
+      Structure& st = structs[id];
+      job = st.job;
+      admin->no_optional = resident + extras + optional > budget;
+      if (admin->no_optional) optional = 0;
+      extras += optional;
+      st.extra = optional;
+    }
+    const int64_t before = orbs_optional_bytes(job->orbs);
+    lcp_status s = lcp_job_prepare(admin, job);
+    int64_t fp = 0;
+    if (s == LCP_OK) s = lcp_job_footprint(job, &fp);
+    const int64_t made = orbs_optional_bytes(job->orbs) - before;
+    std::lock_guard<std::mutex> lk(mu);
+    Structure& st = structs[id];
+    extras += made - st.extra;
+    st.extra = made;
+    if (s == LCP_OK) {
+      resident += fp - made - st.footprint;
+      st.footprint = fp - made;
+    }
+    return s;
   }
 
   // Admits queued structures, in order, while they fit the free budget: their
@@ -239,17 +290,12 @@ struct lcp_server {
         std::lock_guard<std::mutex> lk(mu);
         job = structs[id].job;
       }
-      lcp_status s = lcp_job_prepare(admin, job);
-      int64_t fp = 0;
-      if (s == LCP_OK) s = lcp_job_footprint(job, &fp);
+      int64_t optional = 0;
+      job_footprint_estimate(job, precision, &optional);
+      const lcp_status s = make_tables(id, optional);
       {
         std::lock_guard<std::mutex> lk(mu);
-        Structure& st = structs[id];
-        if (s == LCP_OK) {
-          resident += fp - st.footprint;
-          st.footprint = fp;
-        }
-        st.state = kAdmitted;  // a failure shows up in the structure's requests
+        structs[id].state = kAdmitted;  // a failure shows up in the structure's requests
       }
       if (s != LCP_OK && first == LCP_OK) first = s;
     }
@@ -276,6 +322,7 @@ lcp_status lcp_server_create(int32_t device, int32_t nslots, int32_t precision, 
     lcp_ctx* c = nullptr;
     lcp_status st = lcp_ctx_create(device, &c);
     if (st) return st;
+    c->no_optional = true;  // make_tables decides
     s->slots.push_back(c);
     s->runners.push_back(nullptr);
     cudaStream_t stream;
@@ -333,7 +380,8 @@ void lcp_server_destroy(lcp_server* srv) {
 lcp_status lcp_server_add(lcp_server* srv, lcp_job* job, int32_t nspin, int64_t hsize, int32_t* id) {
   if (!srv || !job || !id) return fail(LCP_EINVAL, "NULL argument");
   if (nspin < 1 || nspin > 4 || hsize < 0) return fail(LCP_EINVAL, "bad nspin / hsize");
-  const int64_t est = job_footprint_estimate(job, srv->precision);
+  int64_t optional = 0;
+  const int64_t est = job_footprint_estimate(job, srv->precision, &optional);
   if (est < 0) return fail(LCP_EINVAL, "the structure's footprint cannot be estimated (bricks)");
   if (est > srv->budget)
     return fail(LCP_ENOMEM, "admission: the structure needs " + std::to_string(est) +
@@ -355,18 +403,15 @@ lcp_status lcp_server_add(lcp_server* srv, lcp_job* job, int32_t nspin, int64_t 
   }
   if (!now) return LCP_OK;  // admitted when removals free the budget
   // the precision's tables are built now, and the footprint measured
-  lcp_status s = lcp_job_prepare(srv->admin, job);
-  int64_t fp = 0;
-  if (s == LCP_OK) s = lcp_job_footprint(job, &fp);
+  const lcp_status s = srv->make_tables(*id, optional);
   std::lock_guard<std::mutex> lk(srv->mu);
   Structure& st = srv->structs[*id];
   if (s != LCP_OK) {
     srv->resident -= st.footprint;
+    srv->extras -= st.extra;
     srv->structs.erase(*id);
     return s;
   }
-  srv->resident += fp - st.footprint;
-  st.footprint = fp;
   st.state = kAdmitted;
   return LCP_OK;
 }
@@ -388,6 +433,7 @@ lcp_status lcp_server_remove(lcp_server* srv, int32_t id) {
         }
     } else {
       srv->resident -= it->second.footprint;
+      srv->extras -= it->second.extra;
     }
     srv->structs.erase(it);
   }
@@ -494,7 +540,7 @@ lcp_status lcp_server_stats(lcp_server* srv, int64_t* out4) {
   std::lock_guard<std::mutex> lk(srv->mu);
   out4[0] = srv->submitted;
   out4[1] = srv->completed;
-  out4[2] = srv->resident;
+  out4[2] = srv->resident + srv->extras;
   out4[3] = srv->budget;
   return LCP_OK;
 }

@@ -850,7 +850,8 @@ class Server:
         It is admitted now when its footprint fits the free budget, else it
         waits in the admission queue (its requests wait with it) until
         removals free the budget.  Raises LCPError (LCP_ENOMEM) only when the
-        footprint exceeds the whole budget."""
+        footprint exceeds the whole budget.  Tables that the precision can do
+        without count only while the budget has room for them."""
         i = ctypes.c_int32()
         check(lib.lcp_server_add(self._h, job._h, job.nspin, job.ucell.Total_Hsize, ctypes.byref(i)))
         self._jobs[i.value] = job

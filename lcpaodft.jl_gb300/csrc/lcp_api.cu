@@ -114,9 +114,10 @@ lcp_status ensure_phi32(lcp_ctx* ctx, lcp_orbs* o) {
   return LCP_OK;
 }
 
-// The overlap lists and work items of the pair kernels (FP32, the force term,
-// the FP64 cells beyond the tensor-core kernels' limits and FP64 steps whose
-// first run is inside a stream capture).
+// The overlap lists and work items of the pair kernels, made for every orbital
+// set: FP32 reads them, and FP64 (with the force term) where the tensor-core
+// kernels do not run (f64_ready): cells beyond their limits, no room for their
+// tables, a first run inside a stream capture.
 static lcp_status make_lens(lcp_ctx* ctx, lcp_orbs* o) {
   cudaStream_t st = ctx->stream;
   const lcp::UCell& u = o->ucell->u;
@@ -194,8 +195,6 @@ static lcp_status make_lens(lcp_ctx* ctx, lcp_orbs* o) {
   return LCP_OK;
 }
 
-// Brick tiling, split-BF16 orbital tables and the ordered pair list of the
-// tensor-core path, built once per tabulation.
 // Blocks of 16 rows that the bricks' rows fill when they are packed: the
 // orbitals of the images' 16-orbital chunks (widths), end to end.
 static std::vector<int64_t> packed_blocks(const lcp::UCell& u, const lcp::Bricks& b, std::vector<uint8_t>& width) {
@@ -260,6 +259,8 @@ static lcp_status pack_rows(lcp_ctx* ctx, lcp_orbs* o) {
   return LCP_OK;
 }
 
+// Brick tiling, split-BF16 orbital tables and the ordered pair list of the
+// tensor-core path, built once per tabulation.
 lcp_status ensure_bricks(lcp_ctx* ctx, lcp_orbs* o) {
   if (o->bricks_ready) return LCP_OK;
   if (o->phi_released) return fail(LCP_ESTATE, "the FP64 orbital tables were released");
@@ -437,10 +438,11 @@ static lcp_status f64_made(lcp_ctx* ctx, lcp_orbs* o, int which, bool* tc) {
 
 // Whether an FP64 contraction takes the tensor-core kernels, with their brick
 // lists and workspaces made if need be.  Always, except for cells beyond the
-// kernels' limits, without the memory for them, and inside a caller's stream capture before anything was
-// made (allocating and synchronising there would break the capture): those
-// take the pair kernels (64-atom 96^3 cell: 36.8 ms for density and matrix
-// elements, against 3.15 ms; 2-atom 24^3 cell: 0.62 ms against 0.145).
+// kernels' limits, without the memory for them (or a server's budget), and
+// inside a caller's stream capture before anything was made (allocating and
+// synchronising there would break the capture): those take the pair kernels
+// (64-atom 96^3 cell: 36.8 ms for density and matrix elements, against 3.15 ms;
+// 2-atom 24^3 cell: 0.62 ms against 0.145).
 static lcp_status f64_ready(lcp_ctx* ctx, const lcp_orbs* orbs, int which, bool* tc) {
   *tc = false;
   if (ctx->precision != LCP_PREC_FP64) return LCP_OK;

@@ -541,7 +541,8 @@ __global__ void __launch_bounds__(256, std::is_same<T, double>::value ? 3 : 4) f
     for (int e = threadIdx.x / W; e < n; e += rows) spec[base + e * estride] = norm(bufs[(size_t)col * S + off + e]);
 }
 
-// Shared-memory budget of a pass 2-4 block: four blocks per SM.
+// Shared-memory budget of a pass 2-4 block: four blocks per SM (of which the FP64
+// form's registers leave three).
 constexpr size_t kColsSmem = 54 * 1024;
 
 // The factors' stride: 2 mod 16 doubles, so the 16 lanes of one 8-byte

@@ -2,14 +2,15 @@
 //
 // GB300 issues 2 FP64 FMAs per clock and SM, and the pair kernels of
 // lcp_kernels_pair.cu keep that pipe 95 % busy: 16.9 ms (density) and 19.9 ms
-// (matrix elements) on the 64-atom 96^3 cell, where the kernels below take 1.5
-// and 1.6 ms.  The tensor cores do 4,096 FP16 multiply-adds per clock and SM
+// (matrix elements) on the 64-atom 96^3 cell, where the kernels below take 1.6
+// ms each.  The tensor cores do 4,096 FP16 multiply-adds per clock and SM
 // with FP32 accumulation, which is exact for integers below 2^24.  So each FP64
 // operand is put on a fixed-point grid of 56 bits,
 //
 //   x = t 2^-55 2^E,  |x| < 2^E,  t = sum_i d_i 256^(7-i),  |d_i| <= 128,
 //
-// whose seven base-256 digits are exact FP16 values, and a contraction of two
+// whose seven base-256 digits are exact FP16 values (the splitting of Ozaki, Ogita,
+// Oishi and Rump, Numer. Algorithms 59, 2012, on fixed grids), and a contraction of two
 // operands is the 28 digit products d_i d_j' with i + j <= 8, each group of
 // equal weight (i + j = d + 1) in its own FP32 accumulator a_d.  Over 64 terms
 // |a_d| <= d 2^20 < 2^24, so every sum is exact in the matrix elements; in the
@@ -21,10 +22,21 @@
 // of itself.  Against 113-bit sums over the same tables, on cells of 2 to 6
 // atoms and 4 to 18 orbitals, the errors over the result's norm are 1.3e-16 to
 // 2.1e-16 in H (pair kernels 2.0e-16 to 3.7e-16) and 1.3e-16 to 1.5e-16 in rho
-// (1.4e-16 to 2.8e-16).  Elements of H far below the largest, where two
-// orbitals' tails meet, carry fewer digits of their own than the pair
-// kernels' (99th percentile of the elements' relative errors 3e-14 to 2e-13,
-// against 1e-14).
+// (1.4e-16 to 2.8e-16).
+//
+// What a value on a grid loses is what lies below 2^-56 of the grid's scale, where
+// an FP64 product keeps 53 bits of its own whatever its neighbours hold:
+//   phi   elements: the row's largest in the brick; density, force: the point's
+//         largest row;
+//   V     2^-62 of the brick's largest where an orbital is (f64_vprep_kernel lists
+//         the bricks where it spans too much for that);
+//   D     density: its column's largest over all pairs of the cell
+//         (f64_btop_kernel lists the bricks that this would cost more than 12 bits);
+//         force: its row's.
+// The listed ("odd") bricks are summed directly in FP64, and so are those with
+// values that are not finite.  Elements of H far below the largest, where two
+// orbitals' tails meet, carry fewer digits of their own than the pair kernels'
+// (99th percentile of the elements' relative errors 3e-14 to 2e-13, against 1e-14).
 //
 // The split is integer work: the mantissa shifted to the scale's grid, rounded,
 // biased by 128 in every byte, and each byte turned into FP16 by placing it
@@ -421,8 +433,8 @@ struct F64HamArgs {
   int* status;
 };
 
-// V of every slot that an image holds, in brick order, as a multiple of 2^-62 of
-// the brick's bound (zero at the other slots, whatever V holds there), and the bounds.
+// V of every slot that an image holds, in brick order, rounded to a multiple of
+// 2^-62 of the brick's bound (zero at the other slots, whatever V holds there), and the bounds.
 //
 // One scale serves all of a brick's pairs, and a pair may hold only those of its
 // points where V is small: what V spans, its elements lose.  So the bricks where
@@ -455,7 +467,7 @@ __global__ void __launch_bounds__(kHP) f64_vprep_kernel(F64Bricks b, const doubl
                         (cover == 0 && (load_brick(b.bricks + k).size & 0xffffu) > 0);
     int e;
     const uint64_t m = mantissa(v, e) << 10;
-    const int64_t t = (int64_t)(m >> min((uint32_t)(E - e), 63u));
+    const int64_t t = (int64_t)(((m >> min((uint32_t)(E - e - 1), 63u)) + 1) >> 1);
     vb[k * kHP + p] = is_odd ? 0 : (v < 0.0 ? -t : t);
     if (p == 0) {
       vexp[k] = is_odd ? 1 : E;
@@ -709,7 +721,7 @@ __global__ void __launch_bounds__(kHThreads, 1) f64_hamiltonian_kernel(const __g
               const uint64_t da = tc::smem_desc(a0 + i * kHADigit + ks * 4096, 2048, 128);
               // digit 0 writes all seven accumulators first
               if (tc::elect_one())
-                tc::mma_bf16(d0 + kWin * i, da, db, idesc_f16_f32(128, kWin * (kDig - i), 0, 0),
+                tc::mma_f16kind(d0 + kWin * i, da, db, idesc_f16_f32(128, kWin * (kDig - i), 0, 0),
                              (ks > 0 || i > 0) ? 1u : 0u);
             }
           }
@@ -1530,7 +1542,7 @@ __global__ void __launch_bounds__(kDThreads, 1) f64_points_kernel(const __grid_c
               for (int i = 0; i < kDig; ++i) {
                 const uint64_t da = tc::smem_desc(a0 + i * kDADigit + ks * 256, 128, 512);
                 if (tc::elect_one())
-                  tc::mma_bf16(d0 + kWin * i, da, db, idesc_f16_f32(128, kWin * (kDig - i), 1, 0),
+                  tc::mma_f16kind(d0 + kWin * i, da, db, idesc_f16_f32(128, kWin * (kDig - i), 1, 0),
                                (r0 > s0 || ks > 0 || i > 0) ? 1u : 0u);
               }
             }

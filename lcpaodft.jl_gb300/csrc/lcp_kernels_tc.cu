@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(128) tc_selftest_kernel(const float* __restric
     for (int ks = 0; ks < K / 16; ++ks) {
       const uint64_t da = tc::smem_desc(tc::smem_u32(sa + 2 * ks * lbo_a), lbo_a, sbo_a);
       const uint64_t db = tc::smem_desc(tc::smem_u32(sb + 2 * ks * lbo_b), lbo_b, sbo_b);
-      tc::mma_bf16(tmem, da, db, idesc, ks > 0 ? 1u : 0u);
+      tc::mma_f16kind(tmem, da, db, idesc, ks > 0 ? 1u : 0u);
     }
     tc::mma_commit(&mbar);
   }
@@ -813,14 +813,14 @@ __global__ void __launch_bounds__(192 + 32 * kDGatherWarps, 1) density_tc_kernel
                          dbl = tc::smem_desc(b0 + 4 * kDBLbo, kDBLbo, 128);
           const uint32_t acc = k > 0 ? 1u : 0u;
           if (tc::elect_one()) {
-            tc::mma_bf16(d0, dah, dbh, idesc, acc);
-            tc::mma_bf16(d1, dah, dbm, idesc, acc);
-            tc::mma_bf16(d1, dam, dbh, idesc, 1u);
-            tc::mma_bf16(d1, dah, dbl, idesc, 1u);
-            tc::mma_bf16(d1, dal, dbh, idesc, 1u);
-            tc::mma_bf16(d1, dam, dbm, idesc, 1u);
-            tc::mma_bf16(d1, dam, dbl, idesc, 1u);
-            tc::mma_bf16(d1, dal, dbm, idesc, 1u);
+            tc::mma_f16kind(d0, dah, dbh, idesc, acc);
+            tc::mma_f16kind(d1, dah, dbm, idesc, acc);
+            tc::mma_f16kind(d1, dam, dbh, idesc, 1u);
+            tc::mma_f16kind(d1, dah, dbl, idesc, 1u);
+            tc::mma_f16kind(d1, dal, dbh, idesc, 1u);
+            tc::mma_f16kind(d1, dam, dbm, idesc, 1u);
+            tc::mma_f16kind(d1, dam, dbl, idesc, 1u);
+            tc::mma_f16kind(d1, dal, dbm, idesc, 1u);
             if (t < c1) {
               // column block t is final once these MMAs finish; the epilogue
               // reads it with phi_t from this stage and then frees the stage
@@ -1139,14 +1139,14 @@ __global__ void __launch_bounds__(kHThreads, 1) hamiltonian_tc_kernel(const __gr
             // hi * [hi, mid, lo] and lo * [hi, mid] whole.
             if (tc::elect_one()) {
               if (ks == 0) {
-                tc::mma_bf16(d0 + 2 * W, dal, dbh, idesc2, 0u);  // lo * [hi, mid] -> acc 2, 3 (first write)
-                tc::mma_bf16(d0, dah, dbh, idesc2, 0u);          // hi * [hi, mid] -> acc 0, 1 (first write)
-                tc::mma_bf16(d0 + 2 * W, dah, dbl, idesc1, 1u);  // hi * lo -> acc 2
+                tc::mma_f16kind(d0 + 2 * W, dal, dbh, idesc2, 0u);  // lo * [hi, mid] -> acc 2, 3 (first write)
+                tc::mma_f16kind(d0, dah, dbh, idesc2, 0u);          // hi * [hi, mid] -> acc 0, 1 (first write)
+                tc::mma_f16kind(d0 + 2 * W, dah, dbl, idesc1, 1u);  // hi * lo -> acc 2
               } else {
-                tc::mma_bf16(d0, dah, dbh, idesc3, 1u);          // hi * [hi, mid, lo] -> acc 0, 1, 2
-                tc::mma_bf16(d0 + 2 * W, dal, dbh, idesc2, 1u);  // lo * [hi, mid] -> acc 2, 3
+                tc::mma_f16kind(d0, dah, dbh, idesc3, 1u);          // hi * [hi, mid, lo] -> acc 0, 1, 2
+                tc::mma_f16kind(d0 + 2 * W, dal, dbh, idesc2, 1u);  // lo * [hi, mid] -> acc 2, 3
               }
-              tc::mma_bf16(d0 + W, dam, dbh, idesc3, 1u);        // mid * [hi, mid, lo] -> acc 1, 2, 3
+              tc::mma_f16kind(d0 + W, dam, dbh, idesc3, 1u);        // mid * [hi, mid, lo] -> acc 1, 2, 3
             }
           }
           if (tc::elect_one()) {

@@ -891,9 +891,6 @@ lcp_status ucell_host_lists(const lcp_ucell* c) {
   return LCP_OK;
 }
 
-namespace lcp {
-}  // namespace lcp
-
 extern "C" {
 
 lcp_status lcp_ucell_create_device(lcp_ctx* ctx, int32_t nspin, const double* latvecs, int32_t natom,

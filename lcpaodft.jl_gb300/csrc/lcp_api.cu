@@ -448,6 +448,7 @@ static lcp_status f64_ready(lcp_ctx* ctx, const lcp_orbs* orbs, int which, bool*
   if (ctx->precision != LCP_PREC_FP64) return LCP_OK;
   lcp_orbs* o = const_cast<lcp_orbs*>(orbs);
   auto built = [&]() {
+    std::lock_guard<std::mutex> lock(o->f64_mutex);  // another context may be making them
     return (!(which & kF64Density) || o->f64_density.state == 1) && (!(which & kF64Elements) || o->f64_elements.state == 1);
   };
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;

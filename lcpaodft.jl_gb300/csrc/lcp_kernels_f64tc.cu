@@ -861,7 +861,8 @@ __global__ void f64_finish_kernel(DevPairs pr, const int32_t* __restrict__ numor
 // without that a chunk took 5,000 clocks, whatever the arithmetic.  With four
 // warps on B, B set the pace (2,900 clocks a chunk); with one of the A warps
 // issuing the copies, that warp did.  Seven warps on B and the copies on the MMA
-// warp took the 64-atom 96^3 cell from 1.79 to 1.53 ms; the integer pipe is the
+// warp took the 64-atom 96^3 cell from 1.79 to 1.53 ms (1.60 since rows come in
+// segments and columns of any size keep their digits); the integer pipe is the
 // busiest unit now (2.5 of 4 instructions a clock issued).
 //
 // The force term's epilogue holds Y's column as one FP64 value times the
